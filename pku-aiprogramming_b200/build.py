@@ -75,6 +75,25 @@ def build_library(force: bool = False, verbose: bool = False) -> str:
     return LIB
 
 
+def build_torch_binding(force: bool = False, verbose: bool = False) -> str:
+    """`lib/_ttorch.so`: functional.py's calls on torch tensors as a CPython extension (links libtt_attn.so)."""
+    import sysconfig
+    src = os.path.join(HOST, "bind_torch.cpp")
+    out = os.path.join(LIB_DIR, "_ttorch.so")
+    newest = max(os.path.getmtime(src), os.path.getmtime(os.path.join(ROOT, "include", "tt_attn.h")))
+    if not force and os.path.exists(out) and os.path.getmtime(out) >= newest:
+        return out
+    import torch
+    base = os.path.dirname(torch.__file__)
+    inc = [os.path.join(base, "include"), os.path.join(base, "include", "torch", "csrc", "api", "include"),
+           sysconfig.get_paths()["include"], "/usr/local/cuda/include", os.path.join(ROOT, "include")]
+    _run(["g++", "-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-shared",
+          "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch.compiled_with_cxx11_abi()), *["-I" + d for d in inc], src, "-o", out,
+          "-L" + LIB_DIR, "-ltt_attn", "-L" + os.path.join(base, "lib"), "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu",
+          "-lc10_cuda", "-lc10", "-Wl,-rpath,$ORIGIN"], verbose)
+    return out
+
+
 HOST = os.path.join(CSRC, "host")
 HOST_DIR = os.path.join(PKG, "host_modules")   # myTensor*.so and myLayer*.so land here
 
@@ -84,6 +103,7 @@ def build_host_modules(force: bool = False, verbose: bool = False):
     import sysconfig
     import pybind11
     build_library(force=False, verbose=verbose)
+    build_torch_binding(force=force, verbose=verbose)
     os.makedirs(HOST_DIR, exist_ok=True)
     suffix = sysconfig.get_config_var("EXT_SUFFIX")
     inc = ["-I" + pybind11.get_include(), "-I" + sysconfig.get_paths()["include"], "-I" + HOST]
@@ -127,5 +147,6 @@ def build_host_modules(force: bool = False, verbose: bool = False):
 if __name__ == "__main__":
     path = build_library(force="--force" in sys.argv, verbose="--verbose" in sys.argv)
     print(path)
+    print(build_torch_binding(force="--force" in sys.argv, verbose="--verbose" in sys.argv))
     for m_ in build_host_modules(force="--force" in sys.argv, verbose="--verbose" in sys.argv):
         print(m_)

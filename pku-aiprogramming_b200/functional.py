@@ -1,18 +1,45 @@
 """Attention calls over torch CUDA tensors.
 
 torch is used for device memory and streams only: every call hands raw device pointers
-to the C ABI (`capi.lib`).  Shapes follow the reference's row-major layout:
+to the C ABI, through the extension `_ttorch` (csrc/host/bind_torch.cpp), which checks the
+arguments and allocates the outputs.  Where it finds that an argument does not fit it returns
+None, and the `_explain_*` functions here say what is wrong.  Shapes follow the reference's row-major layout:
 q/out `[B,H,S,D]`, k/v `[B,Hkv,L,D]` (Hkv = H, or a divisor of H for grouped heads), lse `[B,H,S]` fp32.
 """
 from __future__ import annotations
 
 import ctypes
+import importlib.machinery
+import importlib.util
+import os
 
 import torch
 
 from . import capi
 
+
+def _load_binding():
+    path = os.path.join(os.path.dirname(capi.LIB_PATH), "_ttorch.so")
+    if not os.path.exists(path):
+        raise capi.NativeLibraryMissing(f"{path} not found. Build it with "
+                                        f"`python {os.path.join(os.path.dirname(__file__), 'build.py')}`.")
+    loader = importlib.machinery.ExtensionFileLoader("_ttorch", path)
+    module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_ttorch", loader))
+    loader.exec_module(module)
+    return module
+
+
+_native = _load_binding()
+
 _DT = {torch.float32: capi.TT_F32, torch.bfloat16: capi.TT_BF16}
+
+
+def _done(result, explain, *args):
+    """The result of a native call; None: an argument does not fit, int: the status of a call that failed."""
+    if result is None:
+        explain(*args)
+        raise ValueError("arguments do not fit the call")
+    capi.check(result)
 
 
 def _check_inputs(q, k, v):
@@ -52,90 +79,56 @@ def _check_lens(kv_lens, B, device):
     return kv_lens
 
 
+def _explain_attention(q, k, v, kv_lens=None, out=None, lse=None, dout=None, decode=False):
+    B, H, S, _, _ = _check_inputs(q, k, v)
+    _check_lens(kv_lens, B, q.device)
+    if decode and S != 1:
+        raise ValueError(f"decode needs S == 1, got {S}")
+    if dout is not None:
+        for name, t, shp in (("out", out, q.shape), ("dout", dout, q.shape)):
+            if tuple(t.shape) != tuple(shp) or t.dtype != q.dtype or not t.is_cuda or not t.is_contiguous():
+                raise ValueError(f"{name} must be a contiguous CUDA tensor of shape {tuple(shp)} and dtype {q.dtype}")
+        if tuple(lse.shape) != (B, H, S) or lse.dtype != torch.float32 or not lse.is_cuda or not lse.is_contiguous():
+            raise ValueError("lse must be contiguous CUDA float32 [B,H,S]")
+
+
 def attention_forward(q, k, v, causal=False, scale=None, out=None, lse=None, need_lse=True, kv_lens=None):
     """`softmax(scale * q k^T [+causal]) v` -> (out, lse).  Asynchronous on the current stream.
     `kv_lens` (int32 `[B]`, CUDA): batch entry b attends to its first kv_lens[b] keys only."""
-    B, H, S, L, D = _check_inputs(q, k, v)
-    kv_lens = _check_lens(kv_lens, B, q.device)
-    with torch.cuda.device(q.device):
-        if out is None:
-            out = torch.empty_like(q)
-        if lse is None and need_lse:
-            lse = torch.empty((B, H, S), dtype=torch.float32, device=q.device)
-        d = capi.make_desc(B, H, S, L, D, _DT[q.dtype], causal, scale, Hkv=k.shape[1])
-        if kv_lens is None:
-            capi.check(capi.lib.tt_attn_fwd(ctypes.byref(d), _p(q), _p(k), _p(v), _p(out), _p(lse), _stream_ptr(q)))
-        else:
-            capi.check(capi.lib.tt_attn_fwd_padded(ctypes.byref(d), _p(q), _p(k), _p(v), _p(kv_lens), _p(out), _p(lse),
-                                                   _stream_ptr(q)))
-    return out, lse
+    r = _native.attention_forward(q, k, v, causal, scale, out, lse, need_lse, kv_lens)
+    return r if r.__class__ is tuple else _done(r, _explain_attention, q, k, v, kv_lens)
 
 
 def attention_backward(q, k, v, out, lse, dout, causal=False, scale=None, workspace=None, kv_lens=None):
     """(dq, dk, dv) for upstream gradient `dout`; `out`, `lse` from `attention_forward` (same `kv_lens`)."""
-    B, H, S, L, D = _check_inputs(q, k, v)
-    kv_lens = _check_lens(kv_lens, B, q.device)
-    for name, t, shp in (("out", out, q.shape), ("dout", dout, q.shape)):
-        if tuple(t.shape) != tuple(shp) or t.dtype != q.dtype or not t.is_cuda or not t.is_contiguous():
-            raise ValueError(f"{name} must be a contiguous CUDA tensor of shape {tuple(shp)} and dtype {q.dtype}")
-    if tuple(lse.shape) != (B, H, S) or lse.dtype != torch.float32 or not lse.is_contiguous():
-        raise ValueError("lse must be contiguous float32 [B,H,S]")
-    with torch.cuda.device(q.device):
-        d = capi.make_desc(B, H, S, L, D, _DT[q.dtype], causal, scale, Hkv=k.shape[1])
-        need = int(capi.lib.tt_attn_bwd_workspace_bytes(ctypes.byref(d)))
-        if workspace is None or workspace.numel() * workspace.element_size() < need:
-            workspace = torch.empty(max(need, 256), dtype=torch.uint8, device=q.device)
-        dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-        nbytes = workspace.numel() * workspace.element_size()
-        if kv_lens is None:
-            capi.check(capi.lib.tt_attn_bwd(ctypes.byref(d), _p(q), _p(k), _p(v), _p(out), _p(lse), _p(dout),
-                                            _p(dq), _p(dk), _p(dv), _p(workspace), nbytes, _stream_ptr(q)))
-        else:
-            capi.check(capi.lib.tt_attn_bwd_padded(ctypes.byref(d), _p(q), _p(k), _p(v), _p(kv_lens), _p(out), _p(lse),
-                                                   _p(dout), _p(dq), _p(dk), _p(dv), _p(workspace), nbytes,
-                                                   _stream_ptr(q)))
-    return dq, dk, dv
+    r = _native.attention_backward(q, k, v, out, lse, dout, causal, scale, workspace, kv_lens)
+    return r if r.__class__ is tuple else _done(r, _explain_attention, q, k, v, kv_lens, out, lse, dout)
 
 
-def _varlen_desc(q, k, cu_q, cu_k, max_q, max_k, causal, scale):
+def _explain_varlen(q, k, v, cu_q, cu_k):
     for name, t in (("q", q), ("k", k)):
         if t.dim() != 3 or not t.is_cuda or not t.is_contiguous() or t.dtype != torch.bfloat16:
             raise ValueError(f"{name} must be a contiguous CUDA bfloat16 tensor [tokens, heads, D]")
     for name, t in (("cu_q", cu_q), ("cu_k", cu_k)):
         if t.dtype != torch.int32 or not t.is_cuda or not t.is_contiguous() or t.dim() != 1 or t.numel() != cu_q.numel():
             raise ValueError(f"{name} must be a contiguous CUDA int32 vector of n_seq + 1 cumulative token counts")
-    H, Hkv, D = q.shape[1], k.shape[1], q.shape[2]
-    if k.shape[2] != D or H % Hkv != 0:
+    if k.shape[2] != q.shape[2] or k.shape[1] < 1 or q.shape[1] % k.shape[1] != 0:
         raise ValueError(f"shape mismatch: q {tuple(q.shape)} k {tuple(k.shape)}")
-    return capi.VarlenDesc(cu_q.numel() - 1, H, Hkv, D, capi.TT_BF16, 1 if causal else 0, float(scale) if scale else 0.0,
-                           int(max_q), int(max_k), q.shape[0], k.shape[0])
+    raise ValueError("v, out, lse and dout must be CUDA tensors")
 
 
 def attention_forward_varlen(q, k, v, cu_q, cu_k, max_q, max_k, causal=False, scale=None, out=None, lse=None):
     """Packed variable-length batch: q `[total_q,H,D]`, k, v `[total_k,Hkv,D]`, cu_q / cu_k int32 `[n_seq+1]`
     (CUDA) cumulative token counts, max_q / max_k the longest sequence.  Returns (out `[total_q,H,D]`,
     lse `[H,total_q]`)."""
-    d = _varlen_desc(q, k, cu_q, cu_k, max_q, max_k, causal, scale)
-    with torch.cuda.device(q.device):
-        out = torch.empty_like(q) if out is None else out
-        lse = torch.empty((q.shape[1], q.shape[0]), dtype=torch.float32, device=q.device) if lse is None else lse
-        capi.check(capi.lib.tt_attn_fwd_varlen(ctypes.byref(d), _p(q), _p(k), _p(v), _p(cu_q), _p(cu_k), _p(out), _p(lse),
-                                               _stream_ptr(q)))
-    return out, lse
+    r = _native.attention_forward_varlen(q, k, v, cu_q, cu_k, max_q, max_k, causal, scale, out, lse)
+    return r if r.__class__ is tuple else _done(r, _explain_varlen, q, k, v, cu_q, cu_k)
 
 
 def attention_backward_varlen(q, k, v, cu_q, cu_k, max_q, max_k, out, lse, dout, causal=False, scale=None, workspace=None):
     """(dq, dk, dv) of the packed batch; `out`, `lse` from `attention_forward_varlen`."""
-    d = _varlen_desc(q, k, cu_q, cu_k, max_q, max_k, causal, scale)
-    with torch.cuda.device(q.device):
-        need = int(capi.lib.tt_attn_bwd_varlen_workspace_bytes(ctypes.byref(d)))
-        if workspace is None or workspace.numel() * workspace.element_size() < need:
-            workspace = torch.empty(max(need, 256), dtype=torch.uint8, device=q.device)
-        dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-        capi.check(capi.lib.tt_attn_bwd_varlen(ctypes.byref(d), _p(q), _p(k), _p(v), _p(cu_q), _p(cu_k), _p(out), _p(lse),
-                                               _p(dout), _p(dq), _p(dk), _p(dv), _p(workspace),
-                                               workspace.numel() * workspace.element_size(), _stream_ptr(q)))
-    return dq, dk, dv
+    r = _native.attention_backward_varlen(q, k, v, cu_q, cu_k, max_q, max_k, out, lse, dout, causal, scale, workspace)
+    return r if r.__class__ is tuple else _done(r, _explain_varlen, q, k, v, cu_q, cu_k)
 
 
 def set_backward_deterministic(on: bool) -> None:
@@ -152,32 +145,11 @@ def decode_workspace_bytes(B, H, L, D, dtype=torch.bfloat16, Hkv=None) -> int:
 
 def attention_decode(q, k, v, scale=None, out=None, lse=None, workspace=None, need_lse=True):
     """Single-query attention: q `[B,H,1,D]` against the whole cache k,v `[B,H,L,D]`."""
-    B, H, S, L, D = _check_inputs(q, k, v)
-    if S != 1:
-        raise ValueError(f"decode needs S == 1, got {S}")
-    with torch.cuda.device(q.device):
-        if out is None:
-            out = torch.empty_like(q)
-        if lse is None and need_lse:
-            lse = torch.empty((B, H, 1), dtype=torch.float32, device=q.device)
-        d = capi.make_desc(B, H, 1, L, D, _DT[q.dtype], False, scale, Hkv=k.shape[1])
-        need = int(capi.lib.tt_attn_decode_workspace_bytes(ctypes.byref(d)))
-        if need and (workspace is None or workspace.numel() * workspace.element_size() < need):
-            workspace = torch.empty(need, dtype=torch.uint8, device=q.device)
-        nbytes = workspace.numel() * workspace.element_size() if workspace is not None else 0
-        capi.check(capi.lib.tt_attn_decode(ctypes.byref(d), _p(q), _p(k), _p(v), _p(out), _p(lse),
-                                           _p(workspace), nbytes, _stream_ptr(q)))
-    return out, lse
+    r = _native.attention_decode(q, k, v, scale, out, lse, workspace, need_lse)
+    return r if r.__class__ is tuple else _done(r, lambda: _explain_attention(q, k, v, decode=True))
 
 
-def attention_decode_paged(q, k_pool, v_pool, block_table=None, seq_lens=None, max_len=None, scale=None, out=None,
-                           lse=None, workspace=None, need_lse=True):
-    """Single-query attention over a paged and/or ragged cache (bf16, D 64 or 128).
-
-    q `[B,H,1,D]`.  With `block_table` (int32 `[B, max_pages]`, CUDA): k_pool, v_pool are page pools
-    `[pages, Hkv, page_size, D]`.  Without: dense `[B,Hkv,L,D]`.  `seq_lens` (int32 `[B]`, CUDA)
-    limits each batch entry to its first seq_lens[b] keys.  `max_len`: longest possible sequence
-    (default: page_size * max_pages, or L of the dense cache)."""
+def _explain_paged(q, k_pool, v_pool, block_table, seq_lens, max_len):
     if q.dim() != 4 or q.shape[2] != 1 or not q.is_cuda or not q.is_contiguous() or q.dtype != torch.bfloat16:
         raise ValueError("q must be a contiguous CUDA bfloat16 tensor [B,H,1,D]")
     B, H, _, D = q.shape
@@ -196,90 +168,64 @@ def attention_decode_paged(q, k_pool, v_pool, block_table=None, seq_lens=None, m
     if block_table is not None:
         if block_table.dim() != 2 or block_table.shape[0] != B:
             raise ValueError("block_table must be [B, max_pages]")
-        page_size, max_pages = k_pool.shape[2], block_table.shape[1]
-        L = int(max_len) if max_len is not None else page_size * max_pages
     else:
         if k_pool.shape[0] != B:
             raise ValueError("a dense cache must be [B,Hkv,L,D]")
-        page_size, max_pages = 0, 0
-        L = int(max_len) if max_len is not None else k_pool.shape[2]
-        if L > k_pool.shape[2]:
+        if max_len is not None and int(max_len) > k_pool.shape[2]:
             raise ValueError("max_len exceeds the cache length")
-    with torch.cuda.device(q.device):
-        out = torch.empty_like(q) if out is None else out
-        if lse is None and need_lse:
-            lse = torch.empty((B, H, 1), dtype=torch.float32, device=q.device)
-        d = capi.make_desc(B, H, 1, L, D, capi.TT_BF16, False, scale, Hkv=Hkv)
-        need = int(capi.lib.tt_attn_decode_workspace_bytes(ctypes.byref(d)))
-        if need and (workspace is None or workspace.numel() * workspace.element_size() < need):
-            workspace = torch.empty(need, dtype=torch.uint8, device=q.device)
-        nbytes = workspace.numel() * workspace.element_size() if workspace is not None else 0
-        capi.check(capi.lib.tt_attn_decode_paged(ctypes.byref(d), _p(q), _p(k_pool), _p(v_pool), _p(block_table),
-                                                 _p(seq_lens), page_size, max_pages, _p(out), _p(lse), _p(workspace),
-                                                 nbytes, _stream_ptr(q)))
-    return out, lse
+
+
+def attention_decode_paged(q, k_pool, v_pool, block_table=None, seq_lens=None, max_len=None, scale=None, out=None,
+                           lse=None, workspace=None, need_lse=True):
+    """Single-query attention over a paged and/or ragged cache (bf16, D 64 or 128).
+
+    q `[B,H,1,D]`.  With `block_table` (int32 `[B, max_pages]`, CUDA): k_pool, v_pool are page pools
+    `[pages, Hkv, page_size, D]`.  Without: dense `[B,Hkv,L,D]`.  `seq_lens` (int32 `[B]`, CUDA)
+    limits each batch entry to its first seq_lens[b] keys.  `max_len`: longest possible sequence
+    (default: page_size * max_pages, or L of the dense cache)."""
+    r = _native.attention_decode_paged(q, k_pool, v_pool, block_table, seq_lens, max_len, scale, out, lse, workspace, need_lse)
+    return r if r.__class__ is tuple else _done(r, _explain_paged, q, k_pool, v_pool, block_table, seq_lens, max_len)
+
+
+def _explain_softmax_forward(x):
+    raise ValueError("softmax_forward takes a contiguous float32/bfloat16 CUDA tensor")
 
 
 def softmax_forward(x, out=None):
     """Softmax over the last axis of a contiguous CUDA tensor (float32 or bfloat16)."""
-    if not x.is_cuda or not x.is_contiguous() or x.dtype not in _DT:
-        raise ValueError("softmax_forward takes a contiguous float32/bfloat16 CUDA tensor")
-    cols = x.shape[-1]
-    rows = x.numel() // cols if cols else 0
-    with torch.cuda.device(x.device):
-        out = torch.empty_like(x) if out is None else out
-        capi.check(capi.lib.tt_softmax_fwd(_p(x), _p(out), rows, cols, _DT[x.dtype], _stream_ptr(x)))
-    return out
+    r = _native.softmax_forward(x, out)
+    return r if r is not None and r.__class__ is not int else _done(r, _explain_softmax_forward, x)
+
+
+def _explain_softmax_backward(y, dy):
+    raise ValueError("softmax_backward takes two contiguous CUDA tensors of one shape and dtype")
 
 
 def softmax_backward(y, dy, dx=None):
     """dx = y * (dy - sum(dy * y, last axis)) for y = softmax(x)."""
-    if not (y.is_cuda and dy.is_cuda and y.is_contiguous() and dy.is_contiguous()) or y.dtype != dy.dtype \
-            or y.shape != dy.shape or y.dtype not in _DT:
-        raise ValueError("softmax_backward takes two contiguous CUDA tensors of one shape and dtype")
-    cols = y.shape[-1]
-    rows = y.numel() // cols if cols else 0
-    with torch.cuda.device(y.device):
-        dx = torch.empty_like(y) if dx is None else dx
-        capi.check(capi.lib.tt_softmax_bwd(_p(y), _p(dy), _p(dx), rows, cols, _DT[y.dtype], _stream_ptr(y)))
-    return dx
+    r = _native.softmax_backward(y, dy, dx)
+    return r if r is not None and r.__class__ is not int else _done(r, _explain_softmax_backward, y, dy)
 
 
-def _fc_check(x, w):
+def _explain_fc(x, w, bias=None, dy=None):
     if not (x.is_cuda and w.is_cuda and x.is_contiguous() and w.is_contiguous()) or x.dtype != w.dtype \
             or x.dtype not in _DT or w.dim() != 2 or x.dim() < 1 or x.shape[-1] != w.shape[0]:
         raise ValueError("fc takes contiguous CUDA tensors x [..., in] and w [in, out] of one dtype (float32/bfloat16)")
-    return x.numel() // x.shape[-1] if x.shape[-1] else 0, w.shape[0], w.shape[1]
+    if dy is not None:
+        raise ValueError("dy must be a contiguous CUDA tensor shaped like the layer's output")
+    raise ValueError(f"bias must be a CUDA tensor of shape ({w.shape[1]},) and dtype {x.dtype}")
 
 
 def fc_forward(x, w, bias=None, out=None):
     """y = x @ w + bias for x `[..., in]`, w `[in, out]`, bias `[out]` or None."""
-    rows, fin, fout = _fc_check(x, w)
-    if bias is not None and (bias.dtype != x.dtype or tuple(bias.shape) != (fout,) or not bias.is_cuda):
-        raise ValueError(f"bias must be a CUDA tensor of shape ({fout},) and dtype {x.dtype}")
-    with torch.cuda.device(x.device):
-        if out is None:
-            out = torch.empty(tuple(x.shape[:-1]) + (fout,), dtype=x.dtype, device=x.device)
-        capi.check(capi.lib.tt_fc_fwd(_p(x), _p(w), _p(bias), _p(out), rows, fin, fout, _DT[x.dtype], _stream_ptr(x)))
-    return out
+    r = _native.fc_forward(x, w, bias, out)
+    return r if r is not None and r.__class__ is not int else _done(r, _explain_fc, x, w, bias)
 
 
 def fc_backward(x, w, dy, need_dx=True, need_dw=True, need_db=True, scalar_bias=False, workspace=None):
     """(dx, dw, db) of `fc_forward` for upstream gradient dy `[..., out]`; skipped ones are None."""
-    rows, fin, fout = _fc_check(x, w)
-    if dy.dtype != x.dtype or not dy.is_cuda or not dy.is_contiguous() or tuple(dy.shape) != tuple(x.shape[:-1]) + (fout,):
-        raise ValueError("dy must be a contiguous CUDA tensor shaped like the layer's output")
-    with torch.cuda.device(x.device):
-        dx = torch.empty_like(x) if need_dx else None
-        dw = torch.empty_like(w) if need_dw else None
-        db = torch.empty((1 if scalar_bias else fout,), dtype=x.dtype, device=x.device) if need_db else None
-        need = int(capi.lib.tt_fc_bwd_workspace_bytes(rows, fin, fout, _DT[x.dtype])) if need_db else 0
-        if need and (workspace is None or workspace.numel() * workspace.element_size() < need):
-            workspace = torch.empty(need, dtype=torch.uint8, device=x.device)
-        nbytes = workspace.numel() * workspace.element_size() if workspace is not None else 0
-        capi.check(capi.lib.tt_fc_bwd(_p(x), _p(w), _p(dy), _p(dx), _p(dw), _p(db), int(bool(scalar_bias)), rows, fin, fout,
-                                      _DT[x.dtype], _p(workspace), nbytes, _stream_ptr(x)))
-    return dx, dw, db
+    r = _native.fc_backward(x, w, dy, need_dx, need_dw, need_db, scalar_bias, workspace)
+    return r if r.__class__ is tuple else _done(r, _explain_fc, x, w, None, dy)
 
 
 def check_device_status(device=None):
