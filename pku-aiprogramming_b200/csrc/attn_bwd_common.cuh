@@ -38,7 +38,8 @@ struct BwdParams {
     int causal;
     float scale, scale_log2;
     unsigned int* status;
-    unsigned int* sched_counter;   // zero at launch; work items are taken with atomicAdd
+    unsigned int* sched_counter;   // CTA-pair kernel: zero at launch; work items are taken with atomicAdd
+    int first_wave;                // one-CTA kernels: CTAs that start together (one per SM); the rest are taken over
     int n_items;                   // resident slices * n_tiles
     int group;                     // query heads per key/value head (1 = ordinary multi-head attention)
     const int* kv_lens;            // optional key padding lengths per batch entry (see AttnArgs)

@@ -136,6 +136,8 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
     int* sched_item = reinterpret_cast<int*>(bar_stat + 2);      // [2]
     uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(sched_item + 2);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_base_slot + 1);
+    uint64_t* bar_steal = reinterpret_cast<uint64_t*>(aux + 1024 - 32);
+    uint4* steal_response = reinterpret_cast<uint4*>(bar_steal + 2);
     float* s_stat = reinterpret_cast<float*>(aux + 1024);       // [2 buffers][2: -lse2, -delta][128]
 
     const int warp = uniform_warp_idx();
@@ -143,7 +145,9 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
     const int off = p.L - p.S;
 
     if (threadIdx.x == 0) {
-        *abort_flag = 0;
+        // a CTA that the hardware starts after another one's wait has given up leaves at once
+        *abort_flag = ((int)blockIdx.x >= p.first_wave && *reinterpret_cast<volatile unsigned int*>(p.status) != 0u) ? 1 : 0;
+        mbar_init(bar_steal, 1);
         mbar_init(bar_res_full, 1);
         mbar_init(bar_res_empty, 1);
         for (int s = 0; s < 4; ++s) {
@@ -184,6 +188,8 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
     tc_fence_after();
     const uint32_t tmem_base = *tmem_base_slot;
     WaitCtx wctx{p.status, abort_flag, warp};
+    grid_let_next_start();
+    grid_wait_for_previous();
     constexpr uint32_t kColX = 0, kColY = 128, kColDV = 256, kColDK = 256 + D;
 
     auto next_item = [&](int k) -> int {
@@ -453,11 +459,9 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
                 for (int sb = 0; sb < Cfg::kSub; ++sb) tma_load_3d(dst + sb * Cfg::kSubBytes, tm, bar, sb * 64, row_start, bh);
             };
             uint32_t git = 0;
-            for (int k = 0;; ++k) {
-                int item = 0;
-                if (lane == 0) item = (int)atomicAdd(p.sched_counter, 1u);
-                item = __shfl_sync(0xffffffffu, item, 0);
-                if (item >= p.n_items || *abort_flag) item = -1;   // an aborted CTA takes no further items
+            ItemStream items{bar_steal, steal_response, p.n_items > p.first_wave};
+            int item = *abort_flag ? -1 : (int)blockIdx.x;
+            for (int k = 0;; ++k, item = items.next(wctx, 89, k)) {
                 const int slot = k & 1;
                 mbar_wait(&bar_sched_empty[slot], ((k >> 1) & 1) ^ 1, wctx, 90 + slot, k);
                 __syncwarp();
@@ -495,6 +499,7 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
                     }
                     __syncwarp();
                 }
+                items.request(*abort_flag != 0);   // an aborted CTA takes no further items
             }
         } else if (warp == 8) {
             // ============================================================ MMA issuer (whole warp runs the
@@ -648,6 +653,8 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
 template <int D>
 __global__ void __launch_bounds__(256) attn_bwd_dq_convert_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dq,
                                                                  int S, int n_qt, float scale, int wide) {
+    grid_let_next_start();
+    grid_wait_for_previous();
     const long long blk = blockIdx.x;            // qs * n_qt + t
     const int t = (int)(blk % n_qt);
     const long long qs = blk / n_qt;
@@ -707,7 +714,7 @@ static cudaError_t launch_fused(const AttnArgs& a, void* ws, cudaStream_t st) {
     if (!make_tmap_bf16(&tv, a.v, D, a.L, a.BH / a.group, 128, &why)) return cudaErrorInvalidValue;
     if (!make_tmap_bf16(&tdo, a.dout, D, a.S, a.BH, 128, &why)) return cudaErrorInvalidValue;
     auto M = [](TmapStorage& t) -> CUtensorMap& { return *reinterpret_cast<CUtensorMap*>(t.bytes); };
-    e = cudaFuncSetAttribute(attn_bwd_fused_sm100_kernel<D, kTrace>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
+    e = TT_ALLOW_SMEM((attn_bwd_fused_sm100_kernel<D, kTrace>), Cfg::kSmemBytes);
     if (e != cudaSuccess) return e;
     BwdParams p;
     memset(&p, 0, sizeof(p));
@@ -734,21 +741,14 @@ static cudaError_t launch_fused(const AttnArgs& a, void* ws, cudaStream_t st) {
     p.n_qt = (a.S + 127) / 128;
     p.trace = kTrace ? g_fused_trace : nullptr;
     p.trace_block = g_fused_trace_block;
-    int dev = 0, n_sm = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
-    SchedCounter sc;
-    e = sched_counter_acquire(st, &sc);
-    if (e != cudaSuccess) return e;
-    p.sched_counter = sc.ptr;
+    p.first_wave = sm_count();
     {
         LaunchScope ls(K_BWD_FUSED, st);
-        attn_bwd_fused_sm100_kernel<D, kTrace><<<(unsigned)std::min(p.n_items, n_sm), Cfg::kThreads, Cfg::kSmemBytes, st>>>(
-            M(tk), M(tv), M(tq), M(tdo), p);
+        launch_overlapped(attn_bwd_fused_sm100_kernel<D, kTrace>, (unsigned)p.n_items, Cfg::kThreads, Cfg::kSmemBytes, st, M(tk), M(tv), M(tq), M(tdo), p);
     }
-    sched_counter_release(sc, st);
     {
         LaunchScope ls(K_BWD_DQ_CONVERT, st);
-        attn_bwd_dq_convert_kernel<D><<<(unsigned)(a.BH * p.n_qt), 256, 0, st>>>(dq_acc, (__nv_bfloat16*)a.dq, a.S, p.n_qt, a.scale,
+        launch_overlapped(attn_bwd_dq_convert_kernel<D>, (unsigned)(a.BH * p.n_qt), 256, 0, st, dq_acc, (__nv_bfloat16*)a.dq, a.S, p.n_qt, a.scale,
                                                                                   (reinterpret_cast<uintptr_t>(a.dq) & 31) == 0 ? 1 : 0);
     }
     return cudaGetLastError();

@@ -547,7 +547,7 @@ int max_resident_pairs() {
     if (!cached[dev]) {
         int n_sm = 148;
         cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
-        cudaFuncSetAttribute(attn_bwd_dkv_pair_sm100_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdPairCfg::kSmemBytes);
+        TT_ALLOW_SMEM((attn_bwd_dkv_pair_sm100_kernel), BwdPairCfg::kSmemBytes);
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)n_sm & ~1u);
         cfg.blockDim = dim3(BwdPairCfg::kThreads);
@@ -596,7 +596,7 @@ cudaError_t attn_bwd_dkv_pair(const AttnArgs& a, const float* delta, const float
     if (!make_tmap_bf16(&tdo64, a.dout, D, a.S, a.BH, 64, &why)) return cudaErrorInvalidValue;
     if (!make_tmap_bf16(&tdo128, a.dout, D, a.S, a.BH, 128, &why)) return cudaErrorInvalidValue;
     auto M = [](TmapStorage& t) -> CUtensorMap& { return *reinterpret_cast<CUtensorMap*>(t.bytes); };
-    cudaError_t e = cudaFuncSetAttribute(attn_bwd_dkv_pair_sm100_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
+    cudaError_t e = TT_ALLOW_SMEM((attn_bwd_dkv_pair_sm100_kernel), Cfg::kSmemBytes);
     if (e != cudaSuccess) return e;
     BwdParams p;
     memset(&p, 0, sizeof(p));

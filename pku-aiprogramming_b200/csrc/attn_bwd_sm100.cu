@@ -61,8 +61,8 @@ enum BwdBarId { BB_RES = 0, BB_STFULL = 10, BB_STEMPTY = 20, BB_SFULL = 30, BB_D
             p.trace[((role) * 64 + (iter)) * 8 + (slot)] = clock64();                              \
     } while (0)
 
-// Persistent like the forward: one CTA per SM takes (slice, resident tile) items from a global
-// counter, heavy items of a slice first; the loader runs up to two items ahead and the first
+// Persistent like the forward: one CTA per SM takes (slice, resident tile) items (ItemStream), heavy
+// items of a slice first; the loader runs up to two items ahead and the first
 // MMAs of the next item overlap the write-out of the accumulators of the current one.
 // kTrace: compiled with the cycle stamps (debug aid; launched only while a trace buffer is set).
 // kVarlen: packed variable-length batches (per-item sequence geometry, token-major addressing).
@@ -113,6 +113,8 @@ attn_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmR0, const __grid_con
     int* sched_item = reinterpret_cast<int*>(bar_res_tmem + 1);  // [2]
     uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(sched_item + 2);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_base_slot + 1);
+    uint64_t* bar_steal = reinterpret_cast<uint64_t*>(aux + 1024 - 32);
+    uint4* steal_response = reinterpret_cast<uint4*>(bar_steal + 2);
     float* s_stat = reinterpret_cast<float*>(aux + 1024);     // [2 buffers][2: -lse2, -delta][128]
 
     const int warp = uniform_warp_idx();
@@ -128,7 +130,9 @@ attn_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmR0, const __grid_con
     constexpr uint32_t kColRes = 256;   // Q at [256, 256 + D/2), dO at [256 + D/2, 256 + D)
 
     if (threadIdx.x == 0) {
-        *abort_flag = 0;
+        // a CTA that the hardware starts after another one's wait has given up leaves at once
+        *abort_flag = ((int)blockIdx.x >= p.first_wave && *reinterpret_cast<volatile unsigned int*>(p.status) != 0u) ? 1 : 0;
+        mbar_init(bar_steal, 1);
         mbar_init(bar_res_full, 1);
         // the resident pair may be reloaded when the MMA warp has issued its last reads of it and, where
         // the compute threads copy it to tensor memory, when all of them have done so (short items
@@ -172,6 +176,11 @@ attn_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmR0, const __grid_con
     tc_fence_after();
     const uint32_t tmem_base = *tmem_base_slot;
     WaitCtx wctx{p.status, abort_flag, warp};
+    // The dK/dV pass lets the dQ pass start only behind its own wait, i.e. when the statistics are complete; the
+    // dQ pass needs nothing else, so its CTAs begin to work as the dK/dV pass's last CTAs leave the SMs, and it
+    // waits for that pass at its END (what follows on the stream may rely on both).
+    if (kKeysResident) grid_wait_for_previous();
+    grid_let_next_start();
     constexpr uint32_t kColS = 0, kColDP = 128, kColAcc0 = 256, kColAcc1 = 256 + D;
 
     auto next_item = [&](int k) -> int {
@@ -478,19 +487,18 @@ attn_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmR0, const __grid_con
                 for (int sb = 0; sb < Cfg::kSub; ++sb) tma_load_3d(dst + sb * Cfg::kSubBytes, tm, bar, sb * 64, row_start, bh);
             };
             uint32_t git = 0;
-            for (int k = 0;; ++k) {
-                int item = 0;
+            ItemStream items{bar_steal, steal_response, p.n_items > p.first_wave};
+            int item = *abort_flag ? -1 : (int)blockIdx.x;
+            for (int k = 0;; ++k, item = items.next(wctx, 89, k)) {
                 BwdItem w;
-                for (;;) {
-                    if (lane == 0) item = (int)atomicAdd(p.sched_counter, 1u);
-                    item = __shfl_sync(0xffffffffu, item, 0);
-                    if (item >= p.n_items || *abort_flag) item = -1;   // an aborted CTA takes no further items
-                    if (item < 0) break;
+                while (item >= 0) {
                     w = bwd_decode_item<kKeysResident, kVarlen>(item, p);
                     // packed batches number their items for the longest sequence: what lies past a shorter
                     // sequence's end, or sees nothing under the causal mask, is never published (the
                     // outputs were cleared before the launch)
                     if (!kVarlen || w.n_it > 0) break;
+                    items.request(*abort_flag != 0);
+                    item = items.next(wctx, 89, k);
                 }
                 const int slot = k & 1;
                 mbar_wait(&bar_sched_empty[slot], ((k >> 1) & 1) ^ 1, wctx, 90 + slot, k);
@@ -533,6 +541,7 @@ attn_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmR0, const __grid_con
                     }
                     __syncwarp();
                 }
+                items.request(*abort_flag != 0);   // an aborted CTA takes no further items
             }
         } else if (warp == 8) {
             // ============================================================ MMA issuer (whole warp runs the
@@ -664,6 +673,7 @@ attn_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmR0, const __grid_con
         tc_fence_after();
         tmem_dealloc(tmem_base, Cfg::kTmemCols);
     }
+    if (!kKeysResident) grid_wait_for_previous();
 }
 
 // ---------------------------------------------------------------- preprocessing
@@ -683,6 +693,8 @@ template <int D, bool kVarlen>
 __global__ void __launch_bounds__(256) attn_bwd_prep_kernel(const __nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ dout,
                                                             const float* __restrict__ lse, float* __restrict__ delta,
                                                             float* __restrict__ lse2, long long n_rows, long long total_q, int H) {
+    grid_let_next_start();
+    grid_wait_for_previous();
     constexpr int kLanesPerRow = D / 8, kRowsPerStep = 32 / kLanesPerRow;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int sub = lane / kLanesPerRow, li = lane % kLanesPerRow;
@@ -726,8 +738,7 @@ __global__ void __launch_bounds__(256) attn_bwd_prep_kernel(const __nv_bfloat16*
 template <int D, bool kVarlen>
 static void launch_prep(const AttnArgs& a, float* delta, float* lse2, long long n_rows, cudaStream_t st) {
     const long long per_cta = 8LL * (32 / (D / 8)) * kPrepUnroll;
-    attn_bwd_prep_kernel<D, kVarlen><<<(unsigned)((n_rows + per_cta - 1) / per_cta), 256, 0, st>>>(
-        (const __nv_bfloat16*)a.out, (const __nv_bfloat16*)a.dout, a.lse, delta, lse2, n_rows, a.total_q, a.H);
+    launch_overlapped(attn_bwd_prep_kernel<D, kVarlen>, (unsigned)((n_rows + per_cta - 1) / per_cta), 256, 0, st, (const __nv_bfloat16*)a.out, (const __nv_bfloat16*)a.dout, a.lse, delta, lse2, n_rows, a.total_q, a.H);
 }
 cudaError_t attn_bwd_prep(const AttnArgs& a, float* delta, float* lse2, cudaStream_t st) {
     LaunchScope ls(K_BWD_PREP, st);
@@ -791,9 +802,9 @@ static cudaError_t launch_bwd(const AttnArgs& a, void* ws, cudaStream_t st) {
         if (!make_tmap_bf16(&tdo, a.dout, D, a.S, a.BH, 128, &why)) return cudaErrorInvalidValue;
     }
     auto M = [](TmapStorage& t) -> CUtensorMap& { return *reinterpret_cast<CUtensorMap*>(t.bytes); };
-    e = cudaFuncSetAttribute(attn_bwd_sm100_kernel<D, true, kTrace, kVarlen>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
+    e = TT_ALLOW_SMEM((attn_bwd_sm100_kernel<D, true, kTrace, kVarlen>), Cfg::kSmemBytes);
     if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(attn_bwd_sm100_kernel<D, false, kTrace, kVarlen>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
+    e = TT_ALLOW_SMEM((attn_bwd_sm100_kernel<D, false, kTrace, kVarlen>), Cfg::kSmemBytes);
     if (e != cudaSuccess) return e;
     BwdParams p;
     memset(&p, 0, sizeof(p));
@@ -808,8 +819,7 @@ static cudaError_t launch_bwd(const AttnArgs& a, void* ws, cudaStream_t st) {
     p.trace = g_bwd_trace_mode == 1 ? g_bwd_trace : nullptr;
     p.trace_block = g_bwd_trace_block;
     // dK, dV: keys resident, stream (Q, dO)
-    int dev = 0, n_sm = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
+    p.first_wave = sm_count();
     p.out0 = (__nv_bfloat16*)a.dv;
     p.out1 = (__nv_bfloat16*)a.dk;
     p.group = a.group;
@@ -825,20 +835,12 @@ static cudaError_t launch_bwd(const AttnArgs& a, void* ws, cudaStream_t st) {
     p.n_items = (int)(a.BH / a.group * p.n_tiles);
     p.n_light = a.causal ? p.n_tiles / 4 : 0;
     p.n_items_heavy = (int)(a.BH / a.group * (p.n_tiles - p.n_light));
-    SchedCounter sc;
     if (D == 128 && !kTrace && !kVarlen && attn_bwd_dkv_pair_supported(a)) {
         // same pass on CTA pairs: each MMA reads half of its streamed operand per SM
         if ((e = attn_bwd_dkv_pair(a, delta, lse2, st)) != cudaSuccess) return e;
     } else {
-        e = sched_counter_acquire(st, &sc);
-        if (e != cudaSuccess) return e;
-        p.sched_counter = sc.ptr;
-        {
-            LaunchScope ls(K_BWD_DKV, st);
-            attn_bwd_sm100_kernel<D, true, kTrace, kVarlen><<<(unsigned)std::min(p.n_items, n_sm), Cfg::kThreads, Cfg::kSmemBytes, st>>>(
-                M(tk), M(tv), M(tq), M(tdo), p);
-        }
-        sched_counter_release(sc, st);
+        LaunchScope ls(K_BWD_DKV, st);
+        launch_overlapped(attn_bwd_sm100_kernel<D, true, kTrace, kVarlen>, (unsigned)p.n_items, Cfg::kThreads, Cfg::kSmemBytes, st, M(tk), M(tv), M(tq), M(tdo), p);
     }
     // dQ: queries resident, stream (K, V)
     p.trace = g_bwd_trace_mode == 2 ? g_bwd_trace : nullptr;
@@ -848,15 +850,10 @@ static cudaError_t launch_bwd(const AttnArgs& a, void* ws, cudaStream_t st) {
     p.n_items = (int)(a.BH * p.n_tiles);
     p.n_light = a.causal ? p.n_tiles / 4 : 0;
     p.n_items_heavy = (int)(a.BH * (p.n_tiles - p.n_light));
-    e = sched_counter_acquire(st, &sc);
-    if (e != cudaSuccess) return e;
-    p.sched_counter = sc.ptr;
     {
         LaunchScope ls(K_BWD_DQ, st);
-        attn_bwd_sm100_kernel<D, false, kTrace, kVarlen><<<(unsigned)std::min(p.n_items, n_sm), Cfg::kThreads, Cfg::kSmemBytes, st>>>(
-            M(tq), M(tdo), M(tk), M(tv), p);
+        launch_overlapped(attn_bwd_sm100_kernel<D, false, kTrace, kVarlen>, (unsigned)p.n_items, Cfg::kThreads, Cfg::kSmemBytes, st, M(tq), M(tdo), M(tk), M(tv), p);
     }
-    sched_counter_release(sc, st);
     return cudaGetLastError();
 }
 

@@ -92,6 +92,8 @@ attn_decode_bf16_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16
                         const __nv_bfloat16* __restrict__ v, __nv_bfloat16* __restrict__ out,
                         float* __restrict__ lse, float* __restrict__ partial, int L, int splits, int chunk,
                         float scale_log2, int map_group, DecodeRows rows) {
+    grid_let_next_start();
+    grid_wait_for_previous();
     constexpr int LPR = D / 8;        // lanes per key row
     constexpr int RPI = 32 / LPR;     // rows per warp load instruction
     __shared__ float sm_m[G][kDecWarps], sm_l[G][kDecWarps];
@@ -239,6 +241,8 @@ attn_decode_bf16_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16
 template <int D>
 __global__ void attn_decode_merge_kernel(const float* __restrict__ partial, __nv_bfloat16* __restrict__ out,
                                          float* __restrict__ lse, int splits, int G) {
+    grid_let_next_start();
+    grid_wait_for_previous();
     const long long bh = blockIdx.x;
     const int d = threadIdx.x;
     const long long kvs = bh / G;
@@ -303,8 +307,7 @@ static int decode_tc_splits(const AttnArgs& a) {   // 0: do not use the forward 
     if (!(a.bf16 && a.S == 1 && a.group >= min_group)) return 0;
     if (f && f[0] == 's') return 0;                           // "simt"
     if (!attn_fwd_sm100_supported(decode_as_forward(a, 1))) return 0;
-    int dev = 0, n_sm = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
+    const int n_sm = sm_count();
     const long long slices = a.BH / a.group;
     const bool gq = decode_on_gq_kernel(a);
     const long long min_chunk = gq ? 512 : 256;
@@ -332,8 +335,7 @@ DecodePlan attn_decode_plan(const AttnArgs& a, bool allow_tc) {
             return pl;
         }
     }
-    int dev = 0, n_sm = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
+    const int n_sm = sm_count();
     const long long resident = (long long)n_sm * 4;
     const long long target = resident * 12;
     const long long cta_slices = decode_group_instantiated(a.group) ? a.BH / a.group : a.BH;
@@ -358,6 +360,8 @@ DecodePlan attn_decode_plan(const AttnArgs& a, bool allow_tc) {
 template <int D>
 __global__ void attn_decode_tc_merge_kernel(const __nv_bfloat16* __restrict__ po, const float* __restrict__ plse,
                                             __nv_bfloat16* __restrict__ out, float* __restrict__ lse, int splits, int G) {
+    grid_let_next_start();
+    grid_wait_for_previous();
     const long long bh = blockIdx.x;
     const int d = threadIdx.x;
     const long long kvs = bh / G;
@@ -383,8 +387,7 @@ __global__ void attn_decode_tc_merge_kernel(const __nv_bfloat16* __restrict__ po
 template <int D, int G>
 static void launch_decode_g(const AttnArgs& a, const DecodePlan& pl, void* ws, cudaStream_t st, const DecodeRows& rows) {
     const long long units = (a.BH / G) * pl.splits;
-    attn_decode_bf16_kernel<D, G><<<(unsigned)units, kDecThreads, 0, st>>>(
-        (const __nv_bfloat16*)a.q, (const __nv_bfloat16*)a.k, (const __nv_bfloat16*)a.v, (__nv_bfloat16*)a.out, a.lse,
+    launch_overlapped(attn_decode_bf16_kernel<D, G>, (unsigned)units, kDecThreads, 0, st, (const __nv_bfloat16*)a.q, (const __nv_bfloat16*)a.k, (const __nv_bfloat16*)a.v, (__nv_bfloat16*)a.out, a.lse,
         (float*)ws, a.L, pl.splits, pl.chunk, a.scale * 1.4426950408889634f, a.group, rows);
 }
 
@@ -405,7 +408,7 @@ static cudaError_t launch_decode(const AttnArgs& a, const DecodePlan& pl, void* 
     }
     if (pl.splits > 1) {
         LaunchScope ls(K_DECODE_MERGE, st, allow_timing);
-        attn_decode_merge_kernel<D><<<(unsigned)a.BH, D, 0, st>>>((const float*)ws, (__nv_bfloat16*)a.out, a.lse,
+        launch_overlapped(attn_decode_merge_kernel<D>, (unsigned)a.BH, D, 0, st, (const float*)ws, (__nv_bfloat16*)a.out, a.lse,
                                                                   pl.splits, G);
     }
     return cudaGetLastError();
@@ -430,8 +433,7 @@ static AttnArgs paged_as_forward(const AttnArgs& a, const DecodeView& v, int spl
     return g;
 }
 static void paged_split(const AttnArgs& a, int* splits, int* chunk) {
-    int dev = 0, n_sm = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
+    const int n_sm = sm_count();
     const long long slices = a.BH / a.group;
     *splits = 1;
     *chunk = a.L;
@@ -472,9 +474,9 @@ cudaError_t attn_decode_paged_forward(const AttnArgs& a, const DecodeView& v, in
     if (e != cudaSuccess) return e;
     LaunchScope ls(K_DECODE_MERGE, st);
     if (a.D == 128)
-        attn_decode_tc_merge_kernel<128><<<(unsigned)a.BH, 128, 0, st>>>(po, plse, (__nv_bfloat16*)a.out, a.lse, splits, a.group);
+        launch_overlapped(attn_decode_tc_merge_kernel<128>, (unsigned)a.BH, 128, 0, st, po, plse, (__nv_bfloat16*)a.out, a.lse, splits, a.group);
     else
-        attn_decode_tc_merge_kernel<64><<<(unsigned)a.BH, 64, 0, st>>>(po, plse, (__nv_bfloat16*)a.out, a.lse, splits, a.group);
+        launch_overlapped(attn_decode_tc_merge_kernel<64>, (unsigned)a.BH, 64, 0, st, po, plse, (__nv_bfloat16*)a.out, a.lse, splits, a.group);
     return cudaGetLastError();
 }
 
@@ -491,9 +493,9 @@ cudaError_t attn_decode(const AttnArgs& a, const DecodePlan& pl, void* ws, cudaS
         if (e != cudaSuccess) return e;
         LaunchScope ls(K_DECODE_MERGE, st);
         if (a.D == 128)
-            attn_decode_tc_merge_kernel<128><<<(unsigned)a.BH, 128, 0, st>>>(po, plse, (__nv_bfloat16*)a.out, a.lse, pl.tc_splits, a.group);
+            launch_overlapped(attn_decode_tc_merge_kernel<128>, (unsigned)a.BH, 128, 0, st, po, plse, (__nv_bfloat16*)a.out, a.lse, pl.tc_splits, a.group);
         else
-            attn_decode_tc_merge_kernel<64><<<(unsigned)a.BH, 64, 0, st>>>(po, plse, (__nv_bfloat16*)a.out, a.lse, pl.tc_splits, a.group);
+            launch_overlapped(attn_decode_tc_merge_kernel<64>, (unsigned)a.BH, 64, 0, st, po, plse, (__nv_bfloat16*)a.out, a.lse, pl.tc_splits, a.group);
         return cudaGetLastError();
     }
     if (a.bf16 && a.S == 1 && a.D == 128) return launch_decode<128>(a, pl, ws, st, true, view);
@@ -511,7 +513,6 @@ static __device__ __align__(256) unsigned char g_decode_static_scratch[kStaticSc
 
 // In host code the array's name is only a handle for the runtime, not a device address: the
 // address a kernel can use has to be asked for, per device, with that device current.
-constexpr int kMaxDevices = 64;
 static void* g_static_scratch_addr[kMaxDevices];
 static std::atomic<int> g_static_scratch_ready[kMaxDevices];
 

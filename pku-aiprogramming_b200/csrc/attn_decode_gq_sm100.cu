@@ -101,18 +101,6 @@ attn_decode_gq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
     const int warp = uniform_warp_idx();
     const int lane = threadIdx.x & 31;
 
-    // ---- this CTA's key range
-    const int bh = blockIdx.x;                 // output slice
-    const int qslice = bh / p.q_div;
-    int zslice = bh, key0 = 0, Lv = p.L;
-    if (kCache) {
-        zslice = qslice;                       // key/value slice
-        key0 = (bh - qslice * p.q_div) * p.kv_chunk;
-        const int len = p.kv_lens ? min(p.L, max(0, p.kv_lens[zslice / p.H])) : p.L;
-        Lv = p.kv_chunk > 0 ? max(0, min(len - key0, p.kv_chunk)) : len;
-    }
-    const int n_tiles = (Lv + 127) >> 7;
-
     if (threadIdx.x == 0) {
         *abort_flag = 0;
         mbar_init(bar_q_full, 1);
@@ -143,6 +131,19 @@ attn_decode_gq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     WaitCtx wctx{p.status, abort_flag, warp};
+    grid_wait_for_previous();
+
+    // ---- this CTA's key range
+    const int bh = blockIdx.x;                 // output slice
+    const int qslice = bh / p.q_div;
+    int zslice = bh, key0 = 0, Lv = p.L;
+    if (kCache) {
+        zslice = qslice;                       // key/value slice
+        key0 = (bh - qslice * p.q_div) * p.kv_chunk;
+        const int len = p.kv_lens ? min(p.L, max(0, p.kv_lens[zslice / p.H])) : p.L;
+        Lv = p.kv_chunk > 0 ? max(0, min(len - key0, p.kv_chunk)) : len;
+    }
+    const int n_tiles = (Lv + 127) >> 7;
     constexpr uint32_t kColO = 32;
 
     if (warp < 4) {
@@ -395,6 +396,7 @@ attn_decode_gq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
             tc_commit(&bar_p_free[b]);   // P consumed; also: every MMA issued so far has completed
         }
     }
+    grid_let_next_start();
     tc_fence_before();
     __syncthreads();
     if (warp == 4) {
@@ -422,7 +424,7 @@ cudaError_t launch_gq(const AttnArgs& a, cudaStream_t st) {
         if (!make_tmap_bf16(&tk, a.k, kD, a.L, kv_slices, 128, &why)) return cudaErrorInvalidValue;
         if (!make_tmap_bf16(&tv, a.v, kD, a.L, kv_slices, 128, &why)) return cudaErrorInvalidValue;
     }
-    cudaError_t e = cudaFuncSetAttribute(attn_decode_gq_sm100_kernel<kD, kG, kCache>, cudaFuncAttributeMaxDynamicSharedMemorySize, GqCfg<kD>::kSmemBytes);
+    cudaError_t e = TT_ALLOW_SMEM((attn_decode_gq_sm100_kernel<kD, kG, kCache>), GqCfg<kD>::kSmemBytes);
     if (e != cudaSuccess) return e;
     GqParams p;
     p.out = (__nv_bfloat16*)a.out;
@@ -439,8 +441,7 @@ cudaError_t launch_gq(const AttnArgs& a, cudaStream_t st) {
     p.scale_log2 = a.scale * 1.4426950408889634f;
     p.status = device_status_word();
     LaunchScope ls(K_DECODE_GQ, st);
-    attn_decode_gq_sm100_kernel<kD, kG, kCache><<<(unsigned)a.BH, kThreads, GqCfg<kD>::kSmemBytes, st>>>(
-        *reinterpret_cast<CUtensorMap*>(tq.bytes), *reinterpret_cast<CUtensorMap*>(tk.bytes),
+    launch_overlapped(attn_decode_gq_sm100_kernel<kD, kG, kCache>, (unsigned)a.BH, kThreads, GqCfg<kD>::kSmemBytes, st, *reinterpret_cast<CUtensorMap*>(tq.bytes), *reinterpret_cast<CUtensorMap*>(tk.bytes),
         *reinterpret_cast<CUtensorMap*>(tv.bytes), p);
     return cudaGetLastError();
 }

@@ -17,8 +17,9 @@ struct FwdParams {
     int causal;
     float scale_log2; // scale * log2(e)
     unsigned int* status;
-    unsigned int* sched_counter;   // zero at launch; work items are taken with atomicAdd
+    unsigned int* sched_counter;   // CTA-pair kernel: zero at launch; work items are taken with atomicAdd
     int n_items;                   // slices * n_qblk
+    int first_wave;                // one-CTA kernel: CTAs that start together (one per SM); the rest are taken over
     int group;                     // query heads per key/value head: query slice bh reads key/value slice bh / group
     const int* kv_lens;            // optional key padding lengths per batch entry (see AttnArgs)
     int H;

@@ -493,7 +493,7 @@ int max_resident_pairs() {
     if (!cached[dev]) {
         int n_sm = 148;
         cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
-        cudaFuncSetAttribute(attn_fwd_pair_sm100_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg::kSmemBytes);
+        TT_ALLOW_SMEM((attn_fwd_pair_sm100_kernel), PairCfg::kSmemBytes);
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)n_sm & ~1u);
         cfg.blockDim = dim3(PairCfg::kThreads);
@@ -539,7 +539,7 @@ cudaError_t attn_fwd_pair_sm100(const AttnArgs& a, cudaStream_t st) {
     if (!make_tmap_bf16(&tq, a.q, D, a.S, a.BH, 128, &why)) return cudaErrorInvalidValue;
     if (!make_tmap_bf16(&tk, a.k, D, a.L, a.BH / a.group, 64, &why)) return cudaErrorInvalidValue;
     if (!make_tmap_bf16(&tv, a.v, D, a.L, a.BH / a.group, 128, &why)) return cudaErrorInvalidValue;
-    cudaError_t e = cudaFuncSetAttribute(attn_fwd_pair_sm100_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
+    cudaError_t e = TT_ALLOW_SMEM((attn_fwd_pair_sm100_kernel), Cfg::kSmemBytes);
     if (e != cudaSuccess) return e;
     FwdParams p = {};
     p.out = (__nv_bfloat16*)a.out;

@@ -64,8 +64,8 @@ enum FwdBarId { BAR_QFULL = 0, BAR_KVFULL = 10, BAR_KVEMPTY = 30, BAR_SFULL = 50
             p.trace[((role) * 64 + (iter)) * 8 + (slot)] = clock64();                              \
     } while (0)
 
-// The kernel is persistent: one CTA per SM takes work items (slice, 256-row query block) from a
-// global counter until none are left.  Items are numbered slice-major with the heavy (late)
+// The kernel is persistent: one CTA per SM takes work items (slice, 256-row query block) until none are
+// left (ItemStream).  Items are numbered slice-major with the heavy (late)
 // query blocks of a slice first, so that concurrently running CTAs share a slice's K/V in L2.
 // Causal launches keep the lightest quarter of every slice's blocks for a second pass over the
 // slices, so that the tail of the launch consists of light items.  The loader runs up to two items ahead; the
@@ -173,12 +173,16 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     int* sched_item = reinterpret_cast<int*>(bar_sched_empty + 2);   // [2]
     uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(sched_item + 2);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_base_slot + 1);
+    uint64_t* bar_steal = reinterpret_cast<uint64_t*>(reinterpret_cast<unsigned char*>(bars) + Cfg::kBarBytes - 32);
+    uint4* steal_response = reinterpret_cast<uint4*>(bar_steal + 2);
 
     const int warp = uniform_warp_idx();
     const int lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
-        *abort_flag = 0;
+        // a CTA that the hardware starts after another one's wait has given up leaves at once
+        *abort_flag = ((int)blockIdx.x >= p.first_wave && *reinterpret_cast<volatile unsigned int*>(p.status) != 0u) ? 1 : 0;
+        mbar_init(bar_steal, 1);
         for (int i = 0; i < 2; ++i) {
             mbar_init(&bar_q_full[i], 1);
             mbar_init(&bar_q_empty[i], 1);
@@ -211,6 +215,8 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     tc_fence_after();
     const uint32_t tmem_base = *tmem_base_slot;
     WaitCtx wctx{p.status, abort_flag, warp};
+    grid_let_next_start();
+    grid_wait_for_previous();
 
     // Every role walks the same item sequence.  Items are published by the loader in a two-slot
     // ring; a negative value ends the sequence.
@@ -380,11 +386,9 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             };
             uint32_t t = 0;                    // K/V ring item counter (runs across work items)
             uint32_t q_uses[2] = {0, 0};       // how often each Q buffer has been filled
-            for (int k = 0;; ++k) {
-                int item = 0;
-                if (lane == 0) item = (int)atomicAdd(p.sched_counter, 1u);
-                item = __shfl_sync(0xffffffffu, item, 0);
-                if (item >= p.n_items || *abort_flag) item = -1;   // an aborted CTA takes no further items
+            ItemStream items{bar_steal, steal_response, p.n_items > p.first_wave};
+            int item = *abort_flag ? -1 : (int)blockIdx.x;
+            for (int k = 0;; ++k, item = items.next(wctx, 89, k)) {
                 const int slot = k & 1;
                 mbar_wait(&bar_sched_empty[slot], ((k >> 1) & 1) ^ 1, wctx, 90 + slot, k);
                 __syncwarp();
@@ -440,6 +444,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
                     load_kv(&tmV, j);
                     if (j + 1 < w.n_max) load_kv(&tmK, j + 1);
                 }
+                items.request(*abort_flag != 0);   // an aborted CTA takes no further items
             }
         } else if (warp == 8) {
             // ======================================================= MMA issuer (whole warp runs the
@@ -652,8 +657,7 @@ static cudaError_t launch_fwd(const AttnArgs& a, cudaStream_t st) {
         if (!make_tmap_bf16(&tk, a.k, D, a.L, kv_slices, 128, &why)) return cudaErrorInvalidValue;
         if (!make_tmap_bf16(&tv, a.v, D, a.L, kv_slices, 128, &why)) return cudaErrorInvalidValue;
     }
-    cudaError_t e = cudaFuncSetAttribute(attn_fwd_sm100_kernel<D, kTrace, kPaged, kVarlen>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         Cfg::kSmemBytes);
+    cudaError_t e = TT_ALLOW_SMEM((attn_fwd_sm100_kernel<D, kTrace, kPaged, kVarlen>), Cfg::kSmemBytes);
     if (e != cudaSuccess) return e;
     FwdParams p;
     p.out = (__nv_bfloat16*)a.out;
@@ -689,21 +693,14 @@ static cudaError_t launch_fwd(const AttnArgs& a, cudaStream_t st) {
         p.n_light = a.causal ? p.n_qblk / 4 : 0;
         p.n_items_heavy = (int)(a.BH * (p.n_qblk - p.n_light));
     }
-    SchedCounter sc;
-    e = sched_counter_acquire(st, &sc);
-    if (e != cudaSuccess) return e;
-    p.sched_counter = sc.ptr;
-    int dev = 0, n_sm = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
-    unsigned grid = (unsigned)std::min<long long>(p.n_items, n_sm);
+    p.first_wave = sm_count();
     {
         LaunchScope ls(K_FWD_TC, st);
-        attn_fwd_sm100_kernel<D, kTrace, kPaged, kVarlen><<<grid, Cfg::kThreads, Cfg::kSmemBytes, st>>>(
-            *reinterpret_cast<CUtensorMap*>(tq.bytes), *reinterpret_cast<CUtensorMap*>(tk.bytes),
-            *reinterpret_cast<CUtensorMap*>(tv.bytes), p);
+        e = launch_overlapped(attn_fwd_sm100_kernel<D, kTrace, kPaged, kVarlen>, (unsigned)p.n_items, Cfg::kThreads, Cfg::kSmemBytes,
+                              st, *reinterpret_cast<CUtensorMap*>(tq.bytes), *reinterpret_cast<CUtensorMap*>(tk.bytes),
+                              *reinterpret_cast<CUtensorMap*>(tv.bytes), p);
     }
-    sched_counter_release(sc, st);
-    return cudaGetLastError();
+    return e;
 }
 
 template <int D>
@@ -838,7 +835,7 @@ static cudaError_t launch_probe(const void* a, const void* b, const void* vt, fl
     if (!make_tmap_bf16(&tb, b, 128, 128, 1, 128, &why)) return cudaErrorInvalidValue;
     if (!make_tmap_bf16(&tv, vt, D, 128, 1, 128, &why)) return cudaErrorInvalidValue;
     const int smem = 6 * 128 * 128 + 1024 + 1024;
-    cudaError_t e = cudaFuncSetAttribute(umma_probe_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = TT_ALLOW_SMEM((umma_probe_kernel<D>), smem);
     if (e != cudaSuccess) return e;
     {
         LaunchScope ls(K_PROBE, st);

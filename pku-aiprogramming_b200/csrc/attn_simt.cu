@@ -68,6 +68,7 @@ __global__ void __launch_bounds__(kSimtThreads) attn_fwd_simt_kernel(const T* __
                                                                       const T* __restrict__ v, T* __restrict__ out,
                                                                       float* __restrict__ lse, int S, int L, int D,
                                                                       int causal, float scale, int group, const int* __restrict__ kv_lens, int H) {
+    grid_wait_for_previous();
     extern __shared__ float smem[];
     const int pitch = D + 1;
     float* sQ = smem;
@@ -149,6 +150,7 @@ __global__ void __launch_bounds__(kSimtThreads) attn_fwd_simt_kernel(const T* __
 template <typename T>
 __global__ void attn_bwd_delta_kernel(const T* __restrict__ out, const T* __restrict__ dout,
                                       float* __restrict__ delta, long long n_rows, int D) {
+    grid_wait_for_previous();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     long long row = (long long)blockIdx.x * (blockDim.x >> 5) + warp;
     if (row >= n_rows) return;
@@ -164,6 +166,7 @@ __global__ void __launch_bounds__(kSimtThreads) attn_bwd_dq_simt_kernel(
     const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, const T* __restrict__ dout,
     const float* __restrict__ lse, const float* __restrict__ delta, T* __restrict__ dq, int S, int L, int D,
     int causal, float scale, int group, const int* __restrict__ kv_lens, int H) {
+    grid_wait_for_previous();
     extern __shared__ float smem[];
     const int pitch = D + 1;
     float* sQ = smem;
@@ -249,6 +252,7 @@ __global__ void __launch_bounds__(kSimtThreads) attn_bwd_dkv_simt_kernel(
     const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, const T* __restrict__ dout,
     const float* __restrict__ lse, const float* __restrict__ delta, T* __restrict__ dk, T* __restrict__ dv, int S,
     int L, int D, int causal, float scale, int group, const int* __restrict__ kv_lens, int H) {
+    grid_wait_for_previous();
     extern __shared__ float smem[];
     const int pitch = D + 1;
     float* sK = smem;
@@ -390,6 +394,7 @@ __global__ void __launch_bounds__(kTiledThreads, 2) attn_fwd_simt_tiled_kernel(
     const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, T* __restrict__ out,
     float* __restrict__ lse, int S, int L, int D, int causal, float scale, int group, const int* __restrict__ kv_lens,
     int H) {
+    grid_wait_for_previous();
     constexpr int DP = DMAX + 4;        // pitch: rows 16 bytes apart modulo 128, 128-bit loads conflict-free
     constexpr int NJ = DMAX / 64;       // float4 column groups of O per thread
     extern __shared__ __align__(16) float smem[];
@@ -598,6 +603,7 @@ __global__ void __launch_bounds__(kTiledThreads) attn_bwd_dq_simt_tiled_kernel(
     const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, const T* __restrict__ dout,
     const float* __restrict__ lse, const float* __restrict__ delta, T* __restrict__ dq, int S, int L, int D,
     int causal, float scale, int group, const int* __restrict__ kv_lens, int H) {
+    grid_wait_for_previous();
     constexpr int DP = DMAX + 4, NJ = DMAX / 64;
     extern __shared__ __align__(16) float smem[];
     float* sQ = smem;
@@ -675,6 +681,7 @@ __global__ void __launch_bounds__(kTiledThreads) attn_bwd_dkv_simt_tiled_kernel(
     const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, const T* __restrict__ dout,
     const float* __restrict__ lse, const float* __restrict__ delta, T* __restrict__ dk, T* __restrict__ dv, int S,
     int L, int D, int causal, float scale, int group, const int* __restrict__ kv_lens, int H) {
+    grid_wait_for_previous();
     constexpr int DP = DMAX + 4, NJ = DMAX / 64;
     extern __shared__ __align__(16) float smem[];
     float* sK = smem;
@@ -771,7 +778,7 @@ static cudaError_t launch_fwd_simt(const AttnArgs& a, cudaStream_t st) {
     unsigned grid = (unsigned)(((a.S + kRowsPerBlock - 1) / kRowsPerBlock) * a.BH);
     {
         LaunchScope ls(K_FWD_SIMT, st);
-        attn_fwd_simt_kernel<T, NV><<<grid, kSimtThreads, smem, st>>>((const T*)a.q, (const T*)a.k, (const T*)a.v,
+        launch_overlapped(attn_fwd_simt_kernel<T, NV>, grid, kSimtThreads, smem, st, (const T*)a.q, (const T*)a.k, (const T*)a.v,
                                                                       (T*)a.out, a.lse, a.S, a.L, a.D, a.causal,
                                                                       a.scale, a.group, a.kv_lens, a.H);
     }
@@ -800,15 +807,13 @@ static cudaError_t launch_bwd_simt_tiled(const AttnArgs& a, float* delta, cudaSt
     const unsigned gq = (unsigned)(((a.S + kTiledM - 1) / kTiledM) * a.BH);
     {
         LaunchScope ls(K_BWD_SIMT_DQ, st);
-        attn_bwd_dq_simt_tiled_kernel<T, DMAX><<<gq, kTiledThreads, smem_q, st>>>(
-            (const T*)a.q, (const T*)a.k, (const T*)a.v, (const T*)a.dout, a.lse, delta, (T*)a.dq, a.S, a.L, a.D,
+        launch_overlapped(attn_bwd_dq_simt_tiled_kernel<T, DMAX>, gq, kTiledThreads, smem_q, st, (const T*)a.q, (const T*)a.k, (const T*)a.v, (const T*)a.dout, a.lse, delta, (T*)a.dq, a.S, a.L, a.D,
             a.causal, a.scale, a.group, a.kv_lens, a.H);
     }
     const unsigned gk = (unsigned)(((a.L + kTiledM - 1) / kTiledM) * (a.BH / a.group));
     {
         LaunchScope ls(K_BWD_SIMT_DKV, st);
-        attn_bwd_dkv_simt_tiled_kernel<T, DMAX><<<gk, kTiledThreads, smem_kv, st>>>(
-            (const T*)a.q, (const T*)a.k, (const T*)a.v, (const T*)a.dout, a.lse, delta, (T*)a.dk, (T*)a.dv, a.S,
+        launch_overlapped(attn_bwd_dkv_simt_tiled_kernel<T, DMAX>, gk, kTiledThreads, smem_kv, st, (const T*)a.q, (const T*)a.k, (const T*)a.v, (const T*)a.dout, a.lse, delta, (T*)a.dk, (T*)a.dv, a.S,
             a.L, a.D, a.causal, a.scale, a.group, a.kv_lens, a.H);
     }
     return cudaGetLastError();
@@ -819,7 +824,7 @@ static cudaError_t launch_bwd_simt(const AttnArgs& a, float* delta, cudaStream_t
     long long n_rows = a.BH * (long long)a.S;
     {
         LaunchScope ls(K_BWD_SIMT_DELTA, st);
-        attn_bwd_delta_kernel<T><<<(unsigned)((n_rows + 7) / 8), 256, 0, st>>>((const T*)a.out, (const T*)a.dout,
+        launch_overlapped(attn_bwd_delta_kernel<T>, (unsigned)((n_rows + 7) / 8), 256, 0, st, (const T*)a.out, (const T*)a.dout,
                                                                               delta, n_rows, a.D);
     }
     if (simt_tiled_bwd_ok(a)) return a.D <= 64 ? launch_bwd_simt_tiled<T, 64>(a, delta, st) : launch_bwd_simt_tiled<T, 128>(a, delta, st);
@@ -832,15 +837,13 @@ static cudaError_t launch_bwd_simt(const AttnArgs& a, float* delta, cudaStream_t
     unsigned gq = (unsigned)(((a.S + kRowsPerBlock - 1) / kRowsPerBlock) * a.BH);
     {
         LaunchScope ls(K_BWD_SIMT_DQ, st);
-        attn_bwd_dq_simt_kernel<T, NV><<<gq, kSimtThreads, smem_q, st>>>(
-            (const T*)a.q, (const T*)a.k, (const T*)a.v, (const T*)a.dout, a.lse, delta, (T*)a.dq, a.S, a.L, a.D,
+        launch_overlapped(attn_bwd_dq_simt_kernel<T, NV>, gq, kSimtThreads, smem_q, st, (const T*)a.q, (const T*)a.k, (const T*)a.v, (const T*)a.dout, a.lse, delta, (T*)a.dq, a.S, a.L, a.D,
             a.causal, a.scale, a.group, a.kv_lens, a.H);
     }
     unsigned gk = (unsigned)(((a.L + kRowsPerBlock - 1) / kRowsPerBlock) * (a.BH / a.group));
     {
         LaunchScope ls(K_BWD_SIMT_DKV, st);
-        attn_bwd_dkv_simt_kernel<T, NV><<<gk, kSimtThreads, smem_kv, st>>>(
-            (const T*)a.q, (const T*)a.k, (const T*)a.v, (const T*)a.dout, a.lse, delta, (T*)a.dk, (T*)a.dv, a.S,
+        launch_overlapped(attn_bwd_dkv_simt_kernel<T, NV>, gk, kSimtThreads, smem_kv, st, (const T*)a.q, (const T*)a.k, (const T*)a.v, (const T*)a.dout, a.lse, delta, (T*)a.dk, (T*)a.dv, a.S,
             a.L, a.D, a.causal, a.scale, a.group, a.kv_lens, a.H);
     }
     return cudaGetLastError();
@@ -854,8 +857,7 @@ static cudaError_t launch_fwd_simt_tiled(const AttnArgs& a, cudaStream_t st) {
     const unsigned grid = (unsigned)(((a.S + kTiledM - 1) / kTiledM) * a.BH);
     {
         LaunchScope ls(K_FWD_SIMT, st);
-        attn_fwd_simt_tiled_kernel<T, DMAX><<<grid, kTiledThreads, smem, st>>>(
-            (const T*)a.q, (const T*)a.k, (const T*)a.v, (T*)a.out, a.lse, a.S, a.L, a.D, a.causal, a.scale, a.group,
+        launch_overlapped(attn_fwd_simt_tiled_kernel<T, DMAX>, grid, kTiledThreads, smem, st, (const T*)a.q, (const T*)a.k, (const T*)a.v, (T*)a.out, a.lse, a.S, a.L, a.D, a.causal, a.scale, a.group,
             a.kv_lens, a.H);
     }
     return cudaGetLastError();

@@ -4,6 +4,7 @@
 #include <cuda_bf16.h>
 #include <stddef.h>
 #include <stdint.h>
+#include <atomic>
 
 namespace ttk {
 
@@ -51,6 +52,47 @@ __device__ __forceinline__ int valid_keys(const int* kv_lens, long long b, int L
 }
 
 inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
+
+// What a launch asks of the runtime on every call, kept per device after the first one: the number of SMs,
+// and whether a kernel's dynamic shared-memory limit has been raised (one mask of devices per kernel).
+constexpr int kMaxDevices = 64;
+int current_device();   // 0 .. kMaxDevices - 1
+int sm_count();         // of the current device
+template <typename Kernel>
+cudaError_t allow_smem(Kernel kernel, size_t bytes, std::atomic<unsigned long long>& done) {
+    const unsigned long long bit = 1ull << current_device();
+    if (done.load(std::memory_order_acquire) & bit) return cudaSuccess;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+    return e;
+}
+// `static`: one mask per place of use, i.e. per kernel instantiation in a launcher template
+#define TT_ALLOW_SMEM(kernel, bytes)                                  \
+    ([&]() -> cudaError_t {                                           \
+        static std::atomic<unsigned long long> done__{0};             \
+        return ::ttk::allow_smem(kernel, bytes, done__);              \
+    }())
+
+// Launch with programmatic stream serialization: where the kernel before it on the stream has let its dependents go
+// (grid_let_next_start below), this kernel's CTAs take SMs as that kernel's last CTAs leave them and do their set-up
+// there.  Every kernel launched this way calls grid_wait_for_previous() in all its threads before it touches
+// global memory; that wait ends when the previous grid has completed and its writes are visible.
+template <typename... P, typename... A>
+cudaError_t launch_overlapped(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+__device__ __forceinline__ void grid_let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Error reporting of the C-ABI layer: records the message tt_last_error() returns on this thread and
 // hands back `code` (a tt_status).

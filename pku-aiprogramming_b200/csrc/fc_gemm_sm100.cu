@@ -148,6 +148,8 @@ fc_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     WaitCtx wctx{status, abort_flag, warp};
+    grid_let_next_start();
+    grid_wait_for_previous();
 
     const int total = tiles_m * tiles_n;
     const int kblocks = (K + kBK - 1) / kBK;
@@ -305,6 +307,8 @@ fc_gemm_pair_sm100_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     WaitCtx wctx{status, abort_flag, warp};
+    grid_let_next_start();
+    grid_wait_for_previous();
 
     const int total = tiles_m * tiles_n;   // 256x256 tiles
     const int kblocks = (K + kBK - 1) / kBK;
@@ -426,6 +430,8 @@ template <typename T>
 __global__ void __launch_bounds__(256) fc_gemm_simt_kernel(const T* __restrict__ A, const T* __restrict__ B,
                                                           T* __restrict__ C, const T* __restrict__ bias, int M, int N,
                                                           int K, int a_mn, int b_mn) {
+    grid_let_next_start();
+    grid_wait_for_previous();
     __shared__ float sA[16][64 + 1];
     __shared__ float sB[16][64 + 1];
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
@@ -476,6 +482,8 @@ __global__ void __launch_bounds__(256) fc_gemm_simt_kernel(const T* __restrict__
 template <typename T>
 __global__ void __launch_bounds__(256) colsum_partial_kernel(const T* __restrict__ X, float* __restrict__ partial,
                                                             long long M, int N, int rows_per_split) {
+    grid_let_next_start();
+    grid_wait_for_previous();
     const int col = blockIdx.x * 64 + (threadIdx.x & 63);
     const int sub = threadIdx.x >> 6;   // 4 row phases per CTA
     const long long r0 = (long long)blockIdx.y * rows_per_split;
@@ -492,6 +500,8 @@ __global__ void __launch_bounds__(256) colsum_partial_kernel(const T* __restrict
 template <typename T>
 __global__ void colsum_final_kernel(const float* __restrict__ partial, T* __restrict__ out, int N, int splits,
                                     int scalar_bias) {
+    grid_let_next_start();
+    grid_wait_for_previous();
     if (scalar_bias) {   // one CTA: the reference's single-value bias gets the sum over all columns too
         __shared__ float red[256];
         float s = 0.f;
@@ -513,15 +523,6 @@ __global__ void colsum_final_kernel(const float* __restrict__ partial, T* __rest
     g_st<T>(out, n, s);
 }
 
-int sm_count() {
-    static int cached[64] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64) dev = 0;
-    if (!cached[dev]) cudaDeviceGetAttribute(&cached[dev], cudaDevAttrMultiProcessorCount, dev);
-    return cached[dev] > 0 ? cached[dev] : 148;
-}
-
 template <bool kAMn, bool kBMn>
 cudaError_t launch_tc(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, cudaStream_t st) {
     TmapStorage ta, tb;
@@ -530,13 +531,12 @@ cudaError_t launch_tc(const void* A, const void* B, void* C, const void* bias, i
         return cudaErrorInvalidValue;
     if (!make_tmap_bf16(&tb, B, kBMn ? (uint64_t)N : (uint64_t)K, kBMn ? (uint64_t)K : (uint64_t)N, 1, kBMn ? 64 : kBN, &why))
         return cudaErrorInvalidValue;
-    cudaError_t e = cudaFuncSetAttribute(fc_gemm_sm100_kernel<kAMn, kBMn>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem);
+    cudaError_t e = TT_ALLOW_SMEM((fc_gemm_sm100_kernel<kAMn, kBMn>), kGemmSmem);
     if (e != cudaSuccess) return e;
     const int tiles_m = (M + kBM - 1) / kBM, tiles_n = (N + kBN - 1) / kBN;
     const int grid = std::min(tiles_m * tiles_n, sm_count());
     LaunchScope ls(K_FC_GEMM, st);
-    fc_gemm_sm100_kernel<kAMn, kBMn><<<grid, 192, kGemmSmem, st>>>(
-        *reinterpret_cast<CUtensorMap*>(ta.bytes), *reinterpret_cast<CUtensorMap*>(tb.bytes), (__nv_bfloat16*)C,
+    launch_overlapped(fc_gemm_sm100_kernel<kAMn, kBMn>, grid, 192, kGemmSmem, st, *reinterpret_cast<CUtensorMap*>(ta.bytes), *reinterpret_cast<CUtensorMap*>(tb.bytes), (__nv_bfloat16*)C,
         (const __nv_bfloat16*)bias, M, N, K, tiles_m, tiles_n,
         ((reinterpret_cast<uintptr_t>(C) & 31) == 0 && N % 16 == 0) ? 1 : 0,   // 32-byte stores possible
         device_status_word());
@@ -562,7 +562,7 @@ cudaError_t launch_tc_pair(const void* A, const void* B, void* C, const void* bi
         return cudaErrorInvalidValue;
     if (!make_tmap_bf16(&tb, B, kBMn ? (uint64_t)N : (uint64_t)K, kBMn ? (uint64_t)K : (uint64_t)N, 1, kBMn ? 64 : 128, &why))
         return cudaErrorInvalidValue;
-    cudaError_t e = cudaFuncSetAttribute(fc_gemm_pair_sm100_kernel<kAMn, kBMn>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem);
+    cudaError_t e = TT_ALLOW_SMEM((fc_gemm_pair_sm100_kernel<kAMn, kBMn>), kPairSmem);
     if (e != cudaSuccess) return e;
     const int tiles_m = (M + 255) / 256, tiles_n = (N + 255) / 256;
     // pairs that can be resident at once (a GPC with an odd number of usable SMs leaves one without a partner)
@@ -591,8 +591,7 @@ cudaError_t launch_tc_pair(const void* A, const void* B, void* C, const void* bi
     }
     const int pairs = std::min(tiles_m * tiles_n, max_pairs[dev]);
     LaunchScope ls(K_FC_GEMM, st);
-    fc_gemm_pair_sm100_kernel<kAMn, kBMn><<<2 * pairs, 192, kPairSmem, st>>>(
-        *reinterpret_cast<CUtensorMap*>(ta.bytes), *reinterpret_cast<CUtensorMap*>(tb.bytes), (__nv_bfloat16*)C,
+    launch_overlapped(fc_gemm_pair_sm100_kernel<kAMn, kBMn>, 2 * pairs, 192, kPairSmem, st, *reinterpret_cast<CUtensorMap*>(ta.bytes), *reinterpret_cast<CUtensorMap*>(tb.bytes), (__nv_bfloat16*)C,
         (const __nv_bfloat16*)bias, M, N, K, tiles_m, tiles_n,
         ((reinterpret_cast<uintptr_t>(C) & 31) == 0 && N % 16 == 0) ? 1 : 0, device_status_word());
     return cudaGetLastError();
@@ -629,10 +628,10 @@ cudaError_t fc_gemm(const void* A, const void* B, void* C, const void* bias, lon
     if (grid.y > 65535u) return cudaErrorInvalidValue;
     LaunchScope ls(K_FC_SIMT, st);
     if (bf16)
-        fc_gemm_simt_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>((const __nv_bfloat16*)A, (const __nv_bfloat16*)B,
+        launch_overlapped(fc_gemm_simt_kernel<__nv_bfloat16>, grid, 256, 0, st, (const __nv_bfloat16*)A, (const __nv_bfloat16*)B,
                                                                 (__nv_bfloat16*)C, (const __nv_bfloat16*)bias, (int)M, N, K, a_mn, b_mn);
     else
-        fc_gemm_simt_kernel<float><<<grid, 256, 0, st>>>((const float*)A, (const float*)B, (float*)C, (const float*)bias,
+        launch_overlapped(fc_gemm_simt_kernel<float>, grid, 256, 0, st, (const float*)A, (const float*)B, (float*)C, (const float*)bias,
                                                         (int)M, N, K, a_mn, b_mn);
     return cudaGetLastError();
 }
@@ -648,15 +647,15 @@ cudaError_t fc_colsum(const void* X, void* out, long long M, int N, int bf16, in
     dim3 grid((unsigned)((N + 63) / 64), (unsigned)splits);
     {
         LaunchScope ls(K_FC_COLSUM, st);
-        if (bf16) colsum_partial_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>((const __nv_bfloat16*)X, partial, M, N, rows_per_split);
-        else colsum_partial_kernel<float><<<grid, 256, 0, st>>>((const float*)X, partial, M, N, rows_per_split);
+        if (bf16) launch_overlapped(colsum_partial_kernel<__nv_bfloat16>, grid, 256, 0, st, (const __nv_bfloat16*)X, partial, M, N, rows_per_split);
+        else launch_overlapped(colsum_partial_kernel<float>, grid, 256, 0, st, (const float*)X, partial, M, N, rows_per_split);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
     LaunchScope ls(K_FC_COLSUM, st, false);
     const unsigned fgrid = scalar_bias ? 1u : (unsigned)((N + 255) / 256);
-    if (bf16) colsum_final_kernel<__nv_bfloat16><<<fgrid, 256, 0, st>>>(partial, (__nv_bfloat16*)out, N, splits, scalar_bias);
-    else colsum_final_kernel<float><<<fgrid, 256, 0, st>>>(partial, (float*)out, N, splits, scalar_bias);
+    if (bf16) launch_overlapped(colsum_final_kernel<__nv_bfloat16>, fgrid, 256, 0, st, partial, (__nv_bfloat16*)out, N, splits, scalar_bias);
+    else launch_overlapped(colsum_final_kernel<float>, fgrid, 256, 0, st, partial, (float*)out, N, splits, scalar_bias);
     return cudaGetLastError();
 }
 

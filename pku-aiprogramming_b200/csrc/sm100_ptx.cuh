@@ -93,6 +93,58 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const 
     return false;
 }
 
+// ------------------------------------------------------------------ work items of a persistent kernel
+// A launch has one CTA per work item (item = blockIdx.x), but a CTA that is running asks the hardware for the
+// items whose CTAs have not started yet (cluster launch control) and works on those too, so that its
+// prologue is paid once and the next item's loads run under this one's epilogue.  There is no counter in global
+// memory to clear before the launch (a memset and an event per launch: about 4 us of host time and 2 us on the stream)
+// or to keep apart between launches.  The loader warp owns this object: all 32 lanes call its members together,
+// `request` behind an item's last load and `next` right after it (the answer takes about 530 cycles, measured, and runs
+// under the tiles in flight).  Asked for at the START of an item, the next one waits while other CTAs run dry: three
+// slices of 21120 keys, backward, 0.88 ms instead of 0.61.
+struct ItemStream {
+    uint64_t* bar;     // mbarrier, one arrival
+    uint4* response;   // 16 bytes of shared memory, 16-byte aligned
+    bool dynamic;      // false: every item has an SM of its own, there is nothing to ask for
+    uint32_t phase = 0;
+    bool pending = false;
+
+    __device__ __forceinline__ void request(bool aborted) {
+        pending = dynamic && !aborted;
+        if (!pending) return;
+        if (elect_one()) {
+            fence_proxy_async_smem();   // the previous response has been read
+            mbar_arrive_expect_tx(bar, 16);
+            asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];"
+                         ::"r"(smem_u32(response)), "r"(smem_u32(bar)) : "memory");
+        }
+        __syncwarp();
+    }
+    // the next item, or -1 when none is left
+    __device__ __forceinline__ int next(const WaitCtx& ctx, int bar_id, int iter) {
+        if (!pending) return -1;
+        const bool ok = mbar_wait(bar, phase & 1, ctx, bar_id, iter);
+        ++phase;
+        uint32_t got = 0, id = 0;
+        asm volatile(
+            "{\n\t.reg .b128 h;\n\t.reg .pred p;\n\t"
+            "ld.shared.b128 h, [%2];\n\t"
+            "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t"
+            "mov.u32 %1, 0;\n\t"
+            "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, h;\n\t}"
+            : "=r"(got), "=r"(id)
+            : "r"(smem_u32(response))
+            : "memory");
+        __syncwarp();
+        if (!ok || !got) {   // after a request that found nothing there must be no further one
+            dynamic = false;
+            return -1;
+        }
+        return (int)id;
+    }
+};
+
 // ------------------------------------------------------------------ TMA (tiled, no multicast)
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* m) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(m)) : "memory");

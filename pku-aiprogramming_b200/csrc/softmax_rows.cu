@@ -49,6 +49,8 @@ __device__ __forceinline__ float block_reduce(float x, float* red) {   // 256 th
 template <typename T, int kPer, bool kBlock, bool kBwd>
 __global__ void __launch_bounds__(256) softmax_rows_kernel(const T* __restrict__ a, const T* __restrict__ b,
                                                           T* __restrict__ out, long long rows, int cols) {
+    grid_let_next_start();
+    grid_wait_for_previous();
     __shared__ float red[8];
     const int nthr = kBlock ? 256 : 32;
     const int tid = kBlock ? threadIdx.x : (threadIdx.x & 31);
@@ -97,6 +99,8 @@ __global__ void __launch_bounds__(256) softmax_rows_kernel(const T* __restrict__
 template <typename T, bool kBwd>
 __global__ void __launch_bounds__(256) softmax_rows_long_kernel(const T* __restrict__ a, const T* __restrict__ b,
                                                                T* __restrict__ out, long long rows, int cols) {
+    grid_let_next_start();
+    grid_wait_for_previous();
     __shared__ float red[8];
     const long long base = (long long)blockIdx.x * cols;
     if (!kBwd) {
@@ -123,8 +127,8 @@ static cudaError_t launch_softmax(const void* a, const void* b, void* out, long 
     const T* pb = (const T*)b;
     T* po = (T*)out;
     LaunchScope ls(kBwd ? K_SOFTMAX_BWD : K_SOFTMAX_FWD, st);
-#define TT_SM_WARP(P) softmax_rows_kernel<T, P, false, kBwd><<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(pa, pb, po, rows, cols)
-#define TT_SM_BLOCK(P) softmax_rows_kernel<T, P, true, kBwd><<<(unsigned)rows, 256, 0, st>>>(pa, pb, po, rows, cols)
+#define TT_SM_WARP(P) launch_overlapped(softmax_rows_kernel<T, P, false, kBwd>, (unsigned)((rows + 7) / 8), 256, 0, st, pa, pb, po, rows, cols)
+#define TT_SM_BLOCK(P) launch_overlapped(softmax_rows_kernel<T, P, true, kBwd>, (unsigned)rows, 256, 0, st, pa, pb, po, rows, cols)
     if (cols <= 32) TT_SM_WARP(1);
     else if (cols <= 64) TT_SM_WARP(2);
     else if (cols <= 128) TT_SM_WARP(4);
@@ -135,7 +139,7 @@ static cudaError_t launch_softmax(const void* a, const void* b, void* out, long 
     else if (cols <= 4096) TT_SM_BLOCK(16);
     else if (cols <= 8192) TT_SM_BLOCK(32);
     else if (cols <= 16384) TT_SM_BLOCK(64);
-    else softmax_rows_long_kernel<T, kBwd><<<(unsigned)rows, 256, 0, st>>>(pa, pb, po, rows, cols);
+    else launch_overlapped(softmax_rows_long_kernel<T, kBwd>, (unsigned)rows, 256, 0, st, pa, pb, po, rows, cols);
 #undef TT_SM_WARP
 #undef TT_SM_BLOCK
     return cudaGetLastError();

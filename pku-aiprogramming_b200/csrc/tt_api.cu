@@ -85,19 +85,30 @@ LaunchScope::~LaunchScope() {
 
 // ------------------------------------------------------------------------------ device status word
 __device__ unsigned int g_device_status[4];
-static std::mutex g_status_mu;
-static std::unordered_map<int, unsigned int*> g_status_ptr;
+static std::atomic<unsigned int*> g_status_ptr[kMaxDevices];
 unsigned int* device_status_word() {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    std::lock_guard<std::mutex> lk(g_status_mu);
-    auto it = g_status_ptr.find(dev);
-    if (it != g_status_ptr.end()) return it->second;
-    unsigned int* p = nullptr;
-    if (cudaGetSymbolAddress((void**)&p, g_device_status) != cudaSuccess) p = nullptr;
-    if (p) cudaMemset(p, 0, 4 * sizeof(unsigned int));
-    g_status_ptr[dev] = p;
+    std::atomic<unsigned int*>& slot = g_status_ptr[current_device()];
+    unsigned int* p = slot.load(std::memory_order_acquire);
+    if (p) return p;
+    if (cudaGetSymbolAddress((void**)&p, g_device_status) != cudaSuccess) return nullptr;
+    slot.store(p, std::memory_order_release);   // (the array is zero when the module is loaded)
     return p;
+}
+
+// ------------------------------------------------------------------------------ device facts
+int current_device() {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
+    return dev;
+}
+int sm_count() {
+    static std::atomic<int> cached[kMaxDevices];
+    const int dev = current_device();
+    int n = cached[dev].load(std::memory_order_relaxed);
+    if (n > 0) return n;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) return 148;
+    cached[dev].store(n, std::memory_order_relaxed);
+    return n;
 }
 
 // ------------------------------------------------------------------------------ work-item counters
