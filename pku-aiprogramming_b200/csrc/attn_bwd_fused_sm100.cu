@@ -511,26 +511,30 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
             // (K-major and MN-major view of the base) plus compile-time offsets describe them all.
             const uint32_t smem_addr = __shfl_sync(0xffffffffu, smem_u32(smem), 0);
             const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
-            const uint64_t desc_k = umma_smem_desc(smem_addr, 16, 1024);                  // K-major: rows = M or N, 128 B of K per row
-            const uint64_t desc_mn = umma_smem_desc(smem_addr, Cfg::kSubBytes, 1024);     // MN-major: rows = K, 64 elements of M/N per row
+            constexpr uint32_t hi = umma_desc_hi(1024);
+            const uint32_t desc_k = umma_desc_lo(smem_addr, 16);                  // K-major: rows = M or N, 128 B of K per row
+            const uint32_t desc_mn = umma_desc_lo(smem_addr, Cfg::kSubBytes);     // MN-major: rows = K, 64 elements of M/N per row
             constexpr uint32_t kOffK = 0, kOffV = Cfg::kTileBytes, kOffQ = 2 * Cfg::kTileBytes,
                                kOffdO = (2 + kNQ) * Cfg::kTileBytes, kOffDS = (2 + kNQ + kNdO) * Cfg::kTileBytes;
-            const uint64_t dK_k = umma_desc_advance(desc_k, kOffK);        // K as A of G1
-            const uint64_t dK_mn = umma_desc_advance(desc_mn, kOffK);      // K as B of G5
-            const uint64_t dV_k = umma_desc_advance(desc_k, kOffV);        // V as A of G2
-            const uint64_t dQ_k = umma_desc_advance(desc_k, kOffQ);        // Q as B of G1
-            const uint64_t dQ_mn = umma_desc_advance(desc_mn, kOffQ);      // Q as B of G4
-            const uint64_t ddO_k = umma_desc_advance(desc_k, kOffdO);      // dO as B of G2
-            const uint64_t ddO_mn = umma_desc_advance(desc_mn, kOffdO);    // dO as B of G3
-            const uint64_t dDS_k = umma_desc_advance(desc_k, kOffDS);      // dS^T as A of G4 (K-major: K = queries)
-            const uint64_t dDS_mn = umma_desc_advance(desc_mn, kOffDS);    // dS^T as A of G5 (MN-major: M = queries)
+            const uint32_t dK_k = desc_k + (kOffK >> 4);        // K as A of G1
+            const uint32_t dK_mn = desc_mn + (kOffK >> 4);      // K as B of G5
+            const uint32_t dV_k = desc_k + (kOffV >> 4);        // V as A of G2
+            const uint32_t dQ_k = desc_k + (kOffQ >> 4);        // Q as B of G1
+            const uint32_t dQ_mn = desc_mn + (kOffQ >> 4);      // Q as B of G4
+            const uint32_t ddO_k = desc_k + (kOffdO >> 4);      // dO as B of G2
+            const uint32_t ddO_mn = desc_mn + (kOffdO >> 4);    // dO as B of G3
+            const uint32_t dDS_k = desc_k + (kOffDS >> 4);      // dS^T as A of G4 (K-major: K = queries)
+            const uint32_t dDS_mn = desc_mn + (kOffDS >> 4);    // dS^T as A of G5 (MN-major: M = queries)
             // G1 / G2: tmem[col] = A B^T over K = D, both operands K-major tiles of D/64 sub-blocks
-            auto issue_score = [&](uint64_t a0, uint64_t b0, uint32_t col) {
+            auto issue_score = [&](uint32_t a0, uint32_t b0, uint32_t col) {
+                if (elect_one()) {
 #pragma unroll
-                for (int kk = 0; kk < D / 16; ++kk) {
-                    const uint32_t o = (kk >> 2) * Cfg::kSubBytes + (kk & 3) * 32;
-                    umma_ss(tmem_u + col, umma_desc_advance(a0, o), umma_desc_advance(b0, o), idesc_s, kk > 0);
+                    for (int kk = 0; kk < D / 16; ++kk) {
+                        const uint32_t o = ((kk >> 2) * Cfg::kSubBytes + (kk & 3) * 32) >> 4;
+                        umma_ss_one(tmem_u + col, a0 + o, b0 + o, hi, idesc_s, kk > 0);
+                    }
                 }
+                __syncwarp();
             };
             uint32_t git = 0;      // streamed tiles issued before the current item
             for (int k = 0;; ++k) {
@@ -551,7 +555,7 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
                     mbar_wait(&bar_q_full[f0], (git / kNQ) & 1, wctx, B1_QFULL + f0, (int)git);
                     __syncwarp();
                     tc_fence_after();
-                    issue_score(dK_k, umma_desc_advance(dQ_k, f0 * Cfg::kTileBytes), kColX);
+                    issue_score(dK_k, dQ_k + f0 * (Cfg::kTileBytes >> 4), kColX);
                     tc_commit(bar_s_full);
                     mbar_wait(&bar_do_full[f1], (git / kNdO) & 1, wctx, B1_DOFULL + f1, (int)git);
                     __syncwarp();
@@ -560,7 +564,7 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
                         __syncwarp();
                     }
                     tc_fence_after();
-                    issue_score(dV_k, umma_desc_advance(ddO_k, f1 * Cfg::kTileBytes), kColY);
+                    issue_score(dV_k, ddO_k + f1 * (Cfg::kTileBytes >> 4), kColY);
                     tc_commit(bar_dp_full);
                 }
                 for (int it = 0; it < n_it; ++it) {
@@ -582,11 +586,14 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
                         tc_fence_after();
                     }
                     {
-                        const uint64_t b0 = umma_desc_advance(ddO_mn, os * Cfg::kTileBytes);
+                        const uint32_t b0 = ddO_mn + os * (Cfg::kTileBytes >> 4);
+                        if (elect_one()) {
 #pragma unroll
-                        for (int kk = 0; kk < 8; ++kk)   // K step = 16 queries = 8 columns of bf16 P^T
-                            umma_ts(tmem_u + kColDV, tmem_u + kColX + (kk >> 2) * 64 + (kk & 3) * 8, umma_desc_advance(b0, kk * 2048),
-                                    idesc_kn, (it > 0 || kk > 0) ? 1u : 0u);
+                            for (int kk = 0; kk < 8; ++kk)   // K step = 16 queries = 8 columns of bf16 P^T
+                                umma_ts_one(tmem_u + kColDV, tmem_u + kColX + (kk >> 2) * 64 + (kk & 3) * 8, b0 + kk * 128, hi, idesc_kn,
+                                            (it > 0 || kk > 0) ? 1u : 0u);
+                        }
+                        __syncwarp();
                     }
                     tc_commit(&bar_do_empty[os]);                            // last read of dO(t)
                     // ---- G1(t+1): the next scores, as soon as P^T(t) has been consumed (in order)
@@ -594,7 +601,7 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
                         mbar_wait(&bar_q_full[nqs], ((g + 1) / kNQ) & 1, wctx, B1_QFULL + nqs, it + 1);
                         __syncwarp();
                         tc_fence_after();
-                        issue_score(dK_k, umma_desc_advance(dQ_k, nqs * Cfg::kTileBytes), kColX);
+                        issue_score(dK_k, dQ_k + nqs * (Cfg::kTileBytes >> 4), kColX);
                         tc_commit(bar_s_full);
                     }
                     // ---- G5: dQ_t = dS K  and  G4: dK += dS^T Q
@@ -603,19 +610,22 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
                     __syncwarp();
                     tc_fence_after();
                     if (tr) TT_B1TRACE(2, it, 3);
+                    if (elect_one()) {
 #pragma unroll
-                    for (int kk = 0; kk < 8; ++kk)       // K step = 16 keys = 16 rows of both tiles
-                        umma_ss(tmem_u + kColY, umma_desc_advance(dDS_mn, kk * 2048), umma_desc_advance(dK_mn, kk * 2048), idesc_nn,
-                                kk > 0 ? 1u : 0u);
+                        for (int kk = 0; kk < 8; ++kk)       // K step = 16 keys = 16 rows of both tiles
+                            umma_ss_one(tmem_u + kColY, dDS_mn + kk * 128, dK_mn + kk * 128, hi, idesc_nn, kk > 0 ? 1u : 0u);
+                    }
+                    __syncwarp();
                     tc_commit(bar_dq_full);
                     {
-                        const uint64_t b0 = umma_desc_advance(dQ_mn, qs * Cfg::kTileBytes);
+                        const uint32_t b0 = dQ_mn + qs * (Cfg::kTileBytes >> 4);
+                        if (elect_one()) {
 #pragma unroll
-                        for (int kk = 0; kk < 8; ++kk) { // K step = 16 queries: 32 bytes along a dS^T row, 16 rows of Q
-                            const uint32_t ao = (kk >> 2) * Cfg::kSubBytes + (kk & 3) * 32;
-                            umma_ss(tmem_u + kColDK, umma_desc_advance(dDS_k, ao), umma_desc_advance(b0, kk * 2048), idesc_kn,
-                                    (it > 0 || kk > 0) ? 1u : 0u);
+                            for (int kk = 0; kk < 8; ++kk)   // K step = 16 queries: 32 bytes along a dS^T row, 16 rows of Q
+                                umma_ss_one(tmem_u + kColDK, dDS_k + (((kk >> 2) * Cfg::kSubBytes + (kk & 3) * 32) >> 4), b0 + kk * 128, hi,
+                                            idesc_kn, (it > 0 || kk > 0) ? 1u : 0u);
                         }
+                        __syncwarp();
                     }
                     tc_commit(&bar_q_empty[qs]);                             // last read of Q(t)
                     tc_commit(bar_ds_free);                                  // G4, G5 are done with the dS^T tile
@@ -629,7 +639,7 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
                         __syncwarp();
                         tc_fence_after();
                         if (tr) TT_B1TRACE(2, it, 5);
-                        issue_score(dV_k, umma_desc_advance(ddO_k, nos * Cfg::kTileBytes), kColY);
+                        issue_score(dV_k, ddO_k + nos * (Cfg::kTileBytes >> 4), kColY);
                         tc_commit(bar_dp_full);
                     }
                     if (tr) TT_B1TRACE(2, it, 6);

@@ -552,37 +552,42 @@ attn_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmR0, const __grid_con
             const uint32_t sR_addr = __shfl_sync(0xffffffffu, smem_u32(sR), 0);
             const uint32_t sT_addr = __shfl_sync(0xffffffffu, smem_u32(sT), 0);
             const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
-            const uint64_t dR_base = umma_smem_desc(sR_addr, 16, 1024);                   // K-major
-            const uint64_t dT_base = umma_smem_desc(sT_addr, 16, 1024);                   // K-major
-            const uint64_t dT_mn_base = umma_smem_desc(sT_addr, Cfg::kSubBytes, 1024);    // MN-major
+            constexpr uint32_t hi = umma_desc_hi(1024);
+            const uint32_t dR_base = umma_desc_lo(sR_addr, 16);                   // K-major
+            const uint32_t dT_base = umma_desc_lo(sT_addr, 16);                   // K-major
+            const uint32_t dT_mn_base = umma_desc_lo(sT_addr, Cfg::kSubBytes);    // MN-major
             // G1 / G2: tmem[col] = R_which T^T for the streamed tile at index `tile` of the stream buffers
             auto issue_score = [&](int which, int tile, uint32_t col, bool a_in_tmem = false) {
-                const uint64_t a0 = umma_desc_advance(dR_base, which * Cfg::kTileBytes);
-                const uint64_t b0 = umma_desc_advance(dT_base, tile * Cfg::kTileBytes);
+                const uint32_t a0 = dR_base + ((which * Cfg::kTileBytes) >> 4);
+                const uint32_t b0 = dT_base + ((tile * Cfg::kTileBytes) >> 4);
+                if (elect_one()) {
 #pragma unroll
-                for (int kk = 0; kk < D / 16; ++kk) {
-                    const uint32_t o = (kk >> 2) * Cfg::kSubBytes + (kk & 3) * 32;
-                    if (kResidentInTmem && a_in_tmem)   // A = resident tile in tensor memory: 8 columns per K step of 16
-                        umma_ts(tmem_u + col, tmem_u + kColRes + which * (D / 2) + kk * 8, umma_desc_advance(b0, o), idesc_s,
-                                kk > 0);
-                    else
-                        umma_ss(tmem_u + col, umma_desc_advance(a0, o), umma_desc_advance(b0, o), idesc_s, kk > 0);
+                    for (int kk = 0; kk < D / 16; ++kk) {
+                        const uint32_t o = ((kk >> 2) * Cfg::kSubBytes + (kk & 3) * 32) >> 4;
+                        if (kResidentInTmem && a_in_tmem)   // A = resident tile in tensor memory: 8 columns per K step of 16
+                            umma_ts_one(tmem_u + col, tmem_u + kColRes + which * (D / 2) + kk * 8, b0 + o, hi, idesc_s, kk > 0);
+                        else
+                            umma_ss_one(tmem_u + col, a0 + o, b0 + o, hi, idesc_s, kk > 0);
+                    }
                 }
+                __syncwarp();
             };
             // G3 / G4: tmem[acc] (+)= bf16 A in tensor memory times the streamed tile (MN-major).  A is what
             // phase B left in the dP columns: with queries resident, each warpgroup's 64 dS values in the
             // first 32 of its 64 columns; with keys resident, per 32-column chunk 16 columns of P^T
             // (part = 0) then 16 of dS^T (part = 1).  K step kk covers 16 streamed rows = 8 columns.
             auto issue_acc = [&](int tile, int part, uint32_t acc_col, bool accumulate) {
-                const uint64_t b0 = umma_desc_advance(dT_mn_base, tile * Cfg::kTileBytes);
+                const uint32_t b0 = dT_mn_base + ((tile * Cfg::kTileBytes) >> 4);
+                if (elect_one()) {
 #pragma unroll
-                for (int kk = 0; kk < 8; ++kk) {
-                    const uint32_t in_wg = kKeysResident ? (uint32_t)(((kk & 3) >> 1) * 32 + part * 16 + (kk & 1) * 8)
-                                                         : (uint32_t)((kk & 3) * 8);
-                    const uint32_t a = tmem_u + kColDP + (kk >> 2) * 64 + in_wg;
-                    umma_ts(tmem_u + acc_col, a, umma_desc_advance(b0, kk * 2048), idesc_acc,
-                            (accumulate || kk > 0) ? 1u : 0u);
+                    for (int kk = 0; kk < 8; ++kk) {
+                        const uint32_t in_wg = kKeysResident ? (uint32_t)(((kk & 3) >> 1) * 32 + part * 16 + (kk & 1) * 8)
+                                                             : (uint32_t)((kk & 3) * 8);
+                        const uint32_t a = tmem_u + kColDP + (kk >> 2) * 64 + in_wg;
+                        umma_ts_one(tmem_u + acc_col, a, b0 + ((kk * 2048) >> 4), hi, idesc_acc, (accumulate || kk > 0) ? 1u : 0u);
+                    }
                 }
+                __syncwarp();
             };
             uint32_t git = 0;      // streamed tiles issued before the current item
             for (int k = 0;; ++k) {

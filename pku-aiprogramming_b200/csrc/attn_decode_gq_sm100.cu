@@ -329,24 +329,31 @@ attn_decode_gq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
         constexpr uint32_t idesc_o = umma_idesc_bf16(128, 16, true, false);    // O^T += V^T P: A = V read MN-major
         const uint32_t sKV_addr = __shfl_sync(0xffffffffu, smem_u32(sKV), 0);
         const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
-        const uint64_t dK_base = umma_smem_desc(sKV_addr, 16, 1024);             // K-major A, 128 key rows
-        const uint64_t dV_base = umma_smem_desc(sKV_addr, kSub == 2 ? kSubBytes : 0, 1024);   // MN-major A: M = d over two 64-wide blocks (D = 64: the same block twice)
-        const uint64_t dQ = umma_smem_desc(__shfl_sync(0xffffffffu, smem_u32(sQ), 0), 16, 1024);   // K-major B, 16 rows
-        const uint64_t dP_base = umma_smem_desc(__shfl_sync(0xffffffffu, smem_u32(sP), 0), 16, 1024);
+        constexpr uint32_t hi = umma_desc_hi(1024);
+        const uint32_t dK_base = umma_desc_lo(sKV_addr, 16);             // K-major A, 128 key rows
+        const uint32_t dV_base = umma_desc_lo(sKV_addr, kSub == 2 ? kSubBytes : 0);   // MN-major A: M = d over two 64-wide blocks (D = 64: the same block twice)
+        const uint32_t dQ = umma_desc_lo(__shfl_sync(0xffffffffu, smem_u32(sQ), 0), 16);   // K-major B, 16 rows
+        const uint32_t dP_base = umma_desc_lo(__shfl_sync(0xffffffffu, smem_u32(sP), 0), 16);
         auto issue_s = [&](int j) {
-            const uint64_t a0 = umma_desc_advance(dK_base, ((2 * j) % kStages) * kTileBytes);
+            const uint32_t a0 = dK_base + (((2 * j) % kStages) * kTileBytes >> 4);
+            if (elect_one()) {
 #pragma unroll
-            for (int kk = 0; kk < kD / 16; ++kk)
-                umma_ss(tmem_u + (uint32_t)((j & 1) * 16), umma_desc_advance(a0, (kk >> 2) * kSubBytes + (kk & 3) * 32),
-                        umma_desc_advance(dQ, (kk >> 2) * 2048 + (kk & 3) * 32), idesc_s, kk > 0);
+                for (int kk = 0; kk < kD / 16; ++kk)
+                    umma_ss_one(tmem_u + (uint32_t)((j & 1) * 16), a0 + (((kk >> 2) * kSubBytes + (kk & 3) * 32) >> 4),
+                                dQ + (((kk >> 2) * 2048 + (kk & 3) * 32) >> 4), hi, idesc_s, kk > 0);
+            }
+            __syncwarp();
         };
         auto issue_o = [&](int j) {
-            const uint64_t a0 = umma_desc_advance(dV_base, ((2 * j + 1) % kStages) * kTileBytes);
-            const uint64_t b0 = umma_desc_advance(dP_base, (j & 1) * kPBytes);
+            const uint32_t a0 = dV_base + (((2 * j + 1) % kStages) * kTileBytes >> 4);
+            const uint32_t b0 = dP_base + ((j & 1) * kPBytes >> 4);
+            if (elect_one()) {
 #pragma unroll
-            for (int kk = 0; kk < 8; ++kk)   // 16 keys per step
-                umma_ss(tmem_u + kColO, umma_desc_advance(a0, kk * 2048), umma_desc_advance(b0, (kk >> 2) * 2048 + (kk & 3) * 32),
-                        idesc_o, (j > 0 || kk > 0) ? 1u : 0u);
+                for (int kk = 0; kk < 8; ++kk)   // 16 keys per step
+                    umma_ss_one(tmem_u + kColO, a0 + kk * 128, b0 + (((kk >> 2) * 2048 + (kk & 3) * 32) >> 4), hi, idesc_o,
+                                (j > 0 || kk > 0) ? 1u : 0u);
+            }
+            __syncwarp();
         };
         auto wait_entry = [&](int e) -> bool {
             const bool ok = mbar_wait(&bar_kv_full[e % kStages], (e / kStages) & 1, wctx, 50 + e % kStages, e);

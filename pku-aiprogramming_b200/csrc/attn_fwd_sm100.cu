@@ -454,10 +454,10 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             const uint32_t sQ_addr = __shfl_sync(0xffffffffu, smem_u32(sQ), 0);
             const uint32_t sKV_addr = __shfl_sync(0xffffffffu, smem_u32(sKV), 0);
             const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);   // warp-uniform copy
-            // descriptor templates; per MMA only the 14-bit start-address field moves
-            const uint64_t dq_base = umma_smem_desc(sQ_addr, 16, 1024);
-            const uint64_t dk_base = umma_smem_desc(sKV_addr, 16, 1024);                 // K-major (S = Q K^T)
-            const uint64_t dv_base = umma_smem_desc(sKV_addr, Cfg::kSubBytes, 1024);     // MN-major (O += P V)
+            constexpr uint32_t hi = umma_desc_hi(1024);
+            const uint32_t dq_base = umma_desc_lo(sQ_addr, 16);
+            const uint32_t dk_base = umma_desc_lo(sKV_addr, 16);                 // K-major (S = Q K^T)
+            const uint32_t dv_base = umma_desc_lo(sKV_addr, Cfg::kSubBytes);     // MN-major (O += P V)
             uint32_t t = 0;                  // K/V ring items consumed before the current work item
             uint32_t q_uses[2] = {0, 0}, p_cnt[2] = {0, 0}, o_uses[2] = {0, 0};
             auto wait_item = [&](uint32_t ri) {
@@ -467,24 +467,30 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             };
             auto release_item = [&](uint32_t ri) { tc_commit(&bar_kv_empty[ri % kStages]); };
             auto issue_s = [&](int i, uint32_t ri) {   // S_i = Q_i K^T with K in ring item ri
-                const uint64_t a0 = umma_desc_advance(dq_base, i * Cfg::kTileBytes);
-                const uint64_t b0 = umma_desc_advance(dk_base, (ri % kStages) * Cfg::kTileBytes);
+                const uint32_t a0 = dq_base + ((i * Cfg::kTileBytes) >> 4);
+                const uint32_t b0 = dk_base + (((ri % kStages) * Cfg::kTileBytes) >> 4);
                 const uint32_t d = tmem_u + (uint32_t)(i * 128);
+                if (elect_one()) {
 #pragma unroll
-                for (int kk = 0; kk < D / 16; ++kk) {
-                    const uint32_t o = (kk >> 2) * Cfg::kSubBytes + (kk & 3) * 32;
-                    umma_ss(d, umma_desc_advance(a0, o), umma_desc_advance(b0, o), idesc_s, kk > 0);
+                    for (int kk = 0; kk < D / 16; ++kk) {
+                        const uint32_t o = ((kk >> 2) * Cfg::kSubBytes + (kk & 3) * 32) >> 4;
+                        umma_ss_one(d, a0 + o, b0 + o, hi, idesc_s, kk > 0);
+                    }
                 }
+                __syncwarp();
             };
             auto issue_pv = [&](int i, uint32_t ri, bool accumulate, int half) {   // O_i (+)= P_i V
-                const uint64_t b0 = umma_desc_advance(dv_base, (ri % kStages) * Cfg::kTileBytes);
+                const uint32_t b0 = dv_base + (((ri % kStages) * Cfg::kTileBytes) >> 4);
                 const uint32_t d = tmem_u + (uint32_t)(256 + i * D);
                 const uint32_t a = tmem_u + (uint32_t)(i * 128);
+                if (elect_one()) {
 #pragma unroll
-                for (int k4 = 0; k4 < 4; ++k4) {
-                    const int kk = half * 4 + k4;
-                    umma_ts(d, a + kk * 8, umma_desc_advance(b0, kk * 2048), idesc_pv, (accumulate || kk > 0) ? 1u : 0u);
+                    for (int k4 = 0; k4 < 4; ++k4) {
+                        const int kk = half * 4 + k4;
+                        umma_ts_one(d, a + kk * 8, b0 + ((kk * 2048) >> 4), hi, idesc_pv, (accumulate || kk > 0) ? 1u : 0u);
+                    }
                 }
+                __syncwarp();
             };
             // Causal items give query tile 1 one key/value tile more than tile 0, so in an item's last
             // iteration slot 0 has nothing to do.  That gap is used: the item that follows is fetched

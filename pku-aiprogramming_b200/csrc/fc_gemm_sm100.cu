@@ -213,12 +213,14 @@ fc_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                 tc_fence_after();
                 const uint32_t sA = smem_u32(smem + s * kStageBytes);
                 const uint32_t sB = sA + kABytes;
-                const uint64_t a0 = umma_smem_desc(sA, kAMn ? kSubBytes : 16, 1024);
-                const uint64_t b0 = umma_smem_desc(sB, kBMn ? kSubBytes : 16, 1024);
+                const uint32_t a0 = umma_desc_lo(sA, kAMn ? kSubBytes : 16), b0 = umma_desc_lo(sB, kBMn ? kSubBytes : 16);
+                if (elect_one()) {
 #pragma unroll
-                for (int kk = 0; kk < kBK / 16; ++kk)
-                    umma_ss(d_tmem, umma_desc_advance(a0, kk * a_step), umma_desc_advance(b0, kk * b_step), idesc,
-                            (uint32_t)((kb | kk) != 0));
+                    for (int kk = 0; kk < kBK / 16; ++kk)
+                        umma_ss_one(d_tmem, a0 + (kk * a_step >> 4), b0 + (kk * b_step >> 4), umma_desc_hi(1024), idesc,
+                                    (uint32_t)((kb | kk) != 0));
+                }
+                __syncwarp();
                 tc_commit(&empty[s]);
             }
             if (live) tc_commit(&acc_full[buf]);
