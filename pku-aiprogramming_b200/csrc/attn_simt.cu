@@ -1,12 +1,12 @@
 // SIMT attention kernels with true fp32 FMA arithmetic (no TF32, no tensor cores).
 //
-// They serve the fp32 dtype, whose tolerance (1e-5 relative) rules out tensor-core
-// formats, and every bf16 shape the tcgen05 kernels do not cover (head dims other than
-// 64/128).  Inputs of either dtype are widened to fp32 in shared memory; all dot
+// They serve what the tensor-core kernels do not take: bf16 with head dims other than 64 / 128, and float
+// tensors whose head dim is above 128 or whose rows are not 16-byte vectors (the rest of the float problems run
+// as three bf16 parts on the tensor cores, attn_f32_sm100.cu).  Inputs of either dtype are widened to fp32 in shared memory; all dot
 // products, the softmax and the accumulators are fp32.
 //
 // Two forms of each kernel (forward, dQ pass, dK/dV pass):
-//   register-tiled (head dims that are multiples of 4 up to 128, vector-aligned tensors): a block owns
+//   register-tiled (bf16, head dims that are multiples of 4 up to 128, vector-aligned tensors): a block owns
 //     64 "rows" and walks the "columns" in tiles of 64; each of its 16 x 16 threads holds a 4 x 4 patch
 //     of scores, so a 128-bit shared-memory load feeds 16 FMAs; see the sections further down;
 //   row-per-lane (any D <= 256): a block owns 32 rows, a warp 4 of them, columns in tiles of 32; lane j
@@ -785,16 +785,18 @@ static cudaError_t launch_fwd_simt(const AttnArgs& a, cudaStream_t st) {
     return cudaGetLastError();
 }
 
+static bool forced_rows(const char* name) {   // TT_SIMT_FWD / TT_SIMT_BWD=rows: the row-per-lane kernels (tests)
+    const char* e = getenv(name);
+    return e && e[0] == 'r';
+}
 // the tiled backward kernels: same vector requirements as the tiled forward, for every tensor they touch
 static bool simt_tiled_bwd_ok(const AttnArgs& a) {
-    const char* e = getenv("TT_SIMT_BWD");
-    if (e && e[0] == 'r') return false;
-    const uintptr_t mask = a.bf16 ? 7 : 15;
+    if (!a.bf16 || forced_rows("TT_SIMT_BWD")) return false;
     const uintptr_t ptrs = reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.k) |
                            reinterpret_cast<uintptr_t>(a.v) | reinterpret_cast<uintptr_t>(a.dout) |
                            reinterpret_cast<uintptr_t>(a.dq) | reinterpret_cast<uintptr_t>(a.dk) |
                            reinterpret_cast<uintptr_t>(a.dv);
-    return a.D % 4 == 0 && a.D <= 128 && (ptrs & mask) == 0;
+    return a.D % 4 == 0 && a.D <= 128 && (ptrs & 7) == 0;
 }
 template <typename T, int DMAX>
 static cudaError_t launch_bwd_simt_tiled(const AttnArgs& a, float* delta, cudaStream_t st) {
@@ -827,7 +829,9 @@ static cudaError_t launch_bwd_simt(const AttnArgs& a, float* delta, cudaStream_t
         launch_overlapped(attn_bwd_delta_kernel<T>, (unsigned)((n_rows + 7) / 8), 256, 0, st, (const T*)a.out, (const T*)a.dout,
                                                                               delta, n_rows, a.D);
     }
-    if (simt_tiled_bwd_ok(a)) return a.D <= 64 ? launch_bwd_simt_tiled<T, 64>(a, delta, st) : launch_bwd_simt_tiled<T, 128>(a, delta, st);
+    if constexpr (sizeof(T) == 2) {
+        if (simt_tiled_bwd_ok(a)) return a.D <= 64 ? launch_bwd_simt_tiled<T, 64>(a, delta, st) : launch_bwd_simt_tiled<T, 128>(a, delta, st);
+    }
     size_t smem_q = (size_t)4 * 32 * (a.D + 1) * sizeof(float);
     size_t smem_kv = smem_q + 64 * sizeof(float);
     cudaError_t e = set_smem(attn_bwd_dq_simt_kernel<T, NV>, smem_q);
@@ -862,20 +866,19 @@ static cudaError_t launch_fwd_simt_tiled(const AttnArgs& a, cudaStream_t st) {
     }
     return cudaGetLastError();
 }
-// the register-tiled forward needs 4-element vectors: D a multiple of 4 and 16-byte (fp32) or 8-byte
-// (bf16) aligned tensors; TT_SIMT_FWD=rows keeps the row-per-lane kernel
+// the register-tiled forward needs 4-element vectors: D a multiple of 4 and 8-byte aligned tensors; TT_SIMT_FWD=rows keeps the row-per-lane kernel
 static bool simt_tiled_ok(const AttnArgs& a) {
-    const char* e = getenv("TT_SIMT_FWD");
-    if (e && e[0] == 'r') return false;
-    const uintptr_t mask = a.bf16 ? 7 : 15;
+    if (!a.bf16 || forced_rows("TT_SIMT_FWD")) return false;
     const uintptr_t ptrs = reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.k) |
                            reinterpret_cast<uintptr_t>(a.v) | reinterpret_cast<uintptr_t>(a.out);
-    return a.D % 4 == 0 && a.D <= 128 && (ptrs & mask) == 0;
+    return a.D % 4 == 0 && a.D <= 128 && (ptrs & 7) == 0;
 }
 
 template <typename T>
 static cudaError_t dispatch_fwd(const AttnArgs& a, cudaStream_t st) {
-    if (simt_tiled_ok(a)) return a.D <= 64 ? launch_fwd_simt_tiled<T, 64>(a, st) : launch_fwd_simt_tiled<T, 128>(a, st);
+    if constexpr (sizeof(T) == 2) {
+        if (simt_tiled_ok(a)) return a.D <= 64 ? launch_fwd_simt_tiled<T, 64>(a, st) : launch_fwd_simt_tiled<T, 128>(a, st);
+    }
     if (a.D <= 32) return launch_fwd_simt<T, 1>(a, st);
     if (a.D <= 64) return launch_fwd_simt<T, 2>(a, st);
     if (a.D <= 128) return launch_fwd_simt<T, 4>(a, st);
@@ -890,9 +893,11 @@ static cudaError_t dispatch_bwd(const AttnArgs& a, float* delta, cudaStream_t st
 }
 
 cudaError_t attn_fwd_simt(const AttnArgs& a, cudaStream_t st) {
+    if (attn_f32_sm100_supported(a, false) && !forced_rows("TT_SIMT_FWD")) return attn_fwd_f32_sm100(a, st);
     return a.bf16 ? dispatch_fwd<__nv_bfloat16>(a, st) : dispatch_fwd<float>(a, st);
 }
 cudaError_t attn_bwd_simt(const AttnArgs& a, float* delta, cudaStream_t st) {
+    if (attn_f32_sm100_supported(a, true) && !forced_rows("TT_SIMT_BWD")) return attn_bwd_f32_sm100(a, delta, st);
     return a.bf16 ? dispatch_bwd<__nv_bfloat16>(a, delta, st) : dispatch_bwd<float>(a, delta, st);
 }
 size_t attn_bwd_simt_workspace(const AttnArgs& a) { return align256((size_t)a.BH * a.S * sizeof(float)); }
