@@ -16,6 +16,7 @@
 #include <stdlib.h>
 
 #include "common.h"
+#include <algorithm>
 #include <atomic>
 
 namespace ttk {
@@ -23,6 +24,7 @@ namespace ttk {
 constexpr int kDecThreads = 256;
 constexpr int kDecWarps = kDecThreads / 32;
 constexpr int kUnroll = 4;
+constexpr int kMaxRanges = 128;   // key ranges per slice of the tensor-core routes
 
 __device__ __forceinline__ uint4 ld_stream16(const void* p) {
     uint4 r;
@@ -291,35 +293,67 @@ static AttnArgs decode_as_forward(const AttnArgs& a, int splits) {
     g.kv_lens = nullptr;
     return g;
 }
-// true: the tensor-core route of this decode is the keys-on-rows kernel.  It runs two CTAs per SM, one per
-// (slice, key range).  As many slices as SMs already keep HBM busy (the CTAs share its bandwidth, so a
-// partial last wave costs little: measured, 256 and 512 unsplit slices beat any split); with fewer, the
-// keys are cut into about four ranges per SM of at least 512 keys.
+// true: the tensor-core route of this decode is the keys-on-rows kernel
 static bool decode_on_gq_kernel(const AttnArgs& a) {
     const char* f = getenv("TT_DECODE_GQA_PATH");
     return a.bf16 && (a.D == 128 || a.D == 64) && a.S == 1 && a.group <= 16 && !(f && f[0] == 'f');
 }
-static int decode_tc_splits(const AttnArgs& a) {   // 0: do not use the forward kernel
+// Key ranges of the keys-on-rows kernel: whole 128-key tiles, `*chunk` keys each; returns their number.  Two CTAs share
+// an SM, one per (slice, range), so 2 x SMs of them run at a time (measured on 148 SMs, D = 128 unless said).
+//   One wave or nearly: as many ranges as fit at once.  8 slices of 32768 keys 27.5 us against 30.3 with twice as many, 128 of
+//     8192 81.6 against 84.3; unsplit 256 slices of 2000 keys 43.2 against 48.5 split, 512 of 2048 81.7 against 91.6.
+//   A last wave less than three quarters full: eight ranges per SM, of at least 1024 keys.  152 slices of 8192 keys 118 ->
+//     108 us, 304 of 4096 131 -> 104, 320 of 8192 262 -> 202, 384 of 3001 105 -> 94.
+//   Lengths that differ (`ragged`) and slices enough that one wave would not cut them short: a range is at most a share of
+//     the work, or the longest sequence runs alone at the end.  16 ranges per SM, of at least 1024 keys: 256 slices of 360 to
+//     7588 keys 123 -> 100 us, 512 of 1 to 16384 364 -> 321 (if all are equally long after all, 157 -> 172).
+//   Up to 512 keys (dense caches: 1023) stay one launch.
+static int gq_ranges(const AttnArgs& a, bool ragged, int* chunk) {
+    const long long slices = a.BH / a.group, n_sm = sm_count(), at_once = 2 * n_sm;
+    *chunk = a.L;
+    long long want = std::max(1LL, at_once / slices), least = 256;
+    const long long units = slices * want, waves = (units + at_once - 1) / at_once;
+    if (ragged && 2 * slices > n_sm) {
+        want = 16 * n_sm / slices;
+        least = 1024;
+    } else if (4 * units < 3 * waves * at_once) {
+        want = (8 * n_sm + slices - 1) / slices;
+        least = 1024;
+    }
+    if (want < 2 || a.L <= (ragged ? 512 : 1023)) return 1;
+    long long c = std::max(least, (a.L + want - 1) / want);
+    c = (std::max<long long>(c, (a.L + kMaxRanges - 1) / kMaxRanges) + 127) / 128 * 128;
+    const long long n = (a.L + c - 1) / c;
+    if (n < 2) return 1;
+    *chunk = (int)c;
+    return (int)n;
+}
+// Key ranges of a dense decode on the tensor cores (0: not on them).
+static int decode_tc_splits(const AttnArgs& a) {
     const char* f = getenv("TT_DECODE_GQA_PATH");
+    const bool gq = decode_on_gq_kernel(a);
     // the keys-on-rows kernel takes every group size up to 16 (measured faster than the split-KV kernel even for
     // single heads); larger groups take the forward kernel
-    const int min_group = decode_on_gq_kernel(a) ? 1 : 4;
-    if (!(a.bf16 && a.S == 1 && a.group >= min_group)) return 0;
+    if (!(a.bf16 && a.S == 1 && a.group >= (gq ? 1 : 4))) return 0;
     if (f && f[0] == 's') return 0;                           // "simt"
     if (!attn_fwd_sm100_supported(decode_as_forward(a, 1))) return 0;
+    int chunk;
+    if (gq) return gq_ranges(a, false, &chunk);
     const int n_sm = sm_count();
     const long long slices = a.BH / a.group;
-    const bool gq = decode_on_gq_kernel(a);
-    const long long min_chunk = gq ? 512 : 256;
     if (slices >= n_sm) return 1;
-    // about four (forward kernel: two) items per SM, ranges of at least min_chunk keys that divide L exactly
-    const long long want = ((gq ? 4LL : 2LL) * n_sm + slices - 1) / slices;
-    for (long long s = want; s <= 64 && a.L / s >= min_chunk; ++s)
+    // about two items per SM, ranges of at least 256 keys that divide L exactly
+    const long long want = (2LL * n_sm + slices - 1) / slices;
+    for (long long s = want; s <= 64 && a.L / s >= 256; ++s)
         if (a.L % s == 0) return (int)s;
     for (long long s = want - 1; s >= 2; --s)
-        if (a.L % s == 0 && a.L / s >= min_chunk) return (int)s;
-    if (gq) return 1;                                         // short or indivisible key range: one range per slice
+        if (a.L % s == 0 && a.L / s >= 256) return (int)s;
     return (f && f[0] == 't') ? 1 : 0;                        // "tc": unsplit rather than SIMT
+}
+// Bytes for the partial results of `splits` ranges, floats from the keys-on-rows kernel, bf16 from the forward kernel;
+// their log-sum-exps lie behind them.
+static size_t partial_bytes(const AttnArgs& a, int splits) {
+    return align256((size_t)a.BH * splits * a.D * (decode_on_gq_kernel(a) ? 4 : 2));
 }
 
 DecodePlan attn_decode_plan(const AttnArgs& a, bool allow_tc) {
@@ -328,10 +362,9 @@ DecodePlan attn_decode_plan(const AttnArgs& a, bool allow_tc) {
     if (allow_tc) {
         pl.tc_splits = decode_tc_splits(a);
         if (pl.tc_splits == 1) return pl;
-        if (pl.tc_splits > 1) {   // partial outputs (bf16) and log-sum-exps (fp32) of every key range
+        if (pl.tc_splits > 1) {
             pl.splits = pl.tc_splits;
-            pl.chunk = a.L / pl.tc_splits;
-            pl.ws_bytes = align256((size_t)a.BH * pl.tc_splits * a.D * 2) + align256((size_t)a.BH * pl.tc_splits * 4);
+            pl.ws_bytes = partial_bytes(a, pl.tc_splits) + align256((size_t)a.BH * pl.tc_splits * 4);
             return pl;
         }
     }
@@ -355,33 +388,100 @@ DecodePlan attn_decode_plan(const AttnArgs& a, bool allow_tc) {
     return pl;
 }
 
-// Merge of the forward kernel's per-range results: out[bh] = sum_c w_c O_c / sum_c w_c with
-// w_c = exp(lse_c - max lse); partial O is [kvs, splits, G, D] bf16, partial lse [kvs, splits, G].
-template <int D>
-__global__ void attn_decode_tc_merge_kernel(const __nv_bfloat16* __restrict__ po, const float* __restrict__ plse,
-                                            __nv_bfloat16* __restrict__ out, float* __restrict__ lse, int splits, int G) {
+__device__ __forceinline__ float4 ld_partial4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
+__device__ __forceinline__ float4 ld_partial4(const __nv_bfloat16* p) {
+    const uint2 w = __ldg(reinterpret_cast<const uint2*>(p));
+    return make_float4(bf_lo(w.x), bf_hi(w.x), bf_lo(w.y), bf_hi(w.y));
+}
+// Merge of normalised per-range results: out[bh] = sum_c w_c O_c / sum_c w_c with w_c = exp(lse_c - max lse);
+// partial O is [kvs, splits, G, D], partial lse [kvs, splits, G].  One CTA per output row: D / 4 threads share a
+// range's row, so 128 threads have 4 (D = 128) or 8 ranges in flight each with `kAhead` loads, the first ones issued
+// before the weights are known.  What bounds it is latency, not bytes.
+template <int D, typename T>
+__global__ void __launch_bounds__(128) attn_decode_tc_merge_kernel(const T* __restrict__ po, const float* __restrict__ plse,
+                                                                  __nv_bfloat16* __restrict__ out, float* __restrict__ lse,
+                                                                  int splits, int G) {
+    constexpr int kLanes = D / 4, kRows = 128 / kLanes, kAhead = 4;
+    __shared__ float sm_w[kMaxRanges];
+    __shared__ float sm_o[kRows][D];
     grid_let_next_start();
     grid_wait_for_previous();
-    const long long bh = blockIdx.x;
-    const int d = threadIdx.x;
-    const long long kvs = bh / G;
-    const int g = (int)(bh - kvs * G);
-    float m = -INFINITY;
-    for (int c = 0; c < splits; ++c) m = fmaxf(m, plse[(kvs * splits + c) * G + g]);
-    if (m == -INFINITY) {   // no range held a key (an empty sequence of a paged cache)
-        out[bh * D + d] = __float2bfloat16_rn(0.f);
-        if (d == 0 && lse != nullptr) lse[bh] = -INFINITY;
-        return;
+    const long long bh = blockIdx.x, kvs = bh / G;
+    const int g = (int)(bh - kvs * G), tid = threadIdx.x;
+    const int r0 = tid / kLanes, col = (tid % kLanes) * 4;
+    const T* rows = po + ((kvs * splits) * G + g) * D + col;
+    float4 x[kAhead];
+    auto load = [&](int c0) {
+#pragma unroll
+        for (int i = 0; i < kAhead; ++i) {
+            const int c = c0 + i * kRows;
+            x[i] = c < splits ? ld_partial4(rows + (long long)c * G * D) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    };
+    load(r0);
+    if (tid < 32) {
+        float y[kMaxRanges / 32], m = -INFINITY, den = 0.f;
+#pragma unroll
+        for (int i = 0; i < kMaxRanges / 32; ++i) {
+            const int c = tid + 32 * i;
+            y[i] = c < splits ? plse[(kvs * splits + c) * G + g] : -INFINITY;
+            m = fmaxf(m, y[i]);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+#pragma unroll
+        for (int i = 0; i < kMaxRanges / 32; ++i) {
+            y[i] = y[i] == -INFINITY ? 0.f : expf(y[i] - m);   // a range without keys (all of them: m = -inf) has no weight
+            den += y[i];
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) den += __shfl_xor_sync(0xffffffffu, den, o);
+        const float inv = den > 0.f || den != den ? 1.f / den : 0.f;
+#pragma unroll
+        for (int i = 0; i < kMaxRanges / 32; ++i) sm_w[tid + 32 * i] = y[i] * inv;
+        if (tid == 0 && lse != nullptr) lse[bh] = m == -INFINITY ? -INFINITY : m + logf(den);
     }
-    float den = 0.f, acc = 0.f;
-    for (int c = 0; c < splits; ++c) {
-        const long long row = (kvs * splits + c) * G + g;
-        const float w = expf(plse[row] - m);
-        den += w;
-        acc = fmaf(w, __bfloat162float(po[row * D + d]), acc);
+    __syncthreads();
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int c0 = r0; c0 < splits; c0 += kAhead * kRows) {
+        if (c0 != r0) load(c0);
+#pragma unroll
+        for (int i = 0; i < kAhead; ++i) {
+            const int c = c0 + i * kRows;
+            const float w = c < splits ? sm_w[c] : 0.f;
+            if (w != 0.f) {   // an empty range's row was never written
+                acc.x = fmaf(w, x[i].x, acc.x); acc.y = fmaf(w, x[i].y, acc.y);
+                acc.z = fmaf(w, x[i].z, acc.z); acc.w = fmaf(w, x[i].w, acc.w);
+            }
+        }
     }
-    out[bh * D + d] = __float2bfloat16_rn(acc / den);
-    if (d == 0 && lse != nullptr) lse[bh] = m + logf(den);
+    *reinterpret_cast<float4*>(&sm_o[r0][col]) = acc;
+    __syncthreads();
+    if (tid < D) {
+        float y = 0.f;
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) y += sm_o[r][tid];
+        out[bh * D + tid] = __float2bfloat16_rn(y);
+    }
+}
+template <typename T>
+static void launch_tc_merge(const AttnArgs& a, const T* po, const float* plse, int splits, cudaStream_t st) {
+    LaunchScope ls(K_DECODE_MERGE, st);
+    if (a.D == 128)
+        launch_overlapped(attn_decode_tc_merge_kernel<128, T>, (unsigned)a.BH, 128, 0, st, po, plse, (__nv_bfloat16*)a.out, a.lse, splits, a.group);
+    else
+        launch_overlapped(attn_decode_tc_merge_kernel<64, T>, (unsigned)a.BH, 128, 0, st, po, plse, (__nv_bfloat16*)a.out, a.lse, splits, a.group);
+}
+// Runs the forward view `g` of decode `a`, several key ranges per slice, and merges their results.
+static cudaError_t run_ranges(const AttnArgs& a, AttnArgs g, int splits, void* ws, cudaStream_t st) {
+    float* plse = (float*)((unsigned char*)ws + partial_bytes(a, splits));
+    g.out = ws;
+    g.lse = plse;
+    const cudaError_t e = run_forward_view(g, st);
+    if (e != cudaSuccess) return e;
+    if (attn_decode_gq_sm100_supported(g)) launch_tc_merge(a, (const float*)ws, plse, splits, st);
+    else launch_tc_merge(a, (const __nv_bfloat16*)ws, plse, splits, st);
+    return cudaGetLastError();
 }
 
 template <int D, int G>
@@ -432,18 +532,20 @@ static AttnArgs paged_as_forward(const AttnArgs& a, const DecodeView& v, int spl
     g.max_pages = v.max_pages;
     return g;
 }
-static void paged_split(const AttnArgs& a, int* splits, int* chunk) {
+static void paged_split(const AttnArgs& a, bool ragged, int* splits, int* chunk) {
+    if (decode_on_gq_kernel(a)) {
+        *splits = gq_ranges(a, ragged, chunk);
+        return;
+    }
     const int n_sm = sm_count();
     const long long slices = a.BH / a.group;
     *splits = 1;
     *chunk = a.L;
-    const bool gq = decode_on_gq_kernel(a);
-    if (gq ? slices >= n_sm : 2 * slices >= n_sm) return;
-    // about four (forward kernel: two) items per SM, ranges of whole 128-key tiles
-    const long long want = ((gq ? 4LL : 2LL) * n_sm + slices - 1) / slices;
-    const long long min_chunk = gq ? 512 : 256;
+    if (2 * slices >= n_sm) return;
+    // about two items per SM, ranges of whole 128-key tiles
+    const long long want = (2LL * n_sm + slices - 1) / slices;
     long long c = ((a.L + want - 1) / want + 127) / 128 * 128;
-    if (c < min_chunk) c = min_chunk;
+    if (c < 256) c = 256;
     const long long n = (a.L + c - 1) / c;
     if (n < 2) return;
     *splits = (int)n;
@@ -455,48 +557,27 @@ int attn_decode_paged_on_forward(const AttnArgs& a, const DecodeView& v, size_t*
     const char* f = getenv("TT_DECODE_GQA_PATH");
     if (f && f[0] == 's') return 0;                           // "simt"
     int splits, chunk;
-    paged_split(a, &splits, &chunk);
+    paged_split(a, v.seq_lens != nullptr, &splits, &chunk);
     if (!attn_fwd_sm100_supported(paged_as_forward(a, v, splits, chunk))) return 0;
-    if (splits > 1) *ws_bytes = align256((size_t)a.BH * splits * a.D * 2) + align256((size_t)a.BH * splits * 4);
+    if (splits > 1) *ws_bytes = partial_bytes(a, splits) + align256((size_t)a.BH * splits * 4);
     return splits;
 }
 cudaError_t attn_decode_paged_forward(const AttnArgs& a, const DecodeView& v, int splits, void* ws, cudaStream_t st) {
     int s2, chunk;
-    paged_split(a, &s2, &chunk);
+    paged_split(a, v.seq_lens != nullptr, &s2, &chunk);
     if (s2 != splits) return cudaErrorInvalidValue;
-    AttnArgs g = paged_as_forward(a, v, splits, chunk);
-    if (splits == 1) return run_forward_view(g, st);
-    __nv_bfloat16* po = (__nv_bfloat16*)ws;
-    float* plse = (float*)((unsigned char*)ws + align256((size_t)a.BH * splits * a.D * 2));
-    g.out = po;
-    g.lse = plse;
-    cudaError_t e = run_forward_view(g, st);
-    if (e != cudaSuccess) return e;
-    LaunchScope ls(K_DECODE_MERGE, st);
-    if (a.D == 128)
-        launch_overlapped(attn_decode_tc_merge_kernel<128>, (unsigned)a.BH, 128, 0, st, po, plse, (__nv_bfloat16*)a.out, a.lse, splits, a.group);
-    else
-        launch_overlapped(attn_decode_tc_merge_kernel<64>, (unsigned)a.BH, 64, 0, st, po, plse, (__nv_bfloat16*)a.out, a.lse, splits, a.group);
-    return cudaGetLastError();
+    const AttnArgs g = paged_as_forward(a, v, splits, chunk);
+    return splits == 1 ? run_forward_view(g, st) : run_ranges(a, g, splits, ws, st);
 }
 
 cudaError_t attn_decode(const AttnArgs& a, const DecodePlan& pl, void* ws, cudaStream_t st, const DecodeView* view) {
     const bool plain = !(view && (view->block_table || view->seq_lens));
     if (plain && pl.tc_splits == 1) return run_forward_view(decode_as_forward(a, 1), st);
     if (plain && pl.tc_splits > 1) {
-        AttnArgs g = decode_as_forward(a, pl.tc_splits);
-        __nv_bfloat16* po = (__nv_bfloat16*)ws;
-        float* plse = (float*)((unsigned char*)ws + align256((size_t)a.BH * pl.tc_splits * a.D * 2));
-        g.out = po;
-        g.lse = plse;
-        cudaError_t e = run_forward_view(g, st);
-        if (e != cudaSuccess) return e;
-        LaunchScope ls(K_DECODE_MERGE, st);
-        if (a.D == 128)
-            launch_overlapped(attn_decode_tc_merge_kernel<128>, (unsigned)a.BH, 128, 0, st, po, plse, (__nv_bfloat16*)a.out, a.lse, pl.tc_splits, a.group);
-        else
-            launch_overlapped(attn_decode_tc_merge_kernel<64>, (unsigned)a.BH, 64, 0, st, po, plse, (__nv_bfloat16*)a.out, a.lse, pl.tc_splits, a.group);
-        return cudaGetLastError();
+        if (!decode_on_gq_kernel(a)) return run_ranges(a, decode_as_forward(a, pl.tc_splits), pl.tc_splits, ws, st);
+        int chunk;
+        if (gq_ranges(a, false, &chunk) != pl.tc_splits) return cudaErrorInvalidValue;
+        return run_ranges(a, paged_as_forward(a, DecodeView(), pl.tc_splits, chunk), pl.tc_splits, ws, st);
     }
     if (a.bf16 && a.S == 1 && a.D == 128) return launch_decode<128>(a, pl, ws, st, true, view);
     if (a.bf16 && a.S == 1 && a.D == 64) return launch_decode<64>(a, pl, ws, st, true, view);

@@ -17,9 +17,11 @@
 // columns in tensor memory.
 //
 // One CTA per (key/value slice, key range); two CTAs per SM (110 KB of shared memory, 64 tensor-memory
-// columns each) so that one CTA's set-up and tail overlap the other's stream.  Results per range are
-// normalised (out bf16 [slices*ranges, G, D], log-sum-exp fp32): with more than one range a merge
-// kernel combines them, exactly as for the forward-kernel route this replaces.
+// columns each) so that one CTA's set-up and tail overlap the other's stream.  With one range the result is
+// the output; with more, a range's normalised result goes to the workspace as floats ([slices*ranges, G, D],
+// log-sum-exp beside it) and a merge kernel combines them.  Ranges are whole tiles behind a key offset that
+// the tensor map's coordinates carry, so any key count splits (equal parts of L, as views of K and V, left
+// 5001 keys with 3 ranges and a prime count with one).
 //   warps 0-3  softmax (thread = key of the tile = row d of O^T),  warp 4  MMA issuer,  warp 5  TMA loader
 // Every mbarrier wait is bounded (sm100_ptx.cuh); the one bar.sync per tile among the softmax warps is reached
 // by all 128 threads whatever the waits returned (they never leave the tile loop early).
@@ -49,7 +51,8 @@ struct GqCfg {
 };
 
 struct GqParams {
-    __nv_bfloat16* out;
+    __nv_bfloat16* out; // one range per slice
+    float* part;        // several: normalised partial results (and lse holds theirs)
     float* lse;
     int G;              // query heads per key/value head = query rows of a slice
     int L;              // keys per key/value slice of the K/V tensor maps
@@ -101,6 +104,26 @@ attn_decode_gq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
     const int warp = uniform_warp_idx();
     const int lane = threadIdx.x & 31;
 
+    // ---- this CTA's key range
+    const int bh = blockIdx.x;                 // output slice
+    const int qslice = bh / p.q_div;
+    int zslice = bh, key0 = 0, Lv = p.L;
+    if (kCache) {
+        zslice = qslice;                       // key/value slice
+        key0 = (bh - qslice * p.q_div) * p.kv_chunk;
+        int len = p.L;
+        if (p.kv_lens) {
+            grid_wait_for_previous();
+            len = min(p.L, max(0, p.kv_lens[zslice / p.H]));
+        }
+        Lv = p.kv_chunk > 0 ? max(0, min(len - key0, p.kv_chunk)) : len;
+        if (Lv == 0 && p.part != nullptr) {    // a range past its sequence's end: no weight in the merge, which reads no more of it
+            if (threadIdx.x < p.G) p.lse[(long long)bh * p.G + threadIdx.x] = -INFINITY;
+            return;
+        }
+    }
+    const int n_tiles = (Lv + 127) >> 7;
+
     if (threadIdx.x == 0) {
         *abort_flag = 0;
         mbar_init(bar_q_full, 1);
@@ -133,17 +156,6 @@ attn_decode_gq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
     WaitCtx wctx{p.status, abort_flag, warp};
     grid_wait_for_previous();
 
-    // ---- this CTA's key range
-    const int bh = blockIdx.x;                 // output slice
-    const int qslice = bh / p.q_div;
-    int zslice = bh, key0 = 0, Lv = p.L;
-    if (kCache) {
-        zslice = qslice;                       // key/value slice
-        key0 = (bh - qslice * p.q_div) * p.kv_chunk;
-        const int len = p.kv_lens ? min(p.L, max(0, p.kv_lens[zslice / p.H])) : p.L;
-        Lv = p.kv_chunk > 0 ? max(0, min(len - key0, p.kv_chunk)) : len;
-    }
-    const int n_tiles = (Lv + 127) >> 7;
     constexpr uint32_t kColO = 32;
 
     if (warp < 4) {
@@ -151,7 +163,7 @@ attn_decode_gq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
         const int t = threadIdx.x;
         const uint32_t lane_off = (uint32_t)(warp * 32) << 16;
         const float c = p.scale_log2;
-        if (n_tiles == 0) {   // an empty range (cache mode): zero output, log-sum-exp -inf; the merge gives it no weight
+        if (n_tiles == 0) {   // an empty sequence (cache mode): zero output, log-sum-exp -inf
             if (t < kD)
                 for (int g = 0; g < p.G; ++g) p.out[((long long)bh * p.G + g) * kD + t] = __float2bfloat16_rn(0.f);
             if (t < p.G && p.lse != nullptr) p.lse[(long long)bh * p.G + t] = -INFINITY;
@@ -260,7 +272,12 @@ attn_decode_gq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
             for (int g = 0; g < kG; ++g) {
                 const float l = red_sum[g] + red_sum[16 + g] + red_sum[32 + g] + red_sum[48 + g];
                 if (g < p.G) {
-                    if (t < kD) p.out[((long long)bh * p.G + g) * kD + t] = __float2bfloat16_rn(__uint_as_float(o[g]) / l);
+                    const long long at = ((long long)bh * p.G + g) * kD + t;
+                    const float y = __uint_as_float(o[g]) / l;
+                    if (t < kD) {
+                        if (kCache && p.part != nullptr) p.part[at] = y;
+                        else p.out[at] = __float2bfloat16_rn(y);
+                    }
                     if (t == g && p.lse != nullptr) p.lse[(long long)bh * p.G + g] = (m_ref[g] + log2f(l)) * 0.6931471805599453f;
                 }
             }
@@ -434,7 +451,8 @@ cudaError_t launch_gq(const AttnArgs& a, cudaStream_t st) {
     cudaError_t e = TT_ALLOW_SMEM((attn_decode_gq_sm100_kernel<kD, kG, kCache>), GqCfg<kD>::kSmemBytes);
     if (e != cudaSuccess) return e;
     GqParams p;
-    p.out = (__nv_bfloat16*)a.out;
+    p.out = q_div > 1 ? nullptr : (__nv_bfloat16*)a.out;
+    p.part = q_div > 1 ? (float*)a.out : nullptr;
     p.lse = a.lse;
     p.G = a.S;
     p.L = a.L;
@@ -456,7 +474,8 @@ cudaError_t launch_gq(const AttnArgs& a, cudaStream_t st) {
 }  // namespace
 
 // `a` is the forward view of a grouped decode (see decode_as_forward / paged_as_forward in
-// attn_decode.cu): S = query heads per key/value head, BH = key/value slices x key ranges.
+// attn_decode.cu): S = query heads per key/value head, BH = key/value slices x key ranges; with several ranges
+// (q_div > 1, cache mode) `out` is the workspace of their float results.
 // TT_DECODE_GQA_PATH=fwd keeps such problems on the general forward kernel (tests, measurements).
 bool attn_decode_gq_sm100_supported(const AttnArgs& a) {
     if (!a.bf16 || (a.D != 128 && a.D != 64) || a.causal || a.group != 1 || a.S < 1 || a.S > 16 || a.L < 1 || a.cu_q != nullptr) return false;
@@ -465,7 +484,7 @@ bool attn_decode_gq_sm100_supported(const AttnArgs& a) {
         if (a.q_div > 1 ? !(a.kv_chunk >= 128 && a.kv_chunk % 128 == 0) : a.kv_chunk != 0) return false;
         const int ps = a.page_size;   // paged: whole pages per TMA box
         if (a.block_table != nullptr && !(ps >= 8 && (128 % ps == 0 || ps % 128 == 0) && a.max_pages >= 1)) return false;
-    } else if (a.block_table != nullptr || a.kv_lens != nullptr) {
+    } else if (a.block_table != nullptr || a.kv_lens != nullptr || a.q_div > 1) {
         return false;
     }
     const char* f = getenv("TT_DECODE_GQA_PATH");

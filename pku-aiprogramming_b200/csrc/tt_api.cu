@@ -654,8 +654,8 @@ size_t tt_attn_decode_workspace_bytes(const tt_attn_desc* desc) {
     if (a.S != 1) return 0;
     // enough for every route a call with this descriptor can take (dense, paged or ragged)
     const size_t w1 = attn_decode_plan(a, true).ws_bytes, w2 = attn_decode_plan(a, false).ws_bytes;
-    size_t w3 = 0;
-    {   // the paged route on the forward kernel (its split depends on the shape only; page size 128 stands in)
+    size_t w3 = 0, w4 = 0;
+    {   // the paged routes with and without lengths (their split depends on the shape only; page size 128 stands in)
         static const int one_page = 0;
         DecodeView v;
         v.block_table = &one_page;
@@ -663,8 +663,10 @@ size_t tt_attn_decode_workspace_bytes(const tt_attn_desc* desc) {
         v.max_pages = (a.L + 127) / 128;
         v.hkv = desc->Hkv > 0 ? desc->Hkv : desc->H;
         attn_decode_paged_on_forward(a, v, &w3);
+        v.seq_lens = &one_page;
+        attn_decode_paged_on_forward(a, v, &w4);
     }
-    return std::max(w1, std::max(w2, w3));
+    return std::max(std::max(w1, w2), std::max(w3, w4));
 }
 
 int tt_attn_decode(const tt_attn_desc* desc, const void* q, const void* k, const void* v, void* out, float* lse,

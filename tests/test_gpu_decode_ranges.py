@@ -1,0 +1,45 @@
+"""Decode whose keys are cut into ranges of whole 128-key tiles: key counts that nothing divides, few slices (one wave of ranges), slices
+that would leave a last wave nearly empty, ragged lengths whose later ranges are empty.  Against the oracle, out 2e-2 absolute and
+log-sum-exp 1e-3 as for the base op; partial results are floats, so the ranges add no rounding of their own."""
+import numpy as np
+import pytest
+
+from test_gpu_variants import dense_decode_ref, make_grouped
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+def run(tt, oracle, B, H, Hkv, L, D, lens=None):
+    q, k, v, _ = make_grouped(oracle, L + D, B, H, Hkv, 1, L, D, True)
+    o_r, lse_r = dense_decode_ref(oracle, q, k, v) if lens is None else dense_decode_ref(oracle, q, k, v, np.asarray(lens, np.int32))
+    tq, tk, tv = (torch.from_numpy(a).cuda().bfloat16() for a in (q, k, v))
+    before = tt.capi.launch_count()
+    if lens is None:
+        out, lse = tt.attention_decode(tq, tk, tv)
+    else:
+        out, lse = tt.attention_decode_paged(tq, tk, tv, seq_lens=torch.tensor(lens, dtype=torch.int32, device="cuda"))
+    launches = tt.capi.launch_count() - before
+    tt.check_device_status()
+    assert oracle.max_abs_err(out.float().cpu().numpy(), o_r) <= 2e-2
+    got = lse.cpu().numpy()
+    keep = np.isfinite(lse_r)
+    assert np.array_equal(np.isfinite(got), keep) and oracle.max_abs_err(got[keep], lse_r[keep]) <= 1e-3
+    return launches
+
+
+# the last: one slice whose ranges stay below the merge kernel's limit of 128
+@pytest.mark.parametrize("B,H,Hkv,L,D", [(1, 4, 4, 1024, 64), (1, 8, 2, 1025, 128), (1, 32, 8, 5003, 128), (1, 16, 1, 16385, 128),
+                                          (38, 8, 8, 2051, 64), (1, 2, 1, 66001, 64)])
+def test_dense_ranges(tt, oracle, B, H, Hkv, L, D):
+    assert run(tt, oracle, B, H, Hkv, L, D) == 2
+
+
+def test_short_cache_is_one_launch(tt, oracle):
+    assert run(tt, oracle, 2, 8, 2, 1023, 128) == 1
+
+
+@pytest.mark.parametrize("H,Hkv,D", [(8, 2, 128), (4, 4, 64)])
+def test_ragged_ranges_with_empty_ones(tt, oracle, H, Hkv, D):
+    lens = [0, 1, 1024, 1025, 2048, 2300, 127, 128] * 5
+    assert run(tt, oracle, len(lens), H, Hkv, 2300, D, lens) == 2
