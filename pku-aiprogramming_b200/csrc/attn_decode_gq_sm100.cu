@@ -16,13 +16,15 @@
 // by more than 2^8), in which case every thread -- now as a row d of O^T -- rescales its 16 accumulator
 // columns in tensor memory.
 //
-// One CTA per (key/value slice, key range); two CTAs per SM (110 KB of shared memory, 64 tensor-memory
-// columns each) so that one CTA's set-up and tail overlap the other's stream.  With one range the result is
+// A work item is a (key/value slice, key range); two CTAs per SM (110 KB of shared memory, 64 tensor-memory
+// columns each) so that one CTA's tail overlaps the other's stream.  A CTA that runs takes over items whose CTAs have not
+// started (ItemStream), and its loader goes on into the next item's keys while the last one's tiles are still
+// worked on: with a CTA per item the ring ran empty at each end, 1 to 2 us an item.  With one range the result is
 // the output; with more, a range's normalised result goes to the workspace as floats ([slices*ranges, G, D],
 // log-sum-exp beside it) and a merge kernel combines them.  Ranges are whole tiles behind a key offset that
 // the tensor map's coordinates carry, so any key count splits (equal parts of L, as views of K and V, left
 // 5001 keys with 3 ranges and a prime count with one).
-//   warps 0-3  softmax (thread = key of the tile = row d of O^T),  warp 4  MMA issuer,  warp 5  TMA loader
+//   warps 0-3  softmax (thread = key of the tile = row d of O^T),  warp 4  MMA issuer,  warp 5  TMA loader and scheduler
 // Every mbarrier wait is bounded (sm100_ptx.cuh); the one bar.sync per tile among the softmax warps is reached
 // by all 128 threads whatever the waits returned (they never leave the tile loop early).
 #include "common.h"
@@ -63,6 +65,7 @@ struct GqParams {
     const int* block_table;
     int page_size, max_pages;
     float scale_log2;
+    int resident;       // CTAs that run at once: with no more items there is none to take over
     unsigned int* status;
 };
 
@@ -96,33 +99,21 @@ attn_decode_gq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
     uint64_t* bar_s_free = bar_s_full + 2;           // [2] softmax (scores in registers) -> MMA
     uint64_t* bar_p_full = bar_s_free + 2;           // [2] softmax (P in shared memory) -> MMA
     uint64_t* bar_p_free = bar_p_full + 2;           // [2] MMA (P consumed) -> softmax
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar_p_free + 2);
+    uint64_t* bar_q_free = bar_p_free + 2;           // MMA (an item's last scores done) -> loader
+    uint64_t* bar_o_free = bar_q_free + 1;           // softmax (O^T in registers) -> MMA
+    uint64_t* bar_item_full = bar_o_free + 1;        // [2] loader -> MMA, softmax
+    uint64_t* bar_item_empty = bar_item_full + 2;    // [2]
+    uint64_t* bar_next = bar_item_empty + 2;         // the hardware's answer
+    int2* item_ring = reinterpret_cast<int2*>(bar_next + 1);   // [2] item, its keys (item -1: no more)
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(item_ring + 2);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    int2* item_now = reinterpret_cast<int2*>(aux + 472);
+    uint4* response = reinterpret_cast<uint4*>(aux + 480);
     int* red_max = reinterpret_cast<int*>(aux + 512);        // [2 buffers][4 warps][16]
     float* red_sum = reinterpret_cast<float*>(aux + 1024);   // [4 warps][16]
 
     const int warp = uniform_warp_idx();
     const int lane = threadIdx.x & 31;
-
-    // ---- this CTA's key range
-    const int bh = blockIdx.x;                 // output slice
-    const int qslice = bh / p.q_div;
-    int zslice = bh, key0 = 0, Lv = p.L;
-    if (kCache) {
-        zslice = qslice;                       // key/value slice
-        key0 = (bh - qslice * p.q_div) * p.kv_chunk;
-        int len = p.L;
-        if (p.kv_lens) {
-            grid_wait_for_previous();
-            len = min(p.L, max(0, p.kv_lens[zslice / p.H]));
-        }
-        Lv = p.kv_chunk > 0 ? max(0, min(len - key0, p.kv_chunk)) : len;
-        if (Lv == 0 && p.part != nullptr) {    // a range past its sequence's end: no weight in the merge, which reads no more of it
-            if (threadIdx.x < p.G) p.lse[(long long)bh * p.G + threadIdx.x] = -INFINITY;
-            return;
-        }
-    }
-    const int n_tiles = (Lv + 127) >> 7;
 
     if (threadIdx.x == 0) {
         *abort_flag = 0;
@@ -136,7 +127,12 @@ attn_decode_gq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
             mbar_init(&bar_s_free[b], 4);
             mbar_init(&bar_p_full[b], 4);
             mbar_init(&bar_p_free[b], 1);
+            mbar_init(&bar_item_full[b], 1);
+            mbar_init(&bar_item_empty[b], 2);   // MMA warp, softmax warp 0
         }
+        mbar_init(bar_q_free, 1);
+        mbar_init(bar_o_free, 4);
+        mbar_init(bar_next, 1);
         fence_barrier_init();
         fence_proxy_async_smem();
     }
@@ -157,17 +153,33 @@ attn_decode_gq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
     grid_wait_for_previous();
 
     constexpr uint32_t kColO = 32;
+    // n-th item of this CTA and its keys, -1: no more (or a wait has given up); one warp reads it for each role
+    auto next_item = [&](int n) -> int2 {
+        int2 it = make_int2(-1, 0);
+        if (__all_sync(0xffffffffu, mbar_wait(&bar_item_full[n & 1], (n >> 1) & 1, wctx, 70 + (n & 1), n))) it = item_ring[n & 1];
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bar_item_empty[n & 1]);
+        return it;
+    };
 
     if (warp < 4) {
         // =========================================================== softmax: thread = key of the tile / row d of O^T
         const int t = threadIdx.x;
         const uint32_t lane_off = (uint32_t)(warp * 32) << 16;
         const float c = p.scale_log2;
-        if (n_tiles == 0) {   // an empty sequence (cache mode): zero output, log-sum-exp -inf
-            if (t < kD)
-                for (int g = 0; g < p.G; ++g) p.out[((long long)bh * p.G + g) * kD + t] = __float2bfloat16_rn(0.f);
-            if (t < p.G && p.lse != nullptr) p.lse[(long long)bh * p.G + t] = -INFINITY;
-        } else {
+        int J0 = 0;   // tiles of earlier items
+        for (int n = 0;; ++n) {
+            // Warp 0 reads the item for all four: the named barriers below need the same items and tiles in each, whatever
+            // a wait returned.  Written again only behind the barriers of this item's tiles.
+            if (warp == 0) {
+                const int2 got = next_item(n);
+                if (lane == 0) *item_now = got;
+            }
+            bar_sync_128(1);
+            const int2 it = *item_now;
+            if (it.x < 0) break;
+            const long long bh = it.x;
+            const int Lv = it.y, n_tiles = (Lv + 127) >> 7;
             float m_ref[kG], l_t[kG];
 #pragma unroll
             for (int g = 0; g < kG; ++g) {
@@ -180,8 +192,8 @@ attn_decode_gq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
             // Every thread runs every tile, even after a wait has given up (all later waits then return at
             // once and the results are void): the named barriers below need all 128 threads each time.
             for (int j = 0; j < n_tiles; ++j) {
-                const int b = j & 1;
-                mbar_wait(&bar_s_full[b], (j >> 1) & 1, wctx, 10 + b, j);
+                const int J = J0 + j, b = J & 1;
+                mbar_wait(&bar_s_full[b], (J >> 1) & 1, wctx, 10 + b, j);
                 __syncwarp();
                 tc_fence_after();
                 uint32_t sr[16];
@@ -227,7 +239,7 @@ attn_decode_gq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
                         // O^T *= f, once every MMA up to tile j - 1 has completed: that is the next phase of the
                         // other P buffer's `free` barrier (a thread waits for every phase of these two barriers in
                         // turn, so a phase's parity is never mistaken for an older one's)
-                        mbar_wait(&bar_p_free[(j - 1) & 1], ((j - 1) >> 1) & 1, wctx, 30, j);
+                        mbar_wait(&bar_p_free[(J - 1) & 1], ((J - 1) >> 1) & 1, wctx, 30, j);
                         __syncwarp();
                         tc_fence_after();
                         uint32_t o[16];
@@ -239,7 +251,7 @@ attn_decode_gq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
                         tmem_wait_st();
                     }
                 }
-                mbar_wait(&bar_p_free[b], ((j >> 1) & 1) ^ 1, wctx, 20 + b, j);   // MMAs of tile j - 2 have read this P buffer
+                mbar_wait(&bar_p_free[b], ((J >> 1) & 1) ^ 1, wctx, 20 + b, j);   // MMAs of tile J - 2 have read this P buffer
                 unsigned char* pb = sP + b * kPBytes + p_off;
 #pragma unroll
                 for (int g = 0; g < kG; ++g) {
@@ -254,12 +266,16 @@ attn_decode_gq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
                 if (lane == 0) mbar_arrive(&bar_p_full[b]);
             }
             // ---- result: O^T / l -> bf16, log-sum-exp
-            mbar_wait(&bar_p_free[(n_tiles - 1) & 1], ((n_tiles - 1) >> 1) & 1, wctx, 31, n_tiles);   // the last tile's MMAs have completed
+            J0 += n_tiles;
+            mbar_wait(&bar_p_free[(J0 - 1) & 1], ((J0 - 1) >> 1) & 1, wctx, 31, n_tiles);   // the last tile's MMAs have completed
             __syncwarp();
             tc_fence_after();
             uint32_t o[16];
             tmem_ld16(tmem_base + lane_off + kColO, o);
             tmem_wait_ld();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_o_free);
 #pragma unroll
             for (int g = 0; g < kG; ++g) {
                 float v = l_t[g];
@@ -272,25 +288,43 @@ attn_decode_gq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
             for (int g = 0; g < kG; ++g) {
                 const float l = red_sum[g] + red_sum[16 + g] + red_sum[32 + g] + red_sum[48 + g];
                 if (g < p.G) {
-                    const long long at = ((long long)bh * p.G + g) * kD + t;
+                    const long long at = (bh * p.G + g) * kD + t;
                     const float y = __uint_as_float(o[g]) / l;
                     if (t < kD) {
                         if (kCache && p.part != nullptr) p.part[at] = y;
                         else p.out[at] = __float2bfloat16_rn(y);
                     }
-                    if (t == g && p.lse != nullptr) p.lse[(long long)bh * p.G + g] = (m_ref[g] + log2f(l)) * 0.6931471805599453f;
+                    if (t == g && p.lse != nullptr) p.lse[bh * p.G + g] = (m_ref[g] + log2f(l)) * 0.6931471805599453f;
                 }
             }
         }
     } else if (warp == 5) {
-        // =========================================================== TMA loader
-        if (n_tiles > 0) {
-            if (elect_one()) {
-                mbar_arrive_expect_tx(bar_q_full, kQBytes);
-                // 16 query rows from row qslice * G of q viewed as [rows, D]; rows past the group belong to other
-                // heads (or are zero past the end): their columns of S^T and O^T are never read
-#pragma unroll
-                for (int sb = 0; sb < kSub; ++sb) tma_load_3d(sQ + sb * 2048, &tmQ, bar_q_full, sb * 64, qslice * p.G, 0);
+        // =========================================================== TMA loader, scheduler
+        ItemStream items{bar_next, response, (int)gridDim.x > p.resident};
+        int n = 0, E0 = 0;   // items handed on, ring entries of earlier items
+        for (int bh = blockIdx.x; bh >= 0; bh = items.next(wctx, 80, n)) {
+            const int qslice = bh / p.q_div;
+            int zslice = bh, key0 = 0, Lv = p.L;
+            if (kCache) {
+                zslice = qslice;                       // key/value slice
+                key0 = (bh - qslice * p.q_div) * p.kv_chunk;
+                const int len = p.kv_lens ? min(p.L, max(0, __ldg(p.kv_lens + zslice / p.H))) : p.L;
+                Lv = p.kv_chunk > 0 ? max(0, min(len - key0, p.kv_chunk)) : len;
+            }
+            const int n_tiles = (Lv + 127) >> 7;
+            if (n_tiles == 0) {   // an empty range or sequence: log-sum-exp -inf, no weight in a merge; output zero without one
+                for (int g = lane; g < p.G; g += 32)
+                    if (p.lse != nullptr) p.lse[(long long)bh * p.G + g] = -INFINITY;
+                if (p.part == nullptr)
+                    for (int i = lane; i < p.G * kD; i += 32) p.out[(long long)bh * p.G * kD + i] = __float2bfloat16_rn(0.f);
+                items.request(*abort_flag != 0);
+                continue;
+            }
+            mbar_wait(&bar_item_empty[n & 1], ((n >> 1) & 1) ^ 1, wctx, 72 + (n & 1), n);
+            __syncwarp();
+            if (lane == 0) {
+                item_ring[n & 1] = make_int2(bh, Lv);
+                mbar_arrive(&bar_item_full[n & 1]);
             }
             __syncwarp();
             // paged cache: lane i fetches the i-th page (or 128-row part of a larger page) of a tile.  The table
@@ -304,13 +338,14 @@ attn_decode_gq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
                 return __ldg(p.block_table + (long long)(zslice / p.H) * p.max_pages + key / p.page_size);
             };
             int page_next = page_of(0);
-            for (int e = 0; e < 2 * n_tiles; ++e) {   // entry e: K of tile e/2 (even), V (odd)
-                const int st = e % kStages;
+            bool live = true;
+            for (int e = 0; e < 2 * n_tiles && live; ++e) {   // entry e: K of tile e/2 (even), V (odd)
+                const int E = E0 + e, st = E % kStages;
                 const int tile = e >> 1;
                 const int page = page_next;
                 if (e & 1) page_next = page_of(tile + 1);             // issued now, consumed two entries later
-                if (!mbar_wait(&bar_kv_empty[st], ((e / kStages) & 1) ^ 1, wctx, 40 + st, e)) break;
-                __syncwarp();
+                live = __all_sync(0xffffffffu, mbar_wait(&bar_kv_empty[st], ((E / kStages) & 1) ^ 1, wctx, 40 + st, e));
+                if (!live) break;
                 const CUtensorMap* tm = (e & 1) ? &tmV : &tmK;
                 unsigned char* dst = sKV + st * kTileBytes;
                 const int k_first = tile * 128;                       // first key of the tile inside the range
@@ -338,9 +373,30 @@ attn_decode_gq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
                     }
                     __syncwarp();
                 }
+                if (e == 0) {   // behind the first K tile: the previous item's last scores may still read Q
+                    live = __all_sync(0xffffffffu, mbar_wait(bar_q_free, (n & 1) ^ 1, wctx, 74, n));
+                    if (live && elect_one()) {
+                        mbar_arrive_expect_tx(bar_q_full, kQBytes);
+                        // 16 query rows from row qslice * G of q viewed as [rows, D]; rows past the group belong to other
+                        // heads (or are zero past the end): their columns of S^T and O^T are never read
+#pragma unroll
+                        for (int sb = 0; sb < kSub; ++sb) tma_load_3d(sQ + sb * 2048, &tmQ, bar_q_full, sb * 64, qslice * p.G, 0);
+                    }
+                    __syncwarp();
+                }
             }
+            E0 += 2 * n_tiles;
+            ++n;
+            items.request(!live || *abort_flag != 0);
         }
-    } else if (n_tiles > 0) {
+        mbar_wait(&bar_item_empty[n & 1], ((n >> 1) & 1) ^ 1, wctx, 73, n);
+        __syncwarp();
+        if (lane == 0) {
+            item_ring[n & 1] = make_int2(-1, 0);
+            mbar_arrive(&bar_item_full[n & 1]);
+        }
+        __syncwarp();
+    } else {
         // =========================================================== MMA issuer (warp 4)
         constexpr uint32_t idesc_s = umma_idesc_bf16(128, 16, false, false);   // S^T = K Q^T
         constexpr uint32_t idesc_o = umma_idesc_bf16(128, 16, true, false);    // O^T += V^T P: A = V read MN-major
@@ -351,7 +407,7 @@ attn_decode_gq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
         const uint32_t dV_base = umma_desc_lo(sKV_addr, kSub == 2 ? kSubBytes : 0);   // MN-major A: M = d over two 64-wide blocks (D = 64: the same block twice)
         const uint32_t dQ = umma_desc_lo(__shfl_sync(0xffffffffu, smem_u32(sQ), 0), 16);   // K-major B, 16 rows
         const uint32_t dP_base = umma_desc_lo(__shfl_sync(0xffffffffu, smem_u32(sP), 0), 16);
-        auto issue_s = [&](int j) {
+        auto issue_s = [&](int j) {   // (tiles counted over all items here and below)
             const uint32_t a0 = dK_base + (((2 * j) % kStages) * kTileBytes >> 4);
             if (elect_one()) {
 #pragma unroll
@@ -361,14 +417,14 @@ attn_decode_gq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
             }
             __syncwarp();
         };
-        auto issue_o = [&](int j) {
+        auto issue_o = [&](int j, bool first) {
             const uint32_t a0 = dV_base + (((2 * j + 1) % kStages) * kTileBytes >> 4);
             const uint32_t b0 = dP_base + ((j & 1) * kPBytes >> 4);
             if (elect_one()) {
 #pragma unroll
                 for (int kk = 0; kk < 8; ++kk)   // 16 keys per step
                     umma_ss_one(tmem_u + kColO, a0 + kk * 128, b0 + (((kk >> 2) * 2048 + (kk & 3) * 32) >> 4), hi, idesc_o,
-                                (j > 0 || kk > 0) ? 1u : 0u);
+                                (!first || kk > 0) ? 1u : 0u);
             }
             __syncwarp();
         };
@@ -377,47 +433,53 @@ attn_decode_gq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
             __syncwarp();
             return ok;
         };
-        bool live = mbar_wait(bar_q_full, 0, wctx, 60, 0);
-        __syncwarp();
-        live = live && wait_entry(0);
-        tc_fence_after();
-        if (live) {
-            issue_s(0);
-            tc_commit(&bar_s_full[0]);
-            tc_commit(&bar_kv_empty[0]);
-        }
-        for (int j = 0; j < n_tiles && live; ++j) {
-            const int b = j & 1;
-            if (j + 1 < n_tiles) {   // next tile's scores, under this tile's softmax
-                live = wait_entry(2 * j + 2);
-                if (j + 1 >= 2) live = live && mbar_wait(&bar_s_free[(j + 1) & 1], (((j + 1) >> 1) & 1) ^ 1, wctx, 61, j);
-                __syncwarp();
-                tc_fence_after();
-                if (!live) break;
-                issue_s(j + 1);
-                tc_commit(&bar_s_full[(j + 1) & 1]);
-                tc_commit(&bar_kv_empty[(2 * j + 2) % kStages]);
-            }
-            live = wait_entry(2 * j + 1);   // V_j
-            const int rv = Lv - j * 128;
-            if (rv < 128) {
-                // Rows of the last V tile past the range's end hold whatever memory (or the ring slot) held;
-                // their P is exactly 0, but 0 x NaN is not, so they are zeroed.
-                unsigned char* vt = sKV + ((2 * j + 1) % kStages) * kTileBytes;
-#pragma unroll
-                for (int sb = 0; sb < kSub; ++sb)
-                    for (int o = rv * 128 + lane * 16; o < 128 * 128; o += 32 * 16)
-                        *reinterpret_cast<uint4*>(vt + sb * kSubBytes + o) = make_uint4(0u, 0u, 0u, 0u);
-                fence_proxy_async_smem();
-                __syncwarp();
-            }
-            live = live && mbar_wait(&bar_p_full[b], (j >> 1) & 1, wctx, 62 + b, j);
+        auto start_s = [&](int J, bool last) -> bool {   // scores of tile J; behind an item's last ones Q may be replaced
+            bool ok = wait_entry(2 * J);
+            if (J >= 2) ok = mbar_wait(&bar_s_free[J & 1], ((J >> 1) & 1) ^ 1, wctx, 61, J) && ok;
             __syncwarp();
             tc_fence_after();
-            if (!live) break;
-            issue_o(j);
-            tc_commit(&bar_kv_empty[(2 * j + 1) % kStages]);
-            tc_commit(&bar_p_free[b]);   // P consumed; also: every MMA issued so far has completed
+            if (!__all_sync(0xffffffffu, ok)) return false;
+            issue_s(J);
+            tc_commit(&bar_s_full[J & 1]);
+            tc_commit(&bar_kv_empty[(2 * J) % kStages]);
+            if (last) tc_commit(bar_q_free);
+            return true;
+        };
+        int J0 = 0;
+        bool live = true;
+        for (int n = 0; live; ++n) {
+            const int2 it = next_item(n);
+            if (it.x < 0) break;
+            const int Lv = it.y, n_tiles = (Lv + 127) >> 7;
+            live = __all_sync(0xffffffffu, mbar_wait(bar_q_full, n & 1, wctx, 60, n)) && start_s(J0, n_tiles == 1);
+            for (int j = 0; j < n_tiles && live; ++j) {
+                const int J = J0 + j, b = J & 1;
+                if (j + 1 < n_tiles) live = start_s(J + 1, j + 2 == n_tiles);   // next tile's scores, under this tile's softmax
+                if (!live) break;
+                live = wait_entry(2 * J + 1);   // V
+                const int rv = Lv - j * 128;
+                if (rv < 128) {
+                    // Rows of the last V tile past the range's end hold whatever memory (or the ring slot) held;
+                    // their P is exactly 0, but 0 x NaN is not, so they are zeroed.
+                    unsigned char* vt = sKV + ((2 * J + 1) % kStages) * kTileBytes;
+#pragma unroll
+                    for (int sb = 0; sb < kSub; ++sb)
+                        for (int o = rv * 128 + lane * 16; o < 128 * 128; o += 32 * 16)
+                            *reinterpret_cast<uint4*>(vt + sb * kSubBytes + o) = make_uint4(0u, 0u, 0u, 0u);
+                    fence_proxy_async_smem();
+                    __syncwarp();
+                }
+                if (j == 0) live = mbar_wait(bar_o_free, (n & 1) ^ 1, wctx, 64, n) && live;   // the previous item's O^T is in registers
+                live = mbar_wait(&bar_p_full[b], (J >> 1) & 1, wctx, 62 + b, j) && live;
+                __syncwarp();
+                tc_fence_after();
+                live = __all_sync(0xffffffffu, live);
+                if (!live) break;
+                issue_o(J, j == 0);
+                tc_commit(&bar_kv_empty[(2 * J + 1) % kStages]);
+                tc_commit(&bar_p_free[b]);   // P consumed; also: every MMA issued so far has completed
+            }
+            J0 += n_tiles;
         }
     }
     grid_let_next_start();
@@ -464,6 +526,7 @@ cudaError_t launch_gq(const AttnArgs& a, cudaStream_t st) {
     p.page_size = a.page_size;
     p.max_pages = a.max_pages;
     p.scale_log2 = a.scale * 1.4426950408889634f;
+    p.resident = 2 * sm_count();
     p.status = device_status_word();
     LaunchScope ls(K_DECODE_GQ, st);
     launch_overlapped(attn_decode_gq_sm100_kernel<kD, kG, kCache>, (unsigned)a.BH, kThreads, GqCfg<kD>::kSmemBytes, st, *reinterpret_cast<CUtensorMap*>(tq.bytes), *reinterpret_cast<CUtensorMap*>(tk.bytes),
