@@ -26,6 +26,7 @@
 // the streamed tiles have 32 rows: with 64, shared memory holds one tile of each tensor (every tile's load is exposed)
 // and the row threads' registers do not hold the accumulator row beside two rows of scores.
 #include "common.h"
+#include "f32_parts.cuh"
 #include "sm100_ptx.cuh"
 
 #include <algorithm>
@@ -72,25 +73,6 @@ struct F32Cfg {
     static_assert(kW + 3 * kWPart <= kAcc && kR0 + 3 * DP / 2 <= 512, "tensor memory");
     static_assert(kSmem <= 227 * 1024, "exceeds the shared memory of one CTA");
 };
-// x[0..7] -> three 16-byte groups of bf16
-__device__ __forceinline__ void split8(const float (&x)[8], uint4& h, uint4& m, uint4& l) {
-    uint32_t hh[4], mm[4], ll[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        float a = x[2 * i], b = x[2 * i + 1];
-        hh[i] = pack_bf16x2(a, b);
-        a -= __uint_as_float(hh[i] << 16);
-        b -= __uint_as_float(hh[i] & 0xffff0000u);
-        mm[i] = pack_bf16x2(a, b);
-        a -= __uint_as_float(mm[i] << 16);
-        b -= __uint_as_float(mm[i] & 0xffff0000u);
-        ll[i] = pack_bf16x2(a, b);
-    }
-    h = make_uint4(hh[0], hh[1], hh[2], hh[3]);
-    m = make_uint4(mm[0], mm[1], mm[2], mm[3]);
-    l = make_uint4(ll[0], ll[1], ll[2], ll[3]);
-}
-
 // ROWS x DP floats from row0 on of a [n_rows, D] matrix, 128 threads, 8 consecutive values per thread and step; what
 // lies past n_rows or D reads as zero.
 template <int DP, int ROWS>
@@ -126,10 +108,6 @@ struct TileRegs {
         }
     }
 };
-
-// The kept products, smallest first: (part of A, part of B).
-__host__ __device__ constexpr uint32_t term_a(int t) { return (0x001102u >> (4 * t)) & 3u; }
-__host__ __device__ constexpr uint32_t term_b(int t) { return (0x010120u >> (4 * t)) & 3u; }
 
 // One work item of one mode.
 struct F32Item {

@@ -55,3 +55,21 @@ def test_padded_keys(tt, oracle, D, lens):
                                 ("dv", dv[b:b + 1, :, :n], dv_r)):
             assert float(np.abs(got.cpu().numpy() - want).max()) <= TOL * max(float(np.abs(want).max()), 1.0), (name, n)
         assert float(dk[b, :, n:].abs().max() if n < L else 0.0) == 0.0 and float(dv[b, :, n:].abs().max() if n < L else 0.0) == 0.0
+
+
+def test_largest_finite_values(tt, oracle):
+    """A value next to the largest float keeps its size (its first bf16 part must not round to infinity), and takes no part
+    in the rows that the mask hides it from."""
+    S, D = 150, 64
+    q, k, v, _ = oracle.make_inputs(5, 1, 1, S, S, D)
+    big = np.finfo(np.float32).max
+    want = oracle.closed_form_f64(q, k, v, np.zeros_like(q), True)[0]
+    v[0, 0, S - 1] = -big
+    out, _ = tt.attention_forward(*(torch.from_numpy(x).cuda() for x in (q, k, v)), causal=True)
+    tt.check_device_status()
+    got = out.cpu().numpy()
+    assert float(np.abs(got[:, :, :S - 1] - want[:, :, :S - 1]).max()) <= TOL * max(float(np.abs(want).max()), 1.0)
+    s = (q[0, 0, S - 1].astype(np.float64) @ k[0, 0].T.astype(np.float64)) / np.sqrt(D)
+    p = np.exp(s - s.max())
+    last = -(p / p.sum())[S - 1] * float(big)
+    assert float(np.abs(got[0, 0, S - 1] / last - 1).max()) <= 1e-5
