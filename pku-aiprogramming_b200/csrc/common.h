@@ -91,6 +91,25 @@ cudaError_t launch_overlapped(void (*kernel)(P...), dim3 grid, dim3 block, size_
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
+// The same, as clusters of n_cta CTAs (the grid is a multiple of it).
+template <typename... P, typename... A>
+cudaError_t launch_overlapped_cluster(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, int n_cta, A&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = (unsigned)n_cta;
+    at[1].val.clusterDim.y = 1;
+    at[1].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = n_cta > 1 ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
 __device__ __forceinline__ void grid_let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void grid_wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

@@ -19,11 +19,13 @@
 //   warps 2-5   epilogue: accumulator (256 tensor-memory columns, double buffered so the next
 //               tile's MMAs run meanwhile) -> registers -> + bias -> bf16 -> global
 // Every wait is bounded (see sm100_ptx.cuh); an expired wait aborts the CTA through the common exit.
+#include <cooperative_groups.h>
 #include <cuda.h>
 
 #include <algorithm>
 
 #include "common.h"
+#include "fc_tiles.cuh"
 #include "sm100_ptx.cuh"
 
 namespace ttk {
@@ -37,17 +39,8 @@ constexpr int kBBytes = kBN * kBK * 2;          // 32 KB
 constexpr int kStageBytes = kABytes + kBBytes;  // 48 KB
 constexpr int kSubBytes = 64 * 128;             // one 64-wide MN-major sub-block: 64 K-rows x 128 B
 constexpr int kGemmSmem = kStages * kStageBytes + 1024 /*alignment slack*/ + 256 /*barriers*/;
-constexpr int kBandRows = 16;
-
-__device__ __forceinline__ void tile_coords(int t, int tiles_m, int tiles_n, int& mb, int& nb) {
-    const int per_band = kBandRows * tiles_n;
-    const int band = t / per_band;
-    const int first = band * kBandRows;
-    const int rows = min(kBandRows, tiles_m - first);
-    const int r = t - band * per_band;
-    mb = first + r % rows;
-    nb = r / rows;
-}
+constexpr int kSplitPitch = kBN + 4;             // floats; rows of a share's accumulator in shared memory
+static_assert(kBM * kSplitPitch * 4 <= kStages * kStageBytes, "a share's accumulator takes the ring's place");
 
 // One thread's accumulator row (256 fp32 columns of tensor memory starting at `taddr`) -> + bias -> bf16 ->
 // row `row` of C, columns n0...  Hands the accumulator buffer back (one arrival: on `acc_empty` of this CTA,
@@ -105,7 +98,11 @@ __device__ __forceinline__ void store_acc_row(uint32_t taddr, long long row, int
     }
 }
 
-template <bool kAMn, bool kBMn>
+// kSplit: launched as clusters, one output tile per cluster.  Each CTA sums its share of K; the shares' accumulators go to
+// shared memory (the ring is empty by then), and each CTA adds up its rows of the tile through distributed shared memory,
+// in rank order.  No workspace and no second launch, where few tiles over a long K (the weight gradient of a narrow layer)
+// would leave most SMs idle.
+template <bool kAMn, bool kBMn, bool kSplit>
 __global__ void __launch_bounds__(192, 1)
 fc_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                      __nv_bfloat16* __restrict__ C, const __nv_bfloat16* __restrict__ bias, int M, int N, int K,
@@ -151,16 +148,20 @@ fc_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     grid_let_next_start();
     grid_wait_for_previous();
 
+    namespace cg = cooperative_groups;
     const int total = tiles_m * tiles_n;
-    const int kblocks = (K + kBK - 1) / kBK;
+    const int n_cta = kSplit ? (int)cg::this_cluster().num_blocks() : 1, rank = kSplit ? (int)cg::this_cluster().block_rank() : 0;
+    const int t_first = kSplit ? (int)blockIdx.x / n_cta : (int)blockIdx.x, t_step = kSplit ? total : (int)gridDim.x;
+    const int all_blocks = (K + kBK - 1) / kBK, share = (all_blocks + n_cta - 1) / n_cta;
+    const int kb_first = rank * share, kblocks = max(0, min(share, all_blocks - kb_first));
 
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer
         int it = 0;
         bool live = true;
-        for (int t = blockIdx.x; t < total && live; t += gridDim.x) {
+        for (int t = t_first; t < total && live; t += t_step) {
             int mb, nb;
-            tile_coords(t, tiles_m, tiles_n, mb, nb);
+            fc_tile_coords(t, tiles_m, tiles_n, mb, nb);
             const int m0 = mb * kBM, n0 = nb * kBN;
             for (int kb = 0; kb < kblocks; ++kb, ++it) {
                 const int s = it % kStages;
@@ -172,7 +173,7 @@ fc_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                 if (elect_one()) {
                     unsigned char* sA = smem + s * kStageBytes;
                     unsigned char* sB = sA + kABytes;
-                    const int k0 = kb * kBK;
+                    const int k0 = (kb_first + kb) * kBK;
                     mbar_arrive_expect_tx(&full[s], kStageBytes);
                     if (kAMn) {
                         tma_load_3d(sA, &tmA, &full[s], m0, k0, 0);
@@ -197,7 +198,7 @@ fc_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         constexpr uint32_t b_step = kBMn ? 2048u : 32u;
         int it = 0, lt = 0;
         bool live = true;
-        for (int t = blockIdx.x; t < total && live; t += gridDim.x, ++lt) {
+        for (int t = t_first; t < total && live; t += t_step, ++lt) {
             const int buf = lt & 1;
             const uint32_t use = (uint32_t)(lt >> 1) & 1u;
             if (!__all_sync(0xffffffffu, mbar_wait(&acc_empty[buf], use ^ 1u, wctx, 30 + buf, lt))) break;
@@ -230,13 +231,26 @@ fc_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         const int lane_group = warp & 3;                 // tensor-memory lanes 32*lane_group .. +31
         const uint32_t lane_off = (uint32_t)(lane_group * 32) << 16;
         int lt = 0;
-        for (int t = blockIdx.x; t < total; t += gridDim.x, ++lt) {
+        for (int t = t_first; t < total; t += t_step, ++lt) {
             int mb, nb;
-            tile_coords(t, tiles_m, tiles_n, mb, nb);
+            fc_tile_coords(t, tiles_m, tiles_n, mb, nb);
             const int buf = lt & 1;
             const uint32_t use = (uint32_t)(lt >> 1) & 1u;
             if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[buf], use, wctx, 40 + buf, lt))) break;
             tc_fence_after();
+            if (kSplit) {
+                float* dst = reinterpret_cast<float*>(smem) + (lane_group * 32 + lane) * kSplitPitch;
+#pragma unroll 1
+                for (int c = 0; c < kBN; c += 32) {
+                    uint32_t v[32];
+                    tmem_ld32(tmem_base + lane_off + (uint32_t)c, v);
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int e = 0; e < 32; e += 4)   // a share without blocks has no accumulator
+                        *reinterpret_cast<uint4*>(dst + c + e) = kblocks > 0 ? make_uint4(v[e], v[e + 1], v[e + 2], v[e + 3]) : make_uint4(0u, 0u, 0u, 0u);
+                }
+                break;
+            }
             const long long row = (long long)mb * kBM + lane_group * 32 + lane;
             store_acc_row<false>(tmem_base + lane_off + (uint32_t)(buf * kBN), row, nb * kBN, C, bias, M, N, wide,
                                  &acc_empty[buf], 0u);
@@ -247,6 +261,32 @@ fc_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     if (warp == 0) {
         tc_fence_after();
         tmem_dealloc(tmem_base, 512);
+    }
+    if (kSplit) {
+        cg::cluster_group cluster = cg::this_cluster();
+        cluster.sync();   // every share's accumulator is in shared memory
+        int mb, nb;
+        fc_tile_coords(t_first, tiles_m, tiles_n, mb, nb);
+        const int rows = kBM / n_cta;
+        float* tile = reinterpret_cast<float*>(smem);
+        for (int i = threadIdx.x; i < rows * (kBN / 8); i += 192) {
+            const int r = rank * rows + i / (kBN / 8), c = (i % (kBN / 8)) * 8, m = mb * kBM + r, n = nb * kBN + c;
+            if (m >= M || n >= N) continue;   // N % 8 == 0: a group of 8 columns is inside or outside as a whole
+            float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            for (int q = 0; q < n_cta; ++q) {
+                const float4* x = reinterpret_cast<const float4*>(cluster.map_shared_rank(tile, q) + r * kSplitPitch + c);
+                const float4 x0 = x[0], x1 = x[1];
+                v[0] += x0.x; v[1] += x0.y; v[2] += x0.z; v[3] += x0.w;
+                v[4] += x1.x; v[5] += x1.y; v[6] += x1.z; v[7] += x1.w;
+            }
+            if (bias) {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) v[e] += __bfloat162float(bias[n + e]);
+            }
+            *reinterpret_cast<uint4*>(C + (long long)m * N + n) = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
+        }
+        __syncwarp();
+        cluster.sync();   // a peer may still be reading this CTA's share
     }
 }
 
@@ -321,7 +361,7 @@ fc_gemm_pair_sm100_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
         bool live = true;
         for (int t = pair; t < total && live; t += n_pairs) {
             int mb, nb;
-            tile_coords(t, tiles_m, tiles_n, mb, nb);
+            fc_tile_coords(t, tiles_m, tiles_n, mb, nb);
             const int m0 = mb * 256 + (int)rank * 128, n0 = nb * 256 + (int)rank * 128;
             for (int kb = 0; kb < kblocks; ++kb, ++it) {
                 const int s = it % kPStages;
@@ -400,7 +440,7 @@ fc_gemm_pair_sm100_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
         int lt = 0;
         for (int t = pair; t < total; t += n_pairs, ++lt) {
             int mb, nb;
-            tile_coords(t, tiles_m, tiles_n, mb, nb);
+            fc_tile_coords(t, tiles_m, tiles_n, mb, nb);
             const int buf = lt & 1;
             const uint32_t use = (uint32_t)(lt >> 1) & 1u;
             if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[buf], use, wctx, 40 + buf, lt))) break;
@@ -533,15 +573,21 @@ cudaError_t launch_tc(const void* A, const void* B, void* C, const void* bias, i
         return cudaErrorInvalidValue;
     if (!make_tmap_bf16(&tb, B, kBMn ? (uint64_t)N : (uint64_t)K, kBMn ? (uint64_t)K : (uint64_t)N, 1, kBMn ? 64 : kBN, &why))
         return cudaErrorInvalidValue;
-    cudaError_t e = TT_ALLOW_SMEM((fc_gemm_sm100_kernel<kAMn, kBMn>), kGemmSmem);
-    if (e != cudaSuccess) return e;
     const int tiles_m = (M + kBM - 1) / kBM, tiles_n = (N + kBN - 1) / kBN;
-    const int grid = std::min(tiles_m * tiles_n, sm_count());
+    const int wide = ((reinterpret_cast<uintptr_t>(C) & 31) == 0 && N % 16 == 0) ? 1 : 0;   // 32-byte stores possible
+    const CUtensorMap &ma = *reinterpret_cast<CUtensorMap*>(ta.bytes), &mb = *reinterpret_cast<CUtensorMap*>(tb.bytes);
     LaunchScope ls(K_FC_GEMM, st);
-    launch_overlapped(fc_gemm_sm100_kernel<kAMn, kBMn>, grid, 192, kGemmSmem, st, *reinterpret_cast<CUtensorMap*>(ta.bytes), *reinterpret_cast<CUtensorMap*>(tb.bytes), (__nv_bfloat16*)C,
-        (const __nv_bfloat16*)bias, M, N, K, tiles_m, tiles_n,
-        ((reinterpret_cast<uintptr_t>(C) & 31) == 0 && N % 16 == 0) ? 1 : 0,   // 32-byte stores possible
-        device_status_word());
+    const int n_cta = fc_k_ctas((long long)tiles_m * tiles_n, (K + kBK - 1) / kBK);
+    if (n_cta > 1) {
+        const cudaError_t e = TT_ALLOW_SMEM((fc_gemm_sm100_kernel<kAMn, kBMn, true>), kGemmSmem);
+        if (e != cudaSuccess) return e;
+        return launch_overlapped_cluster(fc_gemm_sm100_kernel<kAMn, kBMn, true>, (unsigned)(tiles_m * tiles_n * n_cta), 192, kGemmSmem, st, n_cta,
+                                         ma, mb, (__nv_bfloat16*)C, (const __nv_bfloat16*)bias, M, N, K, tiles_m, tiles_n, wide, device_status_word());
+    }
+    const cudaError_t e = TT_ALLOW_SMEM((fc_gemm_sm100_kernel<kAMn, kBMn, false>), kGemmSmem);
+    if (e != cudaSuccess) return e;
+    launch_overlapped(fc_gemm_sm100_kernel<kAMn, kBMn, false>, std::min(tiles_m * tiles_n, sm_count()), 192, kGemmSmem, st, ma, mb,
+                      (__nv_bfloat16*)C, (const __nv_bfloat16*)bias, M, N, K, tiles_m, tiles_n, wide, device_status_word());
     return cudaGetLastError();
 }
 
