@@ -208,8 +208,9 @@ int tt_softmax_bwd(const void* y, const void* dy, void* dx, int64_t rows, int32_
  * of src/Layers.cu:42-79: dx = dy . w^T, dw = x^T . dy, db = column sums of dy (db_scalar != 0:
  * one value, the sum over all of dy, for the reference's single-value bias); each of dx, dw, db
  * may be NULL and is then skipped.  bf16 with in % 8 == 0 and out % 8 == 0 runs the tcgen05
- * kernel (fp32 accumulation), float and other shapes an fp32 SIMT kernel; tt_fc_path says
- * which (1 = tensor cores).  The workspace is only needed for db. */
+ * kernel (fp32 accumulation), float of any shape a tcgen05 kernel on three bf16 parts per value,
+ * other shapes an fp32 SIMT kernel; tt_fc_path says which (1 = tensor cores).  The workspace is only
+ * needed for db. */
 int tt_fc_fwd(const void* x, const void* w, const void* bias, void* y, int64_t rows, int32_t in_features,
               int32_t out_features, int32_t dtype, void* stream);
 size_t tt_fc_bwd_workspace_bytes(int64_t rows, int32_t in_features, int32_t out_features, int32_t dtype);

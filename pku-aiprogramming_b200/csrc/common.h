@@ -190,11 +190,15 @@ cudaError_t softmax_rows_bwd(const void* y, const void* dy, void* dx, long long 
 // --- fully connected layer: C[M,N] = op(A) op(B) (+ bias[N]), row-major, fp32 accumulation.
 //   a_mn = 0: A stored [M,K];  a_mn = 1: A stored [K,M] (the product uses its transpose)
 //   b_mn = 1: B stored [K,N];  b_mn = 0: B stored [N,K] (the product uses its transpose)
-// bf16 with 16-byte row pitches runs the tcgen05 kernel, everything else the fp32 SIMT kernel.
+// bf16 with 16-byte row pitches and floats run on the tensor cores, everything else the fp32 SIMT kernel.
 bool fc_gemm_tc_supported(const void* A, const void* B, const void* C, const void* bias, long long M, int N, int K,
                           int a_mn, int b_mn, int bf16);
 cudaError_t fc_gemm(const void* A, const void* B, void* C, const void* bias, long long M, int N, int K, int a_mn,
                     int b_mn, int bf16, cudaStream_t st);
+// float tensors on the tensor cores, three bf16 parts per value (fc_f32_sm100.cu)
+bool fc_f32_tc_supported(long long M, int N, int K, int a_mn, int b_mn, int bf16);
+cudaError_t fc_gemm_f32_sm100(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, int a_mn, int b_mn,
+                              cudaStream_t st);
 // out[n] = sum over rows of X[M,N] (scalar_bias: out[0] = sum of everything); workspace of
 // fc_colsum_workspace(M, N) bytes holds the per-range partial sums.
 size_t fc_colsum_workspace(long long M, int N);

@@ -672,6 +672,7 @@ cudaError_t fc_gemm(const void* A, const void* B, void* C, const void* bias, lon
         if (a_mn && b_mn) return launch_tc<true, true>(A, B, C, bias, (int)M, N, K, st);
         return launch_tc<true, false>(A, B, C, bias, (int)M, N, K, st);
     }
+    if (fc_f32_tc_supported(M, N, K, a_mn, b_mn, bf16)) return fc_gemm_f32_sm100(A, B, C, bias, (int)M, N, K, a_mn, b_mn, st);
     dim3 grid((unsigned)((N + 63) / 64), (unsigned)((M + 63) / 64));
     if (grid.y > 65535u) return cudaErrorInvalidValue;
     LaunchScope ls(K_FC_SIMT, st);

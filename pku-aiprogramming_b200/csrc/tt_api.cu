@@ -794,6 +794,7 @@ int tt_fc_bwd(const void* x, const void* w, const void* dy, void* dx, void* dw, 
 }
 int tt_fc_path(int64_t rows, int32_t in_features, int32_t out_features, int32_t dtype) {
     // alignment of the pointers is checked at the call; pools and torch hand out >= 256-byte alignment
+    if (dtype == TT_F32) return fc_f32_tc_supported(rows, out_features, in_features, 0, 1, 0) ? 1 : 0;
     return fc_gemm_tc_supported(nullptr, nullptr, nullptr, nullptr, rows, out_features, in_features, 0, 1, dtype == TT_BF16) &&
                    fc_gemm_tc_supported(nullptr, nullptr, nullptr, nullptr, in_features, out_features, (int)rows, 1, 1, dtype == TT_BF16)
                ? 1 : 0;

@@ -1,7 +1,9 @@
-"""The fully connected layer where its kernels cut K among the CTAs of a cluster (fc_gemm_sm100.cu), against float64.
+"""The fully connected layer where its kernels cut K among the CTAs of a cluster (fc_gemm_sm100.cu, fc_f32_sm100.cu), and float
+tensors on the tensor cores as three bf16 parts, against float64.
 
 Bounds.  bf16: inputs are exact, sums are float32, the result is rounded once: 2^-8 of the value plus the sums' rounding, below
-2^-20 of the row's sum of magnitudes."""
+2^-20 of the row's sum of magnitudes.  Float: a product loses below 2^-23 to the terms left out, a chunk of 64 a few units of
+2^-23 to truncating additions, chunks are added in float32: 2^-20 of the sum of magnitudes covers it (K up to 64 chunks)."""
 import numpy as np
 import pytest
 
@@ -28,3 +30,39 @@ def test_bf16_cut_along_k(tt, rows, fin, fout):
     g = torch.Generator(device="cuda").manual_seed(rows + fin)
     n = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
     check(tt, n(rows, fin), n(fin, fout), n(fout), n(rows, fout), 2.0 ** -8)
+
+
+# pitches that are and are not multiples of 4 and 8, tile and chunk edges, one CTA per tile and clusters
+@pytest.mark.parametrize("rows,fin,fout", [(128, 128, 128), (129, 65, 127), (640, 333, 130), (64, 1000, 36), (33, 4095, 11), (4099, 129, 260),
+                                           (1500, 1500, 1028), (1, 3, 1)])
+def test_float_parts(tt, rows, fin, fout):
+    g = torch.Generator(device="cuda").manual_seed(rows + fin)
+    n = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    check(tt, n(rows, fin), n(fin, fout), n(fout), n(rows, fout), 2.0 ** -23)
+
+
+def test_float_pointers_off_16_bytes(tt):
+    g = torch.Generator(device="cuda").manual_seed(1)
+    n = lambda r, c: torch.randn(r * c + 1, generator=g, device="cuda")[1:].view(r, c)
+    check(tt, n(200, 256), n(256, 132), torch.randn(132, generator=g, device="cuda"), n(200, 132), 2.0 ** -23)
+
+
+def test_float_extremes(tt):
+    """The largest finite float keeps its value; infinities and NaN give what plain additions and multiplications give, in
+    their rows and columns only."""
+    x = torch.ones(300, 200, device="cuda")
+    w = torch.full((200, 140), 2.0 ** -10, device="cuda")
+    big = torch.finfo(torch.float32).max
+    x[3, 5], x[4, 6] = big, -big
+    y = tt.fc_forward(x, w)
+    assert torch.allclose(y.double(), x.double() @ w.double(), rtol=1e-6, atol=0)
+    x[150, 7], x[151, 8], x[152, 9] = float("inf"), float("-inf"), float("nan")
+    w[0, 139] = float("inf")
+    y = tt.fc_forward(x, w)
+    tt.check_device_status()
+    want = x.double() @ w.double()
+    assert torch.equal(torch.isnan(y), torch.isnan(want))
+    ok = ~torch.isnan(want)
+    assert torch.equal(torch.isinf(y)[ok], torch.isinf(want)[ok]) and torch.equal(torch.sign(y)[ok].double(), torch.sign(want)[ok])
+    fin = torch.isfinite(want)
+    assert torch.allclose(y.double()[fin], want[fin], rtol=1e-6, atol=0)
