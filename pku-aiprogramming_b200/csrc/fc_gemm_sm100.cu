@@ -519,36 +519,64 @@ __global__ void __launch_bounds__(256) fc_gemm_simt_kernel(const T* __restrict__
     }
 }
 
-// Column sums of a row-major [M,N] matrix: partial[split][n] over a fixed row range per split,
-// then a second pass adds the splits in order (deterministic).
-template <typename T>
+// Column sums of a row-major [M,N] matrix: partial[split][n] over a fixed row range per split, then a second pass adds
+// the splits in order (deterministic).  A warp reads 32 x kV consecutive values of a row (16 bytes per lane where
+// the pitch allows it), four rows in flight per thread; 8 warps take every eighth row each.
+template <typename T, int kV>
+__device__ __forceinline__ void add_values(const T* p, float (&s)[kV]) {
+    if constexpr (kV == 1) {
+        s[0] += g_ld<T>(p, 0);
+    } else {
+        const uint4 v = __ldg(reinterpret_cast<const uint4*>(p));
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if constexpr (sizeof(T) == 2) {
+                s[2 * i] += __uint_as_float(w[i] << 16);
+                s[2 * i + 1] += __uint_as_float(w[i] & 0xffff0000u);
+            } else {
+                s[i] += __uint_as_float(w[i]);
+            }
+        }
+    }
+}
+template <typename T, int kV>
 __global__ void __launch_bounds__(256) colsum_partial_kernel(const T* __restrict__ X, float* __restrict__ partial,
                                                             long long M, int N, int rows_per_split) {
     grid_let_next_start();
     grid_wait_for_previous();
-    const int col = blockIdx.x * 64 + (threadIdx.x & 63);
-    const int sub = threadIdx.x >> 6;   // 4 row phases per CTA
+    __shared__ float red[8][32 * kV];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int col0 = blockIdx.x * 32 * kV, col = col0 + lane * kV;
     const long long r0 = (long long)blockIdx.y * rows_per_split;
     const long long r1 = min(M, r0 + rows_per_split);
-    float s = 0.f;
-    if (col < N)
-        for (long long r = r0 + sub; r < r1; r += 4) s += g_ld<T>(X, r * N + col);
-    __shared__ float red[4][64];
-    red[sub][threadIdx.x & 63] = s;
+    float s[kV] = {};
+    if (col < N) {   // kV > 1: N is a multiple of it
+#pragma unroll 4
+        for (long long r = r0 + warp; r < r1; r += 8) add_values<T, kV>(X + r * N + col, s);
+    }
+#pragma unroll
+    for (int e = 0; e < kV; ++e) red[warp][lane * kV + e] = s[e];
     __syncthreads();
-    if (sub == 0 && col < N)
-        partial[(long long)blockIdx.y * N + col] = red[0][threadIdx.x] + red[1][threadIdx.x] + red[2][threadIdx.x] + red[3][threadIdx.x];
+    for (int c = threadIdx.x; c < 32 * kV && col0 + c < N; c += 256) {
+        float v = red[0][c];
+#pragma unroll
+        for (int w = 1; w < 8; ++w) v += red[w][c];
+        partial[(long long)blockIdx.y * N + col0 + c] = v;
+    }
 }
+// A warp adds every eighth split of 32 columns.
 template <typename T>
-__global__ void colsum_final_kernel(const float* __restrict__ partial, T* __restrict__ out, int N, int splits,
-                                    int scalar_bias) {
+__global__ void __launch_bounds__(256) colsum_final_kernel(const float* __restrict__ partial, T* __restrict__ out, int N, int splits,
+                                                          int scalar_bias) {
     grid_let_next_start();
     grid_wait_for_previous();
+    __shared__ float red[256];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    float s = 0.f;
     if (scalar_bias) {   // one CTA: the reference's single-value bias gets the sum over all columns too
-        __shared__ float red[256];
-        float s = 0.f;
-        for (int n = threadIdx.x; n < N; n += 256)
-            for (int p = 0; p < splits; ++p) s += partial[(long long)p * N + n];
+        const long long values = (long long)splits * N;
+        for (long long i = threadIdx.x; i < values; i += 256) s += partial[i];
         red[threadIdx.x] = s;
         __syncthreads();
         for (int o = 128; o > 0; o >>= 1) {
@@ -558,11 +586,18 @@ __global__ void colsum_final_kernel(const float* __restrict__ partial, T* __rest
         if (threadIdx.x == 0) g_st<T>(out, 0, red[0]);
         return;
     }
-    const int n = blockIdx.x * 256 + threadIdx.x;
-    if (n >= N) return;
-    float s = 0.f;
-    for (int p = 0; p < splits; ++p) s += partial[(long long)p * N + n];
-    g_st<T>(out, n, s);
+    const int n = blockIdx.x * 32 + lane;
+    if (n < N) {
+#pragma unroll 4
+        for (int p = warp; p < splits; p += 8) s += partial[(long long)p * N + n];
+    }
+    red[threadIdx.x] = s;
+    __syncthreads();
+    if (warp == 0 && n < N) {
+#pragma unroll
+        for (int w = 1; w < 8; ++w) s += red[w * 32 + lane];
+        g_st<T>(out, n, s);
+    }
 }
 
 template <bool kAMn, bool kBMn>
@@ -685,24 +720,34 @@ cudaError_t fc_gemm(const void* A, const void* B, void* C, const void* bias, lon
     return cudaGetLastError();
 }
 
-int fc_colsum_splits(long long M) { return (int)std::max<long long>(1, std::min<long long>(64, (M + 255) / 256)); }
-size_t fc_colsum_workspace(long long M, int N) { return align256((size_t)fc_colsum_splits(M) * (size_t)N * sizeof(float)); }
+// Row ranges: about four CTAs of 256 columns per SM, each of at least 64 rows (eight per warp).
+static int fc_colsum_splits(long long M, int N) {
+    const long long blocks = (N + 255) / 256, most = std::max(1LL, (4LL * sm_count() + blocks - 1) / blocks);
+    return (int)std::max(1LL, std::min(std::min(most, 256LL), M / 64));
+}
+size_t fc_colsum_workspace(long long M, int N) { return align256((size_t)fc_colsum_splits(M, N) * (size_t)N * sizeof(float)); }
 
+template <typename T>
+static cudaError_t launch_colsum_partial(const void* X, float* partial, long long M, int N, int splits, cudaStream_t st) {
+    constexpr int kV = 16 / sizeof(T);
+    const int rows = (int)((M + splits - 1) / splits);
+    if (N % kV == 0 && ((uintptr_t)X & 15) == 0)
+        return launch_overlapped(colsum_partial_kernel<T, kV>, dim3((unsigned)((N + 32 * kV - 1) / (32 * kV)), (unsigned)splits), 256, 0, st,
+                                 (const T*)X, partial, M, N, rows);
+    return launch_overlapped(colsum_partial_kernel<T, 1>, dim3((unsigned)((N + 31) / 32), (unsigned)splits), 256, 0, st, (const T*)X, partial, M, N, rows);
+}
 cudaError_t fc_colsum(const void* X, void* out, long long M, int N, int bf16, int scalar_bias, void* workspace,
                       cudaStream_t st) {
-    const int splits = fc_colsum_splits(M);
-    const int rows_per_split = (int)((M + splits - 1) / splits);
+    const int splits = fc_colsum_splits(M, N);
     float* partial = (float*)workspace;
-    dim3 grid((unsigned)((N + 63) / 64), (unsigned)splits);
     {
         LaunchScope ls(K_FC_COLSUM, st);
-        if (bf16) launch_overlapped(colsum_partial_kernel<__nv_bfloat16>, grid, 256, 0, st, (const __nv_bfloat16*)X, partial, M, N, rows_per_split);
-        else launch_overlapped(colsum_partial_kernel<float>, grid, 256, 0, st, (const float*)X, partial, M, N, rows_per_split);
-        cudaError_t e = cudaGetLastError();
+        const cudaError_t e = bf16 ? launch_colsum_partial<__nv_bfloat16>(X, partial, M, N, splits, st)
+                                   : launch_colsum_partial<float>(X, partial, M, N, splits, st);
         if (e != cudaSuccess) return e;
     }
     LaunchScope ls(K_FC_COLSUM, st, false);
-    const unsigned fgrid = scalar_bias ? 1u : (unsigned)((N + 255) / 256);
+    const unsigned fgrid = scalar_bias ? 1u : (unsigned)((N + 31) / 32);
     if (bf16) launch_overlapped(colsum_final_kernel<__nv_bfloat16>, fgrid, 256, 0, st, partial, (__nv_bfloat16*)out, N, splits, scalar_bias);
     else launch_overlapped(colsum_final_kernel<float>, fgrid, 256, 0, st, partial, (float*)out, N, splits, scalar_bias);
     return cudaGetLastError();
