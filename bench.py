@@ -643,8 +643,8 @@ def run_fc(tt, dev, peaks, M=16384):
 
 
 def run_fp32(tt, dev, peaks):
-    """The reference's own dtype: fp32 causal forward+backward on the SIMT kernels (true fp32 FMAs;
-    the 1e-5 tolerance rules out the tensor-core formats), Q/K/V [2,8,2048,64].  Reported beside
+    """The reference's own dtype: fp32 causal forward+backward (three bf16 parts per value on the tensor cores,
+    which hold its 1e-5 tolerance), Q/K/V [2,8,2048,64].  Reported beside
     the bf16 step so that the cost of staying in fp32 is visible; not part of the step metric."""
     import torch
     try:
@@ -686,7 +686,7 @@ def main():
     ap.add_argument("--softmax-rows", type=int, default=262144, help="rows of the row-softmax leg")
     ap.add_argument("--no-fc", action="store_true", help="skip the fully connected layer leg at N=1")
     ap.add_argument("--no-softmax", action="store_true", help="skip the row-softmax leg at N=1")
-    ap.add_argument("--no-fp32", action="store_true", help="skip the fp32 (SIMT kernels) side measurement at N=1")
+    ap.add_argument("--no-fp32", action="store_true", help="skip the fp32 side measurement at N=1")
     ap.add_argument("--no-varlen", action="store_true", help="skip the packed variable-length side measurement at N=1")
     ap.add_argument("--no-cfg3", action="store_true", help="skip the S=4096 side measurement at N=1")
     ap.add_argument("--no-cfg2", action="store_true", help="skip the S=1024, D=64 side measurement at N=1")
