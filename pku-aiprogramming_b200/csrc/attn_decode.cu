@@ -24,7 +24,7 @@ namespace ttk {
 constexpr int kDecThreads = 256;
 constexpr int kDecWarps = kDecThreads / 32;
 constexpr int kUnroll = 4;
-constexpr int kMaxRanges = 128;   // key ranges per slice of the tensor-core routes
+constexpr int kMaxRanges = 128;   // key ranges per slice of the keys-on-rows route (a group above 16 can have more)
 
 __device__ __forceinline__ uint4 ld_stream16(const void* p) {
     uint4 r;
@@ -270,15 +270,13 @@ static bool decode_group_instantiated(int g) { return g == 1 || g == 2 || g == 4
 
 // Grouped heads on a dense cache, as a tensor-core problem: the G query heads of a key/value head
 // are contiguous in q [B, Hkv*G, 1, D], i.e. they ARE a [B, Hkv, G, D] tensor of G query rows per
-// key/value head, and out / lse have the matching layout.  The forward kernel then computes the
-// whole group against each K/V tile with two MMAs, which the SIMT kernel cannot keep up with from
+// key/value head, and out / lse have the matching layout.  The SIMT kernel cannot keep up with that from
 // G = 4 on (it is instruction-bound: G dot products and G softmax updates per loaded row).
-// With fewer (batch, key/value head) items than SMs the keys are split as well: K and V viewed as
-// [slices * splits, L / splits, D] are `splits` independent problems per slice (the forward kernel
-// reads the query rows of slice s / splits), whose normalised partial outputs and log-sum-exps a
-// second kernel merges.
-// The forward view of a grouped decode runs on the keys-on-rows decode kernel where that takes it (head
-// dim 128, groups of up to 16), else on the general forward kernel.
+// With few (batch, key/value head) items the keys are split as well, and a second kernel merges the ranges' normalised
+// partial outputs and log-sum-exps:
+//   groups up to 16 (head dim 64 or 128): the keys-on-rows decode kernel, ranges of whole 128-key tiles behind a key offset;
+//   larger groups: the general forward kernel on K and V viewed as [slices * splits, L / splits, D], `splits` independent
+//     problems per slice (it reads the query rows of slice s / splits); paged caches in ranges of whole 128-key tiles.
 static cudaError_t run_forward_view(const AttnArgs& g, cudaStream_t st) {
     return attn_decode_gq_sm100_supported(g) ? attn_decode_gq_sm100(g, st) : attn_fwd_sm100(g, st);
 }
@@ -396,13 +394,15 @@ __device__ __forceinline__ float4 ld_partial4(const __nv_bfloat16* p) {
 // Merge of normalised per-range results: out[bh] = sum_c w_c O_c / sum_c w_c with w_c = exp(lse_c - max lse);
 // partial O is [kvs, splits, G, D], partial lse [kvs, splits, G].  One CTA per output row: D / 4 threads share a
 // range's row, so 128 threads have 4 (D = 128) or 8 ranges in flight each with `kAhead` loads, the first ones issued
-// before the weights are known.  What bounds it is latency, not bytes.
+// before the weights are known.  What bounds it is latency, not bytes.  Any number of ranges: the weights are in
+// dynamic shared memory, one float each; up to kBatch log-sum-exps stay in the first warp's registers between the
+// maximum and the weights, more are read again.
 template <int D, typename T>
 __global__ void __launch_bounds__(128) attn_decode_tc_merge_kernel(const T* __restrict__ po, const float* __restrict__ plse,
                                                                   __nv_bfloat16* __restrict__ out, float* __restrict__ lse,
                                                                   int splits, int G) {
-    constexpr int kLanes = D / 4, kRows = 128 / kLanes, kAhead = 4;
-    __shared__ float sm_w[kMaxRanges];
+    constexpr int kLanes = D / 4, kRows = 128 / kLanes, kAhead = 4, kBatch = 128;
+    extern __shared__ float sm_w[];   // [splits]
     __shared__ float sm_o[kRows][D];
     grid_let_next_start();
     grid_wait_for_previous();
@@ -420,25 +420,34 @@ __global__ void __launch_bounds__(128) attn_decode_tc_merge_kernel(const T* __re
     };
     load(r0);
     if (tid < 32) {
-        float y[kMaxRanges / 32], m = -INFINITY, den = 0.f;
+        float y[kBatch / 32], m = -INFINITY, den = 0.f;
+        auto load_lse = [&](int base) {
 #pragma unroll
-        for (int i = 0; i < kMaxRanges / 32; ++i) {
-            const int c = tid + 32 * i;
-            y[i] = c < splits ? plse[(kvs * splits + c) * G + g] : -INFINITY;
-            m = fmaxf(m, y[i]);
+            for (int i = 0; i < kBatch / 32; ++i) {
+                const int c = base + tid + 32 * i;
+                y[i] = c < splits ? plse[(kvs * splits + c) * G + g] : -INFINITY;
+            }
+        };
+        for (int base = 0; base < splits; base += kBatch) {
+            load_lse(base);
+#pragma unroll
+            for (int i = 0; i < kBatch / 32; ++i) m = fmaxf(m, y[i]);
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        for (int base = 0; base < splits; base += kBatch) {
+            if (splits > kBatch) load_lse(base);
 #pragma unroll
-        for (int i = 0; i < kMaxRanges / 32; ++i) {
-            y[i] = y[i] == -INFINITY ? 0.f : expf(y[i] - m);   // a range without keys (all of them: m = -inf) has no weight
-            den += y[i];
+            for (int i = 0; i < kBatch / 32; ++i) {
+                y[i] = y[i] == -INFINITY ? 0.f : expf(y[i] - m);   // a range without keys (all of them: m = -inf) has no weight
+                den += y[i];
+                if (base + tid + 32 * i < splits) sm_w[base + tid + 32 * i] = y[i];
+            }
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) den += __shfl_xor_sync(0xffffffffu, den, o);
         const float inv = den > 0.f || den != den ? 1.f / den : 0.f;
-#pragma unroll
-        for (int i = 0; i < kMaxRanges / 32; ++i) sm_w[tid + 32 * i] = y[i] * inv;
+        for (int c = tid; c < splits; c += 32) sm_w[c] *= inv;
         if (tid == 0 && lse != nullptr) lse[bh] = m == -INFINITY ? -INFINITY : m + logf(den);
     }
     __syncthreads();
@@ -465,12 +474,13 @@ __global__ void __launch_bounds__(128) attn_decode_tc_merge_kernel(const T* __re
     }
 }
 template <typename T>
-static void launch_tc_merge(const AttnArgs& a, const T* po, const float* plse, int splits, cudaStream_t st) {
+static cudaError_t launch_tc_merge(const AttnArgs& a, const T* po, const float* plse, int splits, cudaStream_t st) {
+    const size_t smem = (size_t)splits * sizeof(float);
+    if (smem > 40 * 1024) return cudaErrorInvalidValue;   // (the split rules stay below 2 ranges per SM)
     LaunchScope ls(K_DECODE_MERGE, st);
     if (a.D == 128)
-        launch_overlapped(attn_decode_tc_merge_kernel<128, T>, (unsigned)a.BH, 128, 0, st, po, plse, (__nv_bfloat16*)a.out, a.lse, splits, a.group);
-    else
-        launch_overlapped(attn_decode_tc_merge_kernel<64, T>, (unsigned)a.BH, 128, 0, st, po, plse, (__nv_bfloat16*)a.out, a.lse, splits, a.group);
+        return launch_overlapped(attn_decode_tc_merge_kernel<128, T>, (unsigned)a.BH, 128, smem, st, po, plse, (__nv_bfloat16*)a.out, a.lse, splits, a.group);
+    return launch_overlapped(attn_decode_tc_merge_kernel<64, T>, (unsigned)a.BH, 128, smem, st, po, plse, (__nv_bfloat16*)a.out, a.lse, splits, a.group);
 }
 // Runs the forward view `g` of decode `a`, several key ranges per slice, and merges their results.
 static cudaError_t run_ranges(const AttnArgs& a, AttnArgs g, int splits, void* ws, cudaStream_t st) {
@@ -479,9 +489,8 @@ static cudaError_t run_ranges(const AttnArgs& a, AttnArgs g, int splits, void* w
     g.lse = plse;
     const cudaError_t e = run_forward_view(g, st);
     if (e != cudaSuccess) return e;
-    if (attn_decode_gq_sm100_supported(g)) launch_tc_merge(a, (const float*)ws, plse, splits, st);
-    else launch_tc_merge(a, (const __nv_bfloat16*)ws, plse, splits, st);
-    return cudaGetLastError();
+    if (attn_decode_gq_sm100_supported(g)) return launch_tc_merge(a, (const float*)ws, plse, splits, st);
+    return launch_tc_merge(a, (const __nv_bfloat16*)ws, plse, splits, st);
 }
 
 template <int D, int G>
