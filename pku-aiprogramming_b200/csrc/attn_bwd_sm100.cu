@@ -176,11 +176,10 @@ attn_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmR0, const __grid_con
     tc_fence_after();
     const uint32_t tmem_base = *tmem_base_slot;
     WaitCtx wctx{p.status, abort_flag, warp};
-    // The dK/dV pass lets the dQ pass start only behind its own wait, i.e. when the statistics are complete; the
-    // dQ pass needs nothing else, so its CTAs begin to work as the dK/dV pass's last CTAs leave the SMs, and it
-    // waits for that pass at its END (what follows on the stream may rely on both).
-    if (kKeysResident) grid_wait_for_previous();
+    // Both passes: a grid that does not wait itself is promised nothing of what ran before, so the dQ pass waits for the
+    // whole dK/dV pass although it reads only the statistics and the inputs.
     grid_let_next_start();
+    grid_wait_for_previous();
     constexpr uint32_t kColS = 0, kColDP = 128, kColAcc0 = 256, kColAcc1 = 256 + D;
 
     auto next_item = [&](int k) -> int {
@@ -678,7 +677,6 @@ attn_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmR0, const __grid_con
         tc_fence_after();
         tmem_dealloc(tmem_base, Cfg::kTmemCols);
     }
-    if (!kKeysResident) grid_wait_for_previous();
 }
 
 // ---------------------------------------------------------------- preprocessing
