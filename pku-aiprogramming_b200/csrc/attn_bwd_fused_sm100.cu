@@ -145,8 +145,7 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
     const int off = p.L - p.S;
 
     if (threadIdx.x == 0) {
-        // a CTA that the hardware starts after another one's wait has given up leaves at once
-        *abort_flag = ((int)blockIdx.x >= p.first_wave && *reinterpret_cast<volatile unsigned int*>(p.status) != 0u) ? 1 : 0;
+        *abort_flag = 0;
         mbar_init(bar_steal, 1);
         mbar_init(bar_res_full, 1);
         mbar_init(bar_res_empty, 1);
@@ -188,6 +187,7 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
     tc_fence_after();
     const uint32_t tmem_base = *tmem_base_slot;
     WaitCtx wctx{p.status, abort_flag, warp};
+    ItemStream items{bar_steal, steal_response, p.n_items > p.first_wave};   // the loader warp's
     grid_let_next_start();
     grid_wait_for_previous();
     constexpr uint32_t kColX = 0, kColY = 128, kColDV = 256, kColDK = 256 + D;
@@ -459,8 +459,7 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
                 for (int sb = 0; sb < Cfg::kSub; ++sb) tma_load_3d(dst + sb * Cfg::kSubBytes, tm, bar, sb * 64, row_start, bh);
             };
             uint32_t git = 0;
-            ItemStream items{bar_steal, steal_response, p.n_items > p.first_wave};
-            int item = *abort_flag ? -1 : (int)blockIdx.x;
+            int item = (int)blockIdx.x;
             for (int k = 0;; ++k, item = items.next(wctx, 89, k)) {
                 const int slot = k & 1;
                 mbar_wait(&bar_sched_empty[slot], ((k >> 1) & 1) ^ 1, wctx, 90 + slot, k);
@@ -655,6 +654,7 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
         tc_fence_after();
         tmem_dealloc(tmem_base, Cfg::kTmemCols);
     }
+    if (warp == 9 && *abort_flag) items.drop_rest(wctx.budget);
 }
 
 // dq[slice][row][:] = bf16(scale * accumulator): one block per (query slice, 128-row query tile), thread

@@ -130,8 +130,7 @@ attn_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmR0, const __grid_con
     constexpr uint32_t kColRes = 256;   // Q at [256, 256 + D/2), dO at [256 + D/2, 256 + D)
 
     if (threadIdx.x == 0) {
-        // a CTA that the hardware starts after another one's wait has given up leaves at once
-        *abort_flag = ((int)blockIdx.x >= p.first_wave && *reinterpret_cast<volatile unsigned int*>(p.status) != 0u) ? 1 : 0;
+        *abort_flag = 0;
         mbar_init(bar_steal, 1);
         mbar_init(bar_res_full, 1);
         // the resident pair may be reloaded when the MMA warp has issued its last reads of it and, where
@@ -176,6 +175,7 @@ attn_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmR0, const __grid_con
     tc_fence_after();
     const uint32_t tmem_base = *tmem_base_slot;
     WaitCtx wctx{p.status, abort_flag, warp};
+    ItemStream items{bar_steal, steal_response, p.n_items > p.first_wave};   // the loader warp's
     // Both passes: a grid that does not wait itself is promised nothing of what ran before, so the dQ pass waits for the
     // whole dK/dV pass although it reads only the statistics and the inputs.
     grid_let_next_start();
@@ -486,8 +486,7 @@ attn_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmR0, const __grid_con
                 for (int sb = 0; sb < Cfg::kSub; ++sb) tma_load_3d(dst + sb * Cfg::kSubBytes, tm, bar, sb * 64, row_start, bh);
             };
             uint32_t git = 0;
-            ItemStream items{bar_steal, steal_response, p.n_items > p.first_wave};
-            int item = *abort_flag ? -1 : (int)blockIdx.x;
+            int item = (int)blockIdx.x;
             for (int k = 0;; ++k, item = items.next(wctx, 89, k)) {
                 BwdItem w;
                 while (item >= 0) {
@@ -677,6 +676,7 @@ attn_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmR0, const __grid_con
         tc_fence_after();
         tmem_dealloc(tmem_base, Cfg::kTmemCols);
     }
+    if (warp == 9 && *abort_flag) items.drop_rest(wctx.budget);
 }
 
 // ---------------------------------------------------------------- preprocessing

@@ -578,11 +578,13 @@ __global__ void __launch_bounds__(kThreads, 1) attn_f32_sm100_kernel(const F32Pa
     sh.t1_empty = bars + 17;  // [2]
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 19);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    uint64_t* bar_next = bars + 24;   // for a CTA that has given up only: a CTA has one item
+    uint4* response = reinterpret_cast<uint4*>(bars + 26);
     sh.stat = reinterpret_cast<float*>(aux + 1024);
     const int warp = uniform_warp_idx();
     if (threadIdx.x == 0) {
-        // a CTA of a later wave leaves at once when a wait has given up elsewhere
-        *abort_flag = ((int)blockIdx.x >= p.first_wave && *reinterpret_cast<volatile unsigned int*>(p.status) != 0u) ? 1 : 0;
+        *abort_flag = 0;
+        mbar_init(bar_next, 1);
         for (int i = 0; i < 19; ++i) {
             const bool rows_or_converters = i == 0 || i == 1 || i == 3 || i == 7 || i == 8 || (i >= 9 && i < 12) || i == 15 || i == 16;
             mbar_init(&bars[i], rows_or_converters ? 128 : 1);
@@ -615,6 +617,10 @@ __global__ void __launch_bounds__(kThreads, 1) attn_f32_sm100_kernel(const F32Pa
     if (warp == 8) {
         tc_fence_after();
         tmem_dealloc(sh.tmem, 512);
+        if (*abort_flag) {
+            ItemStream rest{bar_next, response, (int)gridDim.x > p.first_wave};
+            rest.drop_rest(ctx.budget);
+        }
     }
 }
 

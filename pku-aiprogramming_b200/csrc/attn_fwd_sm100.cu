@@ -180,8 +180,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     const int lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
-        // a CTA that the hardware starts after another one's wait has given up leaves at once
-        *abort_flag = ((int)blockIdx.x >= p.first_wave && *reinterpret_cast<volatile unsigned int*>(p.status) != 0u) ? 1 : 0;
+        *abort_flag = 0;
         mbar_init(bar_steal, 1);
         for (int i = 0; i < 2; ++i) {
             mbar_init(&bar_q_full[i], 1);
@@ -215,6 +214,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     tc_fence_after();
     const uint32_t tmem_base = *tmem_base_slot;
     WaitCtx wctx{p.status, abort_flag, warp};
+    ItemStream items{bar_steal, steal_response, p.n_items > p.first_wave};   // the loader warp's
     grid_let_next_start();
     grid_wait_for_previous();
 
@@ -386,8 +386,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             };
             uint32_t t = 0;                    // K/V ring item counter (runs across work items)
             uint32_t q_uses[2] = {0, 0};       // how often each Q buffer has been filled
-            ItemStream items{bar_steal, steal_response, p.n_items > p.first_wave};
-            int item = *abort_flag ? -1 : (int)blockIdx.x;
+            int item = (int)blockIdx.x;
             for (int k = 0;; ++k, item = items.next(wctx, 89, k)) {
                 const int slot = k & 1;
                 mbar_wait(&bar_sched_empty[slot], ((k >> 1) & 1) ^ 1, wctx, 90 + slot, k);
@@ -616,6 +615,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         tc_fence_after();
         tmem_dealloc(tmem_base, Cfg::kTmemCols);
     }
+    if (warp == 9 && *abort_flag) items.drop_rest(wctx.budget);
 }
 
 // ------------------------------------------------------------------------------ host side
@@ -855,22 +855,29 @@ static cudaError_t launch_probe(const void* a, const void* b, const void* vt, fl
 
 // Exercises the bounded-wait path: one warp waits on an mbarrier that nothing ever arrives on.
 // The wait gives up after `budget_cycles`, records itself in the status word and the kernel
-// returns normally (no trap, no hang); the host then sees TT_ERR_TIMEOUT.
-__global__ void wait_timeout_kernel(unsigned int* status, long long budget_cycles) {
-    __shared__ uint64_t bar;
+// returns normally (no trap, no hang); the host then sees TT_ERR_TIMEOUT.  Of several CTAs, those that have given up drop the
+// ones that have not started; `started` (if any) counts the others.
+__global__ void wait_timeout_kernel(unsigned int* status, long long budget_cycles, unsigned int* started) {
+    __shared__ uint64_t bar, bar_next;
+    __shared__ __align__(16) uint4 response;
     __shared__ int abort_flag;
     if (threadIdx.x == 0) {
         abort_flag = 0;
         mbar_init(&bar, 1);
+        mbar_init(&bar_next, 1);
         fence_barrier_init();
+        if (started) atomicAdd(started, 1u);
     }
     __syncthreads();
     WaitCtx ctx{status, &abort_flag, 0, budget_cycles};
     mbar_wait(&bar, 0, ctx, 99, 7);
+    __syncwarp();
+    ItemStream rest{&bar_next, &response, gridDim.x > 1};
+    rest.drop_rest(budget_cycles);
 }
-cudaError_t wait_timeout_probe(long long budget_cycles, cudaStream_t st) {
+cudaError_t wait_timeout_probe(long long budget_cycles, int ctas, unsigned int* started, cudaStream_t st) {
     LaunchScope ls(K_PROBE, st);
-    wait_timeout_kernel<<<1, 32, 0, st>>>(device_status_word(), budget_cycles);
+    wait_timeout_kernel<<<ctas, 32, 0, st>>>(device_status_word(), budget_cycles, started);
     return cudaGetLastError();
 }
 

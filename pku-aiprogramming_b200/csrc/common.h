@@ -178,7 +178,7 @@ cudaError_t attn_bwd_sm100(const AttnArgs& a, void* workspace, cudaStream_t st);
 // 1 = always the two passes (seven GEMMs, every result bit-reproducible).
 void attn_bwd_set_deterministic(int on);
 int attn_bwd_deterministic();
-cudaError_t wait_timeout_probe(long long budget_cycles, cudaStream_t st);
+cudaError_t wait_timeout_probe(long long budget_cycles, int ctas, unsigned int* started, cudaStream_t st);
 cudaError_t umma_probe(const void* a, const void* b, const void* vt, int D, float* s_out, float* o_out,
                        cudaStream_t st);
 

@@ -120,10 +120,27 @@ struct ItemStream {
         }
         __syncwarp();
     }
-    // the next item, or -1 when none is left
+    // the next item, or -1 when none is left (or the wait gave up: the request is then still pending)
     __device__ __forceinline__ int next(const WaitCtx& ctx, int bar_id, int iter) {
-        if (!pending) return -1;
-        const bool ok = mbar_wait(bar, phase & 1, ctx, bar_id, iter);
+        if (!pending || !__all_sync(0xffffffffu, mbar_wait(bar, phase & 1, ctx, bar_id, iter))) return -1;
+        return answer();
+    }
+    // For a CTA whose wait has given up: takes the CTAs of its own launch that have not started, and drops them.  The launch
+    // then ends about one wait's limit later, not one per wave of CTAs; a flag in global memory that later CTAs look at
+    // would do it for the launches after this one as well.
+    __device__ __forceinline__ void drop_rest(long long budget) {
+        while (dynamic) {
+            if (!pending) request(false);
+            const long long t0 = clock64();
+            bool ok;
+            do ok = __all_sync(0xffffffffu, mbar_try_wait(bar, phase & 1));
+            while (!ok && !__any_sync(0xffffffffu, clock64() - t0 > budget));
+            if (!ok) return;
+            answer();
+        }
+    }
+    __device__ __forceinline__ int answer() {
+        pending = false;
         ++phase;
         uint32_t got = 0, id = 0;
         asm volatile(
@@ -137,7 +154,7 @@ struct ItemStream {
             : "r"(smem_u32(response))
             : "memory");
         __syncwarp();
-        if (!ok || !got) {   // after a request that found nothing there must be no further one
+        if (!got) {   // after a request that found nothing there must be no further one
             dynamic = false;
             return -1;
         }

@@ -854,14 +854,21 @@ int tt_attn_decode_paged(const tt_attn_desc* desc, const void* q, const void* k_
     return TT_OK;
 }
 
-int tt_debug_wait_timeout(int64_t budget_cycles, void* stream) {
+static int wait_timeout(const char* who, int64_t budget_cycles, int32_t ctas, uint32_t* started, void* stream) {
     if (budget_cycles < 1 || budget_cycles > 4000000000LL)
-        return fail(TT_ERR_BAD_SHAPE, "tt_debug_wait_timeout: budget of %lld cycles outside 1..4e9", (long long)budget_cycles);
+        return fail(TT_ERR_BAD_SHAPE, "%s: budget of %lld cycles outside 1..4e9", who, (long long)budget_cycles);
+    if (ctas < 1) return fail(TT_ERR_BAD_SHAPE, "%s: %d CTAs", who, ctas);
     int rc = check_device();
     if (rc != TT_OK) return rc;
-    cudaError_t e = wait_timeout_probe(budget_cycles, (cudaStream_t)stream);
-    if (e != cudaSuccess) return cuda_fail(e, "tt_debug_wait_timeout: launch");
+    cudaError_t e = wait_timeout_probe(budget_cycles, ctas, started, (cudaStream_t)stream);
+    if (e != cudaSuccess) return cuda_fail(e, who);
     return TT_OK;
+}
+int tt_debug_wait_timeout(int64_t budget_cycles, void* stream) {
+    return wait_timeout("tt_debug_wait_timeout", budget_cycles, 1, nullptr, stream);
+}
+int tt_debug_wait_timeout_grid(int64_t budget_cycles, int32_t ctas, uint32_t* started, void* stream) {
+    return wait_timeout("tt_debug_wait_timeout_grid", budget_cycles, ctas, started, stream);
 }
 
 int tt_debug_fwd_trace(void* device_buf, int32_t block, int32_t item) {

@@ -22,6 +22,10 @@ int tt_debug_fwd_trace(void* device_buf, int32_t block, int32_t item);
  * launch, 3 the single-pass kernel. */
 int tt_debug_bwd_trace(void* device_buf, int32_t block, int32_t pass);
 
+/* tt_debug_wait_timeout (tt_attn.h) on `ctas` CTAs: those whose wait has given up drop the ones that have not started;
+ * `started` (device memory, set to 0 by the caller) counts the others. */
+int tt_debug_wait_timeout_grid(int64_t budget_cycles, int32_t ctas, uint32_t* started, void* stream);
+
 /* A failure made on the host, for tests of the error exits of the host-buffer calls (tt_attn_*_host):
  * the (checks+1)-th CUDA runtime result those calls inspect from now on is reported as cudaErrorUnknown
  * although the runtime call was made and succeeded, so the entry point returns TT_ERR_CUDA in the middle
