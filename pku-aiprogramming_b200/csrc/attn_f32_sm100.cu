@@ -22,6 +22,11 @@
 // The streamed tiles are in shared memory; R0, R1 and the bf16 parts of P / dS are A operands in tensor memory: an MMA with
 // 64 columns takes 32 cycles that way and 48 with both operands in shared memory (measured; 16 against 40 with 32 columns).
 // At head dim 128 DK and DQ keep R0 in shared memory, there is no room for both.
+// Parts do what a float does only while nothing overflows: the parts of an infinity sum to NaN, and the part products of two
+// factors whose product overflows are infinities of either sign.  A wrong score of -infinity would pass unseen (its P is 0),
+// so the operands of the scores are watched for magnitudes above 2^60, below which no score overflows; every other
+// infinity or NaN reaches the row's result.  Rows of an item that has met such a magnitude, and rows whose result is not
+// finite, are computed again with plain multiply-adds by their thread (f32_plain_row); what the mask hides takes no part there.
 // The S accumulator is double buffered and the next tile's S is issued before this tile's P is ready.  At head dim 128
 // the streamed tiles have 32 rows: with 64, shared memory holds one tile of each tensor (every tile's load is exposed)
 // and the row threads' registers do not hold the accumulator row beside two rows of scores.
@@ -51,6 +56,7 @@ struct F32Params {
     unsigned int* status;
 };
 
+constexpr float kLarge = 1152921504606846976.f;   // 2^60: 128 products of two values up to it are below 2^128
 constexpr int kRows = 128, kThreads = 384;   // warps 9-11 only complete the third warpgroup
 // registers per thread after setmaxnreg; the sum draws on what the launch allocated (384 x 168)
 constexpr int kRegsRows = 232, kRegsConvert = 168, kRegsIssue = 104;
@@ -94,8 +100,10 @@ struct TileRegs {
     }
     // part p of the tile at dst + p * part bytes; row r of 64-column block s at s * ROWS * 128 + r * 128, 16-byte chunks
     // swizzled.  Eight neighbouring threads write one 128-byte row: no bank conflicts.
-    __device__ __forceinline__ void store(unsigned char* dst, int tid) const {
+    // Returns the largest magnitude.
+    __device__ __forceinline__ float store(unsigned char* dst, int tid) const {
         constexpr int kPart = (DP / 64) * ROWS * 128;
+        float top = 0.f;
 #pragma unroll
         for (int i = 0; i < kSteps; ++i) {
             const int idx = i * 128 + tid, r = idx / (DP / 8), c = idx % (DP / 8);
@@ -105,7 +113,10 @@ struct TileRegs {
             *reinterpret_cast<uint4*>(p) = h;
             *reinterpret_cast<uint4*>(p + kPart) = m;
             *reinterpret_cast<uint4*>(p + 2 * kPart) = l;
+#pragma unroll
+            for (int e = 0; e < 8; e += 2) top = fmax3(top, fabsf(x[i][e]), fabsf(x[i][e + 1]));
         }
+        return top;
     }
 };
 
@@ -146,6 +157,7 @@ __device__ __forceinline__ F32Item f32_item(int idx, const F32Params& p) {
 struct F32Shared {
     unsigned char *res, *t0, *t1;     // resident R0, rings of streamed tiles
     uint64_t *r0_full, *r1_full, *t0_full, *t0_empty, *t1_full, *t1_empty, *s_full, *s_free, *dp_full, *w_full, *acc_full;
+    volatile int* large;              // a magnitude above kLarge in R0 or T0
     float* stat;                      // DV, DK: [8 x 128]: -lse, then -delta, of the streamed rows
     uint32_t tmem;
 };
@@ -184,10 +196,11 @@ __device__ __forceinline__ void f32_convert(const F32Params& p, const F32Item& w
         load_a(0);
         load_b(0);
     }
+    float top = 0.f;
     for (int u = 0; u < w.n_it; ++u) {
         const int s0 = u % Cfg::kN0, s1 = u % Cfg::kN1;
         mbar_wait(&sh.t0_empty[s0], ((u / Cfg::kN0) & 1) ^ 1, ctx, 10 + s0, u);
-        a.store(sh.t0 + s0 * Cfg::kStr, tid);
+        top = fmaxf(top, a.store(sh.t0 + s0 * Cfg::kStr, tid));
         if (kKeys && tid < 2 * kCols) sh.stat[(u & 7) * 128 + tid] = stat_a;   // row threads lag by at most five tiles
         fence_proxy_async_smem();
         mbar_arrive(&sh.t0_full[s0]);
@@ -198,6 +211,9 @@ __device__ __forceinline__ void f32_convert(const F32Params& p, const F32Item& w
         mbar_arrive(&sh.t1_full[s1]);
         if (u + 1 < w.n_it) load_b(u + 1);
     }
+    if (top > kLarge) *sh.large = 1;
+    __syncwarp();
+    asm volatile("bar.arrive 1, 256;" ::: "memory");   // with the row threads, for `large`
 }
 
 // ---------------------------------------------------------------------------- MMA issuer (one warp)
@@ -327,9 +343,11 @@ __device__ __forceinline__ void load_cols(uint32_t taddr, float (&x)[N]) {
     for (int e = 0; e < N; ++e) x[e] = __uint_as_float(a[e / 32][e % 32]);
 }
 
-// One row of DP floats (zero past D, or everywhere if !ok) -> its bf16 parts at `taddr`, DP / 2 columns each.
+// One row of DP floats (zero past D, or everywhere if !ok) -> its bf16 parts at `taddr`, DP / 2 columns each.  Returns
+// the largest magnitude.
 template <int DP>
-__device__ __forceinline__ void row_to_tmem(const float* src, bool ok, int D, uint32_t taddr) {
+__device__ __forceinline__ float row_to_tmem(const float* src, bool ok, int D, uint32_t taddr) {
+    float top = 0.f;
 #pragma unroll 1
     for (int g = 0; g < DP / 32; ++g) {
         uint32_t h[16], m[16], l[16];
@@ -342,6 +360,7 @@ __device__ __forceinline__ void row_to_tmem(const float* src, bool ok, int D, ui
                 float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (ok && d < D) v = __ldg(reinterpret_cast<const float4*>(src + d));
                 y[4 * e] = v.x; y[4 * e + 1] = v.y; y[4 * e + 2] = v.z; y[4 * e + 3] = v.w;
+                top = fmax3(fmax3(top, fabsf(v.x), fabsf(v.y)), fabsf(v.z), fabsf(v.w));
             }
             uint4 a, b, c;
             split8(y, a, b, c);
@@ -356,10 +375,12 @@ __device__ __forceinline__ void row_to_tmem(const float* src, bool ok, int D, ui
     }
     tmem_wait_st();
     tc_fence_before();
+    return top;
 }
 
+// Returns whether the row has to be computed again by plain arithmetic.
 template <int DP, int MODE>
-__device__ __forceinline__ void f32_rows(const F32Params& p, const F32Item& w, const F32Shared& sh, const WaitCtx& ctx, int tid) {
+__device__ __forceinline__ bool f32_rows(const F32Params& p, const F32Item& w, const F32Shared& sh, const WaitCtx& ctx, int tid) {
     using Cfg = F32Cfg<DP>;
     constexpr int kCols = Cfg::kCols;
     constexpr bool kKeys = MODE == DV || MODE == DK, kHasDP = MODE == DK || MODE == DQ;
@@ -371,8 +392,9 @@ __device__ __forceinline__ void f32_rows(const F32Params& p, const F32Item& w, c
     // resident tiles: every thread its own row into tensor memory; R0 of DK / DQ at head dim 128 into shared memory
     constexpr bool kR0Tmem = DP == 64 || !kHasDP;
     const long long first = (long long)w.slice * (kKeys ? p.L : p.S) + w.r0;
+    float top = 0.f;
     if (kR0Tmem) {
-        row_to_tmem<DP>((kKeys ? p.k : p.q) + (first + tid) * p.D, row < res_rows, p.D, lane_base + Cfg::kR0);
+        top = row_to_tmem<DP>((kKeys ? p.k : p.q) + (first + tid) * p.D, row < res_rows, p.D, lane_base + Cfg::kR0);
         mbar_arrive(sh.r0_full);
     } else {
 #pragma unroll 1
@@ -389,6 +411,8 @@ __device__ __forceinline__ void f32_rows(const F32Params& p, const F32Item& w, c
                 *reinterpret_cast<uint4*>(q) = a;
                 *reinterpret_cast<uint4*>(q + Cfg::kResPart) = b;
                 *reinterpret_cast<uint4*>(q + 2 * Cfg::kResPart) = d;
+#pragma unroll
+                for (int e = 0; e < 8; e += 2) top = fmax3(top, fabsf(r.x[i][e]), fabsf(r.x[i][e + 1]));
             }
         }
         fence_proxy_async_smem();
@@ -398,6 +422,7 @@ __device__ __forceinline__ void f32_rows(const F32Params& p, const F32Item& w, c
         row_to_tmem<DP>((kKeys ? p.v : p.dout) + (first + tid) * p.D, row < res_rows, p.D, lane_base + Cfg::kR1);
         mbar_arrive(sh.r1_full);
     }
+    if (top > kLarge) *sh.large = 1;
     uint64_t row_nlse = pack_f32x2(-INFINITY, -INFINITY), row_ndelta = 0;
     if (MODE == DQ && row < p.S) {
         const float nl = -p.lse[(long long)w.slice * p.S + row], nd = -p.delta[(long long)w.slice * p.S + row];
@@ -518,6 +543,11 @@ __device__ __forceinline__ void f32_rows(const F32Params& p, const F32Item& w, c
         wait_acc(w.n_it - 1);
         take_acc(1.f);
     }
+    asm volatile("bar.sync 1, 256;" ::: "memory");   // with the converters, for `large`
+    float zero[4] = {MODE == FWD ? l * 0.f : 0.f, 0.f, 0.f, 0.f};   // NaN where something is not finite
+#pragma unroll
+    for (int d = 0; d < DP; ++d) zero[d & 3] = fmaf(acc[d], 0.f, zero[d & 3]);
+    const bool finite = zero[0] + zero[1] + zero[2] + zero[3] == 0.f;
 
     const int n_rows = kKeys ? p.L : p.S;
     if (row < n_rows) {
@@ -531,26 +561,99 @@ __device__ __forceinline__ void f32_rows(const F32Params& p, const F32Item& w, c
                                                            : make_float4(acc[d] * mul, acc[d + 1] * mul, acc[d + 2] * mul, acc[d + 3] * mul);
         if (MODE == FWD && p.lse_out != nullptr) p.lse_out[(long long)w.slice * p.S + row] = fmaf(m, p.scale, logf(l));
     }
+    return w.n_it > 0 && row < res_rows && (*sh.large || !finite);
 }
 
 template <int DP, int MODE, int ROLE>
-__device__ __forceinline__ void f32_role(int idx, const F32Params& p, const F32Shared& sh, const WaitCtx& ctx) {
+__device__ __forceinline__ bool f32_role(int idx, const F32Params& p, const F32Shared& sh, const WaitCtx& ctx) {
     const F32Item w = f32_item<MODE, F32Cfg<DP>::kCols>(idx, p);
-    if (ROLE == 0) f32_rows<DP, MODE>(p, w, sh, ctx, threadIdx.x);
+    if (ROLE == 0) return f32_rows<DP, MODE>(p, w, sh, ctx, threadIdx.x);
     if (ROLE == 1) f32_convert<DP, MODE>(p, w, sh, ctx, threadIdx.x - 128);
     if (ROLE == 2) f32_issue<DP, MODE>(w, sh, ctx);
+    return false;
 }
 template <int DP, bool kBwd, int ROLE>
-__device__ __forceinline__ void f32_run(const F32Params& p, const F32Shared& sh, const WaitCtx& ctx) {
+__device__ __forceinline__ bool f32_run(const F32Params& p, const F32Shared& sh, const WaitCtx& ctx) {
     const int idx = blockIdx.x;
-    if (!kBwd) {
-        f32_role<DP, FWD, ROLE>(idx, p, sh, ctx);
-        return;
-    }
+    if (!kBwd) return f32_role<DP, FWD, ROLE>(idx, p, sh, ctx);
     const int n_k = p.n_kt * p.kv_slices, n_q = p.n_qt * p.q_slices;
-    if (idx < n_k) f32_role<DP, DK, ROLE>(idx, p, sh, ctx);
-    else if (idx < n_k + n_q) f32_role<DP, DQ, ROLE>(idx - n_k, p, sh, ctx);
-    else f32_role<DP, DV, ROLE>(idx - n_k - n_q, p, sh, ctx);
+    if (idx < n_k) return f32_role<DP, DK, ROLE>(idx, p, sh, ctx);
+    if (idx < n_k + n_q) return f32_role<DP, DQ, ROLE>(idx - n_k, p, sh, ctx);
+    return f32_role<DP, DV, ROLE>(idx - n_k - n_q, p, sh, ctx);
+}
+
+// Row `tid` of this CTA's item with plain multiply-adds over the streamed rows that it sees, written like f32_rows does.  One
+// form for all modes, behind everything else of the kernel: inside f32_rows its code alone cost [2,8,2048,64] 10 us of
+// 300.  Streamed rows are the same for all lanes; the own rows R0, R1 are in shared memory (what the tiles took), rows
+// 16 bytes apart modulo 128.
+__device__ __forceinline__ float plain_dot(const float* a, const float* b, int D) {
+    float s = 0.f;
+#pragma unroll 4
+    for (int d = 0; d < D; d += 4) {
+        const float4 x = *reinterpret_cast<const float4*>(a + d), y = __ldg(reinterpret_cast<const float4*>(b + d));
+        s = fmaf(x.x, y.x, s); s = fmaf(x.y, y.y, s); s = fmaf(x.z, y.z, s); s = fmaf(x.w, y.w, s);
+    }
+    return s;
+}
+template <int DP, bool kBwd>
+__device__ __forceinline__ void f32_plain_row(const F32Params& p, unsigned char* smem, int tid) {
+    using Cfg = F32Cfg<DP>;
+    constexpr int kCols = Cfg::kCols, kPlainPitch = DP + 4, kPlainCols = 32;
+    static_assert(2 * kRows * kPlainPitch * 4 <= Cfg::kRes + (Cfg::kN0 + Cfg::kN1) * Cfg::kStr, "own rows take the tiles' place");
+    const int n_k = p.n_kt * p.kv_slices, n_q = p.n_qt * p.q_slices, idx = blockIdx.x;
+    const int mode = !kBwd ? FWD : idx < n_k ? DK : idx < n_k + n_q ? DQ : DV;
+    const bool keys = mode == DK || mode == DV, has_dp = mode == DK || mode == DQ;
+    const F32Item w = mode == FWD ? f32_item<FWD, kCols>(idx, p) : mode == DQ ? f32_item<DQ, kCols>(idx - n_k, p)
+                                  : f32_item<DK, kCols>(mode == DK ? idx : idx - n_k - n_q, p);
+    const int row = w.r0 + tid, off = p.L - p.S, own_rows = keys ? p.L : p.S, rows = keys ? p.S : p.L;
+    const int lo = keys && p.causal ? max(0, row - off) : 0;
+    const int hi = keys ? p.S : p.causal ? min(w.Lv, row + off + 1) : w.Lv;
+    const long long own = (long long)w.slice * own_rows + row;
+    const float *src0 = (keys ? p.k : p.q) + own * p.D, *src1 = has_dp ? (keys ? p.v : p.dout) + own * p.D : src0;
+    float *r0 = reinterpret_cast<float*>(smem) + tid * kPlainPitch, *r1 = r0 + kRows * kPlainPitch;
+    for (int d = 0; d < p.D; ++d) {
+        r0[d] = src0[d];
+        r1[d] = src1[d];
+    }
+    float m = -INFINITY;
+    if (mode == FWD) {
+        const float* t0 = p.k + (long long)(w.slice / p.group) * rows * p.D;
+#pragma unroll 1
+        for (int c = lo; c < hi; ++c) m = fmaxf(m, plain_dot(r0, t0 + (long long)c * p.D, p.D));
+    }
+    float* dst = (mode == FWD ? p.out : mode == DV ? p.dv : mode == DK ? p.dk : p.dq) + own * p.D;
+#pragma unroll 1
+    for (int d0 = 0; d0 < p.D; d0 += kPlainCols) {   // the weights again for each group of columns: no more registers than the rest
+        float acc[kPlainCols] = {}, l = 0.f;
+#pragma unroll 1
+        for (int hh = 0; hh < (keys ? p.group : 1); ++hh) {
+            const long long slice = keys ? (long long)w.slice * p.group + hh : w.slice / p.group;
+            const float* t0 = (keys ? p.q : p.k) + slice * rows * p.D;
+            const float* t1 = (keys ? p.dout : p.v) + slice * rows * p.D;
+#pragma unroll 1
+            for (int c = lo; c < hi; ++c) {
+                const float s = plain_dot(r0, t0 + (long long)c * p.D, p.D);
+                const long long q_row = keys ? slice * p.S + c : own;
+                float x = mode == FWD ? expf((s - m) * p.scale) : expf(fmaf(s, p.scale, -p.lse[q_row]));
+                l += x;
+                if (has_dp) x *= plain_dot(r1, t1 + (long long)c * p.D, p.D) - p.delta[q_row];
+                const float* t = (has_dp ? t0 : t1) + (long long)c * p.D + d0;
+#pragma unroll
+                for (int d = 0; d < kPlainCols; d += 4)
+                    if (d0 + d < p.D) {
+                        const float4 y = __ldg(reinterpret_cast<const float4*>(t + d));
+                        acc[d] = fmaf(x, y.x, acc[d]); acc[d + 1] = fmaf(x, y.y, acc[d + 1]);
+                        acc[d + 2] = fmaf(x, y.z, acc[d + 2]); acc[d + 3] = fmaf(x, y.w, acc[d + 3]);
+                    }
+            }
+        }
+        const float mul = mode == FWD ? 1.f / l : mode == DV ? 1.f : p.scale;
+#pragma unroll
+        for (int d = 0; d < kPlainCols; d += 4)
+            if (d0 + d < p.D)
+                *reinterpret_cast<float4*>(dst + d0 + d) = make_float4(acc[d] * mul, acc[d + 1] * mul, acc[d + 2] * mul, acc[d + 3] * mul);
+        if (mode == FWD && d0 == 0 && p.lse_out != nullptr) p.lse_out[own] = fmaf(m, p.scale, logf(l));
+    }
 }
 
 // kBwd: one launch holds the items of DK, DQ and DV one after the other.
@@ -580,10 +683,12 @@ __global__ void __launch_bounds__(kThreads, 1) attn_f32_sm100_kernel(const F32Pa
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     uint64_t* bar_next = bars + 24;   // for a CTA that has given up only: a CTA has one item
     uint4* response = reinterpret_cast<uint4*>(bars + 26);
+    sh.large = abort_flag + 1;
     sh.stat = reinterpret_cast<float*>(aux + 1024);
     const int warp = uniform_warp_idx();
     if (threadIdx.x == 0) {
         *abort_flag = 0;
+        *sh.large = 0;
         mbar_init(bar_next, 1);
         for (int i = 0; i < 19; ++i) {
             const bool rows_or_converters = i == 0 || i == 1 || i == 3 || i == 7 || i == 8 || (i >= 9 && i < 12) || i == 15 || i == 16;
@@ -602,9 +707,10 @@ __global__ void __launch_bounds__(kThreads, 1) attn_f32_sm100_kernel(const F32Pa
     WaitCtx ctx{p.status, abort_flag, warp};
     grid_let_next_start();
     grid_wait_for_previous();
+    bool again = false;
     if (warp < 4) {
         setmaxnreg_inc<kRegsRows>();
-        f32_run<DP, kBwd, 0>(p, sh, ctx);
+        again = f32_run<DP, kBwd, 0>(p, sh, ctx);
     } else if (warp < 8) {
         setmaxnreg_dec<kRegsConvert>();   // (what the launch gave)
         f32_run<DP, kBwd, 1>(p, sh, ctx);
@@ -622,6 +728,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_f32_sm100_kernel(const F32Pa
             rest.drop_rest(ctx.budget);
         }
     }
+    if (again) f32_plain_row<DP, kBwd>(p, smem, threadIdx.x);
 }
 
 // delta = rowsum(dO * O): 8 lanes share a row, four rows per warp and step; HBM-bound.

@@ -73,3 +73,61 @@ def test_largest_finite_values(tt, oracle):
     p = np.exp(s - s.max())
     last = -(p / p.sum())[S - 1] * float(big)
     assert float(np.abs(got[0, 0, S - 1] / last - 1).max()) <= 1e-5
+
+
+def visible_f32(q, k, v, do):
+    """One slice, causal, in float32 over the pairs that the mask leaves: what it hides takes no part, not even as 0 x infinity."""
+    S, D = q.shape
+    scale = np.float32(1 / np.sqrt(D))
+    out, lse, dq, dk, dv = np.zeros_like(q), np.zeros(S, np.float32), np.zeros_like(q), np.zeros_like(k), np.zeros_like(v)
+    with np.errstate(all="ignore"):
+        for i in range(S):
+            K, V = k[:i + 1], v[:i + 1]
+            s = (K * q[i]).sum(1) * scale
+            m = np.fmax.reduce(s)
+            e = np.exp(s - m)
+            p = e / e.sum()
+            lse[i], out[i] = m + np.log(e.sum()), (p[:, None] * V).sum(0)
+            ds = p * ((V * do[i]).sum(1) - (out[i] * do[i]).sum())
+            dq[i] = (ds[:, None] * K).sum(0) * scale
+            dk[:i + 1] += ds[:, None] * q[i] * scale
+            dv[:i + 1] += p[:, None] * do[i]
+    return out, lse, dq, dk, dv
+
+
+inf, nan = float("inf"), float("nan")
+
+
+# an infinity or a NaN in each input; an infinity behind what early rows see; scores that overflow to -infinity (weight 0), from an
+# infinity and from finite factors, and to +infinity; a product of finite gradients that overflows; a first part that rounds up
+# (1.0039) and one that does not, because the signs of the cross terms come from the remainders
+@pytest.mark.parametrize("D", [64, 128, 40])
+@pytest.mark.parametrize("name,row,value", [("q", 9, inf), ("k", 150, inf), ("v", 150, inf), ("do", 150, -inf), ("q", 130, nan), ("k", 3, nan),
+                                            ("v", 199, nan), ("do", 0, nan), ("k", 3, -inf), ("k", 150, -3e38), ("k", 7, 1.0039e30),
+                                            ("k", 7, 1.0009e30), ("do", 60, 1.0039e38)])
+def test_infinities_nan_and_overflow(tt, oracle, D, name, row, value):
+    S = 200
+    x = dict(zip(("q", "k", "v", "do"), (a[0, 0] for a in oracle.make_inputs(D, 1, 1, S, S, D))))
+    if name == "k" and not np.isnan(value):
+        x["q"] = np.abs(x["q"]) + np.float32(0.5)       # scores of that key have one sign, whatever the order of the sum
+        if 1e30 < value < 1.1e30:
+            x["q"][100] = 1e20                          # +infinity in this row alone; the others give key 7 all their weight
+    if name == "do" and np.isfinite(value):
+        x["v"] = np.abs(x["v"]) + np.float32(0.5)       # dP of that row overflows to +infinity, its delta too
+    x[name][row] = value
+    want = visible_f32(x["q"], x["k"], x["v"], x["do"])
+    q, k, v, do = (torch.from_numpy(x[n]).cuda()[None, None] for n in ("q", "k", "v", "do"))
+    out, lse = tt.attention_forward(q, k, v, causal=True)
+    got = (out, lse, *tt.attention_backward(q, k, v, out, lse, do, causal=True))
+    tt.check_device_status()
+    for what, g, r in zip(("out", "lse", "dq", "dk", "dv"), got, want):
+        if what[0] == "d" and 1e30 < value < 1.1e30:
+            break                                       # exp(score - lse) of scores near 1e30 is nothing but their rounding
+        g = g.cpu().numpy().reshape(r.shape)
+        assert np.array_equal(np.isnan(g), np.isnan(r)), what
+        assert np.array_equal(np.where(np.isinf(g), np.sign(g), 0), np.where(np.isinf(r), np.sign(r), 0)), what
+        ok = np.isfinite(r)
+        # two float32 sums of up to 200 terms in different orders; values beyond 1e6 come from the large input: relative to them
+        rows = np.abs(np.where(ok, r, 0)).reshape(S, -1).max(1)
+        err = np.abs(np.where(ok, g - r, 0)).reshape(S, -1).max(1)
+        assert bool((err <= 2e-5 * np.maximum(rows, 1.0)).all()), (what, float((err / np.maximum(rows, 1.0)).max()))
