@@ -4,7 +4,8 @@
 
 namespace ttk {
 
-// x[0..7] -> three 16-byte groups of bf16 whose sum is x exactly.  The first part saturates: rounding a value next to
+// x[0..7] -> three 16-byte groups of bf16 whose sum is x, exactly from 2^-110 on (below, the last part falls under bf16's smallest
+// subnormal, 2^-133) and for finite x.  The first part saturates: rounding a value next to
 // the largest float up to infinity would leave a remainder of infinity, where the sum of the parts is finite.
 __device__ __forceinline__ uint32_t pack_bf16x2_sat(float lo, float hi) {
     uint32_t r;

@@ -20,7 +20,9 @@
 // 1.08 ms, [16384,64]x[64,64] 1709 -> 69 us, [300,300]x[300,300] 118 -> 48 us against the FMA kernel.  Errors (2-norm, against
 // float64) 5e-8 to 1.7e-7; the FMA kernel's 6e-8 to 2.3e-6, growing with K.
 //
-// The parts of an infinity sum to NaN.  A CTA that meets one computes its share again with plain fused multiply-adds.
+// The parts of an infinity sum to NaN, and the part products of two factors whose product overflows are infinities of
+// either sign.  Both reach the accumulator, so a thread whose share of a row is not finite computes it again with plain
+// fused multiply-adds.
 #include <cooperative_groups.h>
 #include <stdlib.h>
 
@@ -80,9 +82,8 @@ struct ChunkRegs {
             }
         }
     }
-    // -> three parts at dst; returns the largest magnitude
-    __device__ __forceinline__ float store(unsigned char* dst, int tid) const {
-        float top = 0.f;
+    // -> three parts at dst
+    __device__ __forceinline__ void store(unsigned char* dst, int tid) const {
 #pragma unroll
         for (int i = 0; i < kGroups; ++i) {
             const int idx = i * kConvert + tid, r = idx / (COLS / 8), c = idx % (COLS / 8);
@@ -92,10 +93,7 @@ struct ChunkRegs {
             *reinterpret_cast<uint4*>(p) = h;
             *reinterpret_cast<uint4*>(p + kPart) = m;
             *reinterpret_cast<uint4*>(p + 2 * kPart) = l;
-#pragma unroll
-            for (int e = 0; e < 8; e += 2) top = fmax3(top, fabsf(x[i][e]), fabsf(x[i][e + 1]));
         }
-        return top;
     }
 };
 
@@ -110,11 +108,9 @@ __global__ void __launch_bounds__(kThreads, 1) fc_f32_sm100_kernel(const FcF32Pa
     uint64_t* acc_free = full + 6;    // [2] accumulating threads -> MMA
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(full + 8);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-    volatile int* infinite = abort_flag + 1;
     const int warp = uniform_warp_idx(), lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         *abort_flag = 0;
-        *infinite = 0;
         for (int b = 0; b < 2; ++b) {
             mbar_init(&full[b], kConvert);
             mbar_init(&empty[b], 1);
@@ -167,10 +163,11 @@ __global__ void __launch_bounds__(kThreads, 1) fc_f32_sm100_kernel(const FcF32Pa
             tc_fence_before();
             mbar_arrive(&acc_free[b]);
         }
-        // Every chunk's MMAs are done, nothing uses the operands' shared memory any more; the barrier is for `infinite`.
-        asm volatile("bar.sync 1, 512;" ::: "memory");
         const int r = (warp & 3) * 32 + lane, c0 = (warp >> 2) * 64;
-        if (*infinite) {
+        float zero[4] = {};   // NaN where something is not finite
+#pragma unroll
+        for (int e = 0; e < 64; ++e) zero[e & 3] = fmaf(acc[e], 0.f, zero[e & 3]);
+        if (zero[0] + zero[1] + zero[2] + zero[3] != 0.f) {
             const int m = m0 + r, k_end = min(p.K, (u0 + n_it) * kK);
 #pragma unroll
             for (int e = 0; e < 64; ++e) acc[e] = 0.f;
@@ -183,6 +180,7 @@ __global__ void __launch_bounds__(kThreads, 1) fc_f32_sm100_kernel(const FcF32Pa
                 }
             }
         }
+        // Every chunk's MMAs are done: nothing uses the operands' shared memory any more.
 #pragma unroll
         for (int e = 0; e < 64; e += 4)
             *reinterpret_cast<float4*>(tile + r * kAccPitch + c0 + e) = make_float4(acc[e], acc[e + 1], acc[e + 2], acc[e + 3]);
@@ -206,21 +204,17 @@ __global__ void __launch_bounds__(kThreads, 1) fc_f32_sm100_kernel(const FcF32Pa
             load_a(0);
             load_b(0);
         }
-        float top = 0.f;
         for (int u = 0; u < n_it; ++u) {
             const int s = u & 1;
             mbar_wait(&empty[s], ((u >> 1) & 1) ^ 1, ctx, 10 + s, u);
             unsigned char* dst = smem + s * kStage;
-            top = fmaxf(top, a.store(dst, tid));
+            a.store(dst, tid);
             if (u + 1 < n_it) load_a(u + 1);
-            top = fmaxf(top, b.store(dst + kOperand, tid));
+            b.store(dst + kOperand, tid);
             fence_proxy_async_smem();
             mbar_arrive(&full[s]);
             if (u + 1 < n_it) load_b(u + 1);
         }
-        if (top == INFINITY) *infinite = 1;
-        __syncwarp();
-        asm volatile("bar.arrive 1, 512;" ::: "memory");
     } else {
         setmaxnreg_dec<kRegsIssue>();
     }

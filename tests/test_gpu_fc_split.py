@@ -66,3 +66,23 @@ def test_float_extremes(tt):
     assert torch.equal(torch.isinf(y)[ok], torch.isinf(want)[ok]) and torch.equal(torch.sign(y)[ok].double(), torch.sign(want)[ok])
     fin = torch.isfinite(want)
     assert torch.allclose(y.double()[fin], want[fin], rtol=1e-6, atol=0)
+
+
+@pytest.mark.parametrize("fin", [64, 1000, 8192])   # one CTA per tile, and clusters that cut K
+def test_float_products_that_overflow(tt, fin):
+    """Finite factors whose product overflows give the infinity of the product's sign, whatever the signs of their parts'
+    remainders (1.0039 rounds up to its first part, 1.0009 down), forward and in both gradients; products that just fit stay finite."""
+    x, w = torch.ones(150, fin, device="cuda"), torch.ones(fin, 136, device="cuda")
+    x[0], x[1], x[2], x[140] = 1.0039e30, -4 * 1.0039e30, 16 * 1.0009e30, -64 * 1.0009e30   # (sums that do not cancel)
+    w[:, 3], w[:, 135] = 1e20, -4e20
+    x[5, 7], w[7, 9] = 1.8e19, 1.8e19            # 3.24e38: finite
+    dy = torch.ones(150, 136, device="cuda")
+    dy[0, 3] = 1.0039e20                         # dx[0] = dy w^T and dw[:, 3] = x^T dy overflow
+    y = tt.fc_forward(x, w)
+    dx, dw, _ = tt.fc_backward(x, w, dy)
+    tt.check_device_status()
+    for name, got, want in (("y", y, x.double() @ w.double()), ("dx", dx, dy.double() @ w.double().t()), ("dw", dw, x.double().t() @ dy.double())):
+        over = want.abs() > torch.finfo(torch.float32).max
+        assert bool((got[over] == want[over].sign().float() * float("inf")).all()), name
+        assert torch.allclose(got[~over].double(), want[~over], rtol=1e-5, atol=0), name
+    assert bool(torch.isinf(y).any()) and bool(torch.isinf(dx).any()) and bool(torch.isinf(dw).any())
