@@ -720,10 +720,13 @@ cudaError_t fc_gemm(const void* A, const void* B, void* C, const void* bias, lon
     return cudaGetLastError();
 }
 
-// Row ranges: about four CTAs of 256 columns per SM, each of at least 64 rows (eight per warp).
+// Row ranges: about four CTAs of 256 columns per SM, each of at least 64 rows (eight per warp); for the sake of precision never
+// fewer than one per 256 rows up to 64, because a thread adds the rows of a range one after the other.  Float [16384,152000]:
+// error 2.2e-7 in one range, 1431 us, 4.9e-8 in 64, 1384 us (two-level sums inside one range: 5.4e-8, 1512 us).
 static int fc_colsum_splits(long long M, int N) {
     const long long blocks = (N + 255) / 256, most = std::max(1LL, (4LL * sm_count() + blocks - 1) / blocks);
-    return (int)std::max(1LL, std::min(std::min(most, 256LL), M / 64));
+    const long long least = std::min(64LL, (M + 255) / 256);
+    return (int)std::max(std::max(1LL, least), std::min(std::min(most, 256LL), M / 64));
 }
 size_t fc_colsum_workspace(long long M, int N) { return align256((size_t)fc_colsum_splits(M, N) * (size_t)N * sizeof(float)); }
 

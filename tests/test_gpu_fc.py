@@ -183,3 +183,19 @@ def test_fc_large_shape_takes_the_pair_kernel_and_matches(tt, oracle, torch_cuda
         assert torch.equal(a, b)
     ref = x[:256].float() @ w.float()
     assert bf16_close(oracle, got[0][:256].float().cpu().numpy(), ref.cpu().numpy())
+
+
+# a wide matrix (64 ranges, 32 rows per warp); a pitch that takes one value per load; many ranges of a narrow one; one range
+@pytest.mark.parametrize("rows,fout", [(16384, 151552), (4096, 150001), (70000, 520), (65, 1000)])
+def test_bias_gradient_of_many_rows_adds_in_short_chains(tt, torch_cuda, rows, fout):
+    """Column sums of positive floats, where every rounding shows.  A chain of n additions of equal terms has an error of at most
+    2^-23 / sqrt(12) * sqrt(n / 3) of its sum in the root mean square (3.4e-8 sqrt(n / 3)), and k chains next to one another
+    divide it by sqrt(k).  Here at most 45 rows by each of 8 warps, 8 warps, then 32 ranges by each of 8 warps and 8 warps again:
+    1.0e-7 together, a third more taken.  One chain over the 2048 rows of a warp, in a single range, gives 2.2e-7."""
+    torch = torch_cuda
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    dy = torch.rand(rows, fout, generator=g, device="cuda")
+    db = tt.fc_backward(torch.zeros(rows, 4, device="cuda"), torch.zeros(4, fout, device="cuda"), dy, need_dx=False, need_dw=False)[2]
+    tt.check_device_status()
+    want = sum(c.double().sum(0) for c in dy.split(512))
+    assert float((db.double() - want).norm() / want.norm()) <= 1.3e-7
