@@ -69,21 +69,25 @@ struct OnDevice {
     }
 };
 
-// float argument or None; `zero_is_none`: 0.0 also selects the default scale
+// float argument or None: whatever float() takes
 bool scale_arg(PyObject* o, float* out) {
     *out = 0.f;
     if (o == Py_None) return true;
-    const double x = PyFloat_AsDouble(o);
-    if (x == -1.0 && PyErr_Occurred()) return false;
-    *out = (float)x;
+    PyObject* x = PyNumber_Float(o);
+    if (!x) return false;
+    *out = (float)PyFloat_AS_DOUBLE(x);
+    Py_DECREF(x);
     return true;
 }
-bool int_arg(PyObject* o, int32_t* out) {
-    const long x = PyLong_AsLong(o);
-    if (x == -1 && PyErr_Occurred()) return false;
-    *out = (int32_t)x;
-    return true;
+// integer argument: whatever int() takes
+bool int_arg(PyObject* o, int64_t* out) {
+    PyObject* x = PyNumber_Long(o);
+    if (!x) return false;
+    *out = PyLong_AsLongLong(x);
+    Py_DECREF(x);
+    return !(*out == -1 && PyErr_Occurred());
 }
+bool fits32(int64_t x) { return x == (int32_t)x; }
 
 PyObject* wrap(const Tensor& t) { return THPVariable_Wrap(t); }
 PyObject* wrap_or(PyObject* given, const Tensor& made) {   // the caller's own object where it gave one
@@ -229,13 +233,14 @@ bool varlen_args(PyObject* const* a, const Tensor** q, const Tensor** k, const T
     for (const Tensor* c : {*cq, *ck})
         if (c->scalar_type() != at::kInt || c->dim() != 1 || c->numel() != (*cq)->numel()) return false;
     if (tk.size(2) != tq.size(2) || tk.size(1) < 1 || tq.size(1) % tk.size(1) != 0) return false;
-    int32_t mq, mk;
+    int64_t mq, mk;
     if (!int_arg(a[5], &mq) || !int_arg(a[6], &mk)) {
         *raised = true;
         return false;
     }
-    *d = tt_varlen_desc{(int32_t)(*cq)->numel() - 1, (int32_t)tq.size(1), (int32_t)tk.size(1), (int32_t)tq.size(2), TT_BF16, 0, 0.f, mq,
-                        mk, tq.size(0), tk.size(0)};
+    if (!fits32(mq) || !fits32(mk)) return false;
+    *d = tt_varlen_desc{(int32_t)(*cq)->numel() - 1, (int32_t)tq.size(1), (int32_t)tk.size(1), (int32_t)tq.size(2), TT_BF16, 0, 0.f, (int32_t)mq,
+                        (int32_t)mk, tq.size(0), tk.size(0)};
     return true;
 }
 
@@ -329,7 +334,8 @@ PyObject* attention_decode_paged(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const int64_t B = q->size(0), H = q->size(1), hkv = k->size(1);
         const int32_t* lens;
         if (hkv < 1 || H % hkv != 0 || !lens_arg(a[4], B, &lens)) Py_RETURN_NONE;
-        int32_t page = 0, max_pages = 0, L = (int32_t)k->size(2);
+        int32_t page = 0, max_pages = 0;
+        int64_t L = k->size(2);
         const int32_t* table = nullptr;
         if (a[3] != Py_None) {
             const Tensor* t = cuda_arg(a[3]);
@@ -337,17 +343,17 @@ PyObject* attention_decode_paged(PyObject*, PyObject* const* a, Py_ssize_t n) {
             table = (const int32_t*)t->data_ptr();
             page = (int32_t)k->size(2);
             max_pages = (int32_t)t->size(1);
-            L = page * max_pages;
+            L = (int64_t)page * max_pages;
         } else if (k->size(0) != B) {
             Py_RETURN_NONE;
         }
         if (a[5] != Py_None && !int_arg(a[5], &L)) return nullptr;
-        if (!table && L > k->size(2)) Py_RETURN_NONE;
+        if ((!table && L > k->size(2)) || !fits32(L)) Py_RETURN_NONE;
         bool fits = true;
         const Tensor *out = opt_arg(a[7], &fits), *lse = opt_arg(a[8], &fits), *ws = opt_arg(a[9], &fits);
         const int need_lse = PyObject_IsTrue(a[10]);
         if (!fits) Py_RETURN_NONE;
-        tt_attn_desc d{(int32_t)B, (int32_t)H, 1, L, (int32_t)q->size(3), TT_BF16, 0, 0.f, (int32_t)hkv};
+        tt_attn_desc d{(int32_t)B, (int32_t)H, 1, (int32_t)L, (int32_t)q->size(3), TT_BF16, 0, 0.f, (int32_t)hkv};
         if (need_lse < 0 || !scale_arg(a[6], &d.scale)) return nullptr;
         OnDevice dev(*q);
         Tensor new_out, new_lse, made;

@@ -114,7 +114,7 @@ def _explain_varlen(q, k, v, cu_q, cu_k):
             raise ValueError(f"{name} must be a contiguous CUDA int32 vector of n_seq + 1 cumulative token counts")
     if k.shape[2] != q.shape[2] or k.shape[1] < 1 or q.shape[1] % k.shape[1] != 0:
         raise ValueError(f"shape mismatch: q {tuple(q.shape)} k {tuple(k.shape)}")
-    raise ValueError("v, out, lse and dout must be CUDA tensors")
+    raise ValueError("v, out, lse and dout must be CUDA tensors, max_q and max_k 32-bit integers")
 
 
 def attention_forward_varlen(q, k, v, cu_q, cu_k, max_q, max_k, causal=False, scale=None, out=None, lse=None):
@@ -173,6 +173,7 @@ def _explain_paged(q, k_pool, v_pool, block_table, seq_lens, max_len):
             raise ValueError("a dense cache must be [B,Hkv,L,D]")
         if max_len is not None and int(max_len) > k_pool.shape[2]:
             raise ValueError("max_len exceeds the cache length")
+    raise ValueError("out, lse and workspace must be CUDA tensors, and lengths 32-bit integers")
 
 
 def attention_decode_paged(q, k_pool, v_pool, block_table=None, seq_lens=None, max_len=None, scale=None, out=None,
