@@ -64,8 +64,11 @@ struct OnDevice {
         }
         stream = (void*)c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)want).stream();
     }
-    ~OnDevice() {
-        if (before >= 0) c10::cuda::set_device((c10::DeviceIndex)before);
+    ~OnDevice() {   // an error here was the call's own already; a destructor that throws ends the process
+        try {
+            if (before >= 0) c10::cuda::set_device((c10::DeviceIndex)before);
+        } catch (const std::exception&) {
+        }
     }
 };
 
@@ -126,12 +129,16 @@ PyObject* guarded(F&& f) {
     return nullptr;
 }
 
-#define TT_CALL(rc, expr)      \
-    int rc;                    \
-    Py_BEGIN_ALLOW_THREADS     \
-    rc = (expr);               \
-    Py_END_ALLOW_THREADS
-
+// the GIL is taken again on every way out
+struct NoGil {
+    PyThreadState* state = PyEval_SaveThread();
+    ~NoGil() { PyEval_RestoreThread(state); }
+};
+#define TT_CALL(rc, expr) \
+    const int rc = [&] {  \
+        NoGil released;   \
+        return (expr);    \
+    }()
 
 // q [B,H,S,D], k and v [B,Hkv,L,D] of one type
 bool attn_args(PyObject* oq, PyObject* ok, PyObject* ov, const Tensor** q, const Tensor** k, const Tensor** v,
