@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(kThreads, 1) fc_f32_sm100_kernel(const FcF32Pa
     int mb, nb;
     fc_tile_coords((int)blockIdx.x / n_cta, p.tiles_m, p.tiles_n, mb, nb);
     const int m0 = mb * kTile, n0 = nb * kTile;
-    const int chunks = (p.K + kK - 1) / kK, share = (chunks + n_cta - 1) / n_cta;
+    const int chunks = (p.K - 1) / kK + 1, share = (chunks + n_cta - 1) / n_cta;
     const int u0 = rank * share, n_it = max(0, min(share, chunks - u0));
 
     float* tile = reinterpret_cast<float*>(smem);
@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(kThreads, 1) fc_f32_sm100_kernel(const FcF32Pa
 #pragma unroll
         for (int e = 0; e < 64; ++e) zero[e & 3] = fmaf(acc[e], 0.f, zero[e & 3]);
         if (zero[0] + zero[1] + zero[2] + zero[3] != 0.f) {
-            const int m = m0 + r, k_end = min(p.K, (u0 + n_it) * kK);
+            const int m = m0 + r, k_end = (int)min((long long)p.K, (long long)(u0 + n_it) * kK);
 #pragma unroll
             for (int e = 0; e < 64; ++e) acc[e] = 0.f;
             for (int k = u0 * kK; k < k_end && m < p.M; ++k) {
@@ -292,7 +292,7 @@ cudaError_t launch(const FcF32Params& p, int n_cta, cudaStream_t st) {
 // Every pitch and alignment; the operand forms of the layer: (a_mn, b_mn) = (0, 1), (0, 0) or (1, 1).
 bool fc_f32_tc_supported(long long M, int N, int K, int a_mn, int b_mn, int bf16) {
     if (bf16 || M < 1 || M > 0x7fffffffLL || N < 1 || K < 1 || (a_mn && !b_mn)) return false;
-    if (((M + kTile - 1) / kTile) * ((N + kTile - 1LL) / kTile) * 8 >= (1LL << 31)) return false;
+    if (((M - 1) / kTile + 1) * ((N - 1) / kTile + 1) * 8 >= (1LL << 31)) return false;
     const char* f = getenv("TT_FC_PATH");
     return !(f && f[0] == 's');   // "simt": force the fp32-arithmetic kernel (tests)
 }
@@ -301,13 +301,13 @@ cudaError_t fc_gemm_f32_sm100(const void* A, const void* B, void* C, const void*
     FcF32Params p = {};
     p.A = (const float*)A; p.B = (const float*)B; p.bias = (const float*)bias; p.C = (float*)C;
     p.M = M; p.N = N; p.K = K;
-    p.tiles_m = (M + kTile - 1) / kTile;
-    p.tiles_n = (N + kTile - 1) / kTile;
+    p.tiles_m = (M - 1) / kTile + 1;
+    p.tiles_n = (N - 1) / kTile + 1;
     p.wide = N % 4 == 0 && ((uintptr_t)C & 15) == 0;
     p.status = device_status_word();
     const int a_ld = a_mn ? M : K, b_ld = b_mn ? N : K;
     const bool vec = a_ld % 4 == 0 && b_ld % 4 == 0 && (((uintptr_t)A | (uintptr_t)B) & 15) == 0;
-    const int n_cta = fc_k_ctas((long long)p.tiles_m * p.tiles_n, (K + kK - 1) / kK);
+    const int n_cta = fc_k_ctas((long long)p.tiles_m * p.tiles_n, (K - 1) / kK + 1);
     if (a_mn && b_mn) return vec ? launch<true, true, true>(p, n_cta, st) : launch<true, true, false>(p, n_cta, st);
     if (!a_mn && b_mn) return vec ? launch<false, true, true>(p, n_cta, st) : launch<false, true, false>(p, n_cta, st);
     return vec ? launch<false, false, true>(p, n_cta, st) : launch<false, false, false>(p, n_cta, st);

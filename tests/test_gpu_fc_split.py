@@ -86,3 +86,14 @@ def test_float_products_that_overflow(tt, fin):
         assert bool((got[over] == want[over].sign().float() * float("inf")).all()), name
         assert torch.allclose(got[~over].double(), want[~over], rtol=1e-5, atol=0), name
     assert bool(torch.isinf(y).any()) and bool(torch.isinf(dx).any()) and bool(torch.isinf(dw).any())
+
+
+def test_float_rows_up_to_the_last_32_bit_number(tt):
+    """2^31 - 1 rows: tiles and row numbers end at the largest int."""
+    rows = 2 ** 31 - 1
+    x = torch.full((rows, 1), 3.0, device="cuda")
+    x[-1], x[-130], x[0] = 5.0, 7.0, 11.0
+    y = tt.fc_forward(x, torch.full((1, 1), 2.0, device="cuda"))
+    tt.check_device_status()
+    for a, b in zip(y.split(1 << 28), x.split(1 << 28)):
+        assert torch.equal(a, 2.0 * b)
