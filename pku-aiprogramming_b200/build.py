@@ -76,13 +76,19 @@ def build_library(force: bool = False, verbose: bool = False) -> str:
 
 
 def build_torch_binding(force: bool = False, verbose: bool = False) -> str:
-    """`lib/_ttorch.so`: functional.py's calls on torch tensors as a CPython extension (links libtt_attn.so)."""
+    """`lib/_ttorch.so`: functional.py's calls on torch tensors as a CPython extension (links libtt_attn.so).  It uses torch's C++
+    classes, so it belongs to the torch and Python that it was built with: `build/_ttorch.built_with` names them."""
+    import importlib.metadata
     import sysconfig
     src = os.path.join(HOST, "bind_torch.cpp")
     out = os.path.join(LIB_DIR, "_ttorch.so")
     newest = max(os.path.getmtime(src), os.path.getmtime(os.path.join(ROOT, "include", "tt_attn.h")))
-    if not force and os.path.exists(out) and os.path.getmtime(out) >= newest:
-        return out
+    stamp = os.path.join(OBJ, "_ttorch.built_with")
+    built_with = "torch %s, %s\n" % (importlib.metadata.version("torch"), sysconfig.get_config_var("EXT_SUFFIX"))
+    if not force and os.path.exists(out) and os.path.getmtime(out) >= newest and os.path.exists(stamp):
+        with open(stamp) as f:
+            if f.read() == built_with:
+                return out
     import torch
     base = os.path.dirname(torch.__file__)
     inc = [os.path.join(base, "include"), os.path.join(base, "include", "torch", "csrc", "api", "include"),
@@ -91,6 +97,8 @@ def build_torch_binding(force: bool = False, verbose: bool = False) -> str:
           "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch.compiled_with_cxx11_abi()), *["-I" + d for d in inc], src, "-o", out,
           "-L" + LIB_DIR, "-ltt_attn", "-L" + os.path.join(base, "lib"), "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu",
           "-lc10_cuda", "-lc10", "-Wl,-rpath,$ORIGIN"], verbose)
+    with open(stamp, "w") as f:
+        f.write(built_with)
     return out
 
 
