@@ -304,7 +304,8 @@ static bool decode_on_gq_kernel(const AttnArgs& a) {
 //     108 us, 304 of 4096 131 -> 104, 320 of 8192 262 -> 202, 384 of 3001 105 -> 94.
 //   Lengths that differ (`ragged`) and slices enough that one wave would not cut them short: a range is at most a share of
 //     the work, or the longest sequence runs alone at the end.  16 ranges per SM, of at least 1024 keys: 256 slices of 360 to
-//     7588 keys 123 -> 100 us, 512 of 1 to 16384 364 -> 321 (if all are equally long after all, 157 -> 172).
+//     7588 keys 123 -> 100 us, 512 of 1 to 16384 364 -> 321.  Lengths that are all equal after all lose: 256 slices of 8192 keys
+//     156 -> 158 us, 512 of 2048 84 -> 88 (differing lengths there 63 -> 61).
 //   Up to 512 keys (dense caches: 1023) stay one launch.
 static int gq_ranges(const AttnArgs& a, bool ragged, int* chunk) {
     const long long slices = a.BH / a.group, n_sm = sm_count(), at_once = 2 * n_sm;

@@ -459,8 +459,8 @@ fc_gemm_pair_sm100_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
     }
 }
 
-// fp32-arithmetic SIMT GEMM for float tensors and for shapes the tensor-core kernel does not
-// take (row pitches that are not multiples of 16 bytes).  64x64 tiles, 4x4 outputs per thread.
+// fp32-arithmetic SIMT GEMM for bf16 shapes the tensor-core kernel does not take (row pitches that are not multiples of
+// 16 bytes), and for floats where TT_FC_PATH=simt asks for it.  64x64 tiles, 4x4 outputs per thread.
 template <typename T> __device__ __forceinline__ float g_ld(const T* p, long long i);
 template <> __device__ __forceinline__ float g_ld<float>(const float* p, long long i) { return p[i]; }
 template <> __device__ __forceinline__ float g_ld<__nv_bfloat16>(const __nv_bfloat16* p, long long i) { return __bfloat162float(p[i]); }

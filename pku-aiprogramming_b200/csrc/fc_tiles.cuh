@@ -19,7 +19,9 @@ __device__ __forceinline__ void fc_tile_coords(int t, int tiles_m, int tiles_n, 
 // CTAs of a cluster that share a tile's sum over K: as many as the SMs that the tiles leave idle, up to 8 (the portable
 // cluster size), each with at least four of the `blocks` steps of 64 along K (the exchange costs about as much as those).
 // bf16 forward [256,8192]x[8192,512] (4 tiles, 128 blocks) 46.5 -> 18.3 us, [2048,4096]x[4096,1024] (64 tiles) 30.1 -> 21.1;
-// with 75 tiles and more every CTA keeps a tile of its own.
+// with 75 tiles and more every CTA keeps a tile of its own.  A cluster lies inside one GPC, so the largest counts of a size
+// do not all run at once: [128 t,8192]x[8192,256] with t = 16, 18, 19 35.1, 36.4, 23.3 us, 33, 37, 38 23.8, 43.3, 30.2 (one CTA
+// per tile 43 to 47).
 inline int fc_k_ctas(long long tiles, int blocks) {
     int n = 1;
     while (n < 8 && tiles * n * 2 <= sm_count() && blocks >= n * 2 * 4) n *= 2;

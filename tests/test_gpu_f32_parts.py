@@ -129,5 +129,5 @@ def test_infinities_nan_and_overflow(tt, oracle, D, name, row, value):
         ok = np.isfinite(r)
         # two float32 sums of up to 200 terms in different orders; values beyond 1e6 come from the large input: relative to them
         rows = np.abs(np.where(ok, r, 0)).reshape(S, -1).max(1)
-        err = np.abs(np.where(ok, g - r, 0)).reshape(S, -1).max(1)
+        err = np.abs(np.where(ok, g, 0) - np.where(ok, r, 0)).reshape(S, -1).max(1)
         assert bool((err <= 2e-5 * np.maximum(rows, 1.0)).all()), (what, float((err / np.maximum(rows, 1.0)).max()))

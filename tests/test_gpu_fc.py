@@ -93,6 +93,20 @@ def test_fc_unaligned_bf16_and_forced_simt_agree(tt, oracle, torch_cuda, monkeyp
     assert float((y_tc.float() - y_simt.float()).abs().max()) <= 2.0 ** -7 * float(y_simt.float().abs().max())
 
 
+def test_fc_forced_simt_on_floats(tt, oracle, torch_cuda, monkeypatch):
+    """The fp32 FMA kernel, which floats take only when TT_FC_PATH=simt asks for it."""
+    torch = torch_cuda
+    rng = np.random.default_rng(10)
+    xn, wn, bn, dyn = (rng.standard_normal(s).astype(np.float32) for s in ((130, 65), (65, 67), (67,), (130, 67)))
+    x, w, b, dy = (torch.from_numpy(a).cuda() for a in (xn, wn, bn, dyn))
+    monkeypatch.setenv("TT_FC_PATH", "simt")
+    assert tt.capi.lib.tt_fc_path(130, 65, 67, tt.capi.TT_F32) == 0
+    y = tt.fc_forward(x, w, b)
+    dx, dw, db = tt.fc_backward(x, w, dy)
+    for got, ref in zip((y, dx, dw, db), (oracle.fc_forward(xn, wn, bn),) + tuple(oracle.fc_backward(xn, wn, dyn))):
+        assert oracle.rel_err(got.cpu().numpy(), ref) <= 1e-5
+
+
 def test_fc_leading_axes_empty_and_errors(tt, oracle, torch_cuda):
     torch = torch_cuda
     x = torch.randn(2, 3, 40, 64, device="cuda").bfloat16(); w = torch.randn(64, 128, device="cuda").bfloat16()

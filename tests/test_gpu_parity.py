@@ -145,11 +145,12 @@ def test_odd_head_dims(tt, oracle, D, dtype):
 
 
 @pytest.mark.parametrize("route", ["tiled", "rows"])
-@pytest.mark.parametrize("D,dtype", [(40, "f32"), (128, "f32"), (50, "f32"), (72, "bf16")])
+@pytest.mark.parametrize("D,dtype", [(40, "f32"), (128, "f32"), (50, "f32"), (72, "bf16"), (40, "bf16"), (60, "bf16"), (50, "bf16")])
 def test_simt_kernel_routes(tt, oracle, monkeypatch, route, D, dtype):
-    """The fp32-arithmetic kernels come in two forms: register-tiled (head dims that are multiples
-    of 4 up to 128) and row-per-lane (everything else, or forced with TT_SIMT_FWD/BWD=rows).  Both
-    must meet the same tolerance on a ragged causal shape with L != S."""
+    """What does not run on bf16 tensor-core tiles: floats with head dims that are multiples of 4 take the kernel on three
+    bf16 parts; bf16 with such head dims (other than 64, 128) the register-tiled fp32 kernels (two widths, up to 64 and up
+    to 128); the rest, or everything with TT_SIMT_FWD/BWD=rows, the row-per-lane fp32 kernels.  All must meet the same
+    tolerance on a ragged causal shape with L != S."""
     if route == "rows":
         monkeypatch.setenv("TT_SIMT_FWD", "rows")
         monkeypatch.setenv("TT_SIMT_BWD", "rows")
@@ -160,9 +161,17 @@ def test_simt_kernel_routes(tt, oracle, monkeypatch, route, D, dtype):
     o_ref, lse_ref, dq_ref, dk_ref, dv_ref = oracle.attention_backward(q, k, v, do, True)
     tdt = torch.float32 if dtype == "f32" else torch.bfloat16
     tq, tk, tv, tdo = (_dev(x, tdt) for x in (q, k, v, do))
+    tt.capi.profile_enable(True)
+    tt.capi.profile_reset()
     out, lse = tt.attention_forward(tq, tk, tv, causal=True)
     dq, dk, dv = tt.attention_backward(tq, tk, tv, out, lse, tdo, causal=True)
+    ran = {name for name, (_, n) in tt.capi.profile_read().items() if n}
+    tt.capi.profile_enable(False)
     tt.check_device_status()
+    if dtype == "f32" and D % 4 == 0 and route == "tiled":
+        assert ran == {"attn_fwd_f32_sm100", "attn_bwd_f32_sm100", "attn_bwd_simt_delta"}
+    else:
+        assert ran == {"attn_fwd_simt", "attn_bwd_simt_delta", "attn_bwd_simt_dq", "attn_bwd_simt_dkv"}
     assert oracle.max_abs_err(_np(lse), lse_ref) <= (1e-4 if dtype == "f32" else 2e-2)
     for got, ref in ((out, o_ref), (dq, dq_ref), (dk, dk_ref), (dv, dv_ref)):
         if dtype == "f32":

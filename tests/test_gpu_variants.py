@@ -83,6 +83,21 @@ def dense_decode_ref(oracle, q, k, v, lens=None):
     return out, lse
 
 
+def key_ranges(torch, slices, L, ragged):
+    """Ranges per slice by the rule of the keys-on-rows decode kernel (groups up to 16): whole 128-key tiles, two CTAs per SM."""
+    n_sm = torch.cuda.get_device_properties(0).multi_processor_count
+    want, least = max(1, 2 * n_sm // slices), 256
+    units = slices * want
+    if ragged and 2 * slices > n_sm:
+        want, least = 16 * n_sm // slices, 1024
+    elif 4 * units < 3 * -(-units // (2 * n_sm)) * 2 * n_sm:
+        want, least = -(-8 * n_sm // slices), 1024
+    if want < 2 or L <= (512 if ragged else 1023):
+        return 1
+    chunk = -(-max(least, -(-L // want), -(-L // 128)) // 128) * 128
+    return -(-L // chunk)
+
+
 @pytest.mark.parametrize("H,Hkv,D", [(8, 8, 128), (8, 4, 128), (8, 2, 64), (8, 1, 128), (6, 2, 128), (16, 2, 64)])
 def test_decode_grouped_heads(tt, oracle, torch_cuda, H, Hkv, D):
     """Group sizes 1, 2, 4, 8 (one pass over K/V per group) and 3 (mapped fallback)."""
@@ -111,8 +126,8 @@ def test_decode_grouped_heads_on_the_forward_kernel(tt, oracle, torch_cuda, monk
         out, lse = tt.attention_decode(tq, tk, tv)
         tt.check_device_status()
         # few slices: the split-KV kernel and the forward kernel (groups above 16) cut the 1000 keys into ranges and
-        # merge them (two launches); the keys-on-rows kernel (groups up to 16) keeps ranges of at least 512 keys
-        # that divide the key count, which 1000 keys do not offer: one launch
+        # merge them (two launches); the keys-on-rows kernel (groups up to 16) leaves dense caches of up to 1023 keys
+        # whole: one launch
         assert tt.capi.launch_count() - before == (1 if (route == "tc" and H // Hkv <= 16) else 2), route
         assert oracle.max_abs_err(out.float().cpu().numpy(), o_r) <= 2e-2, route
         assert oracle.max_abs_err(lse.cpu().numpy(), lse_r) <= 1e-3, route
@@ -121,15 +136,15 @@ def test_decode_grouped_heads_on_the_forward_kernel(tt, oracle, torch_cuda, monk
 
 @pytest.mark.parametrize("B,H,Hkv,L,D", [(2, 8, 2, 4096, 128), (1, 32, 4, 3000, 64), (160, 4, 1, 300, 128)])
 def test_decode_grouped_heads_key_split_on_the_forward_kernel(tt, oracle, torch_cuda, B, H, Hkv, L, D):
-    """Default routing: few (batch, key/value head) slices -> the keys are split into ranges that run as
-    forward-kernel work items and are merged; many slices -> one item per slice, no merge."""
+    """Default routing of groups up to 16, the keys-on-rows kernel: few (batch, key/value head) slices and a long cache
+    -> the keys are split into ranges and merged; else one item per slice, no merge."""
     torch = torch_cuda
     q, k, v, _ = make_grouped(oracle, 170 + H, B, H, Hkv, 1, L, D, True)
     tq, tk, tv = (torch.from_numpy(a).cuda().bfloat16() for a in (q, k, v))
     before = tt.capi.launch_count()
     out, lse = tt.attention_decode(tq, tk, tv)
     tt.check_device_status()
-    assert tt.capi.launch_count() - before == (1 if B * Hkv >= 148 else 2)
+    assert tt.capi.launch_count() - before == (1 if key_ranges(torch, B * Hkv, L, False) == 1 else 2)
     o_r, lse_r = dense_decode_ref(oracle, q, k, v)
     assert oracle.max_abs_err(out.float().cpu().numpy(), o_r) <= 2e-2
     assert oracle.max_abs_err(lse.cpu().numpy(), lse_r) <= 1e-3
@@ -177,10 +192,9 @@ def test_decode_paged_and_ragged(tt, oracle, torch_cuda, H, Hkv, D, page):
     (5, 8, 2, 128, 64, 12, "tc"), (5, 8, 1, 128, 128, 5, "tc"), (4, 16, 4, 64, 16, 40, "tc"), (3, 8, 2, 128, 256, 3, "tc"),
     (3, 4, 1, 64, 8, 50, "tc"), (40, 8, 2, 128, 32, 9, None), (3, 8, 2, 128, 64, 40, None), (3, 32, 4, 64, 32, 70, None), (5, 8, 2, 128, 64, 12, "simt")])
 def test_decode_paged_grouped_heads_on_the_forward_kernel(tt, oracle, torch_cuda, monkeypatch, B, H, Hkv, D, page, max_pages, route):
-    """Paged cache with group >= 4: the forward kernel gathers each key tile page by page.  Rows of
+    """Paged cache with group >= 4: the keys-on-rows kernel gathers each key tile page by page.  Rows of
     the pools that no sequence owns hold NaN (a cache allocated but never written may), sequences are
-    ragged and one is empty; result = oracle on the dense cache, and route `None` checks the default
-    (B * Hkv about fills the GPU -> forward kernel, one launch)."""
+    ragged and one is empty; result = oracle on the dense cache.  The number of launches follows the key ranges."""
     torch = torch_cuda
     rng = np.random.default_rng(B * 1000 + page)
     cap = page * max_pages
@@ -209,11 +223,8 @@ def test_decode_paged_grouped_heads_on_the_forward_kernel(tt, oracle, torch_cuda
     out, lse = tt.attention_decode_paged(tq, tkp, tvp, block_table=table, seq_lens=tl)
     tt.check_device_status()
     if route != "simt":
-        # the tensor-core decode kernel alone when the slices fill the GPU or the cache is short, else over
-        # key ranges (whole 128-key tiles, at least 512 keys, about four ranges per SM) + merge
-        want = -(-4 * 148 // (B * Hkv))
-        chunk = max(512, -(-(-(-cap // want)) // 128) * 128)
-        assert tt.capi.launch_count() - before == (1 if B * Hkv >= 148 or -(-cap // chunk) < 2 else 2)
+        # the keys-on-rows kernel alone, or over key ranges + merge
+        assert tt.capi.launch_count() - before == (1 if key_ranges(torch, B * Hkv, cap, True) == 1 else 2)
     got, got_lse = out.float().cpu().numpy(), lse.cpu().numpy()
     assert np.isfinite(got).all()
     assert np.isneginf(got_lse[1]).all() and float(np.abs(got[1]).max()) == 0.0   # the empty sequence
