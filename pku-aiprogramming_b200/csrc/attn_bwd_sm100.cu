@@ -30,6 +30,7 @@
 // Shared memory: the resident pair plus rings of 3 (T0) and 2 (T1) streamed tiles at D = 128,
 // barriers and 2 KB of per-column statistics: exactly 227 KB.
 #include "attn_bwd_common.cuh"
+#include <limits.h>
 #include <string.h>
 #include <algorithm>
 
@@ -66,11 +67,10 @@ enum BwdBarId { BB_RES = 0, BB_STFULL = 10, BB_STEMPTY = 20, BB_SFULL = 30, BB_D
 // MMAs of the next item overlap the write-out of the accumulators of the current one.
 // kTrace: compiled with the cycle stamps (debug aid; launched only while a trace buffer is set).
 // kVarlen: packed variable-length batches (per-item sequence geometry, token-major addressing).
+// first_item: the item that this CTA starts with.
 template <int D, bool kKeysResident, bool kTrace, bool kVarlen>
-__global__ void __launch_bounds__(BwdCfg<D>::kThreads, 1)
-attn_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmR0, const __grid_constant__ CUtensorMap tmR1,
-                      const __grid_constant__ CUtensorMap tmT0, const __grid_constant__ CUtensorMap tmT1,
-                      const BwdParams p) {
+__device__ __forceinline__ void bwd_cta(const CUtensorMap& tmR0, const CUtensorMap& tmR1, const CUtensorMap& tmT0, const CUtensorMap& tmT1,
+                                        const BwdParams& p, const int first_item) {
     using Cfg = BwdCfg<D>;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem = smem_raw;
@@ -486,7 +486,7 @@ attn_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmR0, const __grid_con
                 for (int sb = 0; sb < Cfg::kSub; ++sb) tma_load_3d(dst + sb * Cfg::kSubBytes, tm, bar, sb * 64, row_start, bh);
             };
             uint32_t git = 0;
-            int item = (int)blockIdx.x;
+            int item = first_item;
             for (int k = 0;; ++k, item = items.next(wctx, 89, k)) {
                 BwdItem w;
                 while (item >= 0) {
@@ -679,6 +679,28 @@ attn_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmR0, const __grid_con
     if (warp == 9 && *abort_flag) items.drop_rest(wctx.budget);
 }
 
+template <int D, bool kKeysResident, bool kTrace, bool kVarlen>
+__global__ void __launch_bounds__(BwdCfg<D>::kThreads, 1)
+attn_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmR0, const __grid_constant__ CUtensorMap tmR1,
+                      const __grid_constant__ CUtensorMap tmT0, const __grid_constant__ CUtensorMap tmT1,
+                      const BwdParams p) {
+    bwd_cta<D, kKeysResident, kTrace, kVarlen>(tmR0, tmR1, tmT0, tmT1, p, (int)blockIdx.x);
+}
+// Both passes in one launch: the dK/dV pass's items (`pk`), then the dQ pass's (`pq`), a CTA for each.  Neither needs the
+// other, only the statistics; as two launches the second waits for the first, which leaves SMs idle where the dK/dV pass has
+// few items.  Backward, two launches -> one (items of each): [1,24,1024,128] (192, 192) 62 -> 49 us, [1,8,4096,128] causal
+// (256, 256) 134 -> 111, 32 query heads on 4 key/value heads, [2,32,2048,128] causal (128, 1024) 309 -> 252; but one wave of
+// items that are all alike, [1,64/8,2048,128] (128, 1024), 358 -> 373, and with (296, 296), [1,37,1024,128], 65 -> 70.
+template <int D, bool kVarlen>
+__global__ void __launch_bounds__(BwdCfg<D>::kThreads, 1)
+attn_bwd_both_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
+                           const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmdO,
+                           const BwdParams pk, const BwdParams pq) {
+    const int item = (int)blockIdx.x;
+    if (item < pk.n_items) bwd_cta<D, true, false, kVarlen>(tmK, tmV, tmQ, tmdO, pk, item);
+    else bwd_cta<D, false, false, kVarlen>(tmQ, tmdO, tmK, tmV, pq, item - pk.n_items);
+}
+
 // ---------------------------------------------------------------- preprocessing
 // delta[row] = sum_d dO*O ; lse2[row] = lse[row] * log2(e).  HBM-bound: D/8 lanes share a row (16 bytes
 // of O and of dO per lane), a warp covers 32/(D/8) rows per load instruction and keeps kPrepUnroll of
@@ -838,24 +860,41 @@ static cudaError_t launch_bwd(const AttnArgs& a, void* ws, cudaStream_t st) {
     p.n_items = (int)(a.BH / a.group * p.n_tiles);
     p.n_light = a.causal ? p.n_tiles / 4 : 0;
     p.n_items_heavy = (int)(a.BH / a.group * (p.n_tiles - p.n_light));
-    if (D == 128 && !kTrace && !kVarlen && attn_bwd_dkv_pair_supported(a)) {
+    // dQ: queries resident, stream (K, V)
+    BwdParams pq = p;
+    pq.trace = g_bwd_trace_mode == 2 ? g_bwd_trace : nullptr;
+    pq.out0 = nullptr;
+    pq.out1 = (__nv_bfloat16*)a.dq;
+    pq.n_tiles = (a.S + 127) / 128;
+    pq.n_items = (int)(a.BH * pq.n_tiles);
+    pq.n_light = a.causal ? pq.n_tiles / 4 : 0;
+    pq.n_items_heavy = (int)(a.BH * (pq.n_tiles - pq.n_light));
+    const bool pair = D == 128 && !kTrace && !kVarlen && attn_bwd_dkv_pair_supported(a);
+    if constexpr (!kTrace) {
+        // Up to 1.8 waves of dK/dV items: the dQ pass's items fill the SMs that those leave idle.  Behind more, or a second wave
+        // nearly full, a launch for each pass, whose CTAs take over items, loses less.  (As the last pass the dQ pass may write
+        // over q or dout, each of its items has read its own rows of them by then; beside the other pass it may not.)
+        const uintptr_t dq = (uintptr_t)a.dq, bytes = (uintptr_t)(kVarlen ? a.total_q * a.H : a.BH * a.S) * D * sizeof(__nv_bfloat16);
+        auto apart = [&](const void* t) { return dq + bytes <= (uintptr_t)t || (uintptr_t)t + bytes <= dq; };
+        if (!pair && 5LL * p.n_items <= 9LL * p.first_wave && apart(a.q) && apart(a.dout)) {
+            e = TT_ALLOW_SMEM((attn_bwd_both_sm100_kernel<D, kVarlen>), Cfg::kSmemBytes);
+            if (e != cudaSuccess) return e;
+            p.first_wave = pq.first_wave = INT_MAX;   // nothing is taken over: the next item may be the other pass's
+            LaunchScope ls(K_BWD_BOTH, st);
+            return launch_overlapped(attn_bwd_both_sm100_kernel<D, kVarlen>, (unsigned)(p.n_items + pq.n_items), Cfg::kThreads, Cfg::kSmemBytes, st,
+                                     M(tk), M(tv), M(tq), M(tdo), p, pq);
+        }
+    }
+    if (pair) {
         // same pass on CTA pairs: each MMA reads half of its streamed operand per SM
         if ((e = attn_bwd_dkv_pair(a, delta, lse2, st)) != cudaSuccess) return e;
     } else {
         LaunchScope ls(K_BWD_DKV, st);
         launch_overlapped(attn_bwd_sm100_kernel<D, true, kTrace, kVarlen>, (unsigned)p.n_items, Cfg::kThreads, Cfg::kSmemBytes, st, M(tk), M(tv), M(tq), M(tdo), p);
     }
-    // dQ: queries resident, stream (K, V)
-    p.trace = g_bwd_trace_mode == 2 ? g_bwd_trace : nullptr;
-    p.out0 = nullptr;
-    p.out1 = (__nv_bfloat16*)a.dq;
-    p.n_tiles = (a.S + 127) / 128;
-    p.n_items = (int)(a.BH * p.n_tiles);
-    p.n_light = a.causal ? p.n_tiles / 4 : 0;
-    p.n_items_heavy = (int)(a.BH * (p.n_tiles - p.n_light));
     {
         LaunchScope ls(K_BWD_DQ, st);
-        launch_overlapped(attn_bwd_sm100_kernel<D, false, kTrace, kVarlen>, (unsigned)p.n_items, Cfg::kThreads, Cfg::kSmemBytes, st, M(tq), M(tdo), M(tk), M(tv), p);
+        launch_overlapped(attn_bwd_sm100_kernel<D, false, kTrace, kVarlen>, (unsigned)pq.n_items, Cfg::kThreads, Cfg::kSmemBytes, st, M(tq), M(tdo), M(tk), M(tv), pq);
     }
     return cudaGetLastError();
 }

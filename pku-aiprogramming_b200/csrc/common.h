@@ -123,7 +123,7 @@ int check_device();   // TT_OK, or TT_ERR_BAD_DEVICE when the current device is 
 enum KernelId {
     K_FWD_TC = 0, K_FWD_SIMT, K_BWD_PREP, K_BWD_DKV, K_BWD_DQ, K_BWD_SIMT_DELTA, K_BWD_SIMT_DQ, K_BWD_SIMT_DKV,
     K_DECODE, K_DECODE_MERGE, K_PROBE, K_SOFTMAX_FWD, K_SOFTMAX_BWD, K_FC_GEMM, K_FC_SIMT, K_FC_COLSUM, K_BWD_FUSED,
-    K_BWD_DQ_CONVERT, K_DECODE_GQ, K_FWD_F32, K_BWD_F32, K_COUNT
+    K_BWD_DQ_CONVERT, K_DECODE_GQ, K_FWD_F32, K_BWD_F32, K_BWD_BOTH, K_COUNT
 };
 // Scoped around ONE kernel launch: counts it and, when timing is enabled, brackets it with
 // CUDA events on the launching stream.
