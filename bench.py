@@ -46,7 +46,7 @@ WORKLOADS = {
 # captured on a few slices of the workload's slice shape and scale with the slice count (the kernels walk
 # the slices one after the other, so a slice's traffic does not depend on how many follow).
 NCU_TRAFFIC_BYTES = {
-    "cfg3": {"attn_fwd_sm100": 591.5e6, "attn_bwd_sm100_dkv": 851.6e6, "attn_bwd_sm100_dq": 728.4e6,
+    "cfg3": {"attn_fwd_sm100": 593.0e6, "attn_bwd_sm100_dkv": 850.5e6, "attn_bwd_sm100_dq": 729.1e6,
              "attn_bwd_fused_sm100": 1507.7e6},
     "cfg2": {"attn_fwd_sm100": 52.3e6, "attn_bwd_fused_sm100": 132.1e6},
     "cfg5_per_slice": {"attn_fwd_sm100": 26.08e6, "attn_bwd_sm100_dkv": 35.10e6, "attn_bwd_sm100_dq": 34.66e6},
