@@ -728,7 +728,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_f32_sm100_kernel(const F32Pa
             rest.drop_rest(ctx.budget);
         }
     }
-    if (again) f32_plain_row<DP, kBwd>(p, smem, threadIdx.x);
+    if (again && !*abort_flag) f32_plain_row<DP, kBwd>(p, smem, threadIdx.x);
 }
 
 // delta = rowsum(dO * O): 8 lanes share a row, four rows per warp and step; HBM-bound.
