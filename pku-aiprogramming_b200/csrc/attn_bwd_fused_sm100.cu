@@ -13,23 +13,29 @@
 //   G3: dV  += P^T dO       (A = bf16 P^T in tensor memory over S^T, B = dO MN-major)
 //   G4: dK  += dS^T Q       (A = bf16 dS^T in SHARED memory, K-major;  B = Q MN-major)
 //   G5: dQ_t = dS K         (A = the same dS^T bytes read MN-major;    B = K MN-major)   -> Y
-// Tensor memory (512 columns): X [0,128) S^T then P^T | Y [128,256) dP^T then dQ_t | dV [256,256+D) |
-// dK [256+D,256+2D).  dS^T cannot stay in tensor memory as in the two-pass kernel: G5 needs it with the
-// queries on the M side, and a tensor-memory operand is always M = lanes = keys here.  So the compute
-// threads write it to a 32 KB shared-memory tile in the 128-byte-swizzled layout both descriptors read.
-// The MMA warp issues, per tile t:   G3(t)  G1(t+1)  G5(t)  G4(t)  G2(t+1)
-// so that the tensor pipe always has work while the compute warpgroups turn S^T into P^T (phase A) and
-// dP^T into dS^T (phase B).  dQ_t leaves through the compute threads in the middle of the next tile's
-// phase A: tensor memory -> registers -> red.global.add.v4.f32 into a [D/4][128 rows][4] block per
-// (query slice, query tile), a layout in which the 32 lanes of a warp add to 512 contiguous bytes.  A
-// small second kernel converts the accumulator to bf16 dQ (times scale).  The additions arrive in no
-// fixed order, so dQ is reproducible to fp32 rounding only; dK and dV are bit-reproducible.
+// Tensor memory (512 columns): X [0,128) S^T | Y [128,256) dP^T | dV [256,256+D) | dK [256+D,256+2D).  At D = 128 that is all
+// of it: P^T overlays X and dQ_t overlays Y, and the MMA warp issues, per tile t, G3(t) G1(t+1) G5(t) G4(t) G2(t+1).  At D = 64
+// dQ_t and P^T have columns of their own, S^T(t+1) is issued as soon as S^T(t) is in registers and dP^T(t+1) as soon as
+// dS^T(t) is: G1(t+1) G3(t) G2(t+1) G5(t) G4(t).
+// dS^T cannot stay in tensor memory as in the two-pass kernel: G5 needs it with the queries on the M side, and a
+// tensor-memory operand is always M = lanes = keys here.  So the compute threads write it to a 32 KB shared-memory tile in
+// the 128-byte-swizzled layout both descriptors read.
 //
-// Roles: warps 0-7 = two compute warpgroups (thread <-> resident key row; warpgroup w owns query
-// columns [64w, 64w+64) of X and Y, and columns [w*D/2, +D/2) of dQ_t, dV, dK), warp 8 = MMA issuer,
-// warp 9 = TMA loader and work-item scheduler.
-// Shared memory at D = 128: K, V, two Q slots, two dO slots, the dS^T tile (7 x 32 KB) + 3 KB of barriers
-// and per-query statistics = exactly 227 KB.
+// dQ_t leaves through a warpgroup of its own: tensor memory -> registers (Y is released at once) -> 16 KB pieces in shared
+// memory -> cp.reduce.async.bulk add.f32 into a [D/4][128 rows][4] block per (query slice, query tile).  A small second
+// kernel converts the accumulator to bf16 dQ (times scale).  The L2 takes about 3-4 KB of fp32 additions per cycle from the
+// whole chip, and what waits for it must not be a warp's memory instruction: with red.global.add the additions held up the
+// memory queue that the compute warps' tensor-memory and shared-memory accesses share, from whichever warps they were
+// issued (cycles per tile, S = 4096 not causal: red from the compute warps 5069 at D = 128, 4546 at D = 64; red from the
+// adding warpgroup 5536, 4727; bulk additions 4043, 3842).  Statistics by bulk copies, already negated and padded to whole
+// tiles, and positions stepped instead of divided out: 3818, 3125.  Of those 3818, the additions of 64 KB take ~3200.
+// The additions arrive in no fixed order, so dQ is reproducible to fp32 rounding only; dK and dV are bit-reproducible.
+//
+// Roles: warps 0-7 = two compute warpgroups (thread <-> resident key row; warpgroup w owns query columns [64w, 64w+64) of X
+// and Y, and columns [w*D/2, +D/2) of dV, dK), warps 8-11 = the adding warpgroup (thread <-> query row), warp 12 = MMA
+// issuer, warp 13 = TMA loader and work-item scheduler.
+// Shared memory at D = 128: K, V, two Q slots, one dO slot, the dS^T tile, 2 x 16 KB of dQ_t pieces (7 x 32 KB) + 2.5 KB of
+// barriers and per-query statistics.
 #include "attn_bwd_common.cuh"
 #include <stdlib.h>
 #include <string.h>
@@ -41,49 +47,66 @@ namespace ttk {
 using namespace sm100;
 
 template <int D>
-struct Bwd1Cfg : BwdRegs {
+struct Bwd1Cfg {
+    // warps 0-7 compute, 8-11 add dQ_t, 12 issues MMAs, 13 loads, 14 and 15 only complete a warpgroup for setmaxnreg
+    static constexpr int kThreads = 512;
+    static constexpr int kRegsLaunch = 128, kRegsCompute = 144, kRegsAdd = 152, kRegsOther = 72;
+    static_assert(256 * kRegsCompute + 128 * kRegsAdd + 128 * kRegsOther <= kThreads * kRegsLaunch, "register split exceeds the CTA's pool");
     static constexpr int kSub = D / 64;
     static constexpr int kSubBytes = 128 * 128;
     static constexpr int kTileBytes = kSub * kSubBytes;
     static constexpr int kDsBytes = 2 * kSubBytes;               // 128 keys x 128 queries, bf16
     // Q(t) is read by G1(t) early and by G4(t) late, Q(t+1) in between; dO(t) by G2(t) and G3(t), and
-    // dO(t+1) only by the last GEMM of the next iteration, so ONE dO slot is enough.  At D = 128 four
-    // streamed slots fit beside K, V and dS^T: three go to Q, whose loads then run a tile further ahead
-    // (the L2 is busy with the dQ additions, and loads come back late: 2 + 2 slots measured 12 % slower
-    // at S = 32768).
-    static constexpr int kNQ = (D == 128) ? 3 : 4;
+    // dO(t+1) only by the last GEMM of the next iteration, so ONE dO slot is enough.
+    static constexpr int kNQ = (D == 128) ? 2 : 4;
     static constexpr int kNdO = (D == 128) ? 1 : 3;
     static_assert(kNQ >= 2 && kNQ <= 4 && kNdO >= 1 && kNdO <= 4, "ring lengths the barrier arrays are sized for");
     static constexpr int kTmemCols = 512;
-    static constexpr int kAuxBytes = 3072;                       // 1 KB barriers + 2 KB lse/delta staging
-    static constexpr int kSmemBytes = (2 + kNQ + kNdO) * kTileBytes + kDsBytes + kAuxBytes;
+    static constexpr int kBarBytes = 512;
+    static constexpr int kStatBytes = 2 * 128 * 4;               // -lse2 and -delta of a tile's 128 queries; two such slots
+    static constexpr int kAuxBytes = kBarBytes + 2 * kStatBytes;
+    static constexpr int kStageBytes = 128 * 32 * 4;             // 32 columns of dQ_t; two such buffers
+    static constexpr int kSmemBytes = (2 + kNQ + kNdO) * kTileBytes + kDsBytes + 2 * kStageBytes + kAuxBytes;
     static_assert(kSmemBytes <= 227 * 1024, "exceeds the shared memory of one CTA");
 };
 
 enum Bwd1BarId { B1_RES = 0, B1_QFULL = 10, B1_QEMPTY = 14, B1_DOFULL = 18, B1_DOEMPTY = 22, B1_SFULL = 30, B1_DPFULL = 31,
                  B1_PFULL = 32, B1_DSFULL = 33, B1_FINAL = 34, B1_STAT = 35, B1_DSFREE = 36, B1_DQFULL = 37, B1_DQFREE = 38,
-                 B1_ACCFREE = 39 };
+                 B1_ACCFREE = 39, B1_SREAD = 40, B1_PFREE = 41 };
 
 // The u-th streamed tile of an item: as in the two-pass kernel (heads of a group one after the other), but
 // without a causal mask every key tile of a slice meets ALL query tiles, and CTAs that started together
 // would walk them in step and add their dQ_t into the same 64 KB at the same moment; so key tile r starts
 // its walk at query tile r and wraps round.  (Under the causal mask key tile r starts at query tile r anyway.)
-__device__ __forceinline__ void fused_stream_tile(const BwdItem& w, int u, int group, int causal, int& t, int& slice) {
-    const int hh = u / w.nt;
-    int i = u - hh * w.nt;
-    if (!causal) {
-        i += (w.r0 >> 7) % w.nt;
-        if (i >= w.nt) i -= w.nt;
+// Walked step by step: the divisions of a position's closed form are some 400 cycles of latency per tile and role.
+struct FusedStream {
+    int t, slice;    // query tile and query slice of the current position
+    int first, j;    // the slice's first tile index (relative to t_begin) and the position in its walk
+    __device__ __forceinline__ FusedStream(const BwdItem& w, int group, int causal)
+        : slice(w.bh * group), first(causal || w.nt == 0 ? 0 : (w.r0 >> 7) % w.nt), j(0) { t = w.t_begin + first; }
+    __device__ __forceinline__ void next(const BwdItem& w) {
+        if (++j == w.nt) {
+            j = 0;
+            ++slice;
+            t = w.t_begin + first;
+        } else if (++t == w.t_end) {
+            t = w.t_begin;
+        }
     }
-    t = w.t_begin + i;
-    slice = w.bh * group + hh;
-}
+};
 
-__device__ __forceinline__ void red_add_v4(float* gptr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};"
-                 ::"l"(gptr), "f"(__uint_as_float(a)), "f"(__uint_as_float(b)), "f"(__uint_as_float(c)), "f"(__uint_as_float(d))
-                 : "memory");
+// Adds `bytes` of floats in shared memory to global memory by the TMA engine (one thread; a bulk group of its own).
+__device__ __forceinline__ void bulk_add_f32(float* gptr, const void* src, uint32_t bytes) {
+    asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;\n\tcp.async.bulk.commit_group;"
+                 ::"l"(gptr), "r"(smem_u32(src)), "r"(bytes) : "memory");
 }
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
+}
+template <int kLeft>   // at most kLeft groups of this thread have shared memory still to be read
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(kLeft) : "memory"); }
+__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
 #define TT_B1TRACE(role, iter, slot)                                                               \
     do {                                                                                           \
@@ -114,7 +137,8 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
     unsigned char* sQ = smem + 2 * Cfg::kTileBytes;             // kNQ slots
     unsigned char* sdO = sQ + kNQ * Cfg::kTileBytes;            // kNdO slots
     unsigned char* sDS = sdO + kNdO * Cfg::kTileBytes;          // dS^T: 2 sub-blocks of [128 keys x 64 queries]
-    unsigned char* aux = sDS + Cfg::kDsBytes;
+    unsigned char* sStage = sDS + Cfg::kDsBytes;                // two buffers of 32 dQ_t columns, [8][128 rows][4] floats
+    unsigned char* aux = sStage + 2 * Cfg::kStageBytes;
     uint64_t* bar_res_full = reinterpret_cast<uint64_t*>(aux);   // TMA -> MMA (K, V of the item)
     uint64_t* bar_res_empty = bar_res_full + 1;                  // MMA (last reads of K, V) -> TMA
     uint64_t* bar_q_full = bar_res_empty + 1;                    // [4]
@@ -132,13 +156,16 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
     uint64_t* bar_acc_free = bar_final + 1;                      // compute (accumulators read out) -> MMA
     uint64_t* bar_sched_full = bar_acc_free + 1;                 // [2]
     uint64_t* bar_sched_empty = bar_sched_full + 2;              // [2]
-    uint64_t* bar_stat = bar_sched_empty + 2;                    // [2] per warpgroup: a tile's statistics are staged
-    int* sched_item = reinterpret_cast<int*>(bar_stat + 2);      // [2]
+    uint64_t* bar_stat_full = bar_sched_empty + 2;               // [2] TMA -> compute: a tile's statistics
+    uint64_t* bar_stat_empty = bar_stat_full + 2;                // [2] compute -> TMA
+    uint64_t* bar_s_read = bar_stat_empty + 2;                        // D = 64, compute -> MMA: S^T(t) is in registers
+    uint64_t* bar_p_free = bar_s_read + 1;                       // D = 64, MMA -> compute: G3(t) is done with P^T(t)
+    int* sched_item = reinterpret_cast<int*>(bar_p_free + 1);    // [2]
     uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(sched_item + 2);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_base_slot + 1);
-    uint64_t* bar_steal = reinterpret_cast<uint64_t*>(aux + 1024 - 32);
+    uint64_t* bar_steal = reinterpret_cast<uint64_t*>(aux + Cfg::kBarBytes - 32);
     uint4* steal_response = reinterpret_cast<uint4*>(bar_steal + 2);
-    float* s_stat = reinterpret_cast<float*>(aux + 1024);       // [2 buffers][2: -lse2, -delta][128]
+    float* s_stat = reinterpret_cast<float*>(aux + Cfg::kBarBytes);   // [2 slots][2: -lse2, -delta][128]
 
     const int warp = uniform_warp_idx();
     const int lane = threadIdx.x & 31;
@@ -156,27 +183,30 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
             mbar_init(&bar_do_empty[s], 1);
         }
         mbar_init(bar_s_full, 1);
-        mbar_init(bar_p_full, 256);
+        mbar_init(bar_p_full, 8);
         mbar_init(bar_dp_full, 1);
-        mbar_init(bar_ds_full, 256);
+        mbar_init(bar_ds_full, 8);
         mbar_init(bar_ds_free, 1);
         mbar_init(bar_dq_full, 1);
-        mbar_init(bar_dq_free, 256);
+        mbar_init(bar_dq_free, 4);
+        mbar_init(bar_s_read, 8);
+        mbar_init(bar_p_free, 1);
         mbar_init(bar_final, 1);
-        mbar_init(bar_acc_free, 256);
+        mbar_init(bar_acc_free, 8);
         for (int i = 0; i < 2; ++i) {
-            mbar_init(&bar_stat[i], 128);
+            mbar_init(&bar_stat_full[i], 1);
+            mbar_init(&bar_stat_empty[i], 8);
             mbar_init(&bar_sched_full[i], 1);
-            mbar_init(&bar_sched_empty[i], 257);   // MMA warp (1) + 256 compute threads
+            mbar_init(&bar_sched_empty[i], 13);   // MMA warp, compute and adding warps
         }
         fence_barrier_init();
         fence_proxy_async_smem();
     }
-    if (warp == 8) {
+    if (warp == 12) {
         tmem_alloc(tmem_base_slot, Cfg::kTmemCols);
         tmem_relinquish();
     }
-    if (warp == 9 && lane == 0) {
+    if (warp == 13 && lane == 0) {
         tma_prefetch_desc(&tmK);
         tma_prefetch_desc(&tmV);
         tma_prefetch_desc(&tmQ);
@@ -191,12 +221,21 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
     grid_let_next_start();
     grid_wait_for_previous();
     constexpr uint32_t kColX = 0, kColY = 128, kColDV = 256, kColDK = 256 + D;
+    // At D = 64 the accumulators leave 128 columns, 64 for dQ_t and 64 for P^T: the scores of the next tile then wait for
+    // nothing but the loads of this tile's.
+    constexpr bool kApart = D == 64;
+    constexpr uint32_t kColDQ = kApart ? 384 : kColY, kColP = kApart ? 448 : kColX, kPitchP = kApart ? 32 : 64;
 
     auto next_item = [&](int k) -> int {
         const int slot = k & 1;
         // a wait that gave up (this CTA has aborted) ends the sequence: the slot may hold anything
         if (!mbar_wait(&bar_sched_full[slot], (k >> 1) & 1, wctx, 80 + slot, k)) return -1;
         return sched_item[slot];
+    };
+    // one arrival per warp, behind what all its threads did
+    auto warp_arrive = [&](uint64_t* bar) {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar);
     };
 
     if (warp < 8) {
@@ -208,117 +247,52 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
         const uint32_t lane_off = (uint32_t)(wq * 32) << 16;
         const uint32_t tX = tmem_base + lane_off + kColX + wg * 64;
         const uint32_t tY = tmem_base + lane_off + kColY + wg * 64;
-        const uint32_t tYq = tmem_base + lane_off + kColY + wg * (D / 2);   // this warpgroup's half of dQ_t
-        const int ctid = threadIdx.x;                          // 0..255 among compute threads
+        const uint32_t tP = tmem_base + lane_off + kColP + wg * kPitchP;
         const uint64_t c2 = pack_f32x2(p.scale_log2, p.scale_log2);
         unsigned char* ds_row = sDS + wg * Cfg::kSubBytes + r_in * 128;    // this thread's 128 bytes of dS^T
         uint32_t git = 0;      // streamed tiles processed so far, over all items (barrier phases)
 
-        // dQ_t leaves in two steps.  dq_take: tensor memory -> registers (this thread's query row, its
-        // warpgroup's D/2 columns), after which Y is released at once: the next dP^T GEMM waits for nothing
-        // but these loads.  dq_add: red.global.add.v4.f32 into the accumulator, a few at a time BETWEEN
-        // stretches of arithmetic and ahead of the waits, spread over a whole tile period: the L2 takes
-        // about 4 KB of such additions per cycle from the whole chip (measured: the 64 KB of a tile need
-        // ~2400 cycles with every SM adding), and a warp that issues sixteen of them back to back sits out
-        // most of that time in the issue stage.
-        uint32_t dqr[D / 64][32];
-        float* dq_base = nullptr;
-        int dq_owed = 0;          // additions of the registers' dQ_t not yet issued (they are issued in order)
-        auto dq_take = [&](int t, int qs, uint32_t g, int it) {
-            mbar_wait(bar_dq_full, g & 1, wctx, B1_DQFULL, it);
-            __syncwarp();
-            tc_fence_after();
-#pragma unroll
-            for (int cc = 0; cc < D / 64; ++cc) tmem_ld32(tYq + cc * 32, dqr[cc]);
-            tmem_wait_ld();
-            tc_fence_before();
-            mbar_arrive(bar_dq_free);
-            dq_base = p.dq_acc + ((size_t)((long long)qs * p.n_qt + t) * (D / 4) + (size_t)wg * (D / 8)) * 512 + r_in * 4;
-            dq_owed = D / 8;
-        };
-        // issues additions [first, first + count) of the D/8 this thread owes for the dQ_t in its registers
-        auto dq_add = [&](int first, int count) {
-            if (dq_owed == 0) return;
-#pragma unroll
-            for (int i = first; i < first + count; ++i) {
-                if (i < D / 8) {
-                    const int cc = i >> 3, j = i & 7;
-                    red_add_v4(dq_base + (size_t)i * 512, dqr[cc][4 * j], dqr[cc][4 * j + 1], dqr[cc][4 * j + 2], dqr[cc][4 * j + 3]);
-                }
-            }
-            if (first + count >= D / 8) dq_owed = 0;
-        };
-        constexpr int kQ = D / 64;     // additions per step of the schedule below (8 steps of kQ make D/8)
-
         for (int k = 0;; ++k) {
             const int item = next_item(k);
-            __syncwarp();
-            mbar_arrive(&bar_sched_empty[k & 1]);
+            warp_arrive(&bar_sched_empty[k & 1]);
             if (item < 0) break;
             const BwdItem w = bwd_decode_item<true>(item, p);
             const int bh = w.bh;
             const int rrow = w.r0 + r_in;                      // this thread's key
             const bool row_dead = rrow >= w.Lv;                // padding, or past the end of the tensor: P = dS = 0
-            // per-query statistics: each warpgroup stages -lse2 and -delta of ITS 64 streamed queries one
-            // tile ahead, split-phase through an mbarrier of its own (see the two-pass kernel)
-            const int stat_j = ctid & 127;
-            const int stat_q = wg * 64 + (stat_j & 63);
-            const int stat_slot = (stat_j >> 6) * 128 + stat_q;
-            const float* stat_src = (stat_j < 64 ? p.lse2 : p.delta);
-            const float stat_oob = (stat_j < 64) ? -INFINITY : 0.f;
-            float stat_raw = 0.f;
-            bool stat_ok = false;
-            auto stat_issue = [&](int u) {
-                int tt, qs;
-                fused_stream_tile(w, u, p.group, p.causal, tt, qs);
-                const int qrow = tt * 128 + stat_q;
-                stat_ok = qrow < p.S;
-                if (stat_ok) stat_raw = stat_src[(long long)qs * p.S + qrow];
-            };
-            auto stat_publish = [&](uint32_t g) {
-                s_stat[(g & 1) * 256 + stat_slot] = stat_ok ? -stat_raw : stat_oob;
-                mbar_arrive(&bar_stat[wg]);
-            };
-            if (w.n_it > 0) {
-                stat_issue(0);
-                stat_publish(git);
-                if (w.n_it > 1) stat_issue(1);
-            }
-            int prev_t = 0, prev_qs = 0;
-            for (int u = 0; u < w.n_it; ++u, ++git) {
-                int t, qs;
-                fused_stream_tile(w, u, p.group, p.causal, t, qs);
-                const int c0 = t * 128;                            // first streamed query of this tile
-                const float* st_nlse = s_stat + (git & 1) * 256;
+            FusedStream pos(w, p.group, p.causal);
+            for (int u = 0; u < w.n_it; ++u, ++git, pos.next(w)) {
+                const int c0 = pos.t * 128;                            // first streamed query of this tile
+                const float* st_nlse = s_stat + (git & 1) * 256 + wg * 64;
                 const float* st_ndelta = st_nlse + 128;
-                const bool tr = kTrace && k == 0 && wq == 0 && lane == 0;
+                const bool tr = kTrace && k == 0 && warp == 0 && lane == 0;
                 if (tr) TT_B1TRACE(wg, u, 0);
-                mbar_wait(&bar_stat[wg], git & 1, wctx, B1_STAT, u);
+                mbar_wait(&bar_stat_full[git & 1], (git >> 1) & 1, wctx, B1_STAT, u);
                 // visible queries of this thread's key inside the tile: [vis_lo, 128)
                 int vis_lo = p.causal ? max(0, rrow - off - c0) : 0;
                 if (row_dead) vis_lo = 128;
                 const bool need_mask = vis_lo > 0;
-                uint64_t stat_reg[2][16];
+                // The statistics of a chunk of 32 queries are fetched ahead of the wait for its scores: inside the phases they
+                // would sit behind the tensor-memory waits, while shared memory is busy feeding the GEMMs.
+                uint64_t stat_reg[16];
                 auto load_stats = [&](const float* src) {
 #pragma unroll
-                    for (int cc = 0; cc < 2; ++cc)
-#pragma unroll
-                        for (int e4 = 0; e4 < 8; ++e4) {
-                            const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(src + wg * 64 + cc * 32 + e4 * 4);
-                            stat_reg[cc][2 * e4] = v.x;
-                            stat_reg[cc][2 * e4 + 1] = v.y;
-                        }
+                    for (int e4 = 0; e4 < 8; ++e4) {
+                        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(src + e4 * 4);
+                        stat_reg[2 * e4] = v.x;
+                        stat_reg[2 * e4 + 1] = v.y;
+                    }
                 };
-                uint32_t pb[32];      // this thread's 64 probabilities as bf16 pairs: what goes to tensor memory, kept for phase B
-                // ---------------- phase A: P^T = exp2(S^T*c - lse2) -> bf16 over the S^T columns just read
+                uint64_t pf2[32];     // this thread's 64 probabilities, fp32 pairs
+                // ---------------- phase A: P^T = exp2(S^T*c - lse2) -> bf16
                 // (the mask test stays OUT of the unrolled loop, see the two-pass kernel; and the tensor-memory
                 // store stays out of the branch: it is a warp-wide instruction and rows differ in need_mask)
-                auto phase_a_body = [&](auto masked_c, int cc, int half, const uint32_t (&sr)[32]) {
+                auto phase_a_body = [&](auto masked_c, int cc, const uint32_t (&sr)[32]) {
                     constexpr bool kMasked = decltype(masked_c)::value;
 #pragma unroll
-                    for (int e = half * 16; e < half * 16 + 16; e += 2) {
+                    for (int e = 0; e < 32; e += 2) {
                         const int col = wg * 64 + cc * 32 + e;
-                        const uint64_t x = fma_f32x2(pack_f32x2(__uint_as_float(sr[e]), __uint_as_float(sr[e + 1])), c2, stat_reg[cc][e >> 1]);
+                        const uint64_t x = fma_f32x2(pack_f32x2(__uint_as_float(sr[e]), __uint_as_float(sr[e + 1])), c2, stat_reg[e >> 1]);
                         float a0, a1;
                         unpack_f32x2(x, a0, a1);
                         float p0 = ex2_approx(a0), p1 = ex2_approx(a1);
@@ -326,79 +300,67 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
                             p0 = (col >= vis_lo) ? p0 : 0.f;
                             p1 = (col + 1 >= vis_lo) ? p1 : 0.f;
                         }
-                        pb[cc * 16 + (e >> 1)] = pack_bf16x2(p0, p1);
+                        pf2[cc * 16 + (e >> 1)] = pack_f32x2(p0, p1);
                     }
                 };
-                auto phase_a_half = [&](int cc, int half, const uint32_t (&sr)[32]) {
-                    if (need_mask) phase_a_body(std::true_type{}, cc, half, sr);
-                    else phase_a_body(std::false_type{}, cc, half, sr);
-                };
-                auto store_p = [&](int cc) {
-                    uint32_t pk[16];
-#pragma unroll
-                    for (int e = 0; e < 16; ++e) pk[e] = pb[cc * 16 + e];
-                    __syncwarp();
-                    tmem_st16(tX + cc * 16, pk);
-                };
                 load_stats(st_nlse);
-                dq_add(6 * kQ, 2 * kQ);           // the last additions of the dQ_t taken a tile ago, ahead of the wait
                 mbar_wait(bar_s_full, git & 1, wctx, B1_SFULL, u);
                 __syncwarp();
                 tc_fence_after();
                 if (tr) TT_B1TRACE(wg, u, 1);
-                {
-                    uint32_t sr[32];
-                    tmem_ld32(tX, sr);
+#pragma unroll
+                for (int cc = 0; cc < 2; ++cc) {
+                    uint32_t sr[32], pk[16];
+                    tmem_ld32(tX + cc * 32, sr);
+                    if (cc == 1) load_stats(st_nlse + 32);
                     tmem_wait_ld();
-                    phase_a_half(0, 0, sr);
-                    phase_a_half(0, 1, sr);
-                    store_p(0);
-                }
-                if (tr) TT_B1TRACE(wg, u, 2);
-                // the previous tile's dQ_t: its GEMM ran during this tile's first exponentials
-                if (u > 0) dq_take(prev_t, prev_qs, git - 1, u);
-                if (tr) TT_B1TRACE(wg, u, 3);
-                {
-                    uint32_t sr[32];
-                    tmem_ld32(tX + 32, sr);
-                    tmem_wait_ld();
-                    dq_add(0, kQ);
-                    phase_a_half(1, 0, sr);
-                    dq_add(kQ, kQ);
-                    phase_a_half(1, 1, sr);
-                    store_p(1);
+                    if (kApart && cc == 1) {
+                        tc_fence_before();
+                        warp_arrive(bar_s_read);
+                    }
+                    if (need_mask) phase_a_body(std::true_type{}, cc, sr);
+                    else phase_a_body(std::false_type{}, cc, sr);
+#pragma unroll
+                    for (int e = 0; e < 16; ++e) {
+                        float q0, q1;
+                        unpack_f32x2(pf2[cc * 16 + e], q0, q1);
+                        pk[e] = pack_bf16x2(q0, q1);
+                    }
+                    __syncwarp();
+                    if (kApart && cc == 0 && git > 0) {   // complete long ago: P^T(t-1) has been read
+                        mbar_wait(bar_p_free, (git - 1) & 1, wctx, B1_PFREE, u);
+                        __syncwarp();
+                        tc_fence_after();
+                    }
+                    tmem_st16(tP + cc * 16, pk);
+                    if (tr) TT_B1TRACE(wg, u, 2 + cc);
                 }
                 tmem_wait_st();
                 tc_fence_before();
-                mbar_arrive(bar_p_full);
+                warp_arrive(bar_p_full);
                 if (tr) TT_B1TRACE(wg, u, 4);
                 load_stats(st_ndelta);
-                if (u + 1 < w.n_it) {
-                    stat_publish(git + 1);                     // its load was issued a tile ago
-                    if (u + 2 < w.n_it) stat_issue(u + 2);
-                }
-                dq_add(2 * kQ, 2 * kQ);
                 // ---------------- phase B: dS^T = P^T * (dP^T - delta) -> bf16 -> shared memory
                 mbar_wait(bar_dp_full, git & 1, wctx, B1_DPFULL, u);
                 __syncwarp();
                 tc_fence_after();
                 if (tr) TT_B1TRACE(wg, u, 5);
                 if (git > 0) mbar_wait(bar_ds_free, (git - 1) & 1, wctx, B1_DSFREE, u);   // complete long ago
+                __syncwarp();
 #pragma unroll
                 for (int cc = 0; cc < 2; ++cc) {
                     uint32_t dr[32];
                     tmem_ld32(tY + cc * 32, dr);
+                    if (cc == 1) load_stats(st_ndelta + 32);
                     tmem_wait_ld();
-                    dq_add((4 + cc) * kQ, kQ);
                     uint32_t pk[16];
 #pragma unroll
-                    for (int e = 0; e < 32; e += 2) {
-                        const uint64_t tdiff = add_f32x2(pack_f32x2(__uint_as_float(dr[e]), __uint_as_float(dr[e + 1])), stat_reg[cc][e >> 1]);
-                        const uint32_t pp = pb[cc * 16 + (e >> 1)];
-                        const uint64_t ds = mul_f32x2(pack_f32x2(__uint_as_float(pp << 16), __uint_as_float(pp & 0xffff0000u)), tdiff);
+                    for (int e = 0; e < 16; ++e) {
+                        const uint64_t tdiff = add_f32x2(pack_f32x2(__uint_as_float(dr[2 * e]), __uint_as_float(dr[2 * e + 1])), stat_reg[e]);
+                        const uint64_t ds = mul_f32x2(pf2[cc * 16 + e], tdiff);
                         float x0, x1;
                         unpack_f32x2(ds, x0, x1);
-                        pk[e >> 1] = pack_bf16x2(x0, x1);
+                        pk[e] = pack_bf16x2(x0, x1);
                     }
                     // 16-byte chunk j of row r sits at chunk j ^ (r & 7) of the row (128-byte swizzle)
 #pragma unroll
@@ -408,15 +370,9 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
                 }
                 fence_proxy_async_smem();          // generic-proxy stores -> visible to the MMA's async-proxy reads
                 tc_fence_before();
-                mbar_arrive(bar_ds_full);
+                warp_arrive(bar_ds_full);
+                if (lane == 0) mbar_arrive(&bar_stat_empty[git & 1]);
                 if (tr) TT_B1TRACE(wg, u, 6);
-                prev_t = t;
-                prev_qs = qs;
-            }
-            if (w.n_it > 0) {   // what is still owed for the last-but-one dQ_t, then the item's last one
-                dq_add(6 * kQ, 2 * kQ);
-                dq_take(prev_t, prev_qs, git - 1, w.n_it);
-                dq_add(0, D / 8);
             }
             // ---------------- epilogue: dV, dK out of tensor memory (then the MMA warp may start the next
             // item in them) -> bf16 -> global; warpgroup w owns columns [w*D/2, +D/2)
@@ -424,34 +380,93 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
             __syncwarp();
             tc_fence_after();
             constexpr int kHalf = D / 2;
-            uint32_t acc[2][kHalf / 32][32];
+            uint32_t o16[2][kHalf / 2];
 #pragma unroll
             for (int a = 0; a < 2; ++a) {
+                uint32_t acc[kHalf];
                 const uint32_t tA = tmem_base + lane_off + (a == 0 ? kColDV : kColDK) + wg * kHalf;
 #pragma unroll
-                for (int cc = 0; cc < kHalf / 32; ++cc) tmem_ld32(tA + cc * 32, acc[a][cc]);
+                for (int cc = 0; cc < kHalf / 32; ++cc) tmem_ld32(tA + cc * 32, reinterpret_cast<uint32_t(&)[32]>(acc[cc * 32]));
+                tmem_wait_ld();
+                const float mul = a == 0 ? 1.0f : p.scale;
+#pragma unroll
+                for (int e = 0; e < kHalf / 2; ++e)   // gradients of padded keys are zero
+                    o16[a][e] = row_dead ? 0u : pack_bf16x2(__uint_as_float(acc[2 * e]) * mul, __uint_as_float(acc[2 * e + 1]) * mul);
             }
-            tmem_wait_ld();
             tc_fence_before();
-            mbar_arrive(bar_acc_free);
+            warp_arrive(bar_acc_free);
             if (rrow < p.L) {
-                if (row_dead) {   // gradients of padded keys are zero
-#pragma unroll
-                    for (int a = 0; a < 2; ++a)
-#pragma unroll
-                        for (int cc = 0; cc < kHalf / 32; ++cc)
-#pragma unroll
-                            for (int e = 0; e < 32; ++e) acc[a][cc][e] = 0u;
-                }
                 const long long o = ((long long)bh * p.L + rrow) * D + wg * kHalf;
-                bwd_store_row<kHalf / 32>(p.out0 + o, acc[0], 1.0f, p.wide_stores);
-                bwd_store_row<kHalf / 32>(p.out1 + o, acc[1], p.scale, p.wide_stores);
+#pragma unroll
+                for (int a = 0; a < 2; ++a) {
+                    __nv_bfloat16* dst = (a == 0 ? p.out0 : p.out1) + o;
+#pragma unroll
+                    for (int e = 0; e < kHalf / 2; e += 8) {
+                        if (p.wide_stores) {
+                            st_global_32B(dst + 2 * e, reinterpret_cast<const uint32_t(&)[8]>(o16[a][e]));
+                        } else {
+                            *reinterpret_cast<uint4*>(dst + 2 * e) = make_uint4(o16[a][e], o16[a][e + 1], o16[a][e + 2], o16[a][e + 3]);
+                            *reinterpret_cast<uint4*>(dst + 2 * e + 8) = make_uint4(o16[a][e + 4], o16[a][e + 5], o16[a][e + 6], o16[a][e + 7]);
+                        }
+                    }
+                }
             }
             __syncwarp();
         }
+    } else if (warp < 12) {
+        setmaxnreg_inc<Cfg::kRegsAdd>();
+
+        // ============================================================ the adding warpgroup: dQ_t out of tensor memory (thread
+        // <-> query row), then red.global.add.v4.f32 into the accumulator.  Its own warps, because the L2 takes about 4 KB
+        // of such additions per cycle from the whole chip (the 64 KB of a tile at D = 128 need ~2400 cycles with every SM
+        // adding) and a warp that issues them sits out most of that time in the issue stage.
+        const int r_in = (warp & 3) * 32 + lane;
+        const uint32_t tDQ = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + kColDQ;
+        uint32_t git = 0, chunk = 0;
+        for (int k = 0;; ++k) {
+            const int item = next_item(k);
+            warp_arrive(&bar_sched_empty[k & 1]);
+            if (item < 0) break;
+            const BwdItem w = bwd_decode_item<true>(item, p);
+            FusedStream pos(w, p.group, p.causal);
+            for (int u = 0; u < w.n_it; ++u, ++git, pos.next(w)) {
+                float* dst = p.dq_acc + (size_t)((long long)pos.slice * p.n_qt + pos.t) * (D / 4) * 512;
+                uint32_t r[D / 32][32];
+                auto add = [&](int cc) {
+                    float4* stage = reinterpret_cast<float4*>(sStage + (chunk & 1) * Cfg::kStageBytes);
+                    if (warp == 8) bulk_wait_read<1>();        // what left this buffer two chunks ago has been read
+                    named_bar_sync(1, 128);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        stage[j * 128 + r_in] = make_float4(__uint_as_float(r[cc][4 * j]), __uint_as_float(r[cc][4 * j + 1]),
+                                                            __uint_as_float(r[cc][4 * j + 2]), __uint_as_float(r[cc][4 * j + 3]));
+                    fence_proxy_async_smem();
+                    named_bar_sync(1, 128);
+                    if (warp == 8 && lane == 0) bulk_add_f32(dst + cc * 8 * 512, stage, Cfg::kStageBytes);
+                    __syncwarp();
+                    ++chunk;
+                };
+                const bool tr = kTrace && k == 0 && warp == 8 && lane == 0;
+                if (tr) TT_B1TRACE(1, u, 0);
+                mbar_wait(bar_dq_full, git & 1, wctx, B1_DQFULL, u);
+                __syncwarp();
+                tc_fence_after();
+                if (tr) TT_B1TRACE(1, u, 1);
+#pragma unroll
+                for (int cc = 0; cc < D / 32; ++cc) tmem_ld32(tDQ + cc * 32, r[cc]);
+                tmem_wait_ld();
+                tc_fence_before();
+                warp_arrive(bar_dq_free);
+                if (tr) TT_B1TRACE(1, u, 2);
+#pragma unroll
+                for (int cc = 0; cc < D / 32; ++cc) add(cc);
+                if (tr) TT_B1TRACE(1, u, 3);
+            }
+        }
+        if (warp == 8) bulk_wait_all();
     } else {
         setmaxnreg_dec<Cfg::kRegsOther>();
-        if (warp == 9) {
+        if (warp == 13) {
             // ============================================================ TMA loader + scheduler (whole
             // warp runs the control flow, one elected lane issues)
             auto load_tile = [&](unsigned char* dst, const CUtensorMap* tm, uint64_t* bar, int row_start, int bh) {
@@ -479,10 +494,19 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
                     load_tile(sV, &tmV, bar_res_full, w.r0, w.bh);
                 }
                 __syncwarp();
-                for (int u = 0; u < w.n_it; ++u, ++git) {
-                    const int s0 = git % kNQ, s1 = git % kNdO;
-                    int t, ts;
-                    fused_stream_tile(w, u, p.group, p.causal, t, ts);
+                FusedStream pos(w, p.group, p.causal);
+                for (int u = 0; u < w.n_it; ++u, ++git, pos.next(w)) {
+                    const int s0 = git % kNQ, s1 = git % kNdO, t = pos.t, ts = pos.slice;
+                    mbar_wait(&bar_stat_empty[git & 1], ((git >> 1) & 1) ^ 1, wctx, B1_STAT + 10, (int)git);
+                    __syncwarp();
+                    if (elect_one()) {
+                        const long long at = ((long long)ts * p.n_qt + t) * 128;
+                        float* dst = s_stat + (git & 1) * 256;
+                        mbar_arrive_expect_tx(&bar_stat_full[git & 1], Cfg::kStatBytes);
+                        bulk_load(dst, p.lse2 + at, Cfg::kStatBytes / 2, &bar_stat_full[git & 1]);
+                        bulk_load(dst + 128, p.delta + at, Cfg::kStatBytes / 2, &bar_stat_full[git & 1]);
+                    }
+                    __syncwarp();
                     mbar_wait(&bar_q_empty[s0], ((git / kNQ) & 1) ^ 1, wctx, B1_QEMPTY + s0, (int)git);
                     __syncwarp();
                     if (elect_one()) {
@@ -500,7 +524,7 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
                 }
                 items.request(*abort_flag != 0);   // an aborted CTA takes no further items
             }
-        } else if (warp == 8) {
+        } else if (warp == 12) {
             // ============================================================ MMA issuer (whole warp runs the
             // control flow; each tcgen05.mma / commit is issued by one elected lane)
             constexpr uint32_t idesc_s = umma_idesc_bf16(128, 128, false, false);   // S^T, dP^T: both K-major
@@ -558,7 +582,7 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
                     tc_commit(bar_s_full);
                     mbar_wait(&bar_do_full[f1], (git / kNdO) & 1, wctx, B1_DOFULL + f1, (int)git);
                     __syncwarp();
-                    if (git > 0) {
+                    if (!kApart && git > 0) {
                         mbar_wait(bar_dq_free, (git - 1) & 1, wctx, B1_DQFREE, (int)git);
                         __syncwarp();
                     }
@@ -571,6 +595,21 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
                     const int qs = g % kNQ, os = g % kNdO;                   // slots of this tile
                     const bool has_next = it + 1 < n_it;
                     const int nqs = (g + 1) % kNQ, nos = (g + 1) % kNdO;     // slots of the next tile
+                    // ---- G1(t+1): the next scores, as soon as the columns of S^T(t) are free: its values are in registers, or
+                    // (P^T in the same columns) G3(t) has been issued
+                    auto next_scores = [&] {
+                        if (!has_next) return;
+                        mbar_wait(&bar_q_full[nqs], ((g + 1) / kNQ) & 1, wctx, B1_QFULL + nqs, it + 1);
+                        __syncwarp();
+                        tc_fence_after();
+                        issue_score(dK_k, dQ_k + nqs * (Cfg::kTileBytes >> 4), kColX);
+                        tc_commit(bar_s_full);
+                    };
+                    if (kApart) {
+                        mbar_wait(bar_s_read, g & 1, wctx, B1_SREAD, it);
+                        __syncwarp();
+                        next_scores();
+                    }
                     // ---- G3: dV += P^T dO
                     const bool tr = kTrace && k == 0 && lane == 0;
                     if (tr) TT_B1TRACE(2, it, 0);
@@ -589,30 +628,46 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
                         if (elect_one()) {
 #pragma unroll
                             for (int kk = 0; kk < 8; ++kk)   // K step = 16 queries = 8 columns of bf16 P^T
-                                umma_ts_one(tmem_u + kColDV, tmem_u + kColX + (kk >> 2) * 64 + (kk & 3) * 8, b0 + kk * 128, hi, idesc_kn,
+                                umma_ts_one(tmem_u + kColDV, tmem_u + kColP + (kk >> 2) * kPitchP + (kk & 3) * 8, b0 + kk * 128, hi, idesc_kn,
                                             (it > 0 || kk > 0) ? 1u : 0u);
                         }
                         __syncwarp();
                     }
                     tc_commit(&bar_do_empty[os]);                            // last read of dO(t)
-                    // ---- G1(t+1): the next scores, as soon as P^T(t) has been consumed (in order)
-                    if (has_next) {
-                        mbar_wait(&bar_q_full[nqs], ((g + 1) / kNQ) & 1, wctx, B1_QFULL + nqs, it + 1);
-                        __syncwarp();
-                        tc_fence_after();
-                        issue_score(dK_k, dQ_k + nqs * (Cfg::kTileBytes >> 4), kColX);
-                        tc_commit(bar_s_full);
-                    }
+                    if (kApart) tc_commit(bar_p_free);
+                    else next_scores();
                     // ---- G5: dQ_t = dS K  and  G4: dK += dS^T Q
                     if (tr) TT_B1TRACE(2, it, 2);
                     mbar_wait(bar_ds_full, g & 1, wctx, B1_DSFULL, it);
                     __syncwarp();
                     tc_fence_after();
                     if (tr) TT_B1TRACE(2, it, 3);
+                    // ---- G2(t+1): the next dP^T, once dP^T(t) is in registers and, where it uses these columns, dQ_t has left
+                    auto next_dp = [&] {
+                        if (!has_next) return;
+                        mbar_wait(&bar_do_full[nos], ((g + 1) / kNdO) & 1, wctx, B1_DOFULL + nos, it + 1);
+                        __syncwarp();
+                        if (!kApart) {
+                            mbar_wait(bar_dq_free, g & 1, wctx, B1_DQFREE, it);
+                            __syncwarp();
+                        }
+                        tc_fence_after();
+                        if (tr) TT_B1TRACE(2, it, 5);
+                        issue_score(dV_k, ddO_k + nos * (Cfg::kTileBytes >> 4), kColY);
+                        tc_commit(bar_dp_full);
+                    };
+                    if (kApart) {
+                        next_dp();
+                        if (g > 0) {
+                            mbar_wait(bar_dq_free, (g - 1) & 1, wctx, B1_DQFREE, it);
+                            __syncwarp();
+                            tc_fence_after();
+                        }
+                    }
                     if (elect_one()) {
 #pragma unroll
                         for (int kk = 0; kk < 8; ++kk)       // K step = 16 keys = 16 rows of both tiles
-                            umma_ss_one(tmem_u + kColY, dDS_mn + kk * 128, dK_mn + kk * 128, hi, idesc_nn, kk > 0 ? 1u : 0u);
+                            umma_ss_one(tmem_u + kColDQ, dDS_mn + kk * 128, dK_mn + kk * 128, hi, idesc_nn, kk > 0 ? 1u : 0u);
                     }
                     __syncwarp();
                     tc_commit(bar_dq_full);
@@ -629,18 +684,8 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
                     tc_commit(&bar_q_empty[qs]);                             // last read of Q(t)
                     tc_commit(bar_ds_free);                                  // G4, G5 are done with the dS^T tile
                     if (!has_next) tc_commit(bar_res_empty);                 // the item's last reads of K and V
-                    // ---- G2(t+1): the next dP^T, once dQ_t has left Y
                     if (tr) TT_B1TRACE(2, it, 4);
-                    if (has_next) {
-                        mbar_wait(&bar_do_full[nos], ((g + 1) / kNdO) & 1, wctx, B1_DOFULL + nos, it + 1);
-                        __syncwarp();
-                        mbar_wait(bar_dq_free, g & 1, wctx, B1_DQFREE, it);
-                        __syncwarp();
-                        tc_fence_after();
-                        if (tr) TT_B1TRACE(2, it, 5);
-                        issue_score(dV_k, ddO_k + nos * (Cfg::kTileBytes >> 4), kColY);
-                        tc_commit(bar_dp_full);
-                    }
+                    if (!kApart) next_dp();
                     if (tr) TT_B1TRACE(2, it, 6);
                 }
                 tc_commit(bar_final);
@@ -650,11 +695,55 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 8) {
+    if (warp == 12) {
         tc_fence_after();
         tmem_dealloc(tmem_base, Cfg::kTmemCols);
     }
-    if (warp == 9 && *abort_flag) items.drop_rest(wctx.budget);
+    if (warp == 13 && *abort_flag) items.drop_rest(wctx.budget);
+}
+
+// Statistics as the kernel above streams them: -lse*log2(e) and -rowsum(dO*O), 128 per query tile of a slice (what lies past
+// the slice's last row makes P and dS zero), and the tile's dQ accumulator cleared.  D/8 lanes share a row.
+template <int D>
+__global__ void __launch_bounds__(256) attn_bwd_fused_prep_kernel(const __nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ dout,
+                                                                  const float* __restrict__ lse, float* __restrict__ ndelta,
+                                                                  float* __restrict__ nlse2, float4* __restrict__ dq_acc, int S, int n_qt) {
+    grid_let_next_start();
+    grid_wait_for_previous();
+    constexpr int kLanes = D / 8, kRows = 256 / kLanes, kSteps = 128 / kRows;   // a CTA takes one query tile
+    const long long blk = blockIdx.x;
+    const long long slice = blk / n_qt;
+    const int row0 = (int)(blk - slice * n_qt) * 128, li = threadIdx.x % kLanes;
+    uint4 a[kSteps], b[kSteps];
+#pragma unroll
+    for (int u = 0; u < kSteps; ++u) {
+        const int r = row0 + u * kRows + (int)threadIdx.x / kLanes;
+        a[u] = b[u] = make_uint4(0u, 0u, 0u, 0u);
+        if (r < S) {
+            const long long at = (slice * S + r) * D + li * 8;
+            a[u] = __ldg(reinterpret_cast<const uint4*>(out + at));
+            b[u] = __ldg(reinterpret_cast<const uint4*>(dout + at));
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < D / 8; ++i) dq_acc[blk * (D * 32) + i * 256 + threadIdx.x] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int u = 0; u < kSteps; ++u) {
+        const int in_tile = u * kRows + (int)threadIdx.x / kLanes, r = row0 + in_tile;
+        const uint32_t aw[4] = {a[u].x, a[u].y, a[u].z, a[u].w}, bw[4] = {b[u].x, b[u].y, b[u].z, b[u].w};
+        float acc = 0.f;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            acc = fmaf(__uint_as_float(aw[e] << 16), __uint_as_float(bw[e] << 16), acc);
+            acc = fmaf(__uint_as_float(aw[e] & 0xffff0000u), __uint_as_float(bw[e] & 0xffff0000u), acc);
+        }
+#pragma unroll
+        for (int o = kLanes / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if (li == 0) {
+            ndelta[blk * 128 + in_tile] = -acc;
+            nlse2[blk * 128 + in_tile] = r < S ? lse[slice * S + r] * -1.4426950408889634f : -INFINITY;
+        }
+    }
 }
 
 // dq[slice][row][:] = bf16(scale * accumulator): one block per (query slice, 128-row query tile), thread
@@ -696,7 +785,7 @@ bool attn_bwd_fused_supported(const AttnArgs& a) {
     return a.bf16 && (a.D == 64 || a.D == 128) && a.BH * (((long long)a.S + 127) / 128) < (1LL << 31);
 }
 size_t attn_bwd_fused_workspace(const AttnArgs& a) {
-    return align256((size_t)a.BH * (size_t)((a.S + 127) / 128) * 128 * a.D * sizeof(float));
+    return (size_t)a.BH * (size_t)((a.S + 127) / 128) * 128 * (a.D + 2) * sizeof(float);   // dQ accumulator, two statistics
 }
 
 static long long* g_fused_trace = nullptr;
@@ -709,14 +798,18 @@ void attn_bwd_fused_set_trace(long long* device_buf, int block) {
 template <int D, bool kTrace>
 static cudaError_t launch_fused(const AttnArgs& a, void* ws, cudaStream_t st) {
     using Cfg = Bwd1Cfg<D>;
-    const size_t stat_b = align256((size_t)a.BH * a.S * sizeof(float));
-    float* delta = reinterpret_cast<float*>(ws);
-    float* lse2 = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(ws) + stat_b);
-    float* dq_acc = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(ws) + 2 * stat_b);
-    cudaError_t e = cudaMemsetAsync(dq_acc, 0, attn_bwd_fused_workspace(a), st);
-    if (e != cudaSuccess) return e;
-    e = attn_bwd_prep(a, delta, lse2, st);
-    if (e != cudaSuccess) return e;
+    const int n_qt = (a.S + 127) / 128;
+    const size_t rows = (size_t)a.BH * n_qt * 128;
+    float* dq_acc = reinterpret_cast<float*>(ws);
+    float* delta = dq_acc + rows * D;
+    float* lse2 = delta + rows;
+    cudaError_t e;
+    {
+        LaunchScope ls(K_BWD_PREP, st);
+        e = launch_overlapped(attn_bwd_fused_prep_kernel<D>, (unsigned)(a.BH * n_qt), 256, 0, st, (const __nv_bfloat16*)a.out, (const __nv_bfloat16*)a.dout,
+                              a.lse, delta, lse2, reinterpret_cast<float4*>(dq_acc), a.S, n_qt);
+        if (e != cudaSuccess) return e;
+    }
     TmapStorage tq, tk, tv, tdo;
     const char* why = nullptr;
     if (!make_tmap_bf16(&tq, a.q, D, a.S, a.BH, 128, &why)) return cudaErrorInvalidValue;
@@ -748,7 +841,7 @@ static cudaError_t launch_fused(const AttnArgs& a, void* ws, cudaStream_t st) {
     p.n_light = a.causal ? p.n_tiles / 4 : 0;
     p.n_items_heavy = (int)(a.BH / a.group * (p.n_tiles - p.n_light));
     p.dq_acc = dq_acc;
-    p.n_qt = (a.S + 127) / 128;
+    p.n_qt = n_qt;
     p.trace = kTrace ? g_fused_trace : nullptr;
     p.trace_block = g_fused_trace_block;
     p.first_wave = sm_count();
