@@ -57,6 +57,7 @@ struct BwdParams {
     const int* cu_k;
     int total_q;
     int Hkv;                       // key/value heads per batch entry
+    int n_seq;                     // single-pass kernel: sequences of the packed batch
 };
 
 __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {

@@ -80,10 +80,10 @@ enum Bwd1BarId { B1_RES = 0, B1_QFULL = 10, B1_QEMPTY = 14, B1_DOFULL = 18, B1_D
 // its walk at query tile r and wraps round.  (Under the causal mask key tile r starts at query tile r anyway.)
 // Walked step by step: the divisions of a position's closed form are some 400 cycles of latency per tile and role.
 struct FusedStream {
-    int t, slice;    // query tile and query slice of the current position
+    int t, slice;    // query tile and query slice (packed batches: query head) of the current position
     int first, j;    // the slice's first tile index (relative to t_begin) and the position in its walk
-    __device__ __forceinline__ FusedStream(const BwdItem& w, int group, int causal)
-        : slice(w.bh * group), first(causal || w.nt == 0 ? 0 : (w.r0 >> 7) % w.nt), j(0) { t = w.t_begin + first; }
+    __device__ __forceinline__ FusedStream(const BwdItem& w, const BwdParams& p, bool packed)
+        : slice((packed ? w.head : w.bh) * p.group), first(p.causal || w.nt == 0 ? 0 : (w.r0 >> 7) % w.nt), j(0) { t = w.t_begin + first; }
     __device__ __forceinline__ void next(const BwdItem& w) {
         if (++j == w.nt) {
             j = 0;
@@ -94,6 +94,34 @@ struct FusedStream {
         }
     }
 };
+
+// What the loader publishes of a packed batch's item, so that the other roles need no search of their own.
+struct PackedItem { int head, r0, S, L, q_lo, k_lo, tile0, pad; };
+struct FusedItem : BwdItem {
+    long long blk0;   // accumulator and statistics of query tile t of query slice s: block s * n_qt + blk0 + t
+};
+template <bool kVarlen>
+__device__ __forceinline__ FusedItem fused_item(int item, const PackedItem* packed, const BwdParams& p) {
+    FusedItem w;
+    if constexpr (kVarlen) {
+        w.head = packed->head;
+        w.r0 = packed->r0;
+        w.S = packed->S;
+        w.L = w.Lv = packed->L;
+        w.q_lo = packed->q_lo;
+        w.k_lo = packed->k_lo;
+        w.blk0 = packed->tile0;
+        w.bh = 0;
+        w.t_end = (w.S + 127) >> 7;
+        w.t_begin = p.causal ? (max(0, w.r0 - (w.L - w.S)) >> 7) : 0;
+        w.nt = max(0, w.t_end - w.t_begin);
+        w.n_it = w.nt * p.group;
+    } else {
+        static_cast<BwdItem&>(w) = bwd_decode_item<true>(item, p);
+        w.blk0 = 0;
+    }
+    return w;
+}
 
 // Adds `bytes` of floats in shared memory to global memory by the TMA engine (one thread; a bulk group of its own).
 __device__ __forceinline__ void bulk_add_f32(float* gptr, const void* src, uint32_t bytes) {
@@ -115,7 +143,9 @@ __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wa
     } while (0)
 
 // kTrace: compiled with the cycle stamps (tuning aid; launched only while a trace buffer is set).
-template <int D, bool kTrace>
+// kVarlen: packed batches; work items are numbered by the batch's key tiles (see packed_seq), so that none but the unused
+// numbers and the tiles that no query sees is empty.
+template <int D, bool kTrace, bool kVarlen>
 __global__ void __launch_bounds__(Bwd1Cfg<D>::kThreads, 1)
 attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                             const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmdO,
@@ -163,13 +193,13 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
     int* sched_item = reinterpret_cast<int*>(bar_p_free + 1);    // [2]
     uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(sched_item + 2);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_base_slot + 1);
+    PackedItem* packed = reinterpret_cast<PackedItem*>(aux + 384);    // [2], beside sched_item
     uint64_t* bar_steal = reinterpret_cast<uint64_t*>(aux + Cfg::kBarBytes - 32);
     uint4* steal_response = reinterpret_cast<uint4*>(bar_steal + 2);
     float* s_stat = reinterpret_cast<float*>(aux + Cfg::kBarBytes);   // [2 slots][2: -lse2, -delta][128]
 
     const int warp = uniform_warp_idx();
     const int lane = threadIdx.x & 31;
-    const int off = p.L - p.S;
 
     if (threadIdx.x == 0) {
         *abort_flag = 0;
@@ -237,6 +267,12 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
         __syncwarp();
         if (lane == 0) mbar_arrive(bar);
     };
+    auto take_item = [&](int k, FusedItem& w) -> bool {   // every role but the loader
+        const int item = next_item(k);
+        if (item >= 0) w = fused_item<kVarlen>(item, &packed[k & 1], p);
+        warp_arrive(&bar_sched_empty[k & 1]);
+        return item >= 0;
+    };
 
     if (warp < 8) {
         // ============================================================ compute warpgroups
@@ -253,14 +289,12 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
         uint32_t git = 0;      // streamed tiles processed so far, over all items (barrier phases)
 
         for (int k = 0;; ++k) {
-            const int item = next_item(k);
-            warp_arrive(&bar_sched_empty[k & 1]);
-            if (item < 0) break;
-            const BwdItem w = bwd_decode_item<true>(item, p);
-            const int bh = w.bh;
+            FusedItem w;
+            if (!take_item(k, w)) break;
+            const int bh = w.bh, off = w.L - w.S;
             const int rrow = w.r0 + r_in;                      // this thread's key
             const bool row_dead = rrow >= w.Lv;                // padding, or past the end of the tensor: P = dS = 0
-            FusedStream pos(w, p.group, p.causal);
+            FusedStream pos(w, p, kVarlen);
             for (int u = 0; u < w.n_it; ++u, ++git, pos.next(w)) {
                 const int c0 = pos.t * 128;                            // first streamed query of this tile
                 const float* st_nlse = s_stat + (git & 1) * 256 + wg * 64;
@@ -395,8 +429,8 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
             }
             tc_fence_before();
             warp_arrive(bar_acc_free);
-            if (rrow < p.L) {
-                const long long o = ((long long)bh * p.L + rrow) * D + wg * kHalf;
+            if (rrow < w.L) {
+                const long long o = (kVarlen ? (long long)(w.k_lo + rrow) * p.Hkv + w.head : (long long)bh * w.L + rrow) * D + wg * kHalf;
 #pragma unroll
                 for (int a = 0; a < 2; ++a) {
                     __nv_bfloat16* dst = (a == 0 ? p.out0 : p.out1) + o;
@@ -424,13 +458,11 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
         const uint32_t tDQ = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + kColDQ;
         uint32_t git = 0, chunk = 0;
         for (int k = 0;; ++k) {
-            const int item = next_item(k);
-            warp_arrive(&bar_sched_empty[k & 1]);
-            if (item < 0) break;
-            const BwdItem w = bwd_decode_item<true>(item, p);
-            FusedStream pos(w, p.group, p.causal);
+            FusedItem w;
+            if (!take_item(k, w)) break;
+            FusedStream pos(w, p, kVarlen);
             for (int u = 0; u < w.n_it; ++u, ++git, pos.next(w)) {
-                float* dst = p.dq_acc + (size_t)((long long)pos.slice * p.n_qt + pos.t) * (D / 4) * 512;
+                float* dst = p.dq_acc + (size_t)((long long)pos.slice * p.n_qt + w.blk0 + pos.t) * (D / 4) * 512;
                 uint32_t r[D / 32][32];
                 auto add = [&](int cc) {
                     float4* stage = reinterpret_cast<float4*>(sStage + (chunk & 1) * Cfg::kStageBytes);
@@ -477,30 +509,62 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
             int item = (int)blockIdx.x;
             for (int k = 0;; ++k, item = items.next(wctx, 89, k)) {
                 const int slot = k & 1;
+                PackedItem pi;
+                while (kVarlen && item >= 0) {
+                    const int x = item / p.Hkv, b = packed_seq<7>(p.cu_k, p.n_seq, x);
+                    bool some = false;
+                    if (b >= 0) {
+                        pi.k_lo = p.cu_k[b];
+                        pi.q_lo = p.cu_q[b];
+                        pi.L = p.cu_k[b + 1] - pi.k_lo;
+                        pi.S = p.cu_q[b + 1] - pi.q_lo;
+                        pi.tile0 = (pi.q_lo >> 7) + b;
+                        const int base = (pi.k_lo >> 7) + b, n = ((pi.k_lo + pi.L) >> 7) + 1 - (pi.k_lo >> 7);   // numbers of the sequence
+                        const int r = item - base * p.Hkv;
+                        pi.head = r / n;
+                        pi.r0 = (r - pi.head * n) * 128;
+                        if (pi.head < p.Hkv && pi.r0 < pi.L) {
+                            some = fused_item<true>(item, &pi, p).n_it > 0;
+                            if (!some) {   // keys that no query sees: zero gradients
+                                const int rows = min(128, pi.L - pi.r0);
+                                for (int i = lane; i < rows * (D / 8); i += 32) {
+                                    const long long o = ((long long)(pi.k_lo + pi.r0 + i / (D / 8)) * p.Hkv + pi.head) * D + i % (D / 8) * 8;
+                                    *reinterpret_cast<uint4*>(p.out0 + o) = make_uint4(0u, 0u, 0u, 0u);
+                                    *reinterpret_cast<uint4*>(p.out1 + o) = make_uint4(0u, 0u, 0u, 0u);
+                                }
+                            }
+                        }
+                    }
+                    if (some) break;
+                    items.request(*abort_flag != 0);
+                    item = items.next(wctx, 89, k);
+                }
                 mbar_wait(&bar_sched_empty[slot], ((k >> 1) & 1) ^ 1, wctx, 90 + slot, k);
                 __syncwarp();
                 if (lane == 0) {
                     sched_item[slot] = item;
+                    if (kVarlen) packed[slot] = pi;
                     mbar_arrive(&bar_sched_full[slot]);
                 }
                 __syncwarp();
                 if (item < 0) break;
-                const BwdItem w = bwd_decode_item<true>(item, p);
+                const FusedItem w = fused_item<kVarlen>(item, &pi, p);
+                const int key_row = (kVarlen ? w.k_lo : 0) + w.r0, key_z = kVarlen ? w.head : w.bh, q_row = kVarlen ? w.q_lo : 0;
                 mbar_wait(bar_res_empty, (k & 1) ^ 1, wctx, B1_RES + 1, k);
                 __syncwarp();
                 if (elect_one()) {
                     mbar_arrive_expect_tx(bar_res_full, 2 * Cfg::kTileBytes);
-                    load_tile(sK, &tmK, bar_res_full, w.r0, w.bh);
-                    load_tile(sV, &tmV, bar_res_full, w.r0, w.bh);
+                    load_tile(sK, &tmK, bar_res_full, key_row, key_z);
+                    load_tile(sV, &tmV, bar_res_full, key_row, key_z);
                 }
                 __syncwarp();
-                FusedStream pos(w, p.group, p.causal);
+                FusedStream pos(w, p, kVarlen);
                 for (int u = 0; u < w.n_it; ++u, ++git, pos.next(w)) {
                     const int s0 = git % kNQ, s1 = git % kNdO, t = pos.t, ts = pos.slice;
                     mbar_wait(&bar_stat_empty[git & 1], ((git >> 1) & 1) ^ 1, wctx, B1_STAT + 10, (int)git);
                     __syncwarp();
                     if (elect_one()) {
-                        const long long at = ((long long)ts * p.n_qt + t) * 128;
+                        const long long at = ((long long)ts * p.n_qt + w.blk0 + t) * 128;
                         float* dst = s_stat + (git & 1) * 256;
                         mbar_arrive_expect_tx(&bar_stat_full[git & 1], Cfg::kStatBytes);
                         bulk_load(dst, p.lse2 + at, Cfg::kStatBytes / 2, &bar_stat_full[git & 1]);
@@ -511,14 +575,14 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
                     __syncwarp();
                     if (elect_one()) {
                         mbar_arrive_expect_tx(&bar_q_full[s0], Cfg::kTileBytes);
-                        load_tile(sQ + s0 * Cfg::kTileBytes, &tmQ, &bar_q_full[s0], t * 128, ts);
+                        load_tile(sQ + s0 * Cfg::kTileBytes, &tmQ, &bar_q_full[s0], q_row + t * 128, ts);
                     }
                     __syncwarp();
                     mbar_wait(&bar_do_empty[s1], ((git / kNdO) & 1) ^ 1, wctx, B1_DOEMPTY + s1, (int)git);
                     __syncwarp();
                     if (elect_one()) {
                         mbar_arrive_expect_tx(&bar_do_full[s1], Cfg::kTileBytes);
-                        load_tile(sdO + s1 * Cfg::kTileBytes, &tmdO, &bar_do_full[s1], t * 128, ts);
+                        load_tile(sdO + s1 * Cfg::kTileBytes, &tmdO, &bar_do_full[s1], q_row + t * 128, ts);
                     }
                     __syncwarp();
                 }
@@ -561,12 +625,9 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
             };
             uint32_t git = 0;      // streamed tiles issued before the current item
             for (int k = 0;; ++k) {
-                const int item = next_item(k);
+                FusedItem w;
+                if (!take_item(k, w)) break;
                 __syncwarp();
-                if (elect_one()) mbar_arrive(&bar_sched_empty[k & 1]);
-                __syncwarp();
-                if (item < 0) break;
-                const BwdItem w = bwd_decode_item<true>(item, p);
                 const int n_it = w.n_it;
                 mbar_wait(bar_res_full, k & 1, wctx, B1_RES, k);
                 __syncwarp();
@@ -704,23 +765,54 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
 
 // Statistics as the kernel above streams them: -lse*log2(e) and -rowsum(dO*O), 128 per query tile of a slice (what lies past
 // the slice's last row makes P and dS zero), and the tile's dQ accumulator cleared.  D/8 lanes share a row.
-template <int D>
+// Packed batches: a block's tile is found in the numbering of packed_seq; tokens of no sequence get zero gradients here.
+struct PackedBatch {
+    const int *cu_q, *cu_k;
+    int n_seq, total_q, total_k, H, Hkv;
+    __nv_bfloat16 *dq, *dk, *dv;
+};
+struct TileRows {
+    int n;                   // rows that exist (none where not positive)
+    long long row0, pitch;   // row r of the tile is row row0 + r * pitch of a [rows, D] array
+    long long stat0;         // its log-sum-exp is lse[stat0 + r]
+};
+template <bool kVarlen>
+__device__ __forceinline__ TileRows tile_rows(long long blk, int S, int n_qt, const PackedBatch& b) {
+    const long long s = blk / n_qt;
+    const int t = (int)(blk - s * n_qt);
+    if constexpr (kVarlen) {
+        const int i = packed_seq<7>(b.cu_q, b.n_seq, t);
+        if (i < 0) return {0, 0, 0, 0};
+        const int lo = b.cu_q[i], r0 = (t - (lo >> 7) - i) * 128;
+        return {min(128, b.cu_q[i + 1] - lo - r0), (long long)(lo + r0) * b.H + s, b.H, s * b.total_q + lo + r0};
+    } else {
+        return {min(128, S - t * 128), s * S + t * 128, 1, s * S + t * 128};
+    }
+}
+__device__ __forceinline__ void zero_other_tokens(__nv_bfloat16* t, const int* cu, int n_seq, int total, int width) {
+    const int lo = cu[0], hi = cu[n_seq], n = lo + total - hi;
+    for (long long i = blockIdx.x; i < n; i += gridDim.x) {
+        uint4* dst = reinterpret_cast<uint4*>(t + (i < lo ? i : i - lo + hi) * width);
+        for (int e = threadIdx.x; e < width / 8; e += blockDim.x) dst[e] = make_uint4(0u, 0u, 0u, 0u);
+    }
+}
+template <int D, bool kVarlen>
 __global__ void __launch_bounds__(256) attn_bwd_fused_prep_kernel(const __nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ dout,
                                                                   const float* __restrict__ lse, float* __restrict__ ndelta,
-                                                                  float* __restrict__ nlse2, float4* __restrict__ dq_acc, int S, int n_qt) {
+                                                                  float* __restrict__ nlse2, float4* __restrict__ dq_acc, int S, int n_qt, const PackedBatch pb) {
     grid_let_next_start();
     grid_wait_for_previous();
     constexpr int kLanes = D / 8, kRows = 256 / kLanes, kSteps = 128 / kRows;   // a CTA takes one query tile
     const long long blk = blockIdx.x;
-    const long long slice = blk / n_qt;
-    const int row0 = (int)(blk - slice * n_qt) * 128, li = threadIdx.x % kLanes;
+    const int li = threadIdx.x % kLanes;
+    const TileRows w = tile_rows<kVarlen>(blk, S, n_qt, pb);
     uint4 a[kSteps], b[kSteps];
 #pragma unroll
     for (int u = 0; u < kSteps; ++u) {
-        const int r = row0 + u * kRows + (int)threadIdx.x / kLanes;
+        const int r = u * kRows + (int)threadIdx.x / kLanes;
         a[u] = b[u] = make_uint4(0u, 0u, 0u, 0u);
-        if (r < S) {
-            const long long at = (slice * S + r) * D + li * 8;
+        if (r < w.n) {
+            const long long at = (w.row0 + r * w.pitch) * D + li * 8;
             a[u] = __ldg(reinterpret_cast<const uint4*>(out + at));
             b[u] = __ldg(reinterpret_cast<const uint4*>(dout + at));
         }
@@ -729,7 +821,7 @@ __global__ void __launch_bounds__(256) attn_bwd_fused_prep_kernel(const __nv_bfl
     for (int i = 0; i < D / 8; ++i) dq_acc[blk * (D * 32) + i * 256 + threadIdx.x] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int u = 0; u < kSteps; ++u) {
-        const int in_tile = u * kRows + (int)threadIdx.x / kLanes, r = row0 + in_tile;
+        const int r = u * kRows + (int)threadIdx.x / kLanes;
         const uint32_t aw[4] = {a[u].x, a[u].y, a[u].z, a[u].w}, bw[4] = {b[u].x, b[u].y, b[u].z, b[u].w};
         float acc = 0.f;
 #pragma unroll
@@ -740,28 +832,32 @@ __global__ void __launch_bounds__(256) attn_bwd_fused_prep_kernel(const __nv_bfl
 #pragma unroll
         for (int o = kLanes / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
         if (li == 0) {
-            ndelta[blk * 128 + in_tile] = -acc;
-            nlse2[blk * 128 + in_tile] = r < S ? lse[slice * S + r] * -1.4426950408889634f : -INFINITY;
+            const float l = r < w.n ? lse[w.stat0 + r] : INFINITY;
+            ndelta[blk * 128 + r] = -acc;
+            nlse2[blk * 128 + r] = (kVarlen && l == -INFINITY) ? -INFINITY : l * -1.4426950408889634f;   // a row that sees no key: P = 0
         }
+    }
+    if (kVarlen) {
+        zero_other_tokens(pb.dq, pb.cu_q, pb.n_seq, pb.total_q, pb.H * D);
+        zero_other_tokens(pb.dk, pb.cu_k, pb.n_seq, pb.total_k, pb.Hkv * D);
+        zero_other_tokens(pb.dv, pb.cu_k, pb.n_seq, pb.total_k, pb.Hkv * D);
     }
 }
 
 // dq[slice][row][:] = bf16(scale * accumulator): one block per (query slice, 128-row query tile), thread
 // (row, half of the head dim).  Reads are 16 bytes per lane and contiguous across the rows of a warp; four
 // of them make the 32 contiguous bytes (one full sector) a lane writes.
-template <int D>
+template <int D, bool kVarlen>
 __global__ void __launch_bounds__(256) attn_bwd_dq_convert_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dq,
-                                                                 int S, int n_qt, float scale, int wide) {
+                                                                 int S, int n_qt, float scale, int wide, const PackedBatch pb) {
     grid_let_next_start();
     grid_wait_for_previous();
     const long long blk = blockIdx.x;            // qs * n_qt + t
-    const int t = (int)(blk % n_qt);
-    const long long qs = blk / n_qt;
+    const TileRows w = tile_rows<kVarlen>(blk, S, n_qt, pb);
     const int r = threadIdx.x & 127, h = threadIdx.x >> 7;
-    const int row = t * 128 + r;
-    if (row >= S) return;
+    if (r >= w.n) return;
     const float4* src = reinterpret_cast<const float4*>(acc) + (size_t)blk * (D / 4) * 128 + r;
-    __nv_bfloat16* dst = dq + ((long long)qs * S + row) * D + h * (D / 2);
+    __nv_bfloat16* dst = dq + (w.row0 + r * w.pitch) * D + h * (D / 2);
 #pragma unroll
     for (int c = 0; c < D / 8; c += 4) {
         uint32_t o8[8];
@@ -782,10 +878,14 @@ __global__ void __launch_bounds__(256) attn_bwd_dq_convert_kernel(const float* _
 
 // ---------------------------------------------------------------- host side
 bool attn_bwd_fused_supported(const AttnArgs& a) {
-    return a.bf16 && (a.D == 64 || a.D == 128) && a.BH * (((long long)a.S + 127) / 128) < (1LL << 31);
+    return a.bf16 && (a.D == 64 || a.D == 128) && a.BH * (((long long)a.S + 127) / 128) < (1LL << 31) &&
+           (!a.cu_q || (a.H * (a.total_q / 128 + a.BH / a.H) < (1LL << 31) && a.H * (a.total_k / 128 + a.BH / a.H) < (1LL << 31)));
 }
+// query tiles: of every slice, or of every head over a packed batch's numbering (packed_seq)
+static int fused_tiles(const AttnArgs& a) { return a.cu_q ? (int)(a.total_q / 128 + a.BH / a.H) : (a.S + 127) / 128; }
+static long long fused_blocks(const AttnArgs& a) { return (a.cu_q ? a.H : a.BH) * (long long)fused_tiles(a); }
 size_t attn_bwd_fused_workspace(const AttnArgs& a) {
-    return (size_t)a.BH * (size_t)((a.S + 127) / 128) * 128 * (a.D + 2) * sizeof(float);   // dQ accumulator, two statistics
+    return (size_t)fused_blocks(a) * 128 * (a.D + 2) * sizeof(float);   // dQ accumulator, two statistics
 }
 
 static long long* g_fused_trace = nullptr;
@@ -795,29 +895,38 @@ void attn_bwd_fused_set_trace(long long* device_buf, int block) {
     g_fused_trace_block = block;
 }
 
-template <int D, bool kTrace>
+template <int D, bool kTrace, bool kVarlen>
 static cudaError_t launch_fused(const AttnArgs& a, void* ws, cudaStream_t st) {
     using Cfg = Bwd1Cfg<D>;
-    const int n_qt = (a.S + 127) / 128;
-    const size_t rows = (size_t)a.BH * n_qt * 128;
+    const int n_qt = fused_tiles(a), hkv = a.H / a.group;
+    const long long n_blk = fused_blocks(a);
+    const size_t rows = (size_t)n_blk * 128;
+    const PackedBatch pb = {a.cu_q, a.cu_k, (int)(a.BH / a.H), (int)a.total_q, (int)a.total_k, a.H, hkv, (__nv_bfloat16*)a.dq, (__nv_bfloat16*)a.dk, (__nv_bfloat16*)a.dv};
     float* dq_acc = reinterpret_cast<float*>(ws);
     float* delta = dq_acc + rows * D;
     float* lse2 = delta + rows;
     cudaError_t e;
     {
         LaunchScope ls(K_BWD_PREP, st);
-        e = launch_overlapped(attn_bwd_fused_prep_kernel<D>, (unsigned)(a.BH * n_qt), 256, 0, st, (const __nv_bfloat16*)a.out, (const __nv_bfloat16*)a.dout,
-                              a.lse, delta, lse2, reinterpret_cast<float4*>(dq_acc), a.S, n_qt);
+        e = launch_overlapped(attn_bwd_fused_prep_kernel<D, kVarlen>, (unsigned)n_blk, 256, 0, st, (const __nv_bfloat16*)a.out, (const __nv_bfloat16*)a.dout,
+                              a.lse, delta, lse2, reinterpret_cast<float4*>(dq_acc), a.S, n_qt, pb);
         if (e != cudaSuccess) return e;
     }
     TmapStorage tq, tk, tv, tdo;
     const char* why = nullptr;
-    if (!make_tmap_bf16(&tq, a.q, D, a.S, a.BH, 128, &why)) return cudaErrorInvalidValue;
-    if (!make_tmap_bf16(&tk, a.k, D, a.L, a.BH / a.group, 128, &why)) return cudaErrorInvalidValue;
-    if (!make_tmap_bf16(&tv, a.v, D, a.L, a.BH / a.group, 128, &why)) return cudaErrorInvalidValue;
-    if (!make_tmap_bf16(&tdo, a.dout, D, a.S, a.BH, 128, &why)) return cudaErrorInvalidValue;
+    if (kVarlen) {
+        if (!make_tmap_bf16_strided(&tq, a.q, D, a.total_q, a.H, (uint64_t)a.H * D, D, 128, &why)) return cudaErrorInvalidValue;
+        if (!make_tmap_bf16_strided(&tdo, a.dout, D, a.total_q, a.H, (uint64_t)a.H * D, D, 128, &why)) return cudaErrorInvalidValue;
+        if (!make_tmap_bf16_strided(&tk, a.k, D, a.total_k, hkv, (uint64_t)hkv * D, D, 128, &why)) return cudaErrorInvalidValue;
+        if (!make_tmap_bf16_strided(&tv, a.v, D, a.total_k, hkv, (uint64_t)hkv * D, D, 128, &why)) return cudaErrorInvalidValue;
+    } else {
+        if (!make_tmap_bf16(&tq, a.q, D, a.S, a.BH, 128, &why)) return cudaErrorInvalidValue;
+        if (!make_tmap_bf16(&tk, a.k, D, a.L, a.BH / a.group, 128, &why)) return cudaErrorInvalidValue;
+        if (!make_tmap_bf16(&tv, a.v, D, a.L, a.BH / a.group, 128, &why)) return cudaErrorInvalidValue;
+        if (!make_tmap_bf16(&tdo, a.dout, D, a.S, a.BH, 128, &why)) return cudaErrorInvalidValue;
+    }
     auto M = [](TmapStorage& t) -> CUtensorMap& { return *reinterpret_cast<CUtensorMap*>(t.bytes); };
-    e = TT_ALLOW_SMEM((attn_bwd_fused_sm100_kernel<D, kTrace>), Cfg::kSmemBytes);
+    e = TT_ALLOW_SMEM((attn_bwd_fused_sm100_kernel<D, kTrace, kVarlen>), Cfg::kSmemBytes);
     if (e != cudaSuccess) return e;
     BwdParams p;
     memset(&p, 0, sizeof(p));
@@ -836,8 +945,12 @@ static cudaError_t launch_fused(const AttnArgs& a, void* ws, cudaStream_t st) {
     p.H = a.H;
     const uintptr_t al = reinterpret_cast<uintptr_t>(a.dk) | reinterpret_cast<uintptr_t>(a.dv);
     p.wide_stores = (al & 31) == 0 ? 1 : 0;
+    p.Hkv = hkv;
+    p.cu_q = a.cu_q;
+    p.cu_k = a.cu_k;
+    p.n_seq = pb.n_seq;
     p.n_tiles = (a.L + 127) / 128;
-    p.n_items = (int)(a.BH / a.group * p.n_tiles);
+    p.n_items = kVarlen ? (int)(hkv * (a.total_k / 128 + pb.n_seq)) : (int)(a.BH / a.group * p.n_tiles);
     p.n_light = a.causal ? p.n_tiles / 4 : 0;
     p.n_items_heavy = (int)(a.BH / a.group * (p.n_tiles - p.n_light));
     p.dq_acc = dq_acc;
@@ -847,19 +960,20 @@ static cudaError_t launch_fused(const AttnArgs& a, void* ws, cudaStream_t st) {
     p.first_wave = sm_count();
     {
         LaunchScope ls(K_BWD_FUSED, st);
-        launch_overlapped(attn_bwd_fused_sm100_kernel<D, kTrace>, (unsigned)p.n_items, Cfg::kThreads, Cfg::kSmemBytes, st, M(tk), M(tv), M(tq), M(tdo), p);
+        launch_overlapped(attn_bwd_fused_sm100_kernel<D, kTrace, kVarlen>, (unsigned)p.n_items, Cfg::kThreads, Cfg::kSmemBytes, st, M(tk), M(tv), M(tq), M(tdo), p);
     }
     {
         LaunchScope ls(K_BWD_DQ_CONVERT, st);
-        launch_overlapped(attn_bwd_dq_convert_kernel<D>, (unsigned)(a.BH * p.n_qt), 256, 0, st, dq_acc, (__nv_bfloat16*)a.dq, a.S, p.n_qt, a.scale,
-                                                                                  (reinterpret_cast<uintptr_t>(a.dq) & 31) == 0 ? 1 : 0);
+        launch_overlapped(attn_bwd_dq_convert_kernel<D, kVarlen>, (unsigned)n_blk, 256, 0, st, dq_acc, (__nv_bfloat16*)a.dq, a.S, n_qt, a.scale,
+                          (reinterpret_cast<uintptr_t>(a.dq) & 31) == 0 ? 1 : 0, pb);
     }
     return cudaGetLastError();
 }
 
 cudaError_t attn_bwd_fused(const AttnArgs& a, void* ws, cudaStream_t st) {
-    if (g_fused_trace != nullptr) return a.D == 128 ? launch_fused<128, true>(a, ws, st) : launch_fused<64, true>(a, ws, st);
-    return a.D == 128 ? launch_fused<128, false>(a, ws, st) : launch_fused<64, false>(a, ws, st);
+    if (a.cu_q != nullptr) return a.D == 128 ? launch_fused<128, false, true>(a, ws, st) : launch_fused<64, false, true>(a, ws, st);
+    if (g_fused_trace != nullptr) return a.D == 128 ? launch_fused<128, true, false>(a, ws, st) : launch_fused<64, true, false>(a, ws, st);
+    return a.D == 128 ? launch_fused<128, false, false>(a, ws, st) : launch_fused<64, false, false>(a, ws, st);
 }
 
 // ---------------------------------------------------------------- choice between the two kernels
@@ -867,18 +981,30 @@ static std::atomic<int> g_bwd_deterministic{0};
 void attn_bwd_set_deterministic(int on) { g_bwd_deterministic.store(on ? 1 : 0); }
 int attn_bwd_deterministic() { return g_bwd_deterministic.load(); }
 
+// The single pass has only the key tiles' items to fill the SMs with, and clears, adds to and converts an accumulator; the two
+// passes execute seven GEMMs for five.  Backward in us, single pass / two passes (items per SM, streamed tiles per item):
+//   D = 64   [8,16,1024] causal 105 / 121 (6.9, 4), [4,16,1024] causal 63 / 67 (3.5, 4), [16,32,512] causal 159 / 168 (14, 2), but
+//            [4,32,300] 42.6 / 40.7 (2.6, 3), [64,32,128] causal 131 / 128 (14, 1), [2,32/4,2048] causal 232 / 188 (0.9, 64)
+//   D = 128  [4,32,4096] causal 1614 / 1700 (28, 16), [1,32,4096] 740 / 775 (6.9, 32), [1,32/8,8192] causal 1550 / 1600 (3.5, 128), but
+//            [4,32,2048] causal 506 / 511 (14, 8), [4,32,1024] causal 186 / 181 (6.9, 4), [1,16,4096] causal 226 / 220 (3.5, 16)
+//   packed (the two passes clear the gradients and number their items for the longest sequence), from three items per SM on:
+//            D = 128, 16 sequences of 300 to 4096, 32 heads, causal 2080 / 2313; 32 of 20 to 200 168 / 178; 8 of 500 to 1000, 16 heads 187 / 222
+static bool single_pass_pays(const AttnArgs& a) {
+    const long long n_seq = a.BH / a.H, hkv = a.H / a.group, n_sm = sm_count();
+    if (a.cu_q) return hkv * ((a.total_k + 127) / 128) >= 3 * n_sm;
+    const long long items = n_seq * hkv * ((a.L + 127) / 128), q_tiles = (a.S + 127) / 128;
+    const long long tiles = a.group * (a.causal ? (q_tiles + 1) / 2 : q_tiles);
+    if (a.D == 64) return items >= 3 * n_sm && tiles >= 2;
+    return (items >= 6 * n_sm && tiles >= 16) || (items >= 3 * n_sm && tiles >= 32);
+}
+
 cudaError_t attn_bwd_sm100(const AttnArgs& a, void* ws, cudaStream_t st) {
-    // TT_BWD_PATH=two_pass|fused overrides the setting (tests run both kernels on the same inputs)
+    // TT_BWD_PATH=two_pass|fused overrides the choice (tests run both kernels on the same inputs)
     const char* f = getenv("TT_BWD_PATH");
-    // By measurement (both kernels alternating in one process on one GPU): at D = 128 the two passes win or
-    // draw everywhere -- S = 4096 causal 1.60 ms against 1.66, S = 32768 x 64 heads 46.4 ms against 47.1 under
-    // the power cap -- because the single pass spends what it saves in GEMMs on its dQ additions (see the
-    // kernel's header); at D = 64 a tile's additions are half the bytes against the same exponentials and the
-    // single pass wins ([8,16,1024,64]: 0.172 ms against 0.201).
-    bool fused = !attn_bwd_deterministic() && a.D == 64;
+    bool fused = !attn_bwd_deterministic() && single_pass_pays(a);
     if (f && f[0] == 't') fused = false;
     if (f && f[0] == 'f') fused = true;
-    if (fused && attn_bwd_fused_supported(a) && a.cu_q == nullptr) return attn_bwd_fused(a, ws, st);   // packed batches: two passes
+    if (fused && attn_bwd_fused_supported(a)) return attn_bwd_fused(a, ws, st);
     return attn_bwd_two_pass(a, ws, st);
 }
 

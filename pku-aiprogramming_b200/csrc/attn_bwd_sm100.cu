@@ -788,7 +788,7 @@ bool attn_bwd_sm100_supported(const AttnArgs& a) {
 static size_t stats_rows(const AttnArgs& a) { return a.cu_q ? (size_t)a.total_q * a.H : (size_t)a.BH * a.S; }
 static size_t stats_bytes(const AttnArgs& a) { return 2 * align256(stats_rows(a) * sizeof(float)); }
 size_t attn_bwd_sm100_workspace(const AttnArgs& a) {
-    return stats_bytes(a) + ((attn_bwd_fused_supported(a) && !a.cu_q) ? attn_bwd_fused_workspace(a) : 0);
+    return stats_bytes(a) + (attn_bwd_fused_supported(a) ? attn_bwd_fused_workspace(a) : 0);
 }
 
 static long long* g_bwd_trace = nullptr;

@@ -51,6 +51,25 @@ __device__ __forceinline__ int valid_keys(const int* kv_lens, long long b, int L
     return kv_lens ? min(L, max(1, kv_lens[b])) : L;
 }
 
+// Packed batches: tiles of 2^kLog tokens are numbered over the whole batch, sequence b's from (cu[b] >> kLog) + b on, which
+// leaves room for all its tiles (and at most one unused number) without a prefix sum over the lengths: n_seq + total / 2^kLog
+// numbers in all.  The last b whose numbers start at or before x, or -1; whole warp, a 32-ary search (the loads of a step are
+// independent of each other).
+template <int kLog>
+__device__ __forceinline__ int packed_seq(const int* cu, int n_seq, int x) {
+    const int lane = threadIdx.x & 31;
+    if ((cu[0] >> kLog) > x) return -1;
+    int lo = 0, n = n_seq;
+    while (n > 1) {
+        const int stride = (n + 31) >> 5, i = lane * stride;
+        const bool ok = i < n && (cu[lo + i] >> kLog) + lo + i <= x;
+        const int at = (__popc(__ballot_sync(0xffffffffu, ok)) - 1) * stride;
+        lo += at;
+        n = min(stride, n - at);
+    }
+    return lo;
+}
+
 inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 // What a launch asks of the runtime on every call, kept per device after the first one: the number of SMs,

@@ -642,7 +642,7 @@ int tt_attn_bwd_varlen(const tt_varlen_desc* desc, const void* q, const void* k,
     a.q = q; a.k = k; a.v = v; a.out = const_cast<void*>(out); a.lse = const_cast<float*>(lse); a.dout = dout;
     a.dq = dq; a.dk = dk; a.dv = dv;
     a.cu_q = cu_q; a.cu_k = cu_k;
-    cudaError_t e = attn_bwd_two_pass(a, workspace, (cudaStream_t)stream);
+    cudaError_t e = attn_bwd_sm100(a, workspace, (cudaStream_t)stream);
     if (e == cudaErrorInvalidValue && g_err[0]) return TT_ERR_CUDA;
     if (e != cudaSuccess) return cuda_fail(e, "tt_attn_bwd_varlen");
     return TT_OK;
