@@ -32,7 +32,7 @@ struct FwdParams {
     // S and L above are the LONGEST sequence's counts (they size the grid); lse is [H, total_q].
     const int* cu_q;
     const int* cu_k;
-    int total_q;
+    int total_q, n_seq;
     long long* trace;   // optional cycle trace of one CTA (debug aid): [3 roles][64 iterations][8 stamps]
     int trace_block;
     int trace_item;     // which of the CTA's work items gets the per-iteration stamps

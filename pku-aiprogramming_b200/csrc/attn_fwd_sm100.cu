@@ -83,11 +83,15 @@ struct FwdItem {
     int out_pitch, out_col;
     long long lse0;       // lse[lse0 + r]
 };
+// What the loader publishes of a packed batch's item, so that the other roles need no search of their own.
+struct PackedBlock { int head, q0, S, L, q_lo, k_lo; };
 template <bool kPaged = false, bool kVarlen = false>
-__device__ __forceinline__ FwdItem fwd_decode_item(int item, const FwdParams& p, int D) {
+__device__ __forceinline__ FwdItem fwd_decode_item(int item, const FwdParams& p, int D, const PackedBlock* packed = nullptr) {
     FwdItem w;
-    int qb;
-    if (item < p.n_items_heavy) {
+    int qb = 0;
+    if (kVarlen) {
+        w.bh = 0;
+    } else if (item < p.n_items_heavy) {
         const int n_heavy = p.n_qblk - p.n_light;
         w.bh = item / n_heavy;
         qb = p.n_qblk - 1 - (item - w.bh * n_heavy);
@@ -96,13 +100,13 @@ __device__ __forceinline__ FwdItem fwd_decode_item(int item, const FwdParams& p,
         w.bh = r / p.n_light;
         qb = p.n_light - 1 - (r - w.bh * p.n_light);
     }
-    w.q0 = qb * 256;
+    if (!kVarlen) w.q0 = qb * 256;
     int S = p.S, L = p.L;
     if (kVarlen) {
-        const int b = w.bh / p.H, h = w.bh - b * p.H;
-        const int q_lo = p.cu_q[b], k_lo = p.cu_k[b];
-        S = p.cu_q[b + 1] - q_lo;
-        L = p.cu_k[b + 1] - k_lo;
+        const int h = packed->head, q_lo = packed->q_lo, k_lo = packed->k_lo;
+        w.q0 = packed->q0;
+        S = packed->S;
+        L = packed->L;
         w.qy0 = q_lo; w.qz = h; w.ky0 = k_lo; w.kz = h / p.group;
         w.out_row0 = q_lo; w.out_pitch = p.H * D; w.out_col = h * D;
         w.lse0 = (long long)h * p.total_q + q_lo;
@@ -173,6 +177,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     int* sched_item = reinterpret_cast<int*>(bar_sched_empty + 2);   // [2]
     uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(sched_item + 2);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_base_slot + 1);
+    PackedBlock* packed = reinterpret_cast<PackedBlock*>(reinterpret_cast<unsigned char*>(bars) + Cfg::kBarBytes - 96);   // [2], beside sched_item
     uint64_t* bar_steal = reinterpret_cast<uint64_t*>(reinterpret_cast<unsigned char*>(bars) + Cfg::kBarBytes - 32);
     uint4* steal_response = reinterpret_cast<uint4*>(bar_steal + 2);
 
@@ -242,9 +247,11 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         for (int k = 0;; ++k) {
             const int item = next_item(k);
             __syncwarp();
+            FwdItem w;
+            if (kVarlen && item >= 0) w = fwd_decode_item<kPaged, kVarlen>(item, p, D, &packed[k & 1]);
             mbar_arrive(&bar_sched_empty[k & 1]);
             if (item < 0) break;
-            const FwdItem w = fwd_decode_item<kPaged, kVarlen>(item, p, D);
+            if (!kVarlen) w = fwd_decode_item<kPaged, kVarlen>(item, p, D);
             const int nt = w.n_tiles[i];
             // per-item stamps of the traced CTA (role slot 0/1 = query tile, row = item number k)
             if (kTrace && p.trace != nullptr && (int)blockIdx.x == p.trace_block && wq == 0 && (threadIdx.x & 31) == 0 && k < 64) {
@@ -389,15 +396,36 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             int item = (int)blockIdx.x;
             for (int k = 0;; ++k, item = items.next(wctx, 89, k)) {
                 const int slot = k & 1;
+                PackedBlock pi;
+                while (kVarlen && item >= 0) {   // the item's sequence, head and 256-row block (see packed_seq)
+                    const int x = item / p.H, b = packed_seq<8>(p.cu_q, p.n_seq, x);
+                    bool some = false;
+                    if (b >= 0) {
+                        pi.q_lo = p.cu_q[b];
+                        pi.k_lo = p.cu_k[b];
+                        pi.S = p.cu_q[b + 1] - pi.q_lo;
+                        pi.L = p.cu_k[b + 1] - pi.k_lo;
+                        const int base = (pi.q_lo >> 8) + b, n = ((pi.q_lo + pi.S) >> 8) + 1 - (pi.q_lo >> 8);   // numbers of the sequence
+                        const int r = item - base * p.H, blocks = (pi.S + 255) >> 8;
+                        pi.head = r / n;
+                        const int rank = r - pi.head * n;
+                        pi.q0 = (blocks - 1 - rank) * 256;   // the late blocks are the heavy ones
+                        some = pi.head < p.H && rank < blocks;
+                    }
+                    if (some) break;
+                    items.request(*abort_flag != 0);
+                    item = items.next(wctx, 89, k);
+                }
                 mbar_wait(&bar_sched_empty[slot], ((k >> 1) & 1) ^ 1, wctx, 90 + slot, k);
                 __syncwarp();
                 if (lane == 0) {
                     sched_item[slot] = item;
+                    if (kVarlen) packed[slot] = pi;
                     mbar_arrive(&bar_sched_full[slot]);
                 }
                 __syncwarp();
                 if (item < 0) break;
-                const FwdItem w = fwd_decode_item<kPaged, kVarlen>(item, p, D);
+                const FwdItem w = fwd_decode_item<kPaged, kVarlen>(item, p, D, &pi);
                 auto load_q = [&](int i) {
                     mbar_wait(&bar_q_empty[i], (q_uses[i] & 1) ^ 1, wctx, 5 + i, k);
                     __syncwarp();
@@ -501,10 +529,13 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
                 const int item = (ahead_item != -2) ? ahead_item : next_item(k);
                 ahead_item = -2;
                 __syncwarp();
+                FwdItem w;
+                if (kVarlen && item >= 0) w = fwd_decode_item<kPaged, kVarlen>(item, p, D, &packed[k & 1]);
+                __syncwarp();
                 if (elect_one()) mbar_arrive(&bar_sched_empty[k & 1]);
                 __syncwarp();
                 if (item < 0) break;
-                const FwdItem w = fwd_decode_item<kPaged, kVarlen>(item, p, D);
+                if (!kVarlen) w = fwd_decode_item<kPaged, kVarlen>(item, p, D);
                 // S_i(0) for both tiles.  The S/P columns are free: the P V MMAs of the previous item
                 // were issued earlier by this warp and execute in order.
                 if (w.n_max > 0) {
@@ -690,7 +721,9 @@ static cudaError_t launch_fwd(const AttnArgs& a, cudaStream_t st) {
     p.trace_item = g_fwd_trace_item;
     p.s0_ahead = (kPaged || kVarlen) ? 0 : 1;
     p.wide_stores = (reinterpret_cast<uintptr_t>(a.out) & 31) == 0 ? 1 : 0;
-    p.n_items = (int)(a.BH * p.n_qblk);
+    // (packed: numbered by the batch's blocks, not by the longest sequence's, of which most items would be empty)
+    p.n_seq = kVarlen ? (int)(a.BH / a.H) : 0;
+    p.n_items = kVarlen ? (int)(a.H * (a.total_q / 256 + p.n_seq)) : (int)(a.BH * p.n_qblk);
     {
         // Causal items weigh in proportion to their query block's position.  With one slice-major
         // numbering the launch ends on the last slice's heaviest blocks while the other CTAs run dry;
