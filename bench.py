@@ -48,8 +48,9 @@ WORKLOADS = {
 NCU_TRAFFIC_BYTES = {
     "cfg3": {"attn_fwd_sm100": 593.0e6, "attn_bwd_sm100_dkv": 850.5e6, "attn_bwd_sm100_dq": 729.1e6,
              "attn_bwd_fused_sm100": 1507.7e6},
-    "cfg2": {"attn_fwd_sm100": 52.3e6, "attn_bwd_fused_sm100": 132.1e6},
-    "cfg5_per_slice": {"attn_fwd_sm100": 26.08e6, "attn_bwd_sm100_dkv": 35.10e6, "attn_bwd_sm100_dq": 34.66e6},
+    "cfg2": {"attn_fwd_sm100": 52.3e6, "attn_bwd_fused_sm100": 128.4e6},
+    "cfg5_per_slice": {"attn_fwd_sm100": 26.08e6, "attn_bwd_sm100_dkv": 35.10e6, "attn_bwd_sm100_dq": 34.66e6,
+                       "attn_bwd_fused_sm100": 61.55e6},
     # config 4 = 8 x the captured batch-8 launch (the full launch holds 8.6 GB, too large a capture)
     "decode": {"attn_decode": 8.637e9, "attn_decode_gq_sm100": 8.622e9},
 }
