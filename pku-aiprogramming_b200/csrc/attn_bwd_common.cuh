@@ -27,8 +27,10 @@ struct BwdRegs {
 struct BwdParams {
     __nv_bfloat16* out0;   // keys resident: dV ; else unused
     __nv_bfloat16* out1;   // keys resident: dK ; else dQ
-    const float* lse2;     // [BH,S]  lse * log2(e)
-    const float* delta;    // [BH,S]
+    // [BH,S] lse * log2(e) and rowsum(dO * O); for the single-pass kernel both negated and padded to whole query tiles,
+    // 128 floats per block of the accumulator below
+    const float* lse2;
+    const float* delta;
     int S, L;
     int n_tiles;           // resident tiles per slice
     // causal: the n_light lightest resident tiles of every slice are numbered after all others, so that
@@ -51,7 +53,7 @@ struct BwdParams {
     int n_qt;
     long long* trace;   // optional cycle trace of one CTA (debug aid): [3 roles][64 iterations][8 stamps]
     int trace_block;
-    // packed variable-length batches (two-pass kernel only; see AttnArgs): per-sequence geometry from cu_q /
+    // packed variable-length batches (see AttnArgs): per-sequence geometry from cu_q /
     // cu_k, token-major tensors, statistics as [H, total_q]; S and L above are the longest sequence's counts
     const int* cu_q;
     const int* cu_k;

@@ -451,9 +451,8 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
         setmaxnreg_inc<Cfg::kRegsAdd>();
 
         // ============================================================ the adding warpgroup: dQ_t out of tensor memory (thread
-        // <-> query row), then red.global.add.v4.f32 into the accumulator.  Its own warps, because the L2 takes about 4 KB
-        // of such additions per cycle from the whole chip (the 64 KB of a tile at D = 128 need ~2400 cycles with every SM
-        // adding) and a warp that issues them sits out most of that time in the issue stage.
+        // <-> query row), through shared memory into the accumulator.  Its own warps, because a piece's buffer is free again only
+        // when the L2 has taken what was in it: the 64 KB of a tile at D = 128 need 2400 to 3200 cycles with every SM adding.
         const int r_in = (warp & 3) * 32 + lane;
         const uint32_t tDQ = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + kColDQ;
         uint32_t git = 0, chunk = 0;
