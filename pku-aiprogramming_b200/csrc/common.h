@@ -58,12 +58,14 @@ __device__ __forceinline__ int valid_keys(const int* kv_lens, long long b, int L
 template <int kLog>
 __device__ __forceinline__ int packed_seq(const int* cu, int n_seq, int x) {
     const int lane = threadIdx.x & 31;
-    if ((cu[0] >> kLog) > x) return -1;
+    if (n_seq == 1) return (cu[0] >> kLog) <= x ? 0 : -1;
     int lo = 0, n = n_seq;
     while (n > 1) {
         const int stride = (n + 31) >> 5, i = lane * stride;
         const bool ok = i < n && (cu[lo + i] >> kLog) + lo + i <= x;
-        const int at = (__popc(__ballot_sync(0xffffffffu, ok)) - 1) * stride;
+        const unsigned before = __ballot_sync(0xffffffffu, ok);
+        if (before == 0) return -1;
+        const int at = (__popc(before) - 1) * stride;
         lo += at;
         n = min(stride, n - at);
     }
