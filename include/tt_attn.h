@@ -91,9 +91,10 @@ int tt_attn_bwd(const tt_attn_desc* desc, const void* q, const void* k, const vo
  * then dq with the queries resident and the scores recomputed): seven GEMMs per tile pair, no atomics,
  * every result bit-reproducible.  One pass that produces dk, dv and dq together (five GEMMs), dq through
  * fp32 additions into the workspace; those arrive in no fixed order, so dq repeats to fp32 rounding (a few
- * 1e-7 relative) rather than bit for bit.  on = 0 (default): whichever measured faster for the shape (one
- * pass from three key tiles per SM on at D = 64 and for packed batches, from more and longer ones at D = 128).
- * on = 1: always the two passes, for packed batches too.  Process-wide; no counterpart in
+ * 1e-7 relative) rather than bit for bit.  on = 1: always the two passes.  on = 0: whichever measured faster
+ * for the shape (the single pass from three key tiles per SM on for packed batches and at D = 64, there with two
+ * streamed tiles each, from more and longer ones at D = 128).  A process that never calls this gets the two
+ * passes for packed batches and at D = 128, and at D = 64 what on = 0 gives.  Process-wide; no counterpart in
  * the reference, whose NumPy reverse sweep (optimizer/autodiff.py:33-61) is deterministic and
  * single-threaded. */
 int tt_attn_bwd_set_deterministic(int on);
@@ -157,8 +158,8 @@ int tt_attn_bwd_padded(const tt_attn_desc* desc, const void* q, const void* k, c
  * Every sequence is its own attention problem with the conventions above (causal: bottom-right aligned
  * per sequence; a row that sees no key -- an empty key sequence, or causal with fewer keys than queries --
  * gets out = 0, lse = -inf and zero gradients).  bf16 with D = 64 or 128 only (tensor-core kernels);
- * anything else returns TT_ERR_UNSUPPORTED.  The backward chooses between the single pass and the two passes as
- * above: under tt_attn_bwd_set_deterministic(1), and for small batches, every result repeats bit for bit.
+ * anything else returns TT_ERR_UNSUPPORTED.  The backward runs the two-pass kernels (bit-reproducible) unless
+ * tt_attn_bwd_set_deterministic(0) has allowed the single pass.
  * Workspace: tt_attn_bwd_varlen_workspace_bytes(), 256-byte aligned. */
 typedef struct tt_varlen_desc {
     int32_t n_seq, H, Hkv;   /* Hkv: 0 or H, or a divisor of H (grouped heads) */

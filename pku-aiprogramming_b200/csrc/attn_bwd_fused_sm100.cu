@@ -976,9 +976,8 @@ cudaError_t attn_bwd_fused(const AttnArgs& a, void* ws, cudaStream_t st) {
 }
 
 // ---------------------------------------------------------------- choice between the two kernels
-static std::atomic<int> g_bwd_deterministic{0};
+static std::atomic<int> g_bwd_deterministic{-1};   // -1: the caller has not said
 void attn_bwd_set_deterministic(int on) { g_bwd_deterministic.store(on ? 1 : 0); }
-int attn_bwd_deterministic() { return g_bwd_deterministic.load(); }
 
 // The single pass has only the key tiles' items to fill the SMs with, and clears, adds to and converts an accumulator; the two
 // passes execute seven GEMMs for five.  Backward in us, single pass / two passes (items per SM, streamed tiles per item):
@@ -997,10 +996,17 @@ static bool single_pass_pays(const AttnArgs& a) {
     return (items >= 6 * n_sm && tiles >= 16) || (items >= 3 * n_sm && tiles >= 32);
 }
 
+// A caller that has not said whether results must repeat gets what repeats to the bit for packed batches and at D = 128, and the
+// faster one at D = 64; it is its choice to give that up for the time (tt_attn_bwd_set_deterministic(0)).
+static bool single_pass_allowed(const AttnArgs& a) {
+    const int det = g_bwd_deterministic.load();
+    return det == 0 || (det < 0 && a.D == 64 && a.cu_q == nullptr);
+}
+
 cudaError_t attn_bwd_sm100(const AttnArgs& a, void* ws, cudaStream_t st) {
     // TT_BWD_PATH=two_pass|fused overrides the choice (tests run both kernels on the same inputs)
     const char* f = getenv("TT_BWD_PATH");
-    bool fused = !attn_bwd_deterministic() && single_pass_pays(a);
+    bool fused = single_pass_allowed(a) && single_pass_pays(a);
     if (f && f[0] == 't') fused = false;
     if (f && f[0] == 'f') fused = true;
     if (fused && attn_bwd_fused_supported(a)) return attn_bwd_fused(a, ws, st);

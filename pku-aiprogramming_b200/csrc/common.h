@@ -194,11 +194,10 @@ void attn_bwd_set_trace(long long* device_buf, int block, int pass);   // pass 1
 bool attn_bwd_sm100_supported(const AttnArgs& a);
 size_t attn_bwd_sm100_workspace(const AttnArgs& a);
 cudaError_t attn_bwd_sm100(const AttnArgs& a, void* workspace, cudaStream_t st);
-// Which tensor-core backward runs: 0 = the faster one for the shape (the single pass -- dQ through fp32 adds
+// Which tensor-core backward may run: 0 = the faster one for the shape (the single pass -- dQ through fp32 adds
 // in global memory, five GEMMs per tile pair, dQ reproducible to fp32 rounding -- or the two passes),
-// 1 = always the two passes (seven GEMMs, every result bit-reproducible).
+// 1 = always the two passes (seven GEMMs, every result bit-reproducible); never called: 0 for dense D = 64, else 1.
 void attn_bwd_set_deterministic(int on);
-int attn_bwd_deterministic();
 cudaError_t wait_timeout_probe(long long budget_cycles, int ctas, unsigned int* started, cudaStream_t st);
 cudaError_t umma_probe(const void* a, const void* b, const void* vt, int D, float* s_out, float* o_out,
                        cudaStream_t st);

@@ -132,9 +132,10 @@ def attention_backward_varlen(q, k, v, cu_q, cu_k, max_q, max_k, out, lse, dout,
 
 
 def set_backward_deterministic(on: bool) -> None:
-    """True: the tensor-core backward always runs its two-pass, bit-reproducible kernels; False (the
-    default): whichever kernel measured faster for the shape; for larger problems that is the single-pass one,
-    whose dq repeats to fp32 rounding only.  Process-wide."""
+    """True: the tensor-core backward always runs its two-pass, bit-reproducible kernels; False: whichever
+    measured faster for the shape, for larger problems the single-pass one, whose dq repeats to fp32 rounding
+    only.  Never called: the two passes for packed batches and at head dim 128, as False at head dim 64.
+    Process-wide."""
     capi.check(capi.lib.tt_attn_bwd_set_deterministic(1 if on else 0))
 
 
