@@ -96,7 +96,7 @@ struct FusedStream {
 };
 
 // What the loader publishes of a packed batch's item, so that the other roles need no search of their own.
-struct PackedItem { int head, r0, S, L, q_lo, k_lo, tile0, pad; };
+struct PackedItem { int head, r0, S, L, q_lo, k_lo, tile0, item; };   // item: the adding warps' copy alone
 struct FusedItem : BwdItem {
     long long blk0;   // accumulator and statistics of query tile t of query slice s: block s * n_qt + blk0 + t
 };
@@ -193,6 +193,7 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
     int* sched_item = reinterpret_cast<int*>(bar_p_free + 1);    // [2]
     uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(sched_item + 2);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_base_slot + 1);
+    PackedItem* add_item = reinterpret_cast<PackedItem*>(aux + 320);  // [2], the adding warps' items as warp 8 read them
     PackedItem* packed = reinterpret_cast<PackedItem*>(aux + 384);    // [2], beside sched_item
     uint64_t* bar_steal = reinterpret_cast<uint64_t*>(aux + Cfg::kBarBytes - 32);
     uint4* steal_response = reinterpret_cast<uint4*>(bar_steal + 2);
@@ -227,7 +228,7 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
             mbar_init(&bar_stat_full[i], 1);
             mbar_init(&bar_stat_empty[i], 8);
             mbar_init(&bar_sched_full[i], 1);
-            mbar_init(&bar_sched_empty[i], 13);   // MMA warp, compute and adding warps
+            mbar_init(&bar_sched_empty[i], 10);   // MMA warp, compute warps, the first adding warp
         }
         fence_barrier_init();
         fence_proxy_async_smem();
@@ -258,8 +259,9 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
 
     auto next_item = [&](int k) -> int {
         const int slot = k & 1;
-        // a wait that gave up (this CTA has aborted) ends the sequence: the slot may hold anything
-        if (!mbar_wait(&bar_sched_full[slot], (k >> 1) & 1, wctx, 80 + slot, k)) return -1;
+        // a wait that gave up (this CTA has aborted) ends the sequence: the slot may hold anything.  Lanes may find that out one by
+        // one, the warp leaves as one: what follows are warp-wide instructions
+        if (!__all_sync(0xffffffffu, mbar_wait(&bar_sched_full[slot], (k >> 1) & 1, wctx, 80 + slot, k))) return -1;
         return sched_item[slot];
     };
     // one arrival per warp, behind what all its threads did
@@ -267,7 +269,7 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
         __syncwarp();
         if (lane == 0) mbar_arrive(bar);
     };
-    auto take_item = [&](int k, FusedItem& w) -> bool {   // every role but the loader
+    auto take_item = [&](int k, FusedItem& w) -> bool {   // compute warps, MMA issuer
         const int item = next_item(k);
         if (item >= 0) w = fused_item<kVarlen>(item, &packed[k & 1], p);
         warp_arrive(&bar_sched_empty[k & 1]);
@@ -457,8 +459,21 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
         const uint32_t tDQ = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + kColDQ;
         uint32_t git = 0, chunk = 0;
         for (int k = 0;; ++k) {
-            FusedItem w;
-            if (!take_item(k, w)) break;
+            // Warp 8 reads the item for all four: the named barriers below need the same items and tiles in each, whatever a
+            // wait returned.  A slot is written again two items on, behind the barrier of the item between.
+            PackedItem* mine = &add_item[k & 1];
+            if (warp == 8) {
+                const int item = next_item(k);
+                if (lane == 0) {
+                    if (kVarlen) *mine = packed[k & 1];
+                    mine->item = item;
+                }
+                warp_arrive(&bar_sched_empty[k & 1]);
+            }
+            named_bar_sync(1, 128);
+            const int item = mine->item;
+            if (item < 0) break;
+            const FusedItem w = fused_item<kVarlen>(item, mine, p);
             FusedStream pos(w, p, kVarlen);
             for (int u = 0; u < w.n_it; ++u, ++git, pos.next(w)) {
                 float* dst = p.dq_acc + (size_t)((long long)pos.slice * p.n_qt + w.blk0 + pos.t) * (D / 4) * 512;
@@ -538,8 +553,8 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
                     items.request(*abort_flag != 0);
                     item = items.next(wctx, 89, k);
                 }
-                mbar_wait(&bar_sched_empty[slot], ((k >> 1) & 1) ^ 1, wctx, 90 + slot, k);
-                __syncwarp();
+                // a wait that gave up: somebody may still read the slot, and parts of two items would name rows of neither
+                if (!__all_sync(0xffffffffu, mbar_wait(&bar_sched_empty[slot], ((k >> 1) & 1) ^ 1, wctx, 90 + slot, k))) break;
                 if (lane == 0) {
                     sched_item[slot] = item;
                     if (kVarlen) packed[slot] = pi;
