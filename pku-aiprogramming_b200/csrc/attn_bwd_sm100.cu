@@ -185,7 +185,7 @@ __device__ __forceinline__ void bwd_cta(const CUtensorMap& tmR0, const CUtensorM
     auto next_item = [&](int k) -> int {
         const int slot = k & 1;
         // a wait that gave up (this CTA has aborted) ends the sequence: the slot may hold anything
-        if (!mbar_wait(&bar_sched_full[slot], (k >> 1) & 1, wctx, 80 + slot, k)) return -1;
+        if (!__all_sync(0xffffffffu, mbar_wait(&bar_sched_full[slot], (k >> 1) & 1, wctx, 80 + slot, k))) return -1;   // a warp leaves as one
         return sched_item[slot];
     };
 

@@ -158,7 +158,7 @@ attn_fwd_pair_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid
     // negative value ends it.
     auto next_item = [&](int k) -> int {
         const int slot = k & 1;
-        if (!mbar_wait_cluster(&bar_sched_full[slot], (k >> 1) & 1, wctx, 80 + slot, k)) return -1;
+        if (!__all_sync(0xffffffffu, mbar_wait_cluster(&bar_sched_full[slot], (k >> 1) & 1, wctx, 80 + slot, k))) return -1;   // a warp leaves as one
         return sched_item[slot];
     };
     const uint32_t sched_empty_r0 = map_to_cta(smem_u32(&bar_sched_empty[0]), 0);   // [slot]: + 8 * slot

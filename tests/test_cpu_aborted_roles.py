@@ -41,7 +41,8 @@ def test_one_warp_reads_the_item_for_its_role(name, role, barrier, reader):
     assert "take_item(" not in head and head.count("next_item(") == 1
 
 
-@pytest.mark.parametrize("name", ["attn_bwd_fused_sm100.cu", "attn_decode_gq_sm100.cu"])
+@pytest.mark.parametrize("name", ["attn_bwd_fused_sm100.cu", "attn_decode_gq_sm100.cu", "attn_fwd_sm100.cu", "attn_bwd_sm100.cu",
+                                  "attn_fwd_pair_sm100.cu", "attn_bwd_pair_sm100.cu"])
 def test_a_warp_takes_or_leaves_an_item_as_one(name):
     src = source(name)
     body = src[src.index("auto next_item ="):]
