@@ -417,8 +417,8 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
                     items.request(*abort_flag != 0);
                     item = items.next(wctx, 89, k);
                 }
-                mbar_wait(&bar_sched_empty[slot], ((k >> 1) & 1) ^ 1, wctx, 90 + slot, k);
-                __syncwarp();
+                // a wait that gave up: somebody may still read the slot, and parts of two packed items would name rows of neither
+                if (!__all_sync(0xffffffffu, mbar_wait(&bar_sched_empty[slot], ((k >> 1) & 1) ^ 1, wctx, 90 + slot, k))) break;
                 if (lane == 0) {
                     sched_item[slot] = item;
                     if (kVarlen) packed[slot] = pi;

@@ -47,3 +47,12 @@ def test_a_warp_takes_or_leaves_an_item_as_one(name):
     src = source(name)
     body = src[src.index("auto next_item ="):]
     assert re.search(r"__all_sync\(0xffffffffu, mbar_wait", body[:body.index("};")])
+
+
+@pytest.mark.parametrize("name", ["attn_bwd_fused_sm100.cu", "attn_fwd_sm100.cu"])
+def test_the_loader_leaves_a_slot_alone_that_was_not_released(name):
+    """These two publish a packed item's geometry beside its number: half of it overwritten would name rows of another sequence."""
+    src = source(name)
+    at = src.index("if (kVarlen) packed[slot] = pi;")
+    wait = src.rindex("mbar_wait(&bar_sched_empty[slot]", 0, at)
+    assert re.search(r"if \(!__all_sync\(0xffffffffu, mbar_wait\(&bar_sched_empty\[slot\].*\) break;", src[wait - 40:at])
