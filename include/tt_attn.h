@@ -160,7 +160,10 @@ int tt_attn_bwd_padded(const tt_attn_desc* desc, const void* q, const void* k, c
  * gets out = 0, lse = -inf and zero gradients).  bf16 with D = 64 or 128 only (tensor-core kernels);
  * anything else returns TT_ERR_UNSUPPORTED.  The backward runs the two-pass kernels (bit-reproducible) unless
  * tt_attn_bwd_set_deterministic(0) has allowed the single pass.
- * Workspace: tt_attn_bwd_varlen_workspace_bytes(), 256-byte aligned. */
+ * Workspace: tt_attn_bwd_varlen_workspace_bytes(), 256-byte aligned: 8 bytes per query row and head for the two
+ * passes.  Where the single pass is allowed and would be taken, H * (total_q / 128 + n_seq) * 128 * (D + 2) * 4
+ * bytes, at most 2 * total_q * H * (D + 2) * 4; a call that is given less than that, but enough for the two
+ * passes, takes them. */
 typedef struct tt_varlen_desc {
     int32_t n_seq, H, Hkv;   /* Hkv: 0 or H, or a divisor of H (grouped heads) */
     int32_t D, dtype, causal;

@@ -169,7 +169,8 @@ __device__ __forceinline__ void bwd_store_row(__nv_bfloat16* dst, const uint32_t
     }
 }
 
-// Two-pass (bit-reproducible) backward and the single-pass one; both take the same workspace.
+// Two-pass (bit-reproducible) backward and the single-pass one, and which of them a call would take.
+bool attn_bwd_single_pass(const AttnArgs& a);
 cudaError_t attn_bwd_two_pass(const AttnArgs& a, void* workspace, cudaStream_t st);
 bool attn_bwd_fused_supported(const AttnArgs& a);
 size_t attn_bwd_fused_workspace(const AttnArgs& a);

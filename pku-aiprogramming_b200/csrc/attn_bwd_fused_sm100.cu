@@ -1004,7 +1004,8 @@ void attn_bwd_set_deterministic(int on) { g_bwd_deterministic.store(on ? 1 : 0);
 //            D = 128, 16 sequences of 300 to 4096, 32 heads, causal 2080 / 2313; 32 of 20 to 200 168 / 178; 8 of 500 to 1000, 16 heads 187 / 222
 static bool single_pass_pays(const AttnArgs& a) {
     const long long n_seq = a.BH / a.H, hkv = a.H / a.group, n_sm = sm_count();
-    if (a.cu_q) return hkv * ((a.total_k + 127) / 128) >= 3 * n_sm;
+    // (packed: not where sequences are so short that the accumulator's whole tiles are more than twice the rows)
+    if (a.cu_q) return hkv * ((a.total_k + 127) / 128) >= 3 * n_sm && n_seq * 128 <= a.total_q;
     const long long items = n_seq * hkv * ((a.L + 127) / 128), q_tiles = (a.S + 127) / 128;
     const long long tiles = a.group * (a.causal ? (q_tiles + 1) / 2 : q_tiles);
     if (a.D == 64) return items >= 3 * n_sm && tiles >= 2;
@@ -1018,13 +1019,17 @@ static bool single_pass_allowed(const AttnArgs& a) {
     return det == 0 || (det < 0 && a.D == 64 && a.cu_q == nullptr);
 }
 
-cudaError_t attn_bwd_sm100(const AttnArgs& a, void* ws, cudaStream_t st) {
+bool attn_bwd_single_pass(const AttnArgs& a) {
     // TT_BWD_PATH=two_pass|fused overrides the choice (tests run both kernels on the same inputs)
     const char* f = getenv("TT_BWD_PATH");
     bool fused = single_pass_allowed(a) && single_pass_pays(a);
     if (f && f[0] == 't') fused = false;
     if (f && f[0] == 'f') fused = true;
-    if (fused && attn_bwd_fused_supported(a)) return attn_bwd_fused(a, ws, st);
+    return fused && attn_bwd_fused_supported(a);
+}
+
+cudaError_t attn_bwd_sm100(const AttnArgs& a, void* ws, size_t ws_bytes, cudaStream_t st) {
+    if (attn_bwd_single_pass(a) && ws_bytes >= attn_bwd_fused_workspace(a)) return attn_bwd_fused(a, ws, st);
     return attn_bwd_two_pass(a, ws, st);
 }
 

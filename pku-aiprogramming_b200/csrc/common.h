@@ -193,7 +193,9 @@ void attn_fwd_set_trace(long long* device_buf, int block, int item);
 void attn_bwd_set_trace(long long* device_buf, int block, int pass);   // pass 1: dK/dV, 2: dQ
 bool attn_bwd_sm100_supported(const AttnArgs& a);
 size_t attn_bwd_sm100_workspace(const AttnArgs& a);
-cudaError_t attn_bwd_sm100(const AttnArgs& a, void* workspace, cudaStream_t st);
+size_t attn_bwd_two_pass_workspace(const AttnArgs& a);
+// (takes the two passes where the workspace has no room for the single pass)
+cudaError_t attn_bwd_sm100(const AttnArgs& a, void* workspace, size_t ws_bytes, cudaStream_t st);
 // Which tensor-core backward may run: 0 = the faster one for the shape (the single pass -- dQ through fp32 adds
 // in global memory, five GEMMs per tile pair, dQ reproducible to fp32 rounding -- or the two passes),
 // 1 = always the two passes (seven GEMMs, every result bit-reproducible); never called: 0 for dense D = 64, else 1.

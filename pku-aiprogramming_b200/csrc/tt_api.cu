@@ -539,7 +539,7 @@ static int attn_bwd_common(const char* who, const tt_attn_desc* desc, const void
     bool al = aligned16(q) && aligned16(k) && aligned16(v) && aligned16(out) && aligned16(dout) && aligned16(dq) &&
               aligned16(dk) && aligned16(dv);
     if (attn_bwd_sm100_supported(a) && al) {
-        e = attn_bwd_sm100(a, workspace, st);
+        e = attn_bwd_sm100(a, workspace, workspace_bytes, st);
         if (e == cudaErrorInvalidValue && g_err[0]) return TT_ERR_CUDA;
     } else {
         e = attn_bwd_simt(a, (float*)workspace, st);
@@ -632,7 +632,8 @@ int tt_attn_bwd_varlen(const tt_varlen_desc* desc, const void* q, const void* k,
     if (!(aligned16(q) && aligned16(k) && aligned16(v) && aligned16(out) && aligned16(dout) && aligned16(dq) && aligned16(dk) &&
           aligned16(dv)))
         return fail(TT_ERR_BAD_SHAPE, "tt_attn_bwd_varlen: tensors must be 16-byte aligned");
-    const size_t need = tt_attn_bwd_varlen_workspace_bytes(desc);
+    a.cu_q = cu_q; a.cu_k = cu_k;
+    const size_t need = attn_bwd_two_pass_workspace(a);
     if (!workspace || workspace_bytes < need)
         return fail(TT_ERR_WORKSPACE, "tt_attn_bwd_varlen: workspace of %zu bytes required, %zu given", need, workspace_bytes);
     if ((reinterpret_cast<uintptr_t>(workspace) & 255) != 0)
@@ -641,8 +642,7 @@ int tt_attn_bwd_varlen(const tt_varlen_desc* desc, const void* q, const void* k,
     g_err[0] = 0;
     a.q = q; a.k = k; a.v = v; a.out = const_cast<void*>(out); a.lse = const_cast<float*>(lse); a.dout = dout;
     a.dq = dq; a.dk = dk; a.dv = dv;
-    a.cu_q = cu_q; a.cu_k = cu_k;
-    cudaError_t e = attn_bwd_sm100(a, workspace, (cudaStream_t)stream);
+    cudaError_t e = attn_bwd_sm100(a, workspace, workspace_bytes, (cudaStream_t)stream);
     if (e == cudaErrorInvalidValue && g_err[0]) return TT_ERR_CUDA;
     if (e != cudaSuccess) return cuda_fail(e, "tt_attn_bwd_varlen");
     return TT_OK;
