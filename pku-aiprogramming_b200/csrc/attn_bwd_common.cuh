@@ -132,7 +132,7 @@ __device__ __forceinline__ BwdItem bwd_decode_item(int item, const BwdParams& p)
         w.t_end = (S + 127) >> 7;
         w.t_begin = p.causal ? (max(0, rt * 128 - off) >> 7) : 0;
         // a key tile that is all padding gets zero gradients: one streamed tile keeps the pipeline's
-        // hand-offs alive, the epilogue writes zeros
+        // hand-offs alive, the epilogue writes zeros (the single-pass kernel's loader writes them and passes over the item)
         if (rt * 128 >= w.Lv) w.t_end = min(w.t_end, w.t_begin + 1);
     } else {
         rt = p.n_tiles - 1 - rank;                                    // late query tiles are the heavy ones

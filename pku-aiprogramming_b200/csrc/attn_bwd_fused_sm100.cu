@@ -521,6 +521,14 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
             };
             uint32_t git = 0;
             int item = (int)blockIdx.x;
+            // keys that no query sees: zero gradients, and nothing of them is read
+            auto zero_keys = [&](long long row, int pitch, int rows) {
+                for (int i = lane; i < rows * (D / 8); i += 32) {
+                    const long long o = (row + (long long)(i / (D / 8)) * pitch) * D + i % (D / 8) * 8;
+                    *reinterpret_cast<uint4*>(p.out0 + o) = make_uint4(0u, 0u, 0u, 0u);
+                    *reinterpret_cast<uint4*>(p.out1 + o) = make_uint4(0u, 0u, 0u, 0u);
+                }
+            };
             for (int k = 0;; ++k, item = items.next(wctx, 89, k)) {
                 const int slot = k & 1;
                 PackedItem pi;
@@ -539,17 +547,17 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
                         pi.r0 = (r - pi.head * n) * 128;
                         if (pi.head < p.Hkv && pi.r0 < pi.L) {
                             some = fused_item<true>(item, &pi, p).n_it > 0;
-                            if (!some) {   // keys that no query sees: zero gradients
-                                const int rows = min(128, pi.L - pi.r0);
-                                for (int i = lane; i < rows * (D / 8); i += 32) {
-                                    const long long o = ((long long)(pi.k_lo + pi.r0 + i / (D / 8)) * p.Hkv + pi.head) * D + i % (D / 8) * 8;
-                                    *reinterpret_cast<uint4*>(p.out0 + o) = make_uint4(0u, 0u, 0u, 0u);
-                                    *reinterpret_cast<uint4*>(p.out1 + o) = make_uint4(0u, 0u, 0u, 0u);
-                                }
-                            }
+                            if (!some) zero_keys((long long)(pi.k_lo + pi.r0) * p.Hkv + pi.head, p.Hkv, min(128, pi.L - pi.r0));
                         }
                     }
                     if (some) break;
+                    items.request(*abort_flag != 0);
+                    item = items.next(wctx, 89, k);
+                }
+                while (!kVarlen && p.kv_lens != nullptr && item >= 0) {   // tiles that are all padding
+                    const FusedItem w = fused_item<false>(item, nullptr, p);
+                    if (w.r0 < w.Lv) break;
+                    zero_keys((long long)w.bh * w.L + w.r0, 1, min(128, w.L - w.r0));
                     items.request(*abort_flag != 0);
                     item = items.next(wctx, 89, k);
                 }
