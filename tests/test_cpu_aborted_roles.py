@@ -46,7 +46,9 @@ def test_one_warp_reads_the_item_for_its_role(name, role, barrier, reader):
 def test_a_warp_takes_or_leaves_an_item_as_one(name):
     src = source(name)
     body = src[src.index("auto next_item ="):]
-    assert re.search(r"__all_sync\(0xffffffffu, mbar_wait", body[:body.index("};")])
+    reads = len(re.findall(r"(?<!auto )next_item\(k", src))      # by its callers where not inside
+    assert re.search(r"__all_sync\(0xffffffffu, mbar_wait", body[:body.index("};")]) or \
+        len(re.findall(r"if \(__any_sync\(0xffffffffu, (ahead_)?item < 0\)\)", src)) == reads
 
 
 @pytest.mark.parametrize("name", ["attn_bwd_fused_sm100.cu", "attn_fwd_sm100.cu"])
