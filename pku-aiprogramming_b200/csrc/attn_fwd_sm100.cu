@@ -24,6 +24,7 @@
 // Shared memory: Q tiles (2) + a ring of K/V tiles, each tile stored by TMA as D/64
 // sub-blocks of [128 rows x 128 bytes] with the 128-byte swizzle.
 #include "attn_fwd_common.cuh"
+#include <limits.h>
 #include <algorithm>
 
 namespace ttk {
@@ -151,8 +152,9 @@ __device__ __forceinline__ FwdItem fwd_decode_item(int item, const FwdParams& p,
 // forward problem: sequences may be empty, an item may cover one key range of its slice, rows
 // behind a sequence's end are zeroed in V, and with a block table the K and V tiles are gathered
 // page by page.
-// kVarlen: packed variable-length batches (see FwdParams): per-item sequence geometry, token-major addressing.
-template <int D, bool kTrace, bool kPaged, bool kVarlen>
+// kVarlen: packed variable-length batches (see FwdParams): per-item sequence geometry, token-major addressing; kLanes: of up to 32
+// sequences.
+template <int D, bool kTrace, bool kPaged, bool kVarlen, bool kLanes>
 __global__ void __launch_bounds__(FwdCfg<D>::kThreads, 1)
 attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                       const __grid_constant__ CUtensorMap tmV, const FwdParams p) {
@@ -395,24 +397,76 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             uint32_t t = 0;                    // K/V ring item counter (runs across work items)
             uint32_t q_uses[2] = {0, 0};       // how often each Q buffer has been filled
             int item = (int)blockIdx.x;
+            // A packed batch of up to 32 sequences has its lengths in this warp's registers, sequence b's in lane b, and its blocks
+            // numbered without gaps, the light ones behind all others: an item's sequence is then a vote and shuffles.  Searched for in
+            // memory it is two loads, one behind the other, ahead of every item's first tile.  Searched / so, us: causal, 16 of 278 to 1112, 4
+            // heads, D = 64 27.9 / 26.0, 28 of 100 to 900, 8 heads 51.0 / 45.8, 31 of 200 to 1200, 8 heads, D = 64 64.4 / 59.8, 12 of 100 to 1600,
+            // 8/2 heads 42.1 / 40.3; 4 of 64 to 256, 8 heads 10.2 / 10.0.
+            int seq_q = 0, seq_k = 0, seq_S = 0, seq_L = 0, heavy0 = INT_MAX, light0 = INT_MAX, n_heavy = 0, n_all = 0;
+            if constexpr (kLanes) {
+                if (lane < p.n_seq) {
+                    seq_q = p.cu_q[lane];
+                    seq_k = p.cu_k[lane];
+                    seq_S = p.cu_q[lane + 1] - seq_q;
+                    seq_L = p.cu_k[lane + 1] - seq_k;
+                }
+                if (p.n_light == 0) {   // one phase: as in packed_seq, without a sum over the lengths
+                    if (lane < p.n_seq) heavy0 = (seq_q >> 8) + lane;
+                    n_heavy = n_all = INT_MAX;
+                } else {
+                    const int blocks = (seq_S + 255) >> 8, light = min(blocks, p.n_light);
+                    int h = blocks - light, l = light;   // inclusive sums over the sequences
+#pragma unroll 1
+                    for (int o = 1; o < p.n_seq; o <<= 1) {
+                        const int h1 = __shfl_up_sync(0xffffffffu, h, o), l1 = __shfl_up_sync(0xffffffffu, l, o);
+                        if (lane >= o) {
+                            h += h1;
+                            l += l1;
+                        }
+                    }
+                    n_heavy = __shfl_sync(0xffffffffu, h, p.n_seq - 1);
+                    n_all = n_heavy + __shfl_sync(0xffffffffu, l, p.n_seq - 1);
+                    if (lane < p.n_seq) {
+                        heavy0 = h - (blocks - light);
+                        light0 = n_heavy + l - light;
+                    }
+                }
+            }
             for (int k = 0;; ++k, item = items.next(wctx, 89, k)) {
                 const int slot = k & 1;
                 PackedBlock pi;
-                while (kVarlen && item >= 0) {   // the item's sequence, head and 256-row block (see packed_seq)
-                    const bool second = item >= p.n_items_heavy;   // two phases: the light blocks last
-                    const int at = second ? item - p.n_items_heavy : item;
-                    const int x = at / p.H, b = packed_seq<8>(p.cu_q, p.n_seq, x);
+                while (kVarlen && item >= 0) {   // the item's sequence, head and 256-row block
                     bool some = false;
-                    if (b >= 0) {
-                        pi.q_lo = p.cu_q[b];
-                        pi.k_lo = p.cu_k[b];
-                        pi.S = p.cu_q[b + 1] - pi.q_lo;
-                        pi.L = p.cu_k[b + 1] - pi.k_lo;
-                        const int blocks = (pi.S + 255) >> 8, rank = x - (pi.q_lo >> 8) - b;
-                        pi.head = at - x * p.H;
-                        // the late blocks, which are the heavy ones, of all heads first: the launch ends on a sequence's light ones
-                        pi.q0 = (blocks - 1 - rank) * 256;
-                        some = rank < blocks && (blocks - 1 - rank < p.n_light) == second;
+                    // the late blocks, which are the heavy ones, of all heads first: the launch ends on a sequence's light ones
+                    if constexpr (kLanes) {
+                        const int x = item / p.H;
+                        pi.head = item - x * p.H;
+                        const bool second = x >= n_heavy;
+                        const int first = second ? light0 : heavy0, b = __popc(__ballot_sync(0xffffffffu, first <= x)) - 1;
+                        if (b >= 0) {
+                            pi.q_lo = __shfl_sync(0xffffffffu, seq_q, b);
+                            pi.k_lo = __shfl_sync(0xffffffffu, seq_k, b);
+                            pi.S = __shfl_sync(0xffffffffu, seq_S, b);
+                            pi.L = __shfl_sync(0xffffffffu, seq_L, b);
+                            const int blocks = (pi.S + 255) >> 8, n = second ? min(blocks, p.n_light) : blocks;
+                            const int rank = x - __shfl_sync(0xffffffffu, first, b);
+                            pi.q0 = (n - 1 - rank) * 256;
+                            some = x < n_all && rank < n;
+                        }
+                    } else {   // see packed_seq; in two phases every number comes twice and is taken in one of them
+                        const bool second = item >= p.n_items_heavy;
+                        const int at = second ? item - p.n_items_heavy : item;
+                        const int x = at / p.H, b = packed_seq<8>(p.cu_q, p.n_seq, x);
+                        if (b >= 0) {
+                            pi.q_lo = p.cu_q[b];
+                            pi.k_lo = p.cu_k[b];
+                            pi.S = p.cu_q[b + 1] - pi.q_lo;
+                            pi.L = p.cu_k[b + 1] - pi.k_lo;
+                            const int blocks = (pi.S + 255) >> 8, rank = x - (pi.q_lo >> 8) - b;
+                            pi.head = at - x * p.H;
+                            pi.q0 = (blocks - 1 - rank) * 256;
+                            some = rank < blocks && (blocks - 1 - rank < p.n_light) == second;
+                        }
                     }
                     if (some) break;
                     items.request(*abort_flag != 0);
@@ -672,7 +726,7 @@ void attn_fwd_set_trace(long long* device_buf, int block, int item) {
     g_fwd_trace_item = item;
 }
 
-template <int D, bool kTrace, bool kPaged = false, bool kVarlen = false>
+template <int D, bool kTrace, bool kPaged = false, bool kVarlen = false, bool kLanes = false>
 static cudaError_t launch_fwd(const AttnArgs& a, cudaStream_t st) {
     using Cfg = FwdCfg<D>;
     TmapStorage tq, tk, tv;
@@ -697,7 +751,7 @@ static cudaError_t launch_fwd(const AttnArgs& a, cudaStream_t st) {
         if (!make_tmap_bf16(&tk, a.k, D, a.L, kv_slices, 128, &why)) return cudaErrorInvalidValue;
         if (!make_tmap_bf16(&tv, a.v, D, a.L, kv_slices, 128, &why)) return cudaErrorInvalidValue;
     }
-    cudaError_t e = TT_ALLOW_SMEM((attn_fwd_sm100_kernel<D, kTrace, kPaged, kVarlen>), Cfg::kSmemBytes);
+    cudaError_t e = TT_ALLOW_SMEM((attn_fwd_sm100_kernel<D, kTrace, kPaged, kVarlen, kLanes>), Cfg::kSmemBytes);
     if (e != cudaSuccess) return e;
     FwdParams p;
     p.out = (__nv_bfloat16*)a.out;
@@ -737,16 +791,18 @@ static cudaError_t launch_fwd(const AttnArgs& a, cudaStream_t st) {
     }
     p.first_wave = sm_count();
     if (kVarlen) {
-        // Packed: two phases (every number twice, taken in one of them) only where the launch is short, so that what it ends on shows:
-        // 6 sequences of 723 to 3615, 8 heads (3.1 items per SM) 115 -> 105 us, 4 of 1000 to 4000, 8 heads (2.3) 90 -> 86; 28 of 100 to 900,
-        // 8 heads (4.5) 48.3 in one phase.
+        // Packed: two phases, the light blocks last, always where the loader numbers the blocks in its registers; where it searches, every
+        // number comes twice and is taken in one of the phases, which pays only where the launch is short, so that what it ends on shows.
+        // us, one phase / two: D = 64, 33 of 200 to 1200, 8 heads (6.8 items per SM) 70.8 / 67.9, 50 of 100 to 1500, 4 heads (5.7) 69.2 / 64.7, 100 of
+        // 300 to 2000, 16 heads (53) 736 / 756; D = 128, 40 of 60 to 900, 4 heads (2.9) 38.4 / 37.7, but the first of these 80.6 / 85.3.
         p.n_items_heavy = p.n_items;
-        if (p.n_items <= 4 * p.first_wave && p.n_light > 0) p.n_items *= 2;
-        else p.n_light = 0;
+        const bool two = kLanes || p.n_items <= (D == 64 ? 8 : 4) * p.first_wave;
+        if (!two) p.n_light = 0;
+        else if (!kLanes && p.n_light > 0) p.n_items *= 2;
     }
     {
         LaunchScope ls(K_FWD_TC, st);
-        e = launch_overlapped(attn_fwd_sm100_kernel<D, kTrace, kPaged, kVarlen>, (unsigned)p.n_items, Cfg::kThreads, Cfg::kSmemBytes,
+        e = launch_overlapped(attn_fwd_sm100_kernel<D, kTrace, kPaged, kVarlen, kLanes>, (unsigned)p.n_items, Cfg::kThreads, Cfg::kSmemBytes,
                               st, *reinterpret_cast<CUtensorMap*>(tq.bytes), *reinterpret_cast<CUtensorMap*>(tk.bytes),
                               *reinterpret_cast<CUtensorMap*>(tv.bytes), p);
     }
@@ -756,6 +812,7 @@ static cudaError_t launch_fwd(const AttnArgs& a, cudaStream_t st) {
 template <int D>
 static cudaError_t launch_fwd_d(const AttnArgs& a, cudaStream_t st) {
     if (a.cache_mode) return launch_fwd<D, false, true>(a, st);
+    if (a.cu_q != nullptr && a.BH / a.H <= 32) return launch_fwd<D, false, false, true, true>(a, st);
     if (a.cu_q != nullptr) return launch_fwd<D, false, false, true>(a, st);
     if (g_fwd_trace != nullptr) return launch_fwd<D, true>(a, st);
     return launch_fwd<D, false>(a, st);
