@@ -92,9 +92,9 @@ int tt_attn_bwd(const tt_attn_desc* desc, const void* q, const void* k, const vo
  * every result bit-reproducible.  One pass that produces dk, dv and dq together (five GEMMs), dq through
  * fp32 additions into the workspace; those arrive in no fixed order, so dq repeats to fp32 rounding (a few
  * 1e-7 relative) rather than bit for bit.  on = 1: always the two passes.  on = 0: whichever measured faster
- * for the shape (the single pass from three key tiles per SM on for packed batches and at D = 64, there with two
- * streamed tiles each, from more and longer ones at D = 128).  A process that never calls this gets the two
- * passes for packed batches and at D = 128, and at D = 64 what on = 0 gives.  Process-wide; no counterpart in
+ * for the shape, the single pass for problems of several key tiles per SM that each meet several query tiles and,
+ * at D = 64, for few queries against many keys.  A process that never calls this gets the two passes for packed
+ * batches and at D = 128, and at D = 64 what on = 0 gives.  Process-wide; no counterpart in
  * the reference, whose NumPy reverse sweep (optimizer/autodiff.py:33-61) is deterministic and
  * single-threaded. */
 int tt_attn_bwd_set_deterministic(int on);

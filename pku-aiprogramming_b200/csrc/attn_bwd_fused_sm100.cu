@@ -1003,21 +1003,41 @@ static std::atomic<int> g_bwd_deterministic{-1};   // -1: the caller has not sai
 void attn_bwd_set_deterministic(int on) { g_bwd_deterministic.store(on ? 1 : 0); }
 
 // The single pass has only the key tiles' items to fill the SMs with, and clears, adds to and converts an accumulator; the two
-// passes execute seven GEMMs for five.  Backward in us, single pass / two passes (items per SM, streamed tiles per item):
-//   D = 64   [8,16,1024] causal 105 / 121 (6.9, 4), [4,16,1024] causal 63 / 67 (3.5, 4), [16,32,512] causal 159 / 168 (14, 2), but
-//            [4,32,300] 42.6 / 40.7 (2.6, 3), [64,32,128] causal 131 / 128 (14, 1), [2,32/4,2048] causal 232 / 188 (0.9, 64)
-//   D = 128  [4,32,4096] causal 1614 / 1700 (28, 16), [1,32,4096] 740 / 775 (6.9, 32), [1,32/8,8192] causal 1550 / 1600 (3.5, 128), but
-//            [4,32,2048] causal 506 / 511 (14, 8), [4,32,1024] causal 186 / 181 (6.9, 4), [1,16,4096] causal 226 / 220 (3.5, 16)
-//   packed (the two passes clear the gradients and number their items for the longest sequence), from three items per SM on:
-//            D = 128, 16 sequences of 300 to 4096, 32 heads, causal 2080 / 2313; 32 of 20 to 200 168 / 178; 8 of 500 to 1000, 16 heads 187 / 222
+// passes execute seven GEMMs for five, and up to 1.8 items per SM run both in one launch, whose items fill the SMs better.
+// Backward in us, single pass / two passes (items per SM; streamed tiles per item):
+//   D = 64   [8,16,1024] causal 105 / 121 (6.9; 4), [16,32,512] causal 159 / 168 (14; 2), [1,8,5000] causal 127 / 153 (2.2; 20), [4,16,700]
+//            58 / 60 (2.6; 6), but [7,8,600] 40.5 / 39.3 (1.9; 5), [4,32,300] causal 42.6 / 40.7 (2.6; 2), [16,32,128] causal 40.0 / 38.6 (3.5; 1).
+//            The dQ pass of few queries is as long as the chain of key tiles that each of its items walks (1800 cycles a tile, 3125 in the
+//            single pass): against 9000 keys [1,4,300] 29 / 80, 12000 [1,4,128] 24 / 94, 3000 [1,8,100] 21 / 31, 4096 [1,64,128] 85 / 88, but
+//            2048 [1,100,128] 72 / 64, 2000 [3,32,100] 66 / 63, 578 [1,2,106] 11.7 / 10.3.
+//            One launch: full waves of long walks pay, [1,16,2048] 76 / 87 (1.7; 16), [1,4,4096] 74 / 82 (0.86; 32), [2,16,1024] 50 / 53
+//            (1.7; 8), but [4,16,512] 36.9 / 35.5 (1.7; 4), [1,8,3000] 107 / 89 (1.3; 24), [1,1,20000] 534 / 483 (1.06; 157); causal ones
+//            where they are longer still, [1,4,8192] 148 / 162 (1.7; 32), [1,2,16384] 237 / 283 (1.7; 64), [2,2,6900] 109 / 120 (1.5; 27),
+//            [1,16/4,8192] 534 / 570, but [1,8,4096] 94.4 / 93.8 (1.7; 16), [1,16/8,4096] 168 / 159, [1,2,12288] 176 / 170 (1.3; 48),
+//            [1,4,4096] 73 / 55 (0.86; 16).
+//   D = 128  [4,32,4096] causal 1614 / 1700 (28; 16), [4,32,2048] causal 517 / 538 (14; 8), [4,32,1536] 509 / 523 (10; 12), [1,32,4096]
+//            740 / 775 (6.9; 32), [1,32/8,8192] causal 1550 / 1600 (3.5; 32 of each head), but [4,32,1024] 259 / 255 (6.9; 8), [1,16,4096]
+//            causal 226 / 220 (3.5; 16), [4,64/8,2048] causal 1053 / 1014 (3.5; 8 of each head).
+//   packed   (the two passes clear the gradients and number their items for the longest sequence) 16 of 300 to 4096, 32 heads, causal
+//            1236 / 1550 at D = 64, 2085 / 2330 at D = 128; 24 of 512 434 / 461, 64 of 256 490 / 483, 64 of 128 156 / 165 at D = 64, but 262 / 239
+//            at D = 128.  Grouped heads at D = 128 have fewer items, and a dQ pass of as many as before: of 512, 32/8 heads 380 / 370, of 768
+//            445 / 444, of 1024 511 / 512; 32/4 heads, of 1024 1009 / 977, of 1536 1284 / 1268, 40 of 100 to 1500 1489 / 1506.
 static bool single_pass_pays(const AttnArgs& a) {
     const long long n_seq = a.BH / a.H, hkv = a.H / a.group, n_sm = sm_count();
-    // (packed: not where sequences are so short that the accumulator's whole tiles are more than twice the rows)
-    if (a.cu_q) return hkv * ((a.total_k + 127) / 128) >= 3 * n_sm && n_seq * 128 <= a.total_q;
+    if (a.cu_q) {
+        // (nor where sequences are so short that the accumulator's whole tiles are more than twice the rows)
+        if (hkv * ((a.total_k + 127) / 128) < 3 * n_sm || n_seq * 128 > a.total_q) return false;
+        return a.D == 64 || a.group == 1 || a.total_k >= n_seq * 128 * (a.group <= 4 ? 6 : 12);
+    }
     const long long items = n_seq * hkv * ((a.L + 127) / 128), q_tiles = (a.S + 127) / 128;
-    const long long tiles = a.group * (a.causal ? (q_tiles + 1) / 2 : q_tiles);
-    if (a.D == 64) return items >= 3 * n_sm && tiles >= 2;
-    return (items >= 6 * n_sm && tiles >= 16) || (items >= 3 * n_sm && tiles >= 32);
+    const long long tiles = a.causal ? (q_tiles + 1) / 2 : q_tiles, walk = a.group * tiles;
+    if (a.D == 128) return (items >= 10 * n_sm && tiles >= 8) || (items >= 6 * n_sm && tiles >= 16) || (items >= 3 * n_sm && tiles >= 32);
+    const long long waves = (items + n_sm - 1) / n_sm;
+    const long long key_tiles = (a.L + 127) / 128;
+    if (key_tiles >= 8 && 7 * waves * a.group * q_tiles < 4 * key_tiles) return true;
+    if (5 * items > 9 * n_sm) return walk >= (items >= 3 * n_sm ? 2 : 6);
+    if (a.causal) return 5 * items >= 7 * n_sm && q_tiles >= 48;
+    return 5 * items >= 4 * waves * n_sm && waves * walk >= 16;
 }
 
 // A caller that has not said whether results must repeat gets what repeats to the bit for packed batches and at D = 128, and the
