@@ -227,11 +227,14 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 
     // Every role walks the same item sequence.  Items are published by the loader in a two-slot
     // ring; a negative value ends the sequence.
+    constexpr bool kVoteHere = !kVarlen || kLanes;
     auto next_item = [&](int k) -> int {
         const int slot = k & 1;
         // a wait that gave up (this CTA has aborted) ends the sequence: the slot may hold anything.  Lanes may find that out one
-        // by one; the callers vote, so that a warp leaves as one (a vote here instead: 2 % of packed forwards at D = 64)
-        if (!mbar_wait(&bar_sched_full[slot], (k >> 1) & 1, wctx, 80 + slot, k)) return -1;
+        // by one, so the warp votes and leaves as one: here, but with the callers in the kernel that searches for its sequences,
+        // where a vote here costs 2 % at D = 64 (elsewhere one with the callers costs 2 % at D = 128)
+        const bool ok = mbar_wait(&bar_sched_full[slot], (k >> 1) & 1, wctx, 80 + slot, k);
+        if (kVoteHere ? !__all_sync(0xffffffffu, ok) : !ok) return -1;
         return sched_item[slot];
     };
 
@@ -253,7 +256,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             FwdItem w;
             if (kVarlen && item >= 0) w = fwd_decode_item<kPaged, kVarlen>(item, p, D, &packed[k & 1]);
             mbar_arrive(&bar_sched_empty[k & 1]);
-            if (__any_sync(0xffffffffu, item < 0)) break;
+            if (kVoteHere ? item < 0 : __any_sync(0xffffffffu, item < 0)) break;
             if (!kVarlen) w = fwd_decode_item<kPaged, kVarlen>(item, p, D);
             const int nt = w.n_tiles[i];
             // per-item stamps of the traced CTA (role slot 0/1 = query tile, row = item number k)
@@ -590,7 +593,7 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
                 __syncwarp();
                 if (elect_one()) mbar_arrive(&bar_sched_empty[k & 1]);
                 __syncwarp();
-                if (__any_sync(0xffffffffu, item < 0)) break;
+                if (kVoteHere ? item < 0 : __any_sync(0xffffffffu, item < 0)) break;
                 if (!kVarlen) w = fwd_decode_item<kPaged, kVarlen>(item, p, D);
                 // S_i(0) for both tiles.  The S/P columns are free: the P V MMAs of the previous item
                 // were issued earlier by this warp and execute in order.
@@ -671,9 +674,8 @@ attn_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
                     if (p.s0_ahead && j + 1 == w.n_max && w.n_tiles[0] < w.n_max) {
                         // last iteration, slot 0 idle: S_0(0) of the next item (its K_0 is ring item t + 2 n_max)
                         ahead_item = next_item(k + 1);
-                        if (__any_sync(0xffffffffu, ahead_item < 0)) {
-                            ahead_item = -1;
-                        } else {
+                        __syncwarp();
+                        if (ahead_item >= 0) {
                             const FwdItem wn = fwd_decode_item<kPaged, kVarlen>(ahead_item, p, D);
                             if (wn.n_tiles[0] > 0) {
                                 const uint32_t tn = t + 2 * (uint32_t)w.n_max;
