@@ -180,8 +180,8 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
     uint64_t* bar_dp_full = bar_p_full + 1;                      // MMA -> compute: dP^T(t) is in Y
     uint64_t* bar_ds_full = bar_dp_full + 1;                     // compute -> MMA: dS^T(t) is in shared memory, Y is read
     uint64_t* bar_ds_free = bar_ds_full + 1;                     // MMA -> compute: G4(t), G5(t) are done with the dS^T tile
-    uint64_t* bar_dq_full = bar_ds_free + 1;                     // MMA -> compute: dQ_t is in Y
-    uint64_t* bar_dq_free = bar_dq_full + 1;                     // compute -> MMA: dQ_t is in registers, Y is free
+    uint64_t* bar_dq_full = bar_ds_free + 1;                     // MMA -> adding warps: dQ_t is in its columns
+    uint64_t* bar_dq_free = bar_dq_full + 1;                     // adding warps -> MMA: dQ_t is in registers
     uint64_t* bar_final = bar_dq_free + 1;                       // MMA -> compute: dV, dK of the item are complete
     uint64_t* bar_acc_free = bar_final + 1;                      // compute (accumulators read out) -> MMA
     uint64_t* bar_sched_full = bar_acc_free + 1;                 // [2]
@@ -281,7 +281,7 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
         setmaxnreg_inc<Cfg::kRegsCompute>();
         const int wg = warp >> 2;
         const int wq = warp & 3;
-        const int r_in = wq * 32 + lane;                       // this thread's TMEM lane: key row, or query row of dQ_t
+        const int r_in = wq * 32 + lane;                       // this thread's TMEM lane: key row
         const uint32_t lane_off = (uint32_t)(wq * 32) << 16;
         const uint32_t tX = tmem_base + lane_off + kColX + wg * 64;
         const uint32_t tY = tmem_base + lane_off + kColY + wg * 64;
@@ -656,7 +656,7 @@ attn_bwd_fused_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
                 if (n_it > 0) {
                     // first scores of the item.  X is free: the G3 that read the previous P^T was issued
                     // earlier by this warp and executes in order.  Y holds the previous tile's dQ_t until
-                    // the compute threads have taken it.
+                    // the adding warps have taken it (D = 64: columns of its own).
                     const int f0 = git % kNQ, f1 = git % kNdO;
                     mbar_wait(&bar_q_full[f0], (git / kNQ) & 1, wctx, B1_QFULL + f0, (int)git);
                     __syncwarp();
@@ -1047,10 +1047,18 @@ static bool single_pass_allowed(const AttnArgs& a) {
     return det == 0 || (det < 0 && a.D == 64 && a.cu_q == nullptr);
 }
 
+// dk, dv over k, v: the single pass reads a key tile once, ahead of writing its gradients; the dQ pass reads k and v behind them.
+// At D = 64, where one pass used to be taken at every size, such calls keep it.
+static bool writes_over_keys(const AttnArgs& a) {
+    const uintptr_t bytes = (uintptr_t)(a.BH / a.group) * a.L * a.D * sizeof(__nv_bfloat16);
+    auto meet = [&](const void* x, const void* y) { return (uintptr_t)x < (uintptr_t)y + bytes && (uintptr_t)y < (uintptr_t)x + bytes; };
+    return meet(a.dk, a.k) || meet(a.dk, a.v) || meet(a.dv, a.k) || meet(a.dv, a.v);
+}
+
 bool attn_bwd_single_pass(const AttnArgs& a) {
     // TT_BWD_PATH=two_pass|fused overrides the choice (tests run both kernels on the same inputs)
     const char* f = getenv("TT_BWD_PATH");
-    bool fused = single_pass_allowed(a) && single_pass_pays(a);
+    bool fused = single_pass_allowed(a) && (single_pass_pays(a) || (a.D == 64 && a.cu_q == nullptr && writes_over_keys(a)));
     if (f && f[0] == 't') fused = false;
     if (f && f[0] == 'f') fused = true;
     return fused && attn_bwd_fused_supported(a);
