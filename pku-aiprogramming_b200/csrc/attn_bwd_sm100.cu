@@ -788,11 +788,11 @@ bool attn_bwd_sm100_supported(const AttnArgs& a) {
 static size_t stats_rows(const AttnArgs& a) { return a.cu_q ? (size_t)a.total_q * a.H : (size_t)a.BH * a.S; }
 static size_t stats_bytes(const AttnArgs& a) { return 2 * align256(stats_rows(a) * sizeof(float)); }
 size_t attn_bwd_two_pass_workspace(const AttnArgs& a) { return stats_bytes(a); }
-// Dense: room for either kernel.  Packed: for the one that would run now, since the single pass's accumulator is whole tiles per
-// (head, sequence), much more than the rows where sequences are short.
+// Dense: room for either kernel (one at a time: the single pass keeps its own statistics).  Packed: for the one that would run now,
+// since the single pass's accumulator is whole tiles per (head, sequence), much more than the rows where sequences are short.
 size_t attn_bwd_sm100_workspace(const AttnArgs& a) {
-    if (a.cu_q) return attn_bwd_single_pass(a) ? std::max(stats_bytes(a), attn_bwd_fused_workspace(a)) : stats_bytes(a);
-    return stats_bytes(a) + (attn_bwd_fused_supported(a) ? attn_bwd_fused_workspace(a) : 0);
+    const bool single = a.cu_q ? attn_bwd_single_pass(a) : attn_bwd_fused_supported(a);
+    return single ? std::max(stats_bytes(a), attn_bwd_fused_workspace(a)) : stats_bytes(a);
 }
 
 static long long* g_bwd_trace = nullptr;

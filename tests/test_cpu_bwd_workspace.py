@@ -1,4 +1,4 @@
-"""Size of the packed backward's workspace: a function of the token count, however many sequences share it."""
+"""Size of the backward's workspace: of a packed batch a function of the token count, however many sequences share it."""
 import ctypes
 
 import pytest
@@ -33,3 +33,9 @@ def test_single_pass_takes_no_more_than_twice_its_rows(tt, n_seq, length, H, D):
     assert got <= max(two_pass_bytes(n_seq * length, H), 2 * rows * (D + 2) * 4)
     if length >= 128:
         assert got >= rows * (D + 2) * 4
+
+
+@pytest.mark.parametrize("B,H,S,D", [(1, 64, 32768, 128), (4, 32, 4096, 128), (8, 16, 1024, 64), (2, 3, 300, 64)])
+def test_dense_calls_need_one_accumulator_and_one_pair_of_statistics(tt, B, H, S, D):
+    d = tt.capi.make_desc(B, H, S, S, D, tt.capi.TT_BF16, True, None)
+    assert int(tt.capi.lib.tt_attn_bwd_workspace_bytes(ctypes.byref(d))) == B * H * (-(-S // 128) * 128) * (D + 2) * 4
