@@ -154,7 +154,8 @@ int tt_attn_bwd_padded(const tt_attn_desc* desc, const void* q, const void* k, c
  * [total_q, H, D]; k, v, dk, dv [total_k, Hkv, D]; lse [H, total_q].  cu_q, cu_k: device arrays of
  * n_seq + 1 int32, cumulative token counts (cu[0] = 0, cu[n_seq] = total): sequence b owns query tokens
  * [cu_q[b], cu_q[b+1]) and key tokens [cu_k[b], cu_k[b+1]).  max_q, max_k: upper bounds of the longest
- * sequence (host values: they size the launch; the kernels read the real lengths from cu_q / cu_k).
+ * sequence (host values: the two-pass backward numbers its work for them, the forward orders its work by them; the
+ * kernels read the real lengths from cu_q / cu_k).
  * Every sequence is its own attention problem with the conventions above (causal: bottom-right aligned
  * per sequence; a row that sees no key -- an empty key sequence, or causal with fewer keys than queries --
  * gets out = 0, lse = -inf and zero gradients).  bf16 with D = 64 or 128 only (tensor-core kernels);
